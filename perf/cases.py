@@ -178,3 +178,26 @@ def tolerance(case):
         return {"rel": min(1e-5, max(2.5e-6, 3e-7 * w * w)), "max": 3e-5}
     rel = min(3e-5, max(3e-6, 1e-6 * w * w))
     return {"rel": rel, "max": 13 * rel}
+
+
+def exact(case, seed):
+    """Where every pair is summed directly: the dense op, and a product whose boxes are all small at the first level (the
+    tree's own approximation is most of the distance of any other product from K b, so those have no such value)."""
+    kind, n = case["kind"], case["n"]
+    small = kind in ("one_shot", "kept") and not case["m"] and case["dist"] == "uniform" and n <= 4 * case["small"]
+    if not (kind == "dense" or small) or n > 40_000:
+        return None
+    s = prepare(case, seed)
+    X, b = s["X"].double(), s["b"].double()
+    val = torch.empty_like(b)
+    grad = torch.empty_like(b)
+    ls = float(case["ls"])
+    for i in range(0, n, 1000):
+        D = torch.zeros(min(1000, n - i), n, dtype=torch.float64, device=X.device)
+        for k in range(case["d"]):
+            D += (X[i:i + 1000, None, k] - X[None, :, k]) ** 2
+        K = torch.exp(D / (-2 * ls * ls))
+        val[i:i + 1000] = K @ b
+        if kind == "dense":
+            grad[i:i + 1000] = (K * D) @ b / ls ** 3
+    return (val, grad) if kind == "dense" else val
