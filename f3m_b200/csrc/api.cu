@@ -343,12 +343,12 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
         pl->stats.far_box_pairs += ll.far.count;
         pl->stats.node_pairs += ll.far.count * (int64_t)P * P;
         pl->stats.near_box_pairs += ll.small.count;
-        accumulate_pair_work(pl, level, ll.small, s);
+        accumulate_pair_work(pl, level, level, ll.small, s);
     }
     pl->levels = level;
     if (level > 0) {
         pl->stats.near_box_pairs += pl->lists[level].keep.count;
-        accumulate_pair_work(pl, level, pl->lists[level].keep, s);
+        accumulate_pair_work(pl, level, PAIRWORK_LISTS - 1, pl->lists[level].keep, s);
     } else {
         // no level was built: the root pair is summed directly
         pl->stats.near_box_pairs = 1;
@@ -358,9 +358,17 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
     pl->stats.shared_tree = pl->same;
     pl->stats.edge0 = edge0;
     pl->last.end(s);
-    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + FL_PAIRWORK, pl->d_flags + FL_PAIRWORK, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + FL_PAIRWORK, pl->d_flags + FL_PAIRWORK, 2 * PAIRWORK_LISTS * sizeof(long long),
+                             cudaMemcpyDeviceToHost, s));
     F3M_CUDA(cudaStreamSynchronize(s));
-    if (level > 0) pl->stats.direct_pairs = *reinterpret_cast<long long *>(pl->h_pinned + FL_PAIRWORK);
+    const long long *work = reinterpret_cast<const long long *>(pl->h_pinned + FL_PAIRWORK);
+    auto take_work = [&](PairCSR &csr, int slot) {
+        csr.pairs = work[2 * slot];
+        csr.row_boxes = work[2 * slot + 1];
+        pl->stats.direct_pairs += csr.pairs;
+    };
+    for (int l = 1; l <= level; l++) take_work(pl->lists[l].small, l);
+    if (level > 0) take_work(pl->lists[level].keep, PAIRWORK_LISTS - 1);
     pl->last.ms[ST_BUILD] = 0.f;
     pl->last.resolve();
     pl->stats.build_ms = pl->last.ms[ST_BUILD];

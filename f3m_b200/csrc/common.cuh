@@ -149,8 +149,9 @@ enum FlagSlot {
     FL_NSMALL = 42,      // target tiles of at most 32 points
     FL_LVTOT = 64,       // boxes per level of the batch being built (F3M_MAX_LEVELS words)
     FL_LVMAX = 96,       // largest box per level (F3M_MAX_LEVELS words)
-    FL_PAIRWORK = 128    // 2 words per level: 64-bit sum of n_x * n_y over the level's direct lists
+    FL_PAIRWORK = 128    // 4 words per direct list (PAIRWORK_LISTS of them): 64-bit sums of n_x * n_y and of n_x over its box pairs
 };
+constexpr int PAIRWORK_LISTS = 22;   // "small" lists of levels 1..20, the near list in slot 21
 
 // ---- tree ------------------------------------------------------------------------------------
 struct Level {
@@ -193,6 +194,8 @@ struct PairCSR {
     DevBuf<int> ptr;  // (boxes_x+1)
     DevBuf<int> idx;  // source box per pair
     int64_t count = 0;
+    // direct lists: pairs of points, and (target point, source box) pairs
+    int64_t pairs = 0, row_boxes = 0;
 };
 
 struct LevelLists {
@@ -314,7 +317,7 @@ void scatter_rows_nonzero(const float *src, const int *perm, float *dst, int64_t
 void build_root(Tree &t, cudaStream_t s);
 void build_levels(Tree &t, int l_last, f3m_plan *pl, cudaStream_t s);   // appends levels up to l_last (<= sorted_depth)
 void build_level_lists(f3m_plan *pl, int level, cudaStream_t s);     // uses lists[level-1].keep
-void accumulate_pair_work(f3m_plan *pl, int level, const PairCSR &csr, cudaStream_t s);   // adds into FL_PAIRWORK (device)
+void accumulate_pair_work(f3m_plan *pl, int level, int slot, const PairCSR &csr, cudaStream_t s);   // FL_PAIRWORK (device)
 
 // ---- far.cu ----------------------------------------------------------------------------------
 int nodes_per_dim(int d, int nr_interpolation);   // get_node_list for perfect powers, floor otherwise
@@ -342,6 +345,9 @@ void shard_rows_to_input_order(const f3m_plan *pl, const float *acc_sorted, int 
 // ---- near.cu ---------------------------------------------------------------------------------
 void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted,
                  int64_t row_begin, int64_t row_end, cudaStream_t s);
+// near_moments.cu: sums a direct list through box moments when its geometry allows; false: sum the pairs
+bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted, int row_begin,
+                 int row_end, cudaStream_t s);
 template <bool GRAD>
 void dense_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,
                cudaStream_t s);

@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) lists_kernel(int pass, int nbx, const int
     if (pass == 0 && lane == 0) { far_ptr[box] = nf; small_ptr[box] = ns; keep_ptr[box] = nk; }
 }
 
-// sum over the rows of a CSR list of n_x * sum n_y  (work accounting only)
+// sums over the rows of a CSR list of n_x * sum n_y and of n_x * (row length)
 __global__ void __launch_bounds__(256) pair_work_kernel(int nbx, const int *__restrict__ ptr, const int *__restrict__ idx,
                                                        const int *__restrict__ off_x, const int *__restrict__ off_y,
                                                        unsigned long long *total) {
@@ -377,14 +377,18 @@ __global__ void __launch_bounds__(256) pair_work_kernel(int nbx, const int *__re
     for (int e = ptr[box] + lane; e < ptr[box + 1]; e += 32) { int by = idx[e]; s += off_y[by + 1] - off_y[by]; }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0 && s) atomicAdd(total, (unsigned long long)(s * (long long)(off_x[box + 1] - off_x[box])));
+    if (lane == 0 && s) {
+        const long long nx = off_x[box + 1] - off_x[box];
+        atomicAdd(total, (unsigned long long)(s * nx));
+        atomicAdd(total + 1, (unsigned long long)(nx * (ptr[box + 1] - ptr[box])));
+    }
 }
 
-// adds the list's pair work to the plan's device-side total, which the host reads once when the plan is complete
-void accumulate_pair_work(f3m_plan *pl, int level, const PairCSR &csr, cudaStream_t s) {
+// the list's pair work in its slot of the plan's device words, which the host reads once when the plan is complete
+void accumulate_pair_work(f3m_plan *pl, int level, int slot, const PairCSR &csr, cudaStream_t s) {
     if (csr.count == 0) return;
     Level &lx = pl->tx.levels[level], &ly = pl->ty->levels[level];
-    unsigned long long *d_tot = reinterpret_cast<unsigned long long *>(pl->d_flags + FL_PAIRWORK);
+    unsigned long long *d_tot = reinterpret_cast<unsigned long long *>(pl->d_flags + FL_PAIRWORK) + 2 * slot;
     pair_work_kernel<<<(unsigned)(((int64_t)lx.nb * 32 + 255) / 256), 256, 0, s>>>(lx.nb, csr.ptr.p, csr.idx.p, lx.off.p,
                                                                                    ly.off.p, d_tot);
     F3M_LAUNCH_CHECK();

@@ -49,11 +49,11 @@ enum f3m_status {
                                --use_fast_math build executes (F3M_src/setup.py:16) -- default */
 #define F3M_MATH_IEEE 1     /* IEEE divide, sqrt, no contraction: what a CPU restatement computes */
 
-/* Optional evaluation of the near field by box moments: when every pair of a near / small list has a provably
- * tiny exponent (boxes much smaller than the lengthscale), the sum over a source box is replaced by its 2nd/3rd
- * order Taylor moments (truncation error <= 1e-6 relative, the size of the ex2.approx error).  The pair lists do
- * not change.  Off by default: the default near field is the direct sum of the reference
- * (near_field_run, F3M_src/n_tree.cu:831-902). */
+/* Near sums through box moments.  Where a near / small list has provably small exponents (boxes small against the
+ * lengthscale) and its source boxes hold enough points, the sum over a source box is taken from its moments of degree
+ * 2..6 instead of pair by pair: the same sums, with a polynomial for part of the exponential whose relative error is below
+ * 1.2e-7 (ex2.approx: 2.4e-7).  The pair lists do not change (near_field_run, F3M_src/n_tree.cu:831-902).  This flag
+ * relaxes the bound to 1e-6 and takes moments also where the pair form would be as fast. */
 #define F3M_FLAG_NEAR_MOMENTS 1
 
 /* Optional evaluation of the direct near sums on the tensor cores (one column, boxes at most half a scaled
@@ -295,8 +295,8 @@ int f3m_plan_last_direct_launches(const f3m_plan *plan);
 /* Which form of the direct-sum kernel those launches took (the host picks it per list from a bound on the
  * exponent, see near_field_run n_tree.cu:831-902 for the sums themselves): counts[0] expanded form with every
  * exponential on the special-function unit, [1] expanded form with 2/5 of the pairs on a degree-2 polynomial,
- * [2] with 1/3 on a degree-3 polynomial, [3] direct form (differences, wide boxes), [4] moment form
- * (F3M_FLAG_NEAR_MOMENTS), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES). */
+ * [2] with 1/3 on a degree-3 polynomial, [3] direct form (differences, wide boxes), [4] moment form (of degree 2 and 3 it
+ * counts in [1] and [2] too: every exponent of the list is in that polynomial), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES). */
 int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]);
 long long f3m_launch_count(void);
 

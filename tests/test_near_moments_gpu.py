@@ -1,0 +1,80 @@
+"""Near sums through box moments against the sums over the pairs."""
+import pytest
+import torch
+
+from cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(X, Y, b, ls, leaf, nodes, cuda):
+    """The default product, and the one whose lists are all summed pair by pair (the tensor-core flag keeps moments out)."""
+    from f3m_b200 import _lib, engine
+    out, forms = [], []
+    for flags in (0, _lib.FLAG_NEAR_TENSOR_CORES):
+        plan = engine.Plan(X.to(cuda), None if Y is None else Y.to(cuda), engine.make_params(ls, leaf, nodes, False, 0.15, nodes, flags=flags))
+        out.append(plan.apply(b.to(cuda)).cpu())
+        forms.append(plan.direct_variants())
+    assert forms[1]["moments"] == 0
+    return out, forms[0], plan
+
+
+def _weights(n, R, g):
+    # positive, so that no sum cancels: truncation 1.2e-7, ex2.approx 2.4e-7 on either side, and FP32 sums of blocks of at most a few
+    # hundred terms, each below 1e-6 of the (positive) result
+    return torch.rand(n, R, generator=g) + 0.5
+
+
+TOL = 2e-6
+
+
+# degrees 2, 3, 4, 5, 6 as the boxes widen; one column, a partial block of four, and a block of four and one column
+@pytest.mark.parametrize("d,ls,R", [(1, 0.4, 1), (1, 0.05, 5), (2, 3.0, 1), (2, 0.5, 2), (2, 0.2, 3), (3, 4.0, 1), (3, 1.6, 5), (3, 0.9, 1),
+                                    (3, 0.7, 4), (3, 0.5, 1), (3, 0.42, 2), (4, 4.0, 1), (4, 2.5, 3), (5, 6.0, 1), (5, 4.0, 2)])
+def test_moments_equal_pair_sums(d, ls, R, cuda):
+    g = torch.Generator().manual_seed(10 * d + R)
+    n = 30011
+    X = torch.rand(n, d, generator=g)
+    (a, b), forms, _ = _both(X, None, _weights(n, R, g), ls, 300.0, 3 ** d if d > 3 else 4 ** d, cuda)
+    assert forms["moments"] > 0, forms
+    assert rel_l2(a, b) <= TOL
+
+
+def test_moments_at_the_corners_of_the_boxes(cuda):
+    """Every point within a hair of a corner of its finest box: the exponents reach the bound the degree is chosen by."""
+    g = torch.Generator().manual_seed(3)
+    corner = torch.randint(0, 9, (40000, 3), generator=g).float() / 8.0
+    X = (corner + (torch.rand(40000, 3, generator=g) - 0.5) * 1e-3)
+    (a, b), forms, _ = _both(X, None, _weights(40000, 1, g), 0.8, 300.0, 64, cuda)
+    assert forms["moments"] > 0, forms
+    assert rel_l2(a, b) <= TOL
+
+
+@pytest.mark.parametrize("n,m", [(1, 70000), (31, 40000), (129, 3000), (40000, 1500), (70001, 33)])
+def test_moments_of_two_point_sets(n, m, cuda):
+    """Source boxes of very different length (blocks of 256 threads, parts of a box added atomically) and few targets."""
+    g = torch.Generator().manual_seed(n + m)
+    X, Y = torch.rand(n, 3, generator=g), torch.rand(m, 3, generator=g)
+    if n == 1:
+        X = torch.cat([X, X + 0.2])
+    (a, b), _, _ = _both(X, Y, _weights(m, 1, g), 2.0, 20.0 if min(n, m) > 20 else 1.0, 27, cuda)
+    assert torch.isfinite(a).all()
+    assert rel_l2(a, b) <= TOL
+
+
+def test_moments_of_a_slice_and_short_boxes(cuda):
+    """Rows outside the slice stay untouched; boxes with fewer sources than the polynomial has terms keep the pair form."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(8)
+    X = torch.rand(30000, 3, generator=g)
+    b = _weights(30000, 1, g)
+    plan = engine.Plan(X.to(cuda), None, engine.make_params(1.6, 300.0, 64, False, 0.15, 64))
+    full = plan.apply(b.to(cuda))
+    cuts = (0, 1, 63, 12345, 30000)
+    parts = sum(plan.apply(b.to(cuda), row_range=(lo, hi)) for lo, hi in zip(cuts, cuts[1:]))
+    assert plan.direct_variants()["moments"] > 0
+    assert rel_l2(parts.cpu(), full.cpu()) <= 5e-7
+    X = torch.rand(30000, 5, generator=g)    # one or two points per box against 21 terms
+    (a, p), forms, plan = _both(X, None, b, 6.0, 20.0, 32, cuda)
+    assert forms["moments"] == 0 and forms["poly2"] + forms["poly3"] > 0, forms
+    assert rel_l2(a, p) <= TOL
