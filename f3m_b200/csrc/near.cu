@@ -1,8 +1,6 @@
-// Direct Gaussian sums: the near / small field of the treecode and the exact dense product.
+// Direct Gaussian sums: the near / small field of the treecode.
 //
-// Replaces near_field_run (F3M_src/n_tree.cu:831-902) with skip_conv_1d_shared
-// (F3M_src/1_d_conv.cu:255-335) and rbf_call / rbf_call_grad (n_tree.cu:185-241) with
-// rbf_1d_reduce_shared_torch(_grad) (1_d_conv.cu:126-214).
+// Replaces near_field_run (F3M_src/n_tree.cu:831-902) with skip_conv_1d_shared (F3M_src/1_d_conv.cu:255-335).
 //
 // The reference gathers every x, y and b through the permutation on every use, runs one target per
 // thread over a block-wide tile with two barriers per tile and repeats all exponentials for every
@@ -48,7 +46,7 @@ __global__ void __launch_bounds__(256) pack_sources(const float *__restrict__ pt
 }
 
 // inner product of one target tile with `cnt` packed source rows held in shared memory
-template <int D, int RB, int TI, bool GRAD>
+template <int D, int RB, int TI>
 __device__ __forceinline__ void tile_accumulate(const float *__restrict__ smem, int cnt, const float (&tx)[TI][D],
                                                 float (&acc)[TI][RB]) {
     constexpr int W = row_width(D, RB);
@@ -71,7 +69,6 @@ __device__ __forceinline__ void tile_accumulate(const float *__restrict__ smem, 
                 nr2 = fmaf(-dk, dk, nr2);
             }
             float e = ex2_approx(nr2);
-            if (GRAD) e *= -nr2;
 #pragma unroll
             for (int r = 0; r < RB; r++) acc[u][r] = fmaf(e, row[D + r], acc[u][r]);
         }
@@ -143,7 +140,7 @@ __global__ void __launch_bounds__(NT) near_kernel(const float *__restrict__ xpts
             float4 *sdst = reinterpret_cast<float4 *>(smem);
             for (int q = threadIdx.x; q < cnt * (W / 4); q += NT) sdst[q] = __ldg(g + q);
             __syncthreads();
-            tile_accumulate<D, RB, TI, false>(smem, cnt, tx, acc);
+            tile_accumulate<D, RB, TI>(smem, cnt, tx, acc);
         }
 #pragma unroll
         for (int u = 0; u < TI; u++)
@@ -799,207 +796,6 @@ void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, i
         case 3: direct_d<3>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
         case 4: direct_d<4>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
         default: direct_d<5>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
-// exact dense products
-// ---------------------------------------------------------------------------------------------
-template <int D, int RB>
-__global__ void __launch_bounds__(256) pack_rows_dense(const float *__restrict__ Y, int64_t n, const float *__restrict__ b, int R,
-                                                      int r0, float scale, float *packed) {
-    constexpr int W = row_width(D, RB);
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    float *dst = packed + (size_t)j * W;
-#pragma unroll
-    for (int k = 0; k < D; k++) dst[k] = scale * Y[j * D + k];
-#pragma unroll
-    for (int r = 0; r < RB; r++) dst[D + r] = (r0 + r < R) ? b[(size_t)j * R + r0 + r] : 0.f;
-#pragma unroll
-    for (int c = D + RB; c < W; c++) dst[c] = 0.f;
-}
-
-template <int D, int RB, bool GRAD>
-__global__ void __launch_bounds__(NT) dense_kernel(const float *__restrict__ X, int64_t n, const float *__restrict__ packed,
-                                                  int64_t m, float scale, float post, int R, int r0, float *out) {
-    constexpr int W = row_width(D, RB);
-    __shared__ __align__(16) float smem[ST * W];
-    const int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x;
-    const int64_t ii = i < n ? i : n - 1;
-    float tx[1][D], tot[1][RB];
-#pragma unroll
-    for (int k = 0; k < D; k++) tx[0][k] = scale * X[ii * D + k];
-#pragma unroll
-    for (int r = 0; r < RB; r++) tot[0][r] = 0.f;
-    for (int64_t base = 0; base < m; base += ST) {
-        const int cnt = (int)min((int64_t)ST, m - base);
-        __syncthreads();
-        const float4 *g = reinterpret_cast<const float4 *>(packed + (size_t)base * W);
-        float4 *sdst = reinterpret_cast<float4 *>(smem);
-        for (int q = threadIdx.x; q < cnt * (W / 4); q += NT) sdst[q] = __ldg(g + q);
-        __syncthreads();
-        float acc[1][RB];
-#pragma unroll
-        for (int r = 0; r < RB; r++) acc[0][r] = 0.f;
-        tile_accumulate<D, RB, 1, GRAD>(smem, cnt, tx, acc);
-#pragma unroll
-        for (int r = 0; r < RB; r++) tot[0][r] += acc[0][r];
-    }
-    if (i < n)
-#pragma unroll
-        for (int r = 0; r < RB; r++)
-            if (r0 + r < R) out[(size_t)i * R + r0 + r] = tot[0][r] * post;
-}
-
-template <int D, bool GRAD>
-static void dense_d(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, float ls, float *out,
-                    cudaStream_t s) {
-    const float lcs = 1.f / (2.f * ls * ls);
-    const float scale = near_scale(lcs);
-    // GRAD: sum r^2 exp(..) b / ls^3 with r^2 = (scaled r^2) / scale^2   (n_tree.cu:222-239)
-    const float post = GRAD ? 1.f / (scale * scale) / (ls * ls * ls) : 1.f;
-    const unsigned gy = (unsigned)((M + 255) / 256), gx = (unsigned)((N + NT - 1) / NT);
-    for (int r0 = 0; r0 < R;) {
-        DevBuf<float> packed;
-        if (R - r0 >= 2) {
-            packed.alloc((size_t)M * row_width(D, 4), s);
-            pack_rows_dense<D, 4><<<gy, 256, 0, s>>>(Y, M, b, R, r0, scale, packed.p);
-            F3M_LAUNCH_CHECK();
-            dense_kernel<D, 4, GRAD><<<gx, NT, 0, s>>>(X, N, packed.p, M, scale, post, R, r0, out);
-            r0 += 4;
-        } else {
-            packed.alloc((size_t)M * row_width(D, 1), s);
-            pack_rows_dense<D, 1><<<gy, 256, 0, s>>>(Y, M, b, R, r0, scale, packed.p);
-            F3M_LAUNCH_CHECK();
-            dense_kernel<D, 1, GRAD><<<gx, NT, 0, s>>>(X, N, packed.p, M, scale, post, R, r0, out);
-            r0 += 1;
-        }
-        F3M_LAUNCH_CHECK();
-    }
-}
-
-template <bool GRAD>
-void dense_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,
-               cudaStream_t s) {
-    switch (d) {
-        case 1: dense_d<1, GRAD>(X, N, Y, M, b, R, ls, out, s); break;
-        case 2: dense_d<2, GRAD>(X, N, Y, M, b, R, ls, out, s); break;
-        case 3: dense_d<3, GRAD>(X, N, Y, M, b, R, ls, out, s); break;
-        case 4: dense_d<4, GRAD>(X, N, Y, M, b, R, ls, out, s); break;
-        default: dense_d<5, GRAD>(X, N, Y, M, b, R, ls, out, s); break;
-    }
-}
-template void dense_f32<false>(const float *, int64_t, const float *, int64_t, const float *, int, int, float, float *, cudaStream_t);
-template void dense_f32<true>(const float *, int64_t, const float *, int64_t, const float *, int, int, float, float *, cudaStream_t);
-
-// float64 dense product with a double-precision exponential (accuracy reference on the device).
-// grid.y slices the sources so that a few thousand target rows still fill the GPU; slices are combined
-// with double atomics into a zeroed output.
-__global__ void __launch_bounds__(128) dense_f64_kernel(const double *__restrict__ X, int64_t n, const double *__restrict__ Y,
-                                                       int64_t m, const double *__restrict__ b, int R, int d, double lcs,
-                                                       double *out) {
-    __shared__ double sy[128 * F3M_MAX_DIM];
-    const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
-    const int64_t per = (m + gridDim.y - 1) / gridDim.y;
-    const int64_t m0 = (int64_t)blockIdx.y * per, m1 = min(m, m0 + per);
-    double xi[F3M_MAX_DIM];
-    for (int k = 0; k < d; k++) xi[k] = X[(i < n ? i : n - 1) * d + k];
-    for (int r = 0; r < R; r++) {
-        double acc = 0.;
-        for (int64_t base = m0; base < m1; base += 128) {
-            int cnt = (int)min((int64_t)128, m1 - base);
-            __syncthreads();
-            for (int q = threadIdx.x; q < cnt * d; q += 128) sy[q] = Y[base * d + q];
-            __syncthreads();
-            for (int j = 0; j < cnt; j++) {
-                double r2 = 0.;
-                for (int k = 0; k < d; k++) { double dk = xi[k] - sy[j * d + k]; r2 += dk * dk; }
-                acc += exp(-r2 * lcs) * b[(base + j) * R + r];
-            }
-        }
-        if (i < n) atomicAdd(&out[i * R + r], acc);
-    }
-}
-
-void dense_f64(const double *X, int64_t N, const double *Y, int64_t M, const double *b, int R, int d, double ls, double *out,
-               cudaStream_t s) {
-    F3M_CUDA(cudaMemsetAsync(out, 0, (size_t)N * R * sizeof(double), s));
-    const unsigned gx = (unsigned)((N + 127) / 128);
-    int64_t want = (int64_t)NUM_SMS_HINT * 16 / gx;
-    unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, (M + 4095) / 4096), 4096));
-    dense_f64_kernel<<<dim3(gx, gy), 128, 0, s>>>(X, N, Y, M, b, R, d, 1.0 / (2.0 * ls * ls), out);
-    F3M_LAUNCH_CHECK();
-}
-
-// ---------------------------------------------------------------------------------------------
-// Exact dense product without any allocation.
-//
-// Some hosts may not touch the CUDA allocator once they are running: a service that handed all device
-// memory to its own pool at start-up, or a control loop with a "no allocation after initialisation"
-// rule, because an allocation can stall the whole device.  For them f3m_rbf_dense_f32_static computes
-// the same product as f3m_rbf_dense_f32 with its only scratch buffer -- the packed source rows -- in a
-// fixed array that is part of the library image.  Every GPU that loads libf3m.so holds this array
-// (F3M_STATIC_SCRATCH_FLOATS floats = 16 MiB) until the process exits.
-//
-// In host code the array's name is only a stand-in, not a device address; the address a kernel can use
-// is obtained once per device, with that device current, through cudaGetSymbolAddress.  The first call
-// on a device performs this look-up, so make that first call before any stream capture starts.
-// All calls share the one array: it keeps whatever the previous call packed (every row a call reads is
-// rewritten by that call first, so nothing has to be cleared), and two calls that overlap on the GPU
-// -- different streams, or different host threads -- race on it.
-// ---------------------------------------------------------------------------------------------
-static __device__ __align__(256) float g_static_scratch[F3M_STATIC_SCRATCH_FLOATS];
-
-static float *static_scratch_for_current_device() {
-    static std::atomic<float *> ptr_of_device[64];   // zero-initialised; two threads may both look the address up, both get the same
-    int dev = 0;
-    F3M_CUDA(cudaGetDevice(&dev));
-    F3M_REQUIRE(dev >= 0 && dev < 64, F3M_ERR_UNSUPPORTED, "device ordinal %d not supported by the static entry point", dev);
-    float *p = ptr_of_device[dev].load(std::memory_order_acquire);
-    if (!p) {
-        F3M_CUDA(cudaGetSymbolAddress((void **)&p, g_static_scratch));
-        ptr_of_device[dev].store(p, std::memory_order_release);
-    }
-    return p;
-}
-
-template <int D>
-static void dense_static_d(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, float ls, float *out,
-                           float *scratch, cudaStream_t s) {
-    const float lcs = 1.f / (2.f * ls * ls);
-    const float scale = near_scale(lcs);
-    const unsigned gy = (unsigned)((M + 255) / 256), gx = (unsigned)((N + NT - 1) / NT);
-    for (int r0 = 0; r0 < R;) {   // column blocks reuse the scratch one after the other on the same stream
-        if (R - r0 >= 2) {
-            pack_rows_dense<D, 4><<<gy, 256, 0, s>>>(Y, M, b, R, r0, scale, scratch);
-            F3M_LAUNCH_CHECK();
-            dense_kernel<D, 4, false><<<gx, NT, 0, s>>>(X, N, scratch, M, scale, 1.f, R, r0, out);
-            r0 += 4;
-        } else {
-            pack_rows_dense<D, 1><<<gy, 256, 0, s>>>(Y, M, b, R, r0, scale, scratch);
-            F3M_LAUNCH_CHECK();
-            dense_kernel<D, 1, false><<<gx, NT, 0, s>>>(X, N, scratch, M, scale, 1.f, R, r0, out);
-            r0 += 1;
-        }
-        F3M_LAUNCH_CHECK();
-    }
-}
-
-void dense_f32_static(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,
-                      cudaStream_t s) {
-    const int64_t width = row_width(d, R >= 2 ? 4 : 1);
-    F3M_REQUIRE(M * width <= (int64_t)F3M_STATIC_SCRATCH_FLOATS, F3M_ERR_TOO_LARGE,
-                "f3m_rbf_dense_f32_static holds %lld packed floats; M=%lld sources of %lld floats each need %lld "
-                "(use f3m_rbf_dense_f32, which allocates)",
-                (long long)F3M_STATIC_SCRATCH_FLOATS, (long long)M, (long long)width, (long long)(M * width));
-    float *scratch = static_scratch_for_current_device();
-    switch (d) {
-        case 1: dense_static_d<1>(X, N, Y, M, b, R, ls, out, scratch, s); break;
-        case 2: dense_static_d<2>(X, N, Y, M, b, R, ls, out, scratch, s); break;
-        case 3: dense_static_d<3>(X, N, Y, M, b, R, ls, out, scratch, s); break;
-        case 4: dense_static_d<4>(X, N, Y, M, b, R, ls, out, scratch, s); break;
-        default: dense_static_d<5>(X, N, Y, M, b, R, ls, out, scratch, s); break;
     }
 }
 
