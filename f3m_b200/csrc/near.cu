@@ -197,41 +197,7 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 }
 __host__ __device__ __forceinline__ int pair_row_start(int off, int box) { return (off + box + 1) & ~1; }
 
-template <int D, int RB>
-__global__ void __launch_bounds__(256) pack_pairs_rel(const float *__restrict__ pts, int n, const float *__restrict__ bs,
-                                                     int R, int r0, float scale, const int *__restrict__ off_y, int nby,
-                                                     const float *__restrict__ ctr_y, const unsigned char *__restrict__ need,
-                                                     float *packed) {
-    constexpr int W = row_width(D, RB);
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const int by = box_of_row(off_y, nby, j);
-    if (need && !need[by]) return;   // a slice of the targets reads only the source boxes its lists name
-    const int s0 = off_y[by], s1 = off_y[by + 1];
-    float row[W];
-    float ny = 0.f;
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-        float yr = scale * (pts[(size_t)k * n + j] - ctr_y[by * D + k]);
-        ny = fmaf(-yr, yr, ny);
-        row[k] = 2.f * yr;
-    }
-    const float wy = ex2_approx(ny);
-#pragma unroll
-    for (int r = 0; r < RB; r++) row[D + r] = (r0 + r < R) ? bs[(size_t)j * R + r0 + r] * wy : 0.f;
-#pragma unroll
-    for (int c = D + RB; c < W; c++) row[c] = 0.f;
-    const int pos = pair_row_start(s0, by) + (j - s0);
-    float *dst = packed + (size_t)(pos >> 1) * (2 * W) + (pos & 1);
-#pragma unroll
-    for (int c = 0; c < W; c++) dst[2 * c] = row[c];
-    if (j == s1 - 1 && !(pos & 1)) {   // last source of an odd box: its partner weighs nothing
-#pragma unroll
-        for (int c = 0; c < W; c++) dst[2 * c + 1] = 0.f;
-    }
-}
-
-// The same packing with one warp per source box (and per part of a long box): boxes no list of this product names
+// Packing with one warp per source box (and per part of a long box): boxes no list of this product names
 // are skipped without touching their points, and no point searches for its box.
 template <int D, int RB>
 __global__ void __launch_bounds__(256) pack_pairs_box(const float *__restrict__ pts, int n, const float *__restrict__ bs, int R,
@@ -273,9 +239,7 @@ __global__ void __launch_bounds__(256) pack_pairs_box(const float *__restrict__ 
     }
 }
 
-// source pairs per shared-memory tile: 6 KB for one column, 12 KB for eight (so that shared memory does not limit the
-// CTAs per SM below what the registers allow)
-template <int RB> __host__ __device__ constexpr int sp2_of() { return RB >= 4 ? 96 : 192; }
+constexpr int SP2 = 192;   // source pairs per shared-memory tile (6 KB)
 
 // POLY = 0: every exponential on the MUFU pipe.  POLY = 2 or 3: PNUM of every PDEN source pairs use the
 // polynomial of that degree instead (the host enables it only when the exponent is provably small).
@@ -325,7 +289,6 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
             for (int r = 0; r < RB; r++) acc[u][r] = pack2(0.f, 0.f);
         }
-        constexpr int SP2 = sp2_of<RB>();
         for (int base = 0; base < npairs; base += SP2) {
             const int np = min(SP2, npairs - base);
             __syncthreads();
@@ -398,161 +361,9 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 }
 
 
-// 16-byte asynchronous copy global -> shared (completion tracked per thread in commit groups)
-__device__ __forceinline__ void cp_async16(float *smem_dst, const float *gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// A tile of at most 32 targets (small boxes: clustered data, four and five dimensions), one warp.  Two things differ
-// from near_tile_x2.  (1) With TS <= 16 targets (TS a power of two) the warp splits into 32 / TS lane groups that hold
-// the same targets and take every (32 / TS)-th source pair; the groups' sums are added by shuffles at the end, so no
-// lane idles.  (2) Source boxes of a dozen points give a handful of pair iterations each, too few to hide the chain
-// list entry -> box offsets -> packed rows behind: the shared-memory tile is two half tiles, the rows of the next chunk
-// arrive by asynchronous copies while the current one is consumed, and the offsets and centres of the two boxes after
-// it are already in registers.
-template <int D, int RB, int POLY, int PNUM, int PDEN>
-__device__ __forceinline__ void near_tile_x2_small(const float *__restrict__ xpts, int n_x, const int *__restrict__ ptr,
-                                                   const int *__restrict__ idx, const int *__restrict__ off_y,
-                                                   const float *__restrict__ ctr_y, const float *__restrict__ packed,
-                                                   float scale, int R, int r0, float *out, float pc0, float pc1, float pc2,
-                                                   float pc3, float *smem, int box, int t0, int t1) {
-    constexpr int W = row_width(D, RB);
-    constexpr int SPH = sp2_of<RB>() / 2;   // source pairs per half tile
-    constexpr int V4 = 2 * W / 4;           // 16-byte pieces of a pair block
-    const int lane = threadIdx.x;
-    const int nt = t1 - t0;
-    const int lg = nt > 16 ? 5 : (nt > 8 ? 4 : (nt > 4 ? 3 : 2));
-    const int TS = 1 << lg, G = 32 >> lg;
-    const int g = lane >> lg;
-    const int ti = t0 + (lane & (TS - 1));
-    float x[D], tot[RB];
-    {
-        const int ii = ti < t1 ? ti : t0;
-#pragma unroll
-        for (int k = 0; k < D; k++) x[k] = xpts[(size_t)k * n_x + ii];
-#pragma unroll
-        for (int r = 0; r < RB; r++) tot[r] = 0.f;
-    }
-    const f32x2 c1 = pack2(pc1, pc1), c2 = pack2(pc2, pc2), c3 = pack2(pc3, pc3), one = pack2(pc0, pc0);
-    const int e0 = ptr[box], e1 = ptr[box + 1];
-    if (e0 == e1) return;
-    struct Src {
-        int npairs;
-        const float *rows;
-        float ctr[D];
-    };
-    auto load_src = [&](int by, Src &sb) {
-        const int s0 = off_y[by];
-        sb.npairs = (off_y[by + 1] - s0 + 1) >> 1;
-        sb.rows = packed + (size_t)pair_row_start(s0, by) * W;
-#pragma unroll
-        for (int k = 0; k < D; k++) sb.ctr[k] = __ldg(ctr_y + by * D + k);
-    };
-    auto issue_copy = [&](float *dst, const Src &sb, int base) {
-        const int pieces = min(SPH, sb.npairs - base) * V4;
-        const float *src = sb.rows + (size_t)base * 2 * W;
-        for (int q = lane; q < pieces; q += NT2) cp_async16(dst + 4 * q, src + 4 * q);
-    };
-    Src cur, n1, n2;
-    load_src(idx[e0], cur);
-    n1 = cur; n2 = cur;
-    if (e0 + 1 < e1) load_src(idx[e0 + 1], n1);
-    if (e0 + 2 < e1) load_src(idx[e0 + 2], n2);
-    int by3 = e0 + 3 < e1 ? idx[e0 + 3] : 0;
-    issue_copy(smem, cur, 0);
-    cp_async_commit();
-    int e = e0, base = 0, pb = 0;
-    f32x2 xr[D], acc[RB];
-    float fx = 0.f;
-    while (true) {
-        const bool more_in_box = base + SPH < cur.npairs;
-        const bool have_next = more_in_box || e + 1 < e1;
-        float *bufc = smem + pb * (SPH * 2 * W), *bufn = smem + (pb ^ 1) * (SPH * 2 * W);
-        if (have_next) {
-            if (more_in_box) issue_copy(bufn, cur, base + SPH);
-            else issue_copy(bufn, n1, 0);
-        }
-        cp_async_commit();
-        cp_async_wait<1>();   // everything but the group just committed has landed
-        __syncthreads();
-        if (base == 0) {
-            float nx = 0.f;
-#pragma unroll
-            for (int k = 0; k < D; k++) {
-                const float v = scale * (x[k] - cur.ctr[k]);
-                nx = fmaf(-v, v, nx);
-                xr[k] = pack2(v, v);
-            }
-            fx = ex2_approx(nx);
-#pragma unroll
-            for (int r = 0; r < RB; r++) acc[r] = pack2(0.f, 0.f);
-        }
-        const int np = min(SPH, cur.npairs - base);
-        int q = 0;
-#pragma unroll 2
-        for (int j = g; j < np; j += G) {
-            f32x2 col[W];
-            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(bufc + j * 2 * W);
-#pragma unroll
-            for (int c = 0; c < W / 2; c++) {
-                const ulonglong2 v = src[c];
-                col[2 * c] = v.x;
-                col[2 * c + 1] = v.y;
-            }
-            f32x2 t = mul2(xr[0], col[0]);
-#pragma unroll
-            for (int k = 1; k < D; k++) t = fma2(xr[k], col[k], t);
-            f32x2 ev;
-            if (POLY && ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN) {
-                ev = (POLY == 2) ? fma2(fma2(c2, t, c1), t, one) : fma2(fma2(fma2(c3, t, c2), t, c1), t, one);
-            } else {
-                float ta, tb;
-                unpack2(t, ta, tb);
-                ev = pack2(ex2_approx(ta), ex2_approx(tb));
-            }
-#pragma unroll
-            for (int r = 0; r < RB; r++) acc[r] = fma2(ev, col[D + r], acc[r]);
-            if (POLY && ++q == PDEN) q = 0;
-        }
-        if (!more_in_box) {
-#pragma unroll
-            for (int r = 0; r < RB; r++) {
-                float lo, hi;
-                unpack2(acc[r], lo, hi);
-                tot[r] = fmaf(fx, lo + hi, tot[r]);
-            }
-        }
-        __syncthreads();   // the copy issued in the next round overwrites the half tile read here
-        if (more_in_box) base += SPH;
-        else {
-            if (++e >= e1) break;
-            base = 0;
-            cur = n1;
-            n1 = n2;
-            if (e + 2 < e1) load_src(by3, n2);
-            by3 = e + 3 < e1 ? idx[e + 3] : 0;
-        }
-        pb ^= 1;
-    }
-    cp_async_wait<0>();
-    for (int o = TS; o < 32; o <<= 1)
-#pragma unroll
-        for (int r = 0; r < RB; r++) tot[r] += __shfl_xor_sync(0xffffffffu, tot[r], o);
-    if (g == 0 && ti < t1) {
-#pragma unroll
-        for (int r = 0; r < RB; r++)
-            if (r0 + r < R) out[(size_t)ti * R + r0 + r] += tot[r];
-    }
-}
-
-// TI = targets per thread.  MIXED: a tile of at most 32 targets runs a one-target form, which does half the work (the
-// pipelined one for small boxes); the host picks this variant only when such tiles exist.
+// TI = targets per thread.  MIXED: a tile of at most 32 targets runs a one-target form, which does half the work; the host picks this variant only when such tiles exist.
 template <int D, int RB, int POLY, int PNUM, int PDEN, bool MIXED>
-__global__ void __launch_bounds__(NT2, RB == 1 ? 32 : (RB <= 4 ? 20 : 12)) near_kernel_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x,
+__global__ void __launch_bounds__(NT2, 32) near_kernel_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x,
                                                      int nbx, const int *__restrict__ tile_off,
                                                      const int *__restrict__ ptr, const int *__restrict__ idx,
                                                      const int *__restrict__ off_y, const float *__restrict__ ctr_y,
@@ -560,18 +371,12 @@ __global__ void __launch_bounds__(NT2, RB == 1 ? 32 : (RB <= 4 ? 20 : 12)) near_
                                                      float *out, float pc0, float pc1, float pc2, float pc3, int row_begin,
                                                      int row_end) {
     constexpr int W = row_width(D, RB);
-    __shared__ __align__(16) float smem[sp2_of<RB>() * 2 * W];
+    __shared__ __align__(16) float smem[SP2 * 2 * W];
     int box, t0, t1;
     item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1, MIXED ? NT2 * TI2 : 0);
     if (MIXED && t1 - t0 <= NT2) {
-        // a box of at most 32 points has neighbours of its own kind (same level, same local density): short source boxes,
-        // where the pipelined form pays; the last tile of a large box meets large source boxes and keeps the plain loop
-        if (RB >= 4 && off_x[box + 1] - off_x[box] <= NT2)   // one column: measured slower than the plain loop on clustered data
-            near_tile_x2_small<D, RB, POLY, PNUM, PDEN>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2,
-                                                        pc3, smem, box, t0, t1);
-        else
-            near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3,
-                                                     smem, box, t0, t1);
+        near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3,
+                                                 smem, box, t0, t1);
     } else
         near_tile_x2<D, RB, POLY, PNUM, PDEN, TI2>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3, smem,
                                                    box, t0, t1);
@@ -632,7 +437,7 @@ static inline float near_scale(float lcs) { return sqrtf(lcs * 1.442695040888963
 // any distance test, and the two cubes have separate origins (n_tree.cu:1096-1098): "small" pairs there are
 // classified by size before distance (1_d_conv.cu:916-920), so their distance is bounded only by the offset
 // between the two cubes.
-static double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
+double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
     const bool final_near = (&csr == &pl->lists[level].keep);
     if (final_near) return 2.5;
     if (level == 1 && !pl->same) {
@@ -777,10 +582,11 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 template <int D>
 static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out, int rb, int re,
                      cudaStream_t s) {
+    // expanded form? (the conditions of direct_impl)
+    const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
+    const bool expanded = level > 0 && se <= 1.0 && D * list_reach(pl, level, csr) * se * se <= TMAX_EXPANDED;
     for (int r0 = 0; r0 < R;) {
-        const int left = R - r0;
-        if (left >= 5) { direct_impl<D, 8>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 8; }
-        else if (left >= 2) { direct_impl<D, 4>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 4; }
+        if (R - r0 >= 2) { column_sums(pl, level, csr, expanded, bs, R, r0, out, rb, re, s); r0 += 8; }
         else { direct_impl<D, 1>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 1; }
     }
 }
