@@ -401,17 +401,19 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     outs.zero();
     pl->last.end(s);
 
+    // A product over all rows may end at a level whose interpolation is exact for all its pairs (far_cut_level)
+    const int cut = row_begin <= 0 && row_end >= N && !pl->ext_mom && !pl->shard.active ? far_cut_level(pl, R) : 0;
     const int L = pl->levels;
     if (L == 0) {
         // largest box already small enough: one direct product over the root pair
         direct_sums(pl, 0, pl->lists[0].keep, bs.p, R, outs.p, row_begin, row_end, s);
     }
-    for (int level = 1; level <= L; level++) {
+    for (int level = 1; level <= (cut ? cut - 1 : L); level++) {
         LevelLists &ll = pl->lists[level];
         direct_sums(pl, level, ll.small, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1018-1020
     }
-    far_field(pl, bs.p, R, outs.p, row_begin, row_end, s);                          // n_tree.cu:1021-1051, all levels
-    if (L > 0) direct_sums(pl, L, pl->lists[L].keep, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1092-1094
+    far_field(pl, bs.p, R, outs.p, row_begin, row_end, cut, s);                     // n_tree.cu:1021-1051, all levels
+    if (L > 0 && !cut) direct_sums(pl, L, pl->lists[L].keep, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1092-1094
 
     pl->last.begin(ST_UNPERMUTE, s);
     if (row_begin <= 0 && row_end >= N) scatter_rows(outs.p, tx.perm.p, out, N, R, s);
@@ -495,7 +497,7 @@ int f3m_plan_moments_range(f3m_plan *plan, const float *b, int32_t R, int64_t sr
         plan->moments_out = mom_out;
         plan->mom_begin = src_begin;
         plan->mom_end = src_end;
-        far_field(plan, bs.p, R, nullptr, 0, 0, s);
+        far_field(plan, bs.p, R, nullptr, 0, 0, 0, s);
         F3M_CUDA(cudaStreamSynchronize(s));
     });
     plan->moments_out = nullptr;
@@ -636,7 +638,7 @@ int f3m_plan_shard_begin(f3m_plan *plan, const float *b, int32_t R, int64_t row_
             plan->mom_end = plan->h_pinned[1];
             plan->mom_box_begin = box_begin;
             plan->mom_box_end = box_end;
-            far_field(plan, sh.bs.p, R, nullptr, 0, 0, s);
+            far_field(plan, sh.bs.p, R, nullptr, 0, 0, 0, s);
         }
         F3M_CUDA(cudaStreamSynchronize(s));
         sh.active = true;
@@ -677,7 +679,7 @@ int f3m_plan_shard_far(f3m_plan *plan, const float *mom, float *acc_sorted, void
         F3M_REQUIRE(sh.active, F3M_ERR_ARG, "f3m_plan_shard_far without f3m_plan_shard_begin");
         F3M_REQUIRE(mom || sh.all_sources, F3M_ERR_ARG, "this product exchanges moments: pass the gathered moment array");
         plan->ext_mom = sh.all_sources ? nullptr : mom;
-        far_field(plan, sh.bs.p, sh.R, acc_sorted, sh.row_begin, sh.row_end, s);
+        far_field(plan, sh.bs.p, sh.R, acc_sorted, sh.row_begin, sh.row_end, 0, s);
         F3M_CUDA(cudaMemcpyAsync(plan->h_pinned, plan->d_flags + FL_ERR, sizeof(int), cudaMemcpyDeviceToHost, s));
         F3M_CUDA(cudaStreamSynchronize(s));
         F3M_REQUIRE(plan->h_pinned[0] == 0, F3M_ERR_INTERNAL, "device-side consistency check failed (code %d)", plan->h_pinned[0]);

@@ -257,6 +257,8 @@ struct f3m_plan {
     f3m::Tree tx, ty_store;
     f3m::Tree *ty = nullptr;
     std::vector<f3m::LevelLists> lists;   // lists[l] for level l (index 0 unused)
+    f3m::LevelLists cut_lists;            // all pairs of the level a product is cut at (count, row pointers and the ordered rows)
+    int cut_level = 0;
     int levels = 0;
     f3m_plan_stats stats{};
     f3m::Timings last;
@@ -266,7 +268,7 @@ struct f3m_plan {
     // LEAF_SMALL points are handled one per warp, the others one per CTA; built on first use
     f3m::DevBuf<int> leaf_small[2], leaf_big[2];
     int n_leaf_small[2] = {0, 0}, n_leaf_big[2] = {0, 0};
-    bool leaf_split[2] = {false, false};
+    int leaf_level[2] = {-1, -1};         // level the two lists were built for
     float *moments_out = nullptr;
     int64_t mom_begin = 0, mom_end = 0;
     int64_t mom_box_begin = -1, mom_box_end = -1;   // >= 0: moments_out covers these source boxes only
@@ -323,9 +325,10 @@ void accumulate_pair_work(f3m_plan *pl, int level, int slot, const PairCSR &csr,
 int nodes_per_dim(int d, int nr_interpolation);   // get_node_list for perfect powers, floor otherwise
 void far_field_level(f3m_plan *pl, int level, const float *b_sorted, int R, float *out_sorted,
                      int64_t row_begin, int64_t row_end, cudaStream_t s);   // per-level path (far.cu)
-void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end,
+void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut,
                cudaStream_t s);                                               // whole product (far_fast.cu)
 int64_t far_moments_size(const f3m_plan *pl, int R);
+int far_cut_level(const f3m_plan *pl, int R);   // level at which a product over all rows may end, 0: none
 
 // ---- shard.cu --------------------------------------------------------------------------------
 const unsigned char *level_source_flags(f3m_plan *pl, int level, cudaStream_t s);   // per source box of the level: named by a direct list?
@@ -353,6 +356,7 @@ void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, con
 // near_moments.cu: sums a direct list through box moments when its geometry allows; false: sum the pairs
 bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted, int row_begin,
                  int row_end, cudaStream_t s);
+double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate
 template <bool GRAD>
 void dense_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,
                cudaStream_t s);

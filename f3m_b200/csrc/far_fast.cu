@@ -297,9 +297,22 @@ __global__ void __launch_bounds__(128, 5) m2l_fast(int nbx, int d, const int *__
 // In four and five dimensions the rank key is the base-8 number of the offsets counted from the lowest one
 // that can occur (tabulated offset 4): 8^4 and 8^5 keys.  An offset outside that window is clamped; if two
 // pairs of a row then share a rank key the row keeps its list order (every order is correct, see above).
+// The row may be spread over several CSR lists (the cut level takes far, small and kept pairs alike): its segments are
+// ordered together and written where a list holding all of them has the row.
+struct ListSet {
+    const int *ptr[3], *idx[3];
+    int n;
+};
+__global__ void __launch_bounds__(256) add_list_ptrs(int count, ListSet ls, int *ptr) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= count) return;
+    int v = 0;
+    for (int l = 0; l < ls.n; l++) v += ls.ptr[l][b];
+    ptr[b] = v;
+}
+
 template <int WPL>   // bitmap words per lane: 4 -> 4096 rank keys, 32 -> 32768
-__global__ void __launch_bounds__(128) far_order_kernel(int nbx, int d, const int *__restrict__ fptr, const int *__restrict__ fidx,
-                                                       const int *__restrict__ cell_x, const int *__restrict__ cell_y,
+__global__ void __launch_bounds__(128) far_order_kernel(int nbx, int d, ListSet ls, const int *__restrict__ cell_x, const int *__restrict__ cell_y,
                                                        Geom2 geo, uint32_t *okey, int *oidx, int *err,
                                                        const int *__restrict__ off_x, int row_begin, int row_end) {
     constexpr int ORD_WORDS = 32 * WPL;
@@ -309,8 +322,22 @@ __global__ void __launch_bounds__(128) far_order_kernel(int nbx, int d, const in
     const int bx = blockIdx.x * 4 + w;
     if (bx >= nbx) return;
     if (off_x[bx + 1] <= row_begin || off_x[bx] >= row_end) return;   // no row of this box in the slice being computed
-    const int e0 = fptr[bx], n = fptr[bx + 1] - e0;
+    int e0 = 0, n = 0, seg[3], cnt[3];
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+        seg[l] = cnt[l] = 0;
+        if (l >= ls.n) continue;
+        seg[l] = ls.ptr[l][bx];
+        cnt[l] = ls.ptr[l][bx + 1] - seg[l];
+        e0 += seg[l];
+        n += cnt[l];
+    }
     if (n == 0) return;
+    auto source = [&](int i) {   // i-th source box of the row
+        if (i < cnt[0]) return ls.idx[0][seg[0] + i];
+        i -= cnt[0];
+        return i < cnt[1] ? ls.idx[1][seg[1] + i] : ls.idx[2][seg[2] + i - cnt[1]];
+    };
     const bool compact = d > 3;
     // key: one nibble per axis, last axis lowest, axis 0 on top; rkey: what the row is ordered by
     auto key_of = [&](int by, uint32_t &rkey) {
@@ -329,7 +356,7 @@ __global__ void __launch_bounds__(128) far_order_kernel(int nbx, int d, const in
     __syncwarp();
     for (int i = lane; i < n; i += 32) {
         uint32_t rkey;
-        key_of(fidx[e0 + i], rkey);
+        key_of(source(i), rkey);
         atomicOr(&bits[w][rkey >> 5], 1u << (rkey & 31u));
     }
     __syncwarp();
@@ -347,11 +374,11 @@ __global__ void __launch_bounds__(128) far_order_kernel(int nbx, int d, const in
     __syncwarp();
     if (distinct != n) {   // cannot happen for d <= 3 (boxes of one level have distinct cells); keep the list order
         if (lane == 0 && !compact) atomicExch(err, 2);
-        for (int i = lane; i < n; i += 32) { int by = fidx[e0 + i]; uint32_t rk; okey[e0 + i] = key_of(by, rk); oidx[e0 + i] = by; }
+        for (int i = lane; i < n; i += 32) { int by = source(i); uint32_t rk; okey[e0 + i] = key_of(by, rk); oidx[e0 + i] = by; }
         return;
     }
     for (int i = lane; i < n; i += 32) {
-        const int by = fidx[e0 + i];
+        const int by = source(i);
         uint32_t rkey;
         const uint32_t key = key_of(by, rkey);
         const int rank = below[w][rkey >> 5] + __popc(bits[w][rkey >> 5] & ((1u << (rkey & 31u)) - 1u));
@@ -778,6 +805,19 @@ template <int PP, int RBB>
 static void launch_m2l_rows(int d, int nbx, const int *fptr, const uint32_t *okey, const int *oidx, const int *offx, int rb, int re,
                             const float *T, const float *mom, float *loc, cudaStream_t s) {
     m2l_rows_dispatch<PP, RBB>(false, d, nbx, fptr, okey, oidx, offx, rb, re, T, mom, loc, s);
+}
+
+// is there a row form for p nodes per dimension and 8 columns?
+static bool rows_form_for(int p, int d) {
+    switch (p) {
+        case 2: return rows_form_available<2, 8>(d);
+        case 3: return rows_form_available<3, 8>(d);
+        case 4: return rows_form_available<4, 8>(d);
+        case 5: return rows_form_available<5, 8>(d);
+        case 6: return rows_form_available<6, 8>(d);
+        case 7: return rows_form_available<7, 8>(d);
+        default: return rows_form_available<8, 8>(d);
+    }
 }
 
 // M2M: one CTA per parent box, warps share the children
@@ -1281,9 +1321,10 @@ __global__ void __launch_bounds__(128) l2p_small3(const float *__restrict__ pts,
     out[(size_t)(a + lane) * R + r0] += v;
 }
 
-// lists of the small and the large finest-level boxes of one tree (0: targets, 1: sources), built once per plan
-static void ensure_leaf_split(f3m_plan *pl, int which, Level &lv, cudaStream_t s) {
-    if (pl->leaf_split[which]) return;
+// lists of the small and the large boxes of the far field's last level, of one tree (0: targets, 1: sources); kept in the plan
+static void ensure_leaf_split(f3m_plan *pl, int which, int level, cudaStream_t s) {
+    if (pl->leaf_level[which] == level) return;
+    Level &lv = (which == 0 ? pl->tx : *pl->ty).levels[level];
     pl->leaf_small[which].alloc((size_t)lv.nb, s);
     pl->leaf_big[which].alloc((size_t)lv.nb, s);
     int *counts = pl->d_flags + FL_LEAF;
@@ -1294,17 +1335,25 @@ static void ensure_leaf_split(f3m_plan *pl, int which, Level &lv, cudaStream_t s
     F3M_CUDA(cudaStreamSynchronize(s));
     pl->n_leaf_small[which] = pl->h_pinned[0];
     pl->n_leaf_big[which] = pl->h_pinned[1];
-    pl->leaf_split[which] = true;
+    pl->leaf_level[which] = level;
 }
 
 // ---------------------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------------------
+// Parts a long box is cut into: at most 8192 points each, and short enough that the parts of all boxes fill the SMs four
+// times over (a cut at level 1 or 2 leaves 8 or 64 boxes), but not below 512 points.
+static int leaf_splits(int max_count, int64_t n) {
+    const int64_t part = std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT)));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(1024, (max_count + part - 1) / part));
+}
+
 template <int PP, int RB>
-static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *out, int rb, int re, int lmin,
+static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *out, int rb, int re, int lmin, int L, int cut,
                            cudaStream_t s) {
+    // L: the level whose boxes the points are interpolated to; cut == L: that level takes far, small and kept pairs
     Tree &tx = pl->tx, &ty = *pl->ty;
-    const int d = pl->d, L = pl->levels;
+    const int d = pl->d;
     int P = 1;
     for (int k = 0; k < d; k++) P *= PP;
     const int PR = P * RB;
@@ -1313,8 +1362,8 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     const KronCfg cfg = make_kron_cfg(d, PP, RB);
     const int n_x = (int)tx.n, n_y = (int)ty.n;
     if (RB == 1 && d == 3) {
-        ensure_leaf_split(pl, 0, tx.levels[L], s);
-        if (!pl->same) ensure_leaf_split(pl, 1, ty.levels[L], s);
+        ensure_leaf_split(pl, 0, L, s);
+        if (!pl->same) ensure_leaf_split(pl, 1, L, s);
     }
 
     if (pl->moments_out) {
@@ -1377,7 +1426,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         Level &ly = ty.levels[L];
         const float factor = 2.f / ly.edge;          // 1_d_conv.cu:473
         if (!pl->ext_mom) {
-            int nsplit = std::max(1, std::min(64, (ly.max_count + 8191) / 8192));
+            const int nsplit = leaf_splits(ly.max_count, ty.n);
             if (nsplit > 1) mom[L].zero();
             size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
             F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1429,9 +1478,18 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         };
         DevBuf<int> cellx, celly;
         for (int l = lmin; l <= L; l++) {
-            LevelLists &ll = pl->lists[l];
+            const bool at_cut = l == cut;
+            LevelLists &level_lists = pl->lists[l];
+            LevelLists &ll = at_cut ? pl->cut_lists : level_lists;
             if (ll.far.count == 0) continue;
             Level &lx = tx.levels[l], &ly = ty.levels[l];
+            const ListSet ls{{level_lists.far.ptr.p, level_lists.small.ptr.p, level_lists.keep.ptr.p},
+                             {level_lists.far.idx.p, level_lists.small.idx.p, level_lists.keep.idx.p}, at_cut ? 3 : 1};
+            if (at_cut && !ll.far_ordered) {
+                ll.far.ptr.alloc((size_t)lx.nb + 1, s);
+                add_list_ptrs<<<(lx.nb + 1 + 255) / 256, 256, 0, s>>>(lx.nb + 1, ls, ll.far.ptr.p);
+                F3M_LAUNCH_CHECK();
+            }
             Geom2 geo{};
             for (int k = 0; k < d; k++) {
                 double sh = pl->same ? 0.0 : (double)ty.origin[k] - (double)tx.origin[k];
@@ -1459,10 +1517,10 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                     ll.far_okey.alloc((size_t)ll.far.count, s);
                     ll.far_oidx.alloc((size_t)ll.far.count, s);
                     if (d <= 4)
-                        far_order_kernel<4><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ll.far.ptr.p, ll.far.idx.p, cellx.p, cy, geo,
+                        far_order_kernel<4><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cellx.p, cy, geo,
                                                                            ll.far_okey.p, ll.far_oidx.p, pl->d_flags, lx.off.p, rb, re);
                     else
-                        far_order_kernel<32><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ll.far.ptr.p, ll.far.idx.p, cellx.p, cy, geo,
+                        far_order_kernel<32><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cellx.p, cy, geo,
                                                                             ll.far_okey.p, ll.far_oidx.p, pl->d_flags, lx.off.p, rb, re);
                     F3M_LAUNCH_CHECK();
                     // kept for later products of this plan only when every box was ordered
@@ -1502,7 +1560,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         }
         Level &lx = tx.levels[L];
         const float factor = 2.f / lx.edge;
-        int nsplit = std::max(1, std::min(64, (lx.max_count + 8191) / 8192));
+        const int nsplit = leaf_splits(lx.max_count, tx.n);
         size_t smem = ((size_t)PR + (size_t)std::max(1, d - 1) * PP * 128) * sizeof(float);
         F3M_CUDA(cudaFuncSetAttribute(l2p_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (RB == 1 && d == 3) {
@@ -1521,14 +1579,14 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
 }
 
 template <int PP>
-static void far_fast_p(f3m_plan *pl, const float *bs, int R, float *out, int rb, int re, int lmin, cudaStream_t s) {
+static void far_fast_p(f3m_plan *pl, const float *bs, int R, float *out, int rb, int re, int lmin, int L, int cut, cudaStream_t s) {
     int P = 1;
     for (int k = 0; k < pl->d; k++) P *= PP;
     // 8 columns at a time when the three per-warp buffers of the translation kernels fit, else one
     const bool wide = R > 1 && (size_t)3 * P * 8 * sizeof(float) + (size_t)pl->d * NOFF2 * mat_stride(PP) * sizeof(float) <= 200 * 1024;
     for (int r0 = 0; r0 < R;) {
-        if (wide) { far_fast_block<PP, 8>(pl, bs, R, r0, out, rb, re, lmin, s); r0 += 8; }
-        else { far_fast_block<PP, 1>(pl, bs, R, r0, out, rb, re, lmin, s); r0 += 1; }
+        if (wide) { far_fast_block<PP, 8>(pl, bs, R, r0, out, rb, re, lmin, L, cut, s); r0 += 8; }
+        else { far_fast_block<PP, 1>(pl, bs, R, r0, out, rb, re, lmin, L, cut, s); r0 += 1; }
     }
 }
 
@@ -1556,16 +1614,87 @@ int64_t far_moments_size(const f3m_plan *pl, int R) {
     return (int64_t)pl->ty->levels[L].nb * P * RB;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Where the tree can stop.  The P-node interpolation converges like (edge / 4 l)^p / sqrt(p!), so some levels below the
+// first it reproduces the kernel to rounding for EVERY pair of boxes, neighbours and the box itself included: there the
+// split into far, small and kept pairs no longer matters, and all child pairs of the kept parents are taken through M2L at
+// once.  That level (the cut) ends the product: no direct sums, no deeper lists, no translations below it.
+//
+// Bound.  The kernel is a product over the axes, so the relative error of a pair is the sum over the axes of that of one axis.
+// There g(u) = exp(-u^2 / 2 l^2) is interpolated in x and in y over an edge e: error <= (1 + Lambda_p) E, with E =
+// max |g^(p)| / p! (e/2)^p / 2^(p-1) and max |g^(p)| <= 1.0865 sqrt(p!) / l^p (Cramer's inequality), Lambda_p <= 1 + (2/pi) ln p;
+// and g is at least exp(-(r e)^2 / 2 l^2), r - 1 the offset of the boxes along the axis.  Offsets (near_moments.cu): on one tree the
+// children of kept parents are (3,3,3,..) or (5,1,..) boxes apart, on two trees below 5 along every axis.  The sum must stay below
+// CUT_EPS = 1.2e-7, half the error of ex2.approx.
+// ---------------------------------------------------------------------------------------------
+constexpr double CUT_EPS = 1.2e-7;
+
+static bool cut_is_exact(const f3m_plan *pl, int level, int p) {
+    const int d = pl->d;
+    const double e = (double)pl->ty->levels[level].edge * sqrt(2.0 * (double)pl->lcs);   // edge / l
+    auto inv_g = [&](double r) { return exp(0.5 * r * r * e * e); };
+    double sum;
+    if (level == 1) {   // children of the root pair, which is kept without a distance test
+        sum = 0.0;
+        for (int k = 0; k < d; k++)
+            sum += inv_g(2.0 + (pl->same ? 0.0 : fabs((double)pl->tx.origin[k] - (double)pl->ty->origin[k]) / (double)pl->ty->levels[1].edge));
+    } else
+        sum = pl->same ? std::max(d * inv_g(4.0), inv_g(6.0) + (d - 1) * inv_g(2.0)) : d * inv_g(6.0);
+    double fact = 1.0;
+    for (int i = 2; i <= p; i++) fact *= i;
+    const double E = 2.0 * 1.0865 * pow(e / 4.0, p) / sqrt(fact);
+    return E * (2.0 + 2.0 / 3.14159265358979323846 * log((double)p)) * sum <= CUT_EPS;
+}
+
+// Level at which the product ends (0: no cut, all lists are used).  Among the levels that qualify the one with the smallest
+// estimated time wins.  Measured rates behind the estimate: M2L 1.25e-12 s per pair, node and column (0.25 ns per pair at 216
+// nodes, 2.5 ns at 243 nodes and 8 columns), translations 8e-12 s per box, node and column, direct lists see
+// direct_list_seconds; a cut orders a list of its own and sets up the level (20 us), which small trees do not win back.
+int far_cut_level(const f3m_plan *pl, int R) {
+    const int L = pl->levels;
+    if (L < 1 || (pl->prm.flags & (F3M_FLAG_NEAR_TENSOR_CORES | F3M_FLAG_NEAR_MOMENTS)) || pl->prm.var_compression) return 0;
+    const int p = pl->lists[1].p, d = pl->d;
+    if (p < 2 || p > PMAX_FAST || d < 2) return 0;
+    int P = 1;
+    for (int k = 0; k < d; k++) P *= p;
+    const size_t tab = (size_t)d * NOFF2 * mat_stride(p) * sizeof(float);
+    if ((size_t)3 * P * sizeof(float) + tab > 200 * 1024) return 0;
+    const bool wide = R > 1 && (size_t)3 * P * 8 * sizeof(float) + tab <= 200 * 1024;
+    // the combined list exists in ordered form only, which these kernels read
+    if (!(wide ? rows_form_for(p, d) : (d <= 3 && P / p <= 64))) return 0;
+    const double cols = wide ? 8.0 * ((R + 7) / 8) : R;
+    auto m2l = [&](const PairCSR &c) { return (double)c.count * P * cols * 1.25e-12; };
+    auto shifts = [&](int l) { return ((double)pl->tx.levels[l].nb + pl->ty->levels[l].nb) * P * cols * 8e-12; };
+    double full = direct_list_seconds(pl, L, pl->lists[L].keep, R);
+    for (int l = 1; l <= L; l++) full += direct_list_seconds(pl, l, pl->lists[l].small, R) + m2l(pl->lists[l].far) + shifts(l);
+    int best = 0;
+    double best_t = full, head = 20e-6;
+    for (int l = 1; l <= L; l++) {
+        const LevelLists &ll = pl->lists[l];
+        const double t = head + m2l(ll.far) + m2l(ll.small) + m2l(ll.keep) + shifts(l);
+        if (t < best_t && ll.far.count + ll.small.count + ll.keep.count <= 0x7fffffffLL && cut_is_exact(pl, l, p)) { best = l; best_t = t; }
+        head += direct_list_seconds(pl, l, ll.small, R) + m2l(ll.far) + shifts(l);
+    }
+    return best;
+}
+
 // Far field of the whole product.  Fast path when every level with far pairs uses the same p <= 8;
 // otherwise (var_compression switching node counts between levels, or more nodes per dimension) the
-// per-level path of far.cu.
-void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end,
+// per-level path of far.cu.  cut > 0 (far_cut_level): the product ends at that level, all of whose pairs are taken here.
+void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut,
                cudaStream_t s) {
-    const int L = pl->levels;
-    int lmin = 0, p = 0;
+    int lmin = 0, llast = 0, p = 0;
     bool uniform = true;
-    for (int l = 1; l <= L; l++) {
-        if (pl->lists[l].far.count == 0) continue;
+    if (cut && pl->cut_level != cut) {   // the number of columns can move the cut
+        LevelLists &ll = pl->lists[cut], &all = pl->cut_lists;
+        all.far_ordered = false;
+        all.far.count = ll.far.count + ll.small.count + ll.keep.count;
+        all.p = ll.p;
+        pl->cut_level = cut;
+    }
+    for (int l = 1; l <= (cut ? cut : pl->levels); l++) {
+        if ((l == cut ? pl->cut_lists.far.count : pl->lists[l].far.count) == 0) continue;
+        llast = l;
         if (!lmin) { lmin = l; p = pl->lists[l].p; }
         else if (pl->lists[l].p != p) uniform = false;
     }
@@ -1574,18 +1703,23 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
     for (int k = 0; k < pl->d; k++) P *= p;
     const bool fits = (size_t)3 * P * sizeof(float) + (size_t)pl->d * NOFF2 * mat_stride(p) * sizeof(float) <= 200 * 1024;
     if (!uniform || p > PMAX_FAST || p < 2 || !fits) {
-        for (int l = lmin; l <= L; l++) far_field_level(pl, l, b_sorted, R, out_sorted, row_begin, row_end, s);
+        for (int l = lmin; l <= pl->levels; l++) far_field_level(pl, l, b_sorted, R, out_sorted, row_begin, row_end, s);
         return;
     }
     const int rb = (int)row_begin, re = (int)row_end;
+    // Points are interpolated to the deepest level that has far pairs: below it there is nothing to translate (a mixture of
+    // 1e7 points has 1.55 M boxes of six points and no far pair on its last level).  Slices of the rows and exchanged
+    // moments are cut at boxes of the last level, so they stay there.
+    const bool whole = rb <= 0 && re >= (int)pl->tx.n && !pl->moments_out && !pl->ext_mom && !pl->shard.active;
+    const int last = whole ? llast : pl->levels;
     switch (p) {
-        case 2: far_fast_p<2>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        case 3: far_fast_p<3>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        case 4: far_fast_p<4>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        case 5: far_fast_p<5>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        case 6: far_fast_p<6>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        case 7: far_fast_p<7>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
-        default: far_fast_p<8>(pl, b_sorted, R, out_sorted, rb, re, lmin, s); break;
+        case 2: far_fast_p<2>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 3: far_fast_p<3>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 4: far_fast_p<4>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 5: far_fast_p<5>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 6: far_fast_p<6>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 7: far_fast_p<7>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        default: far_fast_p<8>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
     }
 }
 
