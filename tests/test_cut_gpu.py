@@ -20,8 +20,8 @@ def _points(n, d, dist, g):
     return torch.randn(n, d, generator=g) * 0.5 + centre[torch.randint(0, 10, (n,), generator=g)]
 
 
-@pytest.mark.parametrize("d,p,n,m,R,ls,dist", [(3, 6, 600011, 0, 1, 1.0, "uniform"), (3, 8, 400000, 0, 1, 0.7, "uniform"), (3, 5, 500000, 0, 1, 4.0, "normal"),
-                                               (3, 6, 700001, 0, 1, 3.0, "mixture"), (2, 6, 900000, 0, 1, 0.3, "uniform"), (3, 6, 500000, 300007, 1, 1.5, "uniform"),
+@pytest.mark.parametrize("d,p,n,m,R,ls,dist", [(3, 6, 600011, 0, 1, 1.0, "uniform"), (3, 8, 400000, 0, 1, 0.7, "uniform"), (3, 5, 500000, 0, 1, 40.0, "normal"),
+                                               (3, 6, 700001, 0, 1, 30.0, "mixture"), (2, 6, 900000, 0, 1, 0.3, "uniform"), (3, 6, 500000, 300007, 1, 1.5, "uniform"),
                                                (3, 6, 300000, 0, 1, 1000.0, "uniform"), (4, 4, 300000, 0, 3, 8.0, "uniform")])
 def test_cut_equals_the_full_lists(d, p, n, m, R, ls, dist, cuda):
     from f3m_b200 import engine

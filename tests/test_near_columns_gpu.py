@@ -16,7 +16,7 @@ def test_columns_against_float64(d, n, m, R, ls, cuda):
     X = torch.rand(n, d, generator=g).to(cuda)
     Y = torch.rand(m, d, generator=g).to(cuda) if m else None
     b = (torch.rand(m or n, R, generator=g) + 0.5).to(cuda)
-    plan = engine.Plan(X, Y, engine.make_params(ls, 5.0 if min(n, m or n) < 100 else 100.0, 2 ** d, False, 0.15, 10 ** 6))
+    plan = engine.Plan(X, Y, engine.make_params(ls, 5.0 if min(n, m or n) < 100 else 100.0, 8 ** d, False, 0.15, 10 ** 6))
     out = plan.apply(b)
     st = plan.stats()
     assert st["far_box_pairs"] == 0 and st["direct_pairs"] == n * (m or n)
