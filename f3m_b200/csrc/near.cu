@@ -195,6 +195,29 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// coefficients of the polynomial part of the exponentials, lowest first
+struct ExpCoef { float c[6]; };
+// 2^t for |t| < 120 on the FMA pipe: t = n + f with |f| <= 1/2 (n rounded off by adding and subtracting 1.5 * 2^23), the
+// degree-5 polynomial through the Chebyshev points of [-1/2, 1/2] for 2^f (relative error below 7.5e-8, a third of
+// ex2.approx's), and n added to the exponent.
+__device__ __forceinline__ f32x2 ex2_on_fma(f32x2 t, const f32x2 (&c)[6]) {
+    const f32x2 magic = pack2(12582912.f, 12582912.f), nmagic = pack2(-12582912.f, -12582912.f), minus1 = pack2(-1.f, -1.f);
+    const f32x2 r = add2(t, magic);
+    const f32x2 f = fma2(add2(r, nmagic), minus1, t);
+    f32x2 p = fma2(c[5], f, c[4]);
+#pragma unroll
+    for (int k = 3; k >= 0; k--) p = fma2(p, f, c[k]);
+    float ra, rb, pa, pb;
+    unpack2(r, ra, rb);
+    unpack2(p, pa, pb);
+    return pack2(__uint_as_float(__float_as_uint(pa) + (__float_as_uint(ra) << 23)),
+                 __uint_as_float(__float_as_uint(pb) + (__float_as_uint(rb) << 23)));
+}
 __host__ __device__ __forceinline__ int pair_row_start(int off, int box) { return (off + box + 1) & ~1; }
 
 // Packing with one warp per source box (and per part of a long box): boxes no list of this product names
@@ -241,14 +264,15 @@ __global__ void __launch_bounds__(256) pack_pairs_box(const float *__restrict__ 
 
 constexpr int SP2 = 192;   // source pairs per shared-memory tile (6 KB)
 
-// POLY = 0: every exponential on the MUFU pipe.  POLY = 2 or 3: PNUM of every PDEN source pairs use the
-// polynomial of that degree instead (the host enables it only when the exponent is provably small).
+// PNUM of every PDEN source pairs evaluate their exponentials on the FMA pipe, the others on the MUFU pipe.  POLY = 2 or 3:
+// by the polynomial of that degree (the host enables it only when the exponent is provably small).  POLY = 5: by
+// ex2_on_fma, for any exponent.  A pair of sources costs 16 MUFU cycles per warp and target against d + 1 packed
+// multiply-adds (8 cycles at d = 3); ex2_on_fma moves them to 16 cycles of the FMA pipe, so one pair in four levels the two.
 template <int D, int RB, int POLY, int PNUM, int PDEN, int TI>
 __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ ptr,
                                              const int *__restrict__ idx, const int *__restrict__ off_y,
                                              const float *__restrict__ ctr_y, const float *__restrict__ packed, float scale, int R,
-                                             int r0, float *out, float pc0, float pc1, float pc2, float pc3, float *smem, int box,
-                                             int t0, int t1) {
+                                             int r0, float *out, const ExpCoef &pc, float *smem, int box, int t0, int t1) {
     constexpr int W = row_width(D, RB);
     float x[TI][D], tot[TI][RB];
     int ti[TI];
@@ -267,7 +291,9 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
         for (int r = 0; r < RB; r++) tot[u][r] = 0.f;
     }
-    const f32x2 c1 = pack2(pc1, pc1), c2 = pack2(pc2, pc2), c3 = pack2(pc3, pc3), one = pack2(pc0, pc0);
+    f32x2 c[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) c[k] = pack2(pc.c[k], pc.c[k]);
     const int e0 = ptr[box], e1 = ptr[box + 1];
     for (int e = e0; e < e1; e++) {
         const int by = idx[e];
@@ -312,8 +338,10 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
                     for (int k = 1; k < D; k++) t = fma2(xr[u][k], col[k], t);
                     f32x2 ev;
-                    if (POLY && poly) {
-                        ev = (POLY == 2) ? fma2(fma2(c2, t, c1), t, one) : fma2(fma2(fma2(c3, t, c2), t, c1), t, one);
+                    if (poly) {
+                        ev = POLY == 5   ? ex2_on_fma(t, c)
+                             : POLY == 2 ? fma2(fma2(c[2], t, c[1]), t, c[0])
+                                         : fma2(fma2(fma2(c[3], t, c[2]), t, c[1]), t, c[0]);
                     } else {
                         float ta, tb;
                         unpack2(t, ta, tb);
@@ -325,15 +353,10 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
             };
             int j = 0;
             const int npl = (TI == 1) ? (np - grp + G - 1) / G : np;   // pairs of this lane group
-            if (POLY) {
 #pragma unroll 1
-                for (; j + PDEN <= npl; j += PDEN) {
+            for (; j + PDEN <= npl; j += PDEN) {
 #pragma unroll
-                    for (int q = 0; q < PDEN; q++) body(j + q, ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN);
-                }
-            } else {
-#pragma unroll 4
-                for (; j + 1 <= npl; j++) body(j, false);
+                for (int q = 0; q < PDEN; q++) body(j + q, ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN);
             }
             for (; j < npl; j++) body(j, false);
         }
@@ -368,18 +391,15 @@ __global__ void __launch_bounds__(NT2, 32) near_kernel_x2(const float *__restric
                                                      const int *__restrict__ ptr, const int *__restrict__ idx,
                                                      const int *__restrict__ off_y, const float *__restrict__ ctr_y,
                                                      const float *__restrict__ packed, float scale, int R, int r0,
-                                                     float *out, float pc0, float pc1, float pc2, float pc3, int row_begin,
-                                                     int row_end) {
+                                                     float *out, ExpCoef pc, int row_begin, int row_end) {
     constexpr int W = row_width(D, RB);
     __shared__ __align__(16) float smem[SP2 * 2 * W];
     int box, t0, t1;
     item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1, MIXED ? NT2 * TI2 : 0);
     if (MIXED && t1 - t0 <= NT2) {
-        near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3,
-                                                 smem, box, t0, t1);
+        near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc, smem, box, t0, t1);
     } else
-        near_tile_x2<D, RB, POLY, PNUM, PDEN, TI2>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3, smem,
-                                                   box, t0, t1);
+        near_tile_x2<D, RB, POLY, PNUM, PDEN, TI2>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc, smem, box, t0, t1);
 }
 
 #include "near_mma.cuh"
@@ -401,14 +421,14 @@ __global__ void __launch_bounds__(256) near_tiles_per_box(int nbx, const int *__
     tiles[b] = t;
 }
 
-// Polynomial of degree deg (<= 3) through the Chebyshev points of [tlo, thi] for 2^t, as monomial coefficients.
+// Polynomial of degree deg (<= 5) through the Chebyshev points of [tlo, thi] for 2^t, as monomial coefficients.
 // Its error is at most h^(deg+1) / (2^deg (deg+1)!) with h = ln2 (thi - tlo) / 2.
-static void exp2_poly_fit(double tlo, double thi, int deg, double (&cf)[4]) {
-    for (int i = 0; i < 4; i++) cf[i] = 0.0;
+static void exp2_poly_fit(double tlo, double thi, int deg, double (&cf)[6]) {
+    for (int i = 0; i < 6; i++) cf[i] = 0.0;
     cf[0] = 1.0;
     if (deg <= 0) return;
     const int m = deg + 1;
-    double tn[4], dd[4];
+    double tn[6], dd[6];
     for (int i = 0; i < m; i++) {
         tn[i] = 0.5 * (thi + tlo) + 0.5 * (thi - tlo) * cos((2 * i + 1) * 3.14159265358979323846 / (2.0 * m));
         dd[i] = exp2(tn[i]);
@@ -508,7 +528,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         const double se = (double)scale * ly.edge;
         const double thi = D * se * se * reach, tlo = -D * se * se * (reach + 0.25);
         const int deg = exp2_poly_degree(0.5 * (thi - tlo));
-        double cf[4];
+        double cf[6];
         exp2_poly_fit(tlo, thi, deg, cf);
         int dev = 0, nsm = 0;
         F3M_CUDA(cudaGetDevice(&dev));
@@ -552,12 +572,15 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     if (expanded) {
         const int poly = exp2_poly_degree(tmax);
         pl->last.direct_variants[poly == 2 ? DV_POLY2 : (poly == 3 ? DV_POLY3 : DV_MUFU)]++;
-        double cf[4];
-        exp2_poly_fit(-tmax, tmax, poly, cf);
+        double cf[6];
+        if (poly) exp2_poly_fit(-tmax, tmax, poly, cf);
+        else exp2_poly_fit(-0.5, 0.5, 5, cf);
+        ExpCoef pc{};
+        for (int k = 0; k < 6; k++) pc.c[k] = (float)cf[k];
 #define F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, MIXED_)                                                                                       \
     near_kernel_x2<D, RB, POLY_, PNUM_, PDEN_, MIXED_><<<items, NT2, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, \
                                                                             csr.idx.p, ly.off.p, ly.ctr.p, packed.p, scale, R, r0, out, \
-                                                                            (float)cf[0], (float)cf[1], (float)cf[2], (float)cf[3], row_begin, row_end)
+                                                                            pc, row_begin, row_end)
 #define F3M_NEAR_EXP(POLY_, PNUM_, PDEN_)                         \
     {                                                             \
         if (small_tiles) F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, true); \
@@ -565,7 +588,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     }
         if (poly == 2) F3M_NEAR_EXP(2, 2, 5)
         else if (poly == 3) F3M_NEAR_EXP(3, 1, 3)
-        else F3M_NEAR_EXP(0, 0, 1)
+        else F3M_NEAR_EXP(5, 1, 4)
 #undef F3M_NEAR_EXP2
 #undef F3M_NEAR_EXP
     }
