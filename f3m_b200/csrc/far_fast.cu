@@ -1341,17 +1341,31 @@ static void ensure_leaf_split(f3m_plan *pl, int which, int level, cudaStream_t s
 // ---------------------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------------------
-// Parts a long box is cut into: at most 8192 points each, and short enough that the parts of all boxes fill the SMs four
-// times over (a cut at level 1 or 2 leaves 8 or 64 boxes), but not below 512 points.
-static int leaf_splits(int max_count, int64_t n) {
-    const int64_t part = std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT)));
-    return (int)std::max<int64_t>(1, std::min<int64_t>(1024, (max_count + part - 1) / part));
+// Parts the boxes of a level are cut into (every box into the same number): `part` points in the longest box.  Levels of
+// uneven occupancy would launch a part for each of a million short boxes because one is long: the number of CTAs is held to the
+// boxes plus four times the parts that an even level would have, but parts never grow beyond what 64 parts of 8192 points give.
+static int box_parts(int max_count, int64_t n, int nb, int64_t part) {
+    const int64_t want = (max_count + part - 1) / part, even = 1 + 4 * n / (part * nb), at_least = std::min(64, (max_count + 8191) / 8192);
+    return (int)std::max<int64_t>(1, std::max<int64_t>(at_least, std::min<int64_t>(want, even)));
 }
+// Target boxes: at most 8192 points, and short enough that the parts of all boxes fill the SMs four times over (a cut at
+// level 1 or 2 leaves 8 or 64 boxes), but not below 512 points.
+static int target_parts(int max_count, int64_t n, int nb) {
+    return box_parts(max_count, n, nb, std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT))));
+}
+// Source boxes: at most 1024 points, so that no running sum is longer than some fifty terms (its rounding grows with the
+// square root); the box level is chosen so that few parts are added up (SRC_LEAF).
+static int source_parts(int max_count, int64_t n, int nb) { return box_parts(max_count, n, nb, 1024); }
+// Sources are interpolated at the first level from L on whose boxes hold at most this many points on average, and moved up by
+// M2M, which adds in a tree: with 375 000 sources per box summed at the cut, 3e6 points and l = 10 were 8.4e-7 from float64,
+// the finest level's 5.6e-7.
+constexpr int64_t SRC_LEAF = 8192;
 
 template <int PP, int RB>
-static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *out, int rb, int re, int lmin, int L, int cut,
+static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *out, int rb, int re, int lmin, int L, int Ls, int cut,
                            cudaStream_t s) {
-    // L: the level whose boxes the points are interpolated to; cut == L: that level takes far, small and kept pairs
+    // L: the last level with pairs, whose local expansions go to the targets; Ls >= L: the level the sources are interpolated
+    // to; cut == L: that level takes far, small and kept pairs
     Tree &tx = pl->tx, &ty = *pl->ty;
     const int d = pl->d;
     int P = 1;
@@ -1363,7 +1377,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     const int n_x = (int)tx.n, n_y = (int)ty.n;
     if (RB == 1 && d == 3) {
         ensure_leaf_split(pl, 0, L, s);
-        if (!pl->same) ensure_leaf_split(pl, 1, L, s);
+        if (!pl->same || Ls != L) ensure_leaf_split(pl, 1, Ls, s);
     }
 
     if (pl->moments_out) {
@@ -1396,11 +1410,13 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         F3M_LAUNCH_CHECK();
         return;
     }
-    std::vector<DevBuf<float>> mom(L + 1), loc(L + 1);
-    std::vector<const float *> momp(L + 1, nullptr);
+    std::vector<DevBuf<float>> mom(Ls + 1), loc(L + 1);
+    std::vector<const float *> momp(Ls + 1, nullptr);
+    for (int l = lmin; l <= Ls; l++) {
+        if (!(l == Ls && pl->ext_mom)) mom[l].alloc((size_t)ty.levels[l].nb * PR, s);
+        momp[l] = (l == Ls && pl->ext_mom) ? pl->ext_mom : mom[l].p;
+    }
     for (int l = lmin; l <= L; l++) {
-        if (!(l == L && pl->ext_mom)) mom[l].alloc((size_t)ty.levels[l].nb * PR, s);
-        momp[l] = (l == L && pl->ext_mom) ? pl->ext_mom : mom[l].p;
         loc[l].alloc((size_t)tx.levels[l].nb * PR, s);
         loc[l].zero();
     }
@@ -1420,33 +1436,33 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         return nw;
     };
 
-    // ---- P2M at the finest level, M2M upwards ---------------------------------------------------
+    // ---- P2M at level Ls, M2M upwards ------------------------------------------------------------
     pl->last.begin(ST_P2M, s);
     {
-        Level &ly = ty.levels[L];
+        Level &ly = ty.levels[Ls];
         const float factor = 2.f / ly.edge;          // 1_d_conv.cu:473
         if (!pl->ext_mom) {
-            const int nsplit = leaf_splits(ly.max_count, ty.n);
-            if (nsplit > 1) mom[L].zero();
+            const int nsplit = source_parts(ly.max_count, ty.n, ly.nb);
+            if (nsplit > 1) mom[Ls].zero();
             size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
             F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             if (RB == 1 && d == 3) {
-                const int wy = pl->same ? 0 : 1;
+                const int wy = pl->same && Ls == L ? 0 : 1;
                 if (pl->n_leaf_big[wy])
                     p2m_leaf3<PP><<<dim3(pl->n_leaf_big[wy], nsplit), 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt,
-                                                                                 nsplit, 0, n_y, mom[L].p, pl->leaf_big[wy].p);
+                                                                                 nsplit, 0, n_y, mom[Ls].p, pl->leaf_big[wy].p);
                 if (pl->n_leaf_small[wy])
                     p2m_small3<PP><<<(pl->n_leaf_small[wy] + 3) / 4, 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, 0,
-                                                                                n_y, mom[L].p, pl->leaf_small[wy].p, pl->n_leaf_small[wy]);
+                                                                                n_y, mom[Ls].p, pl->leaf_small[wy].p, pl->n_leaf_small[wy]);
             } else
             p2m_leaf<PP, RB><<<dim3(ly.nb, nsplit), 256, smem, s>>>(ty.pts.p, n_y, d, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, P,
-                                                                  nsplit, 0, n_y, mom[L].p);
+                                                                  nsplit, 0, n_y, mom[Ls].p);
             F3M_LAUNCH_CHECK();
         }
         const int nw = warps_for(2 * MS * sizeof(float));
         size_t sm2 = (size_t)2 * MS * sizeof(float) + nw * per_warp;
         F3M_CUDA(cudaFuncSetAttribute(m2m_fast<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-        for (int l = L - 1; l >= lmin; l--) {
+        for (int l = Ls - 1; l >= lmin; l--) {
             Level &lp = ty.levels[l], &lc = ty.levels[l + 1];
             m2m_fast<PP><<<lp.nb, 32 * nw, sm2, s>>>(lp.nb, d, lp.child_start.p, lc.code.p, A.p, cfg, momp[l + 1], mom[l].p);
             F3M_LAUNCH_CHECK();
@@ -1560,7 +1576,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         }
         Level &lx = tx.levels[L];
         const float factor = 2.f / lx.edge;
-        const int nsplit = leaf_splits(lx.max_count, tx.n);
+        const int nsplit = target_parts(lx.max_count, tx.n, lx.nb);
         size_t smem = ((size_t)PR + (size_t)std::max(1, d - 1) * PP * 128) * sizeof(float);
         F3M_CUDA(cudaFuncSetAttribute(l2p_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (RB == 1 && d == 3) {
@@ -1579,14 +1595,14 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
 }
 
 template <int PP>
-static void far_fast_p(f3m_plan *pl, const float *bs, int R, float *out, int rb, int re, int lmin, int L, int cut, cudaStream_t s) {
+static void far_fast_p(f3m_plan *pl, const float *bs, int R, float *out, int rb, int re, int lmin, int L, int Ls, int cut, cudaStream_t s) {
     int P = 1;
     for (int k = 0; k < pl->d; k++) P *= PP;
     // 8 columns at a time when the three per-warp buffers of the translation kernels fit, else one
     const bool wide = R > 1 && (size_t)3 * P * 8 * sizeof(float) + (size_t)pl->d * NOFF2 * mat_stride(PP) * sizeof(float) <= 200 * 1024;
     for (int r0 = 0; r0 < R;) {
-        if (wide) { far_fast_block<PP, 8>(pl, bs, R, r0, out, rb, re, lmin, L, cut, s); r0 += 8; }
-        else { far_fast_block<PP, 1>(pl, bs, R, r0, out, rb, re, lmin, L, cut, s); r0 += 1; }
+        if (wide) { far_fast_block<PP, 8>(pl, bs, R, r0, out, rb, re, lmin, L, Ls, cut, s); r0 += 8; }
+        else { far_fast_block<PP, 1>(pl, bs, R, r0, out, rb, re, lmin, L, Ls, cut, s); r0 += 1; }
     }
 }
 
@@ -1712,14 +1728,16 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
     // moments are cut at boxes of the last level, so they stay there.
     const bool whole = rb <= 0 && re >= (int)pl->tx.n && !pl->moments_out && !pl->ext_mom && !pl->shard.active;
     const int last = whole ? llast : pl->levels;
+    int src = last;
+    while (whole && src < pl->levels && pl->ty->n / pl->ty->levels[src].nb > SRC_LEAF) src++;
     switch (p) {
-        case 2: far_fast_p<2>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        case 3: far_fast_p<3>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        case 4: far_fast_p<4>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        case 5: far_fast_p<5>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        case 6: far_fast_p<6>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        case 7: far_fast_p<7>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
-        default: far_fast_p<8>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, cut, s); break;
+        case 2: far_fast_p<2>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        case 3: far_fast_p<3>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        case 4: far_fast_p<4>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        case 5: far_fast_p<5>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        case 6: far_fast_p<6>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        case 7: far_fast_p<7>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
+        default: far_fast_p<8>(pl, b_sorted, R, out_sorted, rb, re, lmin, last, src, cut, s); break;
     }
 }
 
