@@ -348,8 +348,6 @@ void shard_rows_to_input_order(const f3m_plan *pl, const float *acc_sorted, int 
 // ---- near.cu ---------------------------------------------------------------------------------
 void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted,
                  int64_t row_begin, int64_t row_end, cudaStream_t s);
-// upper bound of |x_k - c_k| / edge over the pairs of a direct list (x a target, c the centre of its source box)
-double list_reach(const f3m_plan *pl, int level, const PairCSR &csr);
 // near_cols.cu: up to eight columns of a direct list, starting at r0
 void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, const float *b_sorted, int R, int r0, float *out_sorted,
                  int row_begin, int row_end, cudaStream_t s);

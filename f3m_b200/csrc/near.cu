@@ -457,7 +457,7 @@ static inline float near_scale(float lcs) { return sqrtf(lcs * 1.442695040888963
 // any distance test, and the two cubes have separate origins (n_tree.cu:1096-1098): "small" pairs there are
 // classified by size before distance (1_d_conv.cu:916-920), so their distance is bounded only by the offset
 // between the two cubes.
-double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
+static double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
     const bool final_near = (&csr == &pl->lists[level].keep);
     if (final_near) return 2.5;
     if (level == 1 && !pl->same) {
@@ -605,9 +605,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 template <int D>
 static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out, int rb, int re,
                      cudaStream_t s) {
-    // expanded form? (the conditions of direct_impl)
-    const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
-    const bool expanded = level > 0 && se <= 1.0 && D * list_reach(pl, level, csr) * se * se <= TMAX_EXPANDED;
+    const bool expanded = level > 0 && near_scale(pl->lcs) * pl->tx.levels[level].edge <= 1.0f;   // near_cols.cu
     for (int r0 = 0; r0 < R;) {
         if (R - r0 >= 2) { column_sums(pl, level, csr, expanded, bs, R, r0, out, rb, re, s); r0 += 8; }
         else { direct_impl<D, 1>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 1; }

@@ -57,45 +57,13 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const float (&a)[4], flo
           "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
 
-// Packed sources: groups of eight, [coordinate k][t][sources t, t+4], then B in fragment order [lane][rows t, t+4 of column g].
-__host__ __device__ constexpr int col_group_floats(int D) { return 8 * D + 8 * CR; }
-// first group of a box: boxes are padded to whole groups (ceil(len / 8) never exceeds the distance to the next box's start)
-__host__ __device__ __forceinline__ int64_t col_group_start(int off, int box) { return ((int64_t)off + 7 * (int64_t)box + 7) >> 3; }
-
-// one warp per source box and part
-template <int D, bool DIFF>
-__global__ void __launch_bounds__(256) pack_columns(const float *__restrict__ pts, int n, const float *__restrict__ bs, int R, int r0,
-                                                   float scale, const int *__restrict__ off_y, int nby, const float *__restrict__ ctr_y,
-                                                   const unsigned char *__restrict__ need, int nsplit, float *packed) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int by = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (by >= nby || (need && !need[by])) return;
-    const int s0 = off_y[by], len = off_y[by + 1] - s0, ngr = (len + 7) >> 3;
-    float c[D];
-#pragma unroll
-    for (int k = 0; k < D; k++) c[k] = ctr_y[by * D + k];
-    for (int gr = blockIdx.y; gr < ngr; gr += nsplit) {
-        float *dst = packed + (size_t)(col_group_start(s0, by) + gr) * col_group_floats(D);
-        float b2[2], y2[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int j = gr * 8 + t + 4 * h;
-            b2[h] = y2[h] = 0.f;   // the sources that fill the last group weigh nothing
-            if (j < len) {
-                float n2 = 0.f;
-#pragma unroll
-                for (int k = 0; k < D; k++) {
-                    const float v = scale * (pts[(size_t)k * n + s0 + j] - c[k]);
-                    n2 = fmaf(v, v, n2);
-                    if (k == g) y2[h] = DIFF ? -v : 2.f * v;
-                }
-                if (r0 + g < R) b2[h] = bs[(size_t)(s0 + j) * R + r0 + g] * (DIFF ? 1.f : c_ex2(-n2));
-            }
-        }
-        if (g < D) *reinterpret_cast<float2 *>(dst + g * 8 + t * 2) = make_float2(y2[0], y2[1]);
-        *reinterpret_cast<float2 *>(dst + 8 * D + lane * 2) = make_float2(b2[0], b2[1]);
-    }
-}
+// Group of eight sources in shared memory: [row k][t][sources t, t+4] for the D coordinates and, in the expanded form, minus the
+// squared length; then B in fragment order [lane][rows t, t+4 of column g].
+template <int D, bool DIFF> struct ColGroup {
+    static constexpr int ROWS = DIFF ? D : D + 1;
+    static constexpr int FLOATS = 8 * ROWS + 8 * CR;
+};
+constexpr int CST = 64;      // sources staged per warp: two chunks of 32, so that a full chunk always fits behind a remainder
 
 // tiles[b] = tiles of the rows of target box b inside [row_begin, row_end)
 __global__ void __launch_bounds__(256) col_tiles_per_box(int nbx, const int *__restrict__ off_x, const int *__restrict__ ptr, int row_begin,
@@ -107,63 +75,114 @@ __global__ void __launch_bounds__(256) col_tiles_per_box(int nbx, const int *__r
     tiles[b] = t;
 }
 
-// xs: the tile's coordinates in shared memory, [row block m][k][g] = targets (16 m + g, 16 m + g + 8)
+// The sources of a tile's list arrive as ONE stream, box borders left out: 32 list entries at a time (lane = entry) are prefix-summed,
+// and a lane finds the source of its stream position by bisection.  All coordinates are relative to the centre c of the TARGET box,
+// which keeps them for the whole list: with X = s (x-c), Y = s (y-c) the exponent -|X-Y|^2 is, in the expanded form,
+// (2 X.Y - |Y|^2) - |X|^2, whose last part leaves the sum; |X|^2 is at most d/4 there (boxes up to one scaled unit), so the
+// terms of the bracket cancel by no more than that and no factor overflows.  Wide boxes take the differences.
+// Against packed rows per source box this drops the groups' padding at every box border, the target coordinates per
+// source box and the packing pass: boxes of a few points were two thirds overhead.
 template <int D, bool DIFF, int MT>
-__device__ __forceinline__ void column_tile(const float2 *xs, const int *__restrict__ idx, int e0, int e1, const int *__restrict__ off_y,
-                                            const float *__restrict__ ctr_y, const float *__restrict__ packed, float scale, int R, int r0,
+__device__ __forceinline__ void column_tile(const float2 *xs, float *stage, int *entries, const int *__restrict__ idx, int e0, int e1,
+                                            const int *__restrict__ off_y, const float *__restrict__ ypts, int n_y,
+                                            const float *__restrict__ bs, const float (&c)[D], float scale, int R, int r0, bool vec,
                                             float *out, int t0, int nt) {
-    constexpr int GF = col_group_floats(D);
+    using G = ColGroup<D, DIFF>;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const f32x2 minus1 = c_pack(-1.f, -1.f), scale2 = c_pack(scale, scale);
-    f32x2 tot[MT][2];
+    const f32x2 minus1 = c_pack(-1.f, -1.f);
+    f32x2 xr[MT][D], tot[MT][2], acc[MT][2];
 #pragma unroll
-    for (int m = 0; m < MT; m++) tot[m][0] = tot[m][1] = c_pack(0.f, 0.f);
-    int by = idx[e0], s0 = off_y[by], ngr = (off_y[by + 1] - s0 + 7) >> 3;
-    const float *p = packed + (size_t)col_group_start(s0, by) * GF;
-    float2 ny[D], nb;   // the group after the current one, on its way from L2
-    auto fetch = [&](const float *q) {
+    for (int m = 0; m < MT; m++) {
 #pragma unroll
-        for (int k = 0; k < D; k++) ny[k] = __ldg(reinterpret_cast<const float2 *>(q + k * 8 + t * 2));
-        nb = __ldg(reinterpret_cast<const float2 *>(q + 8 * D + lane * 2));
-    };
-    fetch(p);
-    for (int e = e0; e < e1; e++) {
-        float c[D];
+        for (int k = 0; k < D; k++) {
+            const float2 x = xs[(m * D + k) * 8 + g];
+            xr[m][k] = DIFF ? c_pack(x.x, x.y) : c_pack(2.f * x.x, 2.f * x.y);
+        }
+        tot[m][0] = tot[m][1] = acc[m][0] = acc[m][1] = c_pack(0.f, 0.f);
+    }
+    int e = e0, total = 0, pos = 0;   // entries not loaded yet, stream positions loaded and used
+    int fill = 0, since = 0;          // staged sources, groups since the last flush of acc
+    while (true) {
+        // stage up to 32 more sources
+        if (pos == total && e < e1) {
+            int len = 0, s0 = 0;
+            if (e + lane < e1) {
+                const int by = idx[e + lane];
+                s0 = off_y[by];
+                len = off_y[by + 1] - s0;
+            }
+            int inc = len;
 #pragma unroll
-        for (int k = 0; k < D; k++) c[k] = __ldg(ctr_y + by * D + k);
-        const int by_n = e + 1 < e1 ? idx[e + 1] : by;
-        const int s0_n = off_y[by_n], ngr_n = (off_y[by_n + 1] - s0_n + 7) >> 3;
-        const float *p_n = packed + (size_t)col_group_start(s0_n, by_n) * GF;
-        f32x2 xr[MT][D], acc[MT][2];
-        float fx[MT][2];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            total = __shfl_sync(0xffffffffu, inc, 31);
+            __syncwarp();
+            entries[lane] = inc - len;               // first stream position of the entry
+            entries[32 + lane] = s0 - (inc - len);   // sorted row of stream position p: p + this
+            __syncwarp();
+            pos = 0;
+            e = min(e + 32, e1);
+        }
+        const int take = min(32, total - pos);
+        if (lane < take) {
+            const int p = pos + lane;
+            int lo = 0;
 #pragma unroll
-        for (int m = 0; m < MT; m++) {
-            f32x2 n2 = c_pack(0.f, 0.f);
+            for (int step = 16; step > 0; step >>= 1)
+                if (entries[lo + step] <= p) lo += step;
+            const int j = p + entries[32 + lo];
+            const int q = fill + lane;
+            float *dst = stage + (q >> 3) * G::FLOATS + 2 * (q & 3) + ((q >> 2) & 1);
+            float n2 = 0.f;
 #pragma unroll
             for (int k = 0; k < D; k++) {
-                const float2 x = xs[(m * D + k) * 8 + g];
-                xr[m][k] = c_mul(scale2, c_add(c_pack(x.x, x.y), c_pack(-c[k], -c[k])));
-                if (!DIFF) n2 = c_fma(xr[m][k], xr[m][k], n2);
+                const float v = scale * (ypts[(size_t)k * n_y + j] - c[k]);
+                n2 = fmaf(-v, v, n2);
+                dst[8 * k] = DIFF ? -v : v;
             }
-            if (!DIFF) {
-                float a, b;
-                c_unpack(n2, a, b);
-                fx[m][0] = c_ex2(-a);
-                fx[m][1] = c_ex2(-b);
-            } else
-                fx[m][0] = fx[m][1] = 1.f;
-            acc[m][0] = acc[m][1] = c_pack(0.f, 0.f);
+            if (!DIFF) dst[8 * D] = n2;
+            const float *b = bs + (size_t)j * R + r0;
+            float v[CR];
+            if (vec) {
+                const float4 lo4 = __ldg(reinterpret_cast<const float4 *>(b)), hi4 = __ldg(reinterpret_cast<const float4 *>(b) + 1);
+                v[0] = lo4.x; v[1] = lo4.y; v[2] = lo4.z; v[3] = lo4.w; v[4] = hi4.x; v[5] = hi4.y; v[6] = hi4.z; v[7] = hi4.w;
+            } else {
+#pragma unroll
+                for (int r = 0; r < CR; r++) v[r] = r0 + r < R ? __ldg(b + r) : 0.f;
+            }
+#pragma unroll
+            for (int r = 0; r < CR; r++) dst[8 * G::ROWS + 8 * r] = v[r];
         }
+        pos += take;
+        fill += take;
+        const bool last = pos == total && e >= e1;
+        if (fill < 32 && !last) continue;
+        // the sources that fill the last group weigh nothing
+        int ngr = fill >> 3;
+        if (last && (fill & 7)) {
+            const int q = fill + lane;
+            if (q < 8 * (ngr + 1)) {
+                float *dst = stage + (q >> 3) * G::FLOATS + 2 * (q & 3) + ((q >> 2) & 1);
+#pragma unroll
+                for (int k = 0; k < G::ROWS + CR; k++) dst[8 * k] = 0.f;
+            }
+            ngr++;
+        }
+        __syncwarp();
 #pragma unroll 1
         for (int gr = 0; gr < ngr; gr++) {
-            f32x2 y[2][D];
+            const float *p = stage + gr * G::FLOATS;
+            f32x2 y[2][G::ROWS];
 #pragma unroll
-            for (int k = 0; k < D; k++) {
-                y[0][k] = c_pack(ny[k].x, ny[k].x);
-                y[1][k] = c_pack(ny[k].y, ny[k].y);
+            for (int k = 0; k < G::ROWS; k++) {
+                const float2 v = *reinterpret_cast<const float2 *>(p + 8 * k + 2 * t);
+                y[0][k] = c_pack(v.x, v.x);
+                y[1][k] = c_pack(v.y, v.y);
             }
+            const float2 nb = *reinterpret_cast<const float2 *>(p + 8 * G::ROWS + 2 * lane);
             const float bh0 = tf32_head(nb.x), bh1 = tf32_head(nb.y), bl0 = tf32_head(nb.x - bh0), bl1 = tf32_head(nb.y - bh1);
-            fetch(gr + 1 < ngr ? p + (size_t)(gr + 1) * GF : p_n);
 #pragma unroll
             for (int m = 0; m < MT; m++) {
                 float hi[4], lo[4];
@@ -179,7 +198,7 @@ __device__ __forceinline__ void column_tile(const float2 *xs, const int *__restr
                             v = c_fma(df, df, v);
                         }
                     } else {
-                        v = c_mul(xr[m][0], y[h][0]);
+                        v = c_fma(xr[m][0], y[h][0], y[h][G::ROWS - 1]);
 #pragma unroll
                         for (int k = 1; k < D; k++) v = c_fma(xr[m][k], y[h][k], v);
                     }
@@ -198,16 +217,38 @@ __device__ __forceinline__ void column_tile(const float2 *xs, const int *__restr
                 acc[m][1] = c_add(acc[m][1], c_pack(d[2], d[3]));
             }
         }
+        since += ngr;
+        if (since >= 16 || last) {   // blocked accumulation: partial sums of some 128 to 160 sources
 #pragma unroll
-        for (int m = 0; m < MT; m++)
+            for (int m = 0; m < MT; m++)
 #pragma unroll
-            for (int h = 0; h < 2; h++) tot[m][h] = c_fma(c_pack(fx[m][h], fx[m][h]), acc[m][h], tot[m][h]);
-        by = by_n;
-        ngr = ngr_n;
-        p = p_n;
+                for (int h = 0; h < 2; h++) {
+                    tot[m][h] = c_add(tot[m][h], acc[m][h]);
+                    acc[m][h] = c_pack(0.f, 0.f);
+                }
+            since = 0;
+        }
+        if (last) break;
+        __syncwarp();
+        // the remainder of less than a group moves to the front
+        const int rest = fill & 7;
+        if (rest) {
+            for (int q = lane; q < G::FLOATS; q += 32) stage[q] = stage[(fill >> 3) * G::FLOATS + q];
+            __syncwarp();
+        }
+        fill = rest;
     }
 #pragma unroll
-    for (int m = 0; m < MT; m++)
+    for (int m = 0; m < MT; m++) {
+        float f[2] = {1.f, 1.f};
+        if (!DIFF) {   // 2^(-|X|^2) of the thread's two targets; xr holds 2 X
+            f32x2 n2 = c_pack(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < D; k++) n2 = c_fma(xr[m][k], xr[m][k], n2);
+            c_unpack(n2, f[0], f[1]);
+            f[0] = c_ex2(-0.25f * f[0]);
+            f[1] = c_ex2(-0.25f * f[1]);
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int i = 16 * m + g + 8 * h, r = r0 + 2 * t;
@@ -215,18 +256,22 @@ __device__ __forceinline__ void column_tile(const float2 *xs, const int *__restr
             float a, b;
             c_unpack(tot[m][h], a, b);
             float *o = out + (size_t)(t0 + i) * R + r;
-            if (r < R) o[0] += a;
-            if (r + 1 < R) o[1] += b;
+            if (r < R) o[0] += f[h] * a;
+            if (r + 1 < R) o[1] += f[h] * b;
         }
+    }
 }
 
 template <int D, bool DIFF>
 __global__ void __launch_bounds__(32 * CW, 4) near_columns(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x, int nbx,
-                                                          const int *__restrict__ tile_off, const int *__restrict__ ptr,
-                                                          const int *__restrict__ idx, const int *__restrict__ off_y,
-                                                          const float *__restrict__ ctr_y, const float *__restrict__ packed, float scale,
-                                                          int R, int r0, float *out, int row_begin, int row_end) {
+                                                          const float *__restrict__ ctr_x, const int *__restrict__ tile_off,
+                                                          const int *__restrict__ ptr, const int *__restrict__ idx,
+                                                          const int *__restrict__ off_y, const float *__restrict__ ypts, int n_y,
+                                                          const float *__restrict__ bs, float scale, int R, int r0, bool vec, float *out,
+                                                          int row_begin, int row_end) {
     __shared__ float2 xs_all[CW][4 * D * 8];
+    __shared__ __align__(16) float stage_all[CW][CST / 8 * ColGroup<D, DIFF>::FLOATS];
+    __shared__ int entries_all[CW][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * CW + warp;
     if (item >= tile_off[nbx]) return;      // the grid is sized by a bound on the tiles, no read-back
@@ -236,19 +281,28 @@ __global__ void __launch_bounds__(32 * CW, 4) near_columns(const float *__restri
     const int tile = item - tile_off[box], ntiles = tile_off[box + 1] - tile_off[box], units = (len + 15) >> 4;
     const int t0 = a + 16 * (int)(((long long)units * tile) / ntiles);
     const int nt = min(a + 16 * (int)(((long long)units * (tile + 1)) / ntiles), a + len) - t0;
+    float c[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) c[k] = ctr_x[box * D + k];
+    // scaled coordinates of the tile's targets, [row block m][k][g] = targets (16 m + g, 16 m + g + 8)
     float2 *xs = xs_all[warp];
     const int mt = (nt + 15) >> 4;
     for (int q = lane; q < mt * 8 * D; q += 32) {
         const int gg = q & 7, k = (q >> 3) % D, m = (q >> 3) / D;
-        const int i0 = 16 * m + gg, i1 = i0 + 8;
-        xs[q] = make_float2(xpts[(size_t)k * n_x + t0 + min(i0, nt - 1)], xpts[(size_t)k * n_x + t0 + min(i1, nt - 1)]);
+        const int i0 = min(16 * m + gg, nt - 1), i1 = min(16 * m + gg + 8, nt - 1);
+        const float ck = ctr_x[box * D + k];
+        xs[q] = make_float2(scale * (xpts[(size_t)k * n_x + t0 + i0] - ck), scale * (xpts[(size_t)k * n_x + t0 + i1] - ck));
     }
     __syncwarp();
     const int e0 = ptr[box], e1 = ptr[box + 1];
-    if (mt == 4) column_tile<D, DIFF, 4>(xs, idx, e0, e1, off_y, ctr_y, packed, scale, R, r0, out, t0, nt);
-    else if (mt == 3) column_tile<D, DIFF, 3>(xs, idx, e0, e1, off_y, ctr_y, packed, scale, R, r0, out, t0, nt);
-    else if (mt == 2) column_tile<D, DIFF, 2>(xs, idx, e0, e1, off_y, ctr_y, packed, scale, R, r0, out, t0, nt);
-    else column_tile<D, DIFF, 1>(xs, idx, e0, e1, off_y, ctr_y, packed, scale, R, r0, out, t0, nt);
+    float *st = stage_all[warp];
+    int *en = entries_all[warp];
+#define F3M_TILE(MT_) column_tile<D, DIFF, MT_>(xs, st, en, idx, e0, e1, off_y, ypts, n_y, bs, c, scale, R, r0, vec, out, t0, nt)
+    if (mt == 4) F3M_TILE(4);
+    else if (mt == 3) F3M_TILE(3);
+    else if (mt == 2) F3M_TILE(2);
+    else F3M_TILE(1);
+#undef F3M_TILE
 }
 
 template <int D, bool DIFF>
@@ -262,30 +316,19 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
     col_tiles_per_box<<<(unsigned)((lx.nb + 1 + 255) / 256), 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, row_begin, row_end, tiles.p);
     F3M_LAUNCH_CHECK();
     exclusive_scan_i32(tiles.p, tiles.p, (int64_t)lx.nb + 1, s);
-    // packed sources are kept for the "small" and the near list of one level
-    f3m_plan::PackCache &pc = pl->pack_cache;
-    if (!(pc.level == level && pc.r0 == r0 && pc.rb == CR && pc.expanded == !DIFF)) {
-        pc.buf.alloc((size_t)(col_group_start((int)ty.n, ly.nb) + 1) * col_group_floats(D), s);
-        pc.level = level; pc.r0 = r0; pc.rb = CR; pc.expanded = !DIFF;
-        pl->last.begin(ST_PERMUTE, s);
-        const unsigned char *need = level_source_flags(pl, level, s);
-        const int nsplit = std::max(1, std::min(1024, (ly.max_count + 511) / 512));
-        pack_columns<D, DIFF><<<dim3((unsigned)(((int64_t)ly.nb * 32 + 255) / 256), nsplit), 256, 0, s>>>(
-            ty.pts.p, (int)ty.n, bs, R, r0, scale, ly.off.p, ly.nb, ly.ctr.p, need, nsplit, pc.buf.p);
-        pl->last.end(s);
-        F3M_LAUNCH_CHECK();
-    }
     const int64_t max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1;
+    const bool vec = R % 4 == 0 && r0 + CR <= R;   // rows of b as two 16-byte loads (bs starts on a 256-byte boundary)
     pl->last.begin(ST_DIRECT, s);
     near_columns<D, DIFF><<<(unsigned)((max_items + CW - 1) / CW), 32 * CW, 0, s>>>(
-        tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, csr.idx.p, ly.off.p, ly.ctr.p, pc.buf.p, scale, R, r0, out, row_begin, row_end);
+        tx.pts.p, (int)tx.n, lx.off.p, lx.nb, lx.ctr.p, tiles.p, csr.ptr.p, csr.idx.p, ly.off.p, ty.pts.p, (int)ty.n, bs, scale, R, r0, vec, out,
+        row_begin, row_end);
     pl->last.end(s);
     pl->last.direct_launches++;
     pl->last.direct_variants[DIFF ? DV_DIRECT : DV_MUFU]++;
     F3M_LAUNCH_CHECK();
 }
 
-// up to eight columns starting at r0; expanded: the exponent bound of the list allows the expanded form
+// up to eight columns starting at r0; expanded: boxes at most one scaled unit wide
 void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, const float *bs, int R, int r0, float *out, int row_begin, int row_end,
                  cudaStream_t s) {
     if (row_end <= row_begin) return;
