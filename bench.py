@@ -347,48 +347,41 @@ def main():
         variants = plan.direct_variants()
         peaks = engine.measure_peaks(dev)
         flop_per_pair = 3 * d + 2 * R                      # 3d + 2R
-        # The direct-sum kernel (near_kernel_x2) spends per pair d multiply-adds on the inner product, R on the
-        # accumulation and either one exponential (MUFU) or a degree-DEG polynomial (DEG multiply-adds) -- the share of
-        # polynomial pairs and the degree follow the rule in near.cu (direct_impl): same bound on the exponent here.
+        # Where lists are summed pair by pair the direct-sum kernel (near_kernel_x2) spends per pair d multiply-adds on the inner
+        # product, R on the accumulation and one exponential, a quarter of them as degree-5 polynomials on the FMA pipe.  A
+        # product that ends at a level whose interpolation is exact, or whose lists go through box moments, visits no pairs:
+        # its longest stage is the tree (sort), bound by memory.
         Lv = st["levels"]
-        edge = plan.level(Lv)["edge"] if Lv else 0.0
-        se = math.sqrt(math.log2(math.e) / (2.0 * a.ls * a.ls)) * edge
-        h = d * 2.5 * se * se * math.log(2.0)
-        deg, share = (2, 2 / 5) if h ** 3 / 24 <= 3e-7 else ((3, 1 / 3) if h ** 4 / 192 <= 3e-7 else (0, 0.0))
-        fma_per_pair = d + R + share * deg
-        exp_per_pair = 1.0 - share
+        pairs_summed = direct_ms > 0 and variants["moments"] == 0
+        fma_per_pair, exp_per_pair = d + R + 0.25 * 8, 0.75
         peak_pairs = min(peaks["gfma_per_s"] / fma_per_pair, peaks["gexp_per_s"] / exp_per_pair) * 1e9
-        achieved_pairs = st["direct_pairs"] / (direct_ms * 1e-3)
-        sm_mhz = (clocks or {}).get("sm_mhz") or 1965.0
-        sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        roof = {"bound": "fp32-fma+sfu", "bound_note": "not hbm, not tensor in the default path: inner product + exponential per pair; a source row is reused by every target of a tile",
-                "achieved": achieved_pairs * flop_per_pair / 1e12, "peak": peak_pairs * flop_per_pair / 1e12,
-                "unit": "TFLOP/s", "frac": achieved_pairs / peak_pairs,
-                "kernel": f"near_kernel_x2<{d},{R if R == 1 else 8},{deg},..> (all direct-sum launches of one product; packed f32x2 arithmetic over source pairs; "
-                          f"{share:.2f} of the pairs evaluate 2^t by a degree-{deg} polynomial on the FMA pipe)",
-                "pairs": st["direct_pairs"], "ms": direct_ms, "launches": tm["direct_launches"], "kernel_forms": variants,
-                "peak_source": f"measured in this run by register-only probes: {peaks['gexp_per_s']:.0f} Gexp/s, "
-                               f"{peaks['gfma_per_s']:.0f} Gfma/s; peak = min(fma/{fma_per_pair:.2f}, exp/{exp_per_pair:.2f}) pairs/s x {flop_per_pair} flop",
-                # the probe reads a little under lanes x SMs x clock; with that number as the FMA peak the fraction is:
-                "fma_peak_theoretical_gfma": 128 * sms * sm_mhz * 1e-3,
-                "frac_vs_theoretical_fma": achieved_pairs / (min(128 * sms * sm_mhz * 1e-3 / fma_per_pair,
-                                                                  peaks["gexp_per_s"] / exp_per_pair) * 1e9)}
-        if a.workload == "c2":
-            # DRAM bytes per launch from an ncu capture of this kernel at N=1e7 (profiles/near_kernel_x2_c2_1e7.md), scaled by
-            # N: the traffic is per point (packed sources, targets, output)
-            roof["traffic"] = 37.7 * N
-            roof["traffic_note"] = "37.7 B/point from the ncu capture at N=1e7, scaled to N; algorithmic minimum 36 B/point"
-        else:
-            roof["traffic"] = None
-        line["roofline"] = roof
-        line["stages_ms"] = {k: round(v, 3) for k, v in tm.items() if k != "direct_launches"}
-        # ---- per-stage rooflines from the algorithmic work (bytes against the measured copy bandwidth, multiply-adds
-        # against the FMA peak measured above); the slower of the two is the stage's bound ------------------------------
+        achieved_pairs = st["direct_pairs"] / (direct_ms * 1e-3) if pairs_summed else None
         try:
             with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as fh:
                 hbm_gbs, hbm_src = float(json.load(fh)["hbm_gbs"]), "of measured"
         except Exception:
             hbm_gbs, hbm_src = 6650.0, "of fallback"
+        if pairs_summed:
+            roof = {"bound": "fp32-fma+sfu", "bound_note": "inner product + exponential per pair; a source row is reused by every target of a tile",
+                    "achieved": achieved_pairs * flop_per_pair / 1e12, "peak": peak_pairs * flop_per_pair / 1e12,
+                    "unit": "TFLOP/s", "frac": achieved_pairs / peak_pairs,
+                    "kernel": f"direct sums ({'near_kernel_x2' if R == 1 else 'near_columns'}, all launches of one product)",
+                    "pairs": st["direct_pairs"], "ms": direct_ms, "launches": tm["direct_launches"], "kernel_forms": variants,
+                    "peak_source": f"measured in this run by register-only probes: {peaks['gexp_per_s']:.0f} Gexp/s, "
+                                   f"{peaks['gfma_per_s']:.0f} Gfma/s; peak = min(fma/{fma_per_pair:.2f}, exp/{exp_per_pair:.2f}) pairs/s x {flop_per_pair} flop",
+                    "traffic": None}
+        else:
+            build_ms = statistics.median(t["build"] for t in tms)
+            tree_bytes = N * (2 * 4 * d + 2 * 4 * R + 8)
+            roof = {"bound": "hbm", "bound_note": "no pair is summed one by one (direct lists: none, or through box moments); the tree build is the longest stage",
+                    "achieved": tree_bytes / (build_ms * 1e-3) / 1e9, "peak": hbm_gbs, "unit": "GB/s",
+                    "frac": tree_bytes / (build_ms * 1e-3) / 1e9 / hbm_gbs,
+                    "kernel": "tree build (rs_scatter, morton_hist_kernel, heads_*, lists_kernel, unpack_records)", "ms": build_ms,
+                    "kernel_forms": variants, "peak_source": hbm_src, "traffic": None}
+        line["roofline"] = roof
+        line["stages_ms"] = {k: round(v, 3) for k, v in tm.items() if k != "direct_launches"}
+        # ---- per-stage rooflines from the algorithmic work (bytes against the measured copy bandwidth, multiply-adds
+        # against the FMA peak measured above); the slower of the two is the stage's bound ------------------------------
         if Lv:
             nb_leaf = plan.level(Lv)["boxes_x"]
             pd = plan.level(Lv)["nodes_per_dim"]
@@ -405,8 +398,9 @@ def main():
                 "p2m": stage_roof(tm["p2m"], N * (4 * d + 4 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
                 "m2l": stage_roof(tm["m2l"], 2 * nb_leaf * Pn * R * 4, st["far_box_pairs"] * d * pd * Pn * R),
                 "l2p": stage_roof(tm["l2p"], N * (4 * d + 8 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
-                "direct": {"ms": round(direct_ms, 3), "frac": round(achieved_pairs / peak_pairs, 3)},
-                "note": "m2l multiply-adds counted in the per-pair form (d axis transforms per far pair); the nested kernel does fewer"}
+                "direct": {"ms": round(direct_ms, 3), "frac": round(achieved_pairs / peak_pairs, 3) if pairs_summed else None},
+                "note": "m2l multiply-adds counted in the per-pair form (d axis transforms per far pair of all levels); the nested kernel does "
+                        "fewer, and a product that ends above the last level visits only the lists down to there"}
         line["work"] = {"levels": st["levels"], "direct_pairs": st["direct_pairs"], "far_box_pairs": st["far_box_pairs"],
                         "node_pairs_reference_form": st["node_pairs"]}
         rows = torch.randperm(N, device=dev, generator=g)[:a.check_rows]
@@ -431,10 +425,9 @@ def main():
                 return {"ms_per_step": ms_m, "value": float(N) * float(N) * R / (ms_m * 1e-3), "unit": UNIT,
                         "rel_l2_vs_f64": float((out_m[rows].double() - exact).norm() / exact.norm())}
             # ---- the same product with the optional forms of the near field (not the headline: `value` above is the
-            # default path, whose near field is the direct sum on the CUDA cores) ----------------------------------------
+            # default path) ---------------------------------------------------------------------------------------------
             line["near_moments_mode"] = dict(mode_run(f3m_lib.FLAG_NEAR_MOMENTS),
-                                             note="F3M_FLAG_NEAR_MOMENTS: near sums from 2nd/3rd-order box moments where the exponent "
-                                                  "is provably tiny; same pair lists; optional, off by default")
+                                             note="F3M_FLAG_NEAR_MOMENTS: all levels, near sums from box moments to 1e-6; optional, off by default")
             line["near_tensor_cores_mode"] = dict(mode_run(f3m_lib.FLAG_NEAR_TENSOR_CORES),
                                                   note="F3M_FLAG_NEAR_TENSOR_CORES: exponent tiles as TF32 tcgen05 products of split operands "
                                                        "(TMEM accumulators, bulk copies, mbarrier pipeline); optional, off by default")
