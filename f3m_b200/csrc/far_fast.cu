@@ -1668,7 +1668,7 @@ static bool cut_is_exact(const f3m_plan *pl, int level, int p) {
 // direct_list_seconds; a cut orders a list of its own and sets up the level (20 us), which small trees do not win back.
 int far_cut_level(const f3m_plan *pl, int R) {
     const int L = pl->levels;
-    if (L < 1 || (pl->prm.flags & (F3M_FLAG_NEAR_TENSOR_CORES | F3M_FLAG_NEAR_MOMENTS)) || pl->prm.var_compression) return 0;
+    if (L < 1 || (pl->prm.flags & F3M_FLAG_NEAR_TENSOR_CORES) || pl->prm.var_compression) return 0;
     const int p = pl->lists[1].p, d = pl->d;
     if (p < 2 || p > PMAX_FAST || d < 2) return 0;
     int P = 1;
