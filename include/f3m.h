@@ -53,7 +53,7 @@ enum f3m_status {
  * lengthscale) and its source boxes hold enough points, the sum over a source box is taken from its moments of degree
  * 2..6 instead of pair by pair: the same sums, with a polynomial for part of the exponential whose relative error is below
  * 1.2e-7 (ex2.approx: 2.4e-7).  The pair lists do not change (near_field_run, F3M_src/n_tree.cu:831-902).  This flag
- * relaxes the bound to 1e-6 and takes moments also where the pair form would be as fast. */
+ * relaxes that bound to 1e-6 and takes moments also where the pair form would be as fast. */
 #define F3M_FLAG_NEAR_MOMENTS 1
 
 /* Optional evaluation of the direct near sums on the tensor cores (one column, boxes at most half a scaled
@@ -124,7 +124,8 @@ int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, 
  * near_field_run n_tree.cu:831-902).  b (M,R), out (N,R) overwritten.
  * row_begin/row_end restrict the product to the target boxes whose sorted point range starts
  * inside [row_begin,row_end) (a slice of the sorted target order, used to shard target boxes
- * over GPUs); rows outside the slice are written as 0.  Use 0, N for the whole product. */
+ * over GPUs); rows outside the slice are written as 0.  Use 0, N for the whole product, which may end at the level whose
+ * interpolation is exact for every pair (relative bound 1.2e-7); slices visit all levels. */
 int f3m_plan_apply(f3m_plan *plan, const float *b, int32_t R, float *out, void *stream);
 int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, int64_t row_begin,
                          int64_t row_end, void *stream);
