@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(NT) near_kernel(const float *__restrict__ xpts
                                                  float scale, int R, int r0, float *out, int row_begin, int row_end) {
     constexpr int W = row_width(D, RB);
     __shared__ __align__(16) float smem[ST * W];
+    if ((int)blockIdx.x >= tile_off[nbx]) return;
     int box, t0, t1;
     item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1);
     float tx[TI][D], tot[TI][RB];
@@ -195,29 +196,6 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// coefficients of the polynomial part of the exponentials, lowest first
-struct ExpCoef { float c[6]; };
-// 2^t for |t| < 120 on the FMA pipe: t = n + f with |f| <= 1/2 (n rounded off by adding and subtracting 1.5 * 2^23), the
-// degree-5 polynomial through the Chebyshev points of [-1/2, 1/2] for 2^f (relative error below 7.5e-8, a third of
-// ex2.approx's), and n added to the exponent.
-__device__ __forceinline__ f32x2 ex2_on_fma(f32x2 t, const f32x2 (&c)[6]) {
-    const f32x2 magic = pack2(12582912.f, 12582912.f), nmagic = pack2(-12582912.f, -12582912.f), minus1 = pack2(-1.f, -1.f);
-    const f32x2 r = add2(t, magic);
-    const f32x2 f = fma2(add2(r, nmagic), minus1, t);
-    f32x2 p = fma2(c[5], f, c[4]);
-#pragma unroll
-    for (int k = 3; k >= 0; k--) p = fma2(p, f, c[k]);
-    float ra, rb, pa, pb;
-    unpack2(r, ra, rb);
-    unpack2(p, pa, pb);
-    return pack2(__uint_as_float(__float_as_uint(pa) + (__float_as_uint(ra) << 23)),
-                 __uint_as_float(__float_as_uint(pb) + (__float_as_uint(rb) << 23)));
-}
 __host__ __device__ __forceinline__ int pair_row_start(int off, int box) { return (off + box + 1) & ~1; }
 
 // Packing with one warp per source box (and per part of a long box): boxes no list of this product names
@@ -262,17 +240,18 @@ __global__ void __launch_bounds__(256) pack_pairs_box(const float *__restrict__ 
     }
 }
 
-constexpr int SP2 = 192;   // source pairs per shared-memory tile (6 KB)
+// source pairs per shared-memory tile: 6 KB for one column, 12 KB for eight (so that shared memory does not limit the
+// CTAs per SM below what the registers allow)
+template <int RB> __host__ __device__ constexpr int sp2_of() { return RB >= 4 ? 96 : 192; }
 
-// PNUM of every PDEN source pairs evaluate their exponentials on the FMA pipe, the others on the MUFU pipe.  POLY = 2 or 3:
-// by the polynomial of that degree (the host enables it only when the exponent is provably small).  POLY = 5: by
-// ex2_on_fma, for any exponent.  A pair of sources costs 16 MUFU cycles per warp and target against d + 1 packed
-// multiply-adds (8 cycles at d = 3); ex2_on_fma moves them to 16 cycles of the FMA pipe, so one pair in four levels the two.
+// POLY = 0: every exponential on the MUFU pipe.  POLY = 2 or 3: PNUM of every PDEN source pairs use the
+// polynomial of that degree instead (the host enables it only when the exponent is provably small).
 template <int D, int RB, int POLY, int PNUM, int PDEN, int TI>
 __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ ptr,
                                              const int *__restrict__ idx, const int *__restrict__ off_y,
                                              const float *__restrict__ ctr_y, const float *__restrict__ packed, float scale, int R,
-                                             int r0, float *out, const ExpCoef &pc, float *smem, int box, int t0, int t1) {
+                                             int r0, float *out, float pc0, float pc1, float pc2, float pc3, float *smem, int box,
+                                             int t0, int t1) {
     constexpr int W = row_width(D, RB);
     float x[TI][D], tot[TI][RB];
     int ti[TI];
@@ -291,9 +270,7 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
         for (int r = 0; r < RB; r++) tot[u][r] = 0.f;
     }
-    f32x2 c[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) c[k] = pack2(pc.c[k], pc.c[k]);
+    const f32x2 c1 = pack2(pc1, pc1), c2 = pack2(pc2, pc2), c3 = pack2(pc3, pc3), one = pack2(pc0, pc0);
     const int e0 = ptr[box], e1 = ptr[box + 1];
     for (int e = e0; e < e1; e++) {
         const int by = idx[e];
@@ -315,6 +292,7 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
             for (int r = 0; r < RB; r++) acc[u][r] = pack2(0.f, 0.f);
         }
+        constexpr int SP2 = sp2_of<RB>();
         for (int base = 0; base < npairs; base += SP2) {
             const int np = min(SP2, npairs - base);
             __syncthreads();
@@ -338,10 +316,8 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 #pragma unroll
                     for (int k = 1; k < D; k++) t = fma2(xr[u][k], col[k], t);
                     f32x2 ev;
-                    if (poly) {
-                        ev = POLY == 5   ? ex2_on_fma(t, c)
-                             : POLY == 2 ? fma2(fma2(c[2], t, c[1]), t, c[0])
-                                         : fma2(fma2(fma2(c[3], t, c[2]), t, c[1]), t, c[0]);
+                    if (POLY && poly) {
+                        ev = (POLY == 2) ? fma2(fma2(c2, t, c1), t, one) : fma2(fma2(fma2(c3, t, c2), t, c1), t, one);
                     } else {
                         float ta, tb;
                         unpack2(t, ta, tb);
@@ -353,10 +329,15 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
             };
             int j = 0;
             const int npl = (TI == 1) ? (np - grp + G - 1) / G : np;   // pairs of this lane group
+            if (POLY) {
 #pragma unroll 1
-            for (; j + PDEN <= npl; j += PDEN) {
+                for (; j + PDEN <= npl; j += PDEN) {
 #pragma unroll
-                for (int q = 0; q < PDEN; q++) body(j + q, ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN);
+                    for (int q = 0; q < PDEN; q++) body(j + q, ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN);
+                }
+            } else {
+#pragma unroll 4
+                for (; j + 1 <= npl; j++) body(j, false);
             }
             for (; j < npl; j++) body(j, false);
         }
@@ -384,22 +365,184 @@ __device__ __forceinline__ void near_tile_x2(const float *__restrict__ xpts, int
 }
 
 
-// TI = targets per thread.  MIXED: a tile of at most 32 targets runs a one-target form, which does half the work; the host picks this variant only when such tiles exist.
+// 16-byte asynchronous copy global -> shared (completion tracked per thread in commit groups)
+__device__ __forceinline__ void cp_async16(float *smem_dst, const float *gsrc) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// A tile of at most 32 targets (small boxes: clustered data, four and five dimensions), one warp.  Two things differ
+// from near_tile_x2.  (1) With TS <= 16 targets (TS a power of two) the warp splits into 32 / TS lane groups that hold
+// the same targets and take every (32 / TS)-th source pair; the groups' sums are added by shuffles at the end, so no
+// lane idles.  (2) Source boxes of a dozen points give a handful of pair iterations each, too few to hide the chain
+// list entry -> box offsets -> packed rows behind: the shared-memory tile is two half tiles, the rows of the next chunk
+// arrive by asynchronous copies while the current one is consumed, and the offsets and centres of the two boxes after
+// it are already in registers.
+template <int D, int RB, int POLY, int PNUM, int PDEN>
+__device__ __forceinline__ void near_tile_x2_small(const float *__restrict__ xpts, int n_x, const int *__restrict__ ptr,
+                                                   const int *__restrict__ idx, const int *__restrict__ off_y,
+                                                   const float *__restrict__ ctr_y, const float *__restrict__ packed,
+                                                   float scale, int R, int r0, float *out, float pc0, float pc1, float pc2,
+                                                   float pc3, float *smem, int box, int t0, int t1) {
+    constexpr int W = row_width(D, RB);
+    constexpr int SPH = sp2_of<RB>() / 2;   // source pairs per half tile
+    constexpr int V4 = 2 * W / 4;           // 16-byte pieces of a pair block
+    const int lane = threadIdx.x;
+    const int nt = t1 - t0;
+    const int lg = nt > 16 ? 5 : (nt > 8 ? 4 : (nt > 4 ? 3 : 2));
+    const int TS = 1 << lg, G = 32 >> lg;
+    const int g = lane >> lg;
+    const int ti = t0 + (lane & (TS - 1));
+    float x[D], tot[RB];
+    {
+        const int ii = ti < t1 ? ti : t0;
+#pragma unroll
+        for (int k = 0; k < D; k++) x[k] = xpts[(size_t)k * n_x + ii];
+#pragma unroll
+        for (int r = 0; r < RB; r++) tot[r] = 0.f;
+    }
+    const f32x2 c1 = pack2(pc1, pc1), c2 = pack2(pc2, pc2), c3 = pack2(pc3, pc3), one = pack2(pc0, pc0);
+    const int e0 = ptr[box], e1 = ptr[box + 1];
+    if (e0 == e1) return;
+    struct Src {
+        int npairs;
+        const float *rows;
+        float ctr[D];
+    };
+    auto load_src = [&](int by, Src &sb) {
+        const int s0 = off_y[by];
+        sb.npairs = (off_y[by + 1] - s0 + 1) >> 1;
+        sb.rows = packed + (size_t)pair_row_start(s0, by) * W;
+#pragma unroll
+        for (int k = 0; k < D; k++) sb.ctr[k] = __ldg(ctr_y + by * D + k);
+    };
+    auto issue_copy = [&](float *dst, const Src &sb, int base) {
+        const int pieces = min(SPH, sb.npairs - base) * V4;
+        const float *src = sb.rows + (size_t)base * 2 * W;
+        for (int q = lane; q < pieces; q += NT2) cp_async16(dst + 4 * q, src + 4 * q);
+    };
+    Src cur, n1, n2;
+    load_src(idx[e0], cur);
+    n1 = cur; n2 = cur;
+    if (e0 + 1 < e1) load_src(idx[e0 + 1], n1);
+    if (e0 + 2 < e1) load_src(idx[e0 + 2], n2);
+    int by3 = e0 + 3 < e1 ? idx[e0 + 3] : 0;
+    issue_copy(smem, cur, 0);
+    cp_async_commit();
+    int e = e0, base = 0, pb = 0;
+    f32x2 xr[D], acc[RB];
+    float fx = 0.f;
+    while (true) {
+        const bool more_in_box = base + SPH < cur.npairs;
+        const bool have_next = more_in_box || e + 1 < e1;
+        float *bufc = smem + pb * (SPH * 2 * W), *bufn = smem + (pb ^ 1) * (SPH * 2 * W);
+        if (have_next) {
+            if (more_in_box) issue_copy(bufn, cur, base + SPH);
+            else issue_copy(bufn, n1, 0);
+        }
+        cp_async_commit();
+        cp_async_wait<1>();   // everything but the group just committed has landed
+        __syncthreads();
+        if (base == 0) {
+            float nx = 0.f;
+#pragma unroll
+            for (int k = 0; k < D; k++) {
+                const float v = scale * (x[k] - cur.ctr[k]);
+                nx = fmaf(-v, v, nx);
+                xr[k] = pack2(v, v);
+            }
+            fx = ex2_approx(nx);
+#pragma unroll
+            for (int r = 0; r < RB; r++) acc[r] = pack2(0.f, 0.f);
+        }
+        const int np = min(SPH, cur.npairs - base);
+        int q = 0;
+#pragma unroll 2
+        for (int j = g; j < np; j += G) {
+            f32x2 col[W];
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(bufc + j * 2 * W);
+#pragma unroll
+            for (int c = 0; c < W / 2; c++) {
+                const ulonglong2 v = src[c];
+                col[2 * c] = v.x;
+                col[2 * c + 1] = v.y;
+            }
+            f32x2 t = mul2(xr[0], col[0]);
+#pragma unroll
+            for (int k = 1; k < D; k++) t = fma2(xr[k], col[k], t);
+            f32x2 ev;
+            if (POLY && ((q + 1) * PNUM) / PDEN != (q * PNUM) / PDEN) {
+                ev = (POLY == 2) ? fma2(fma2(c2, t, c1), t, one) : fma2(fma2(fma2(c3, t, c2), t, c1), t, one);
+            } else {
+                float ta, tb;
+                unpack2(t, ta, tb);
+                ev = pack2(ex2_approx(ta), ex2_approx(tb));
+            }
+#pragma unroll
+            for (int r = 0; r < RB; r++) acc[r] = fma2(ev, col[D + r], acc[r]);
+            if (POLY && ++q == PDEN) q = 0;
+        }
+        if (!more_in_box) {
+#pragma unroll
+            for (int r = 0; r < RB; r++) {
+                float lo, hi;
+                unpack2(acc[r], lo, hi);
+                tot[r] = fmaf(fx, lo + hi, tot[r]);
+            }
+        }
+        __syncthreads();   // the copy issued in the next round overwrites the half tile read here
+        if (more_in_box) base += SPH;
+        else {
+            if (++e >= e1) break;
+            base = 0;
+            cur = n1;
+            n1 = n2;
+            if (e + 2 < e1) load_src(by3, n2);
+            by3 = e + 3 < e1 ? idx[e + 3] : 0;
+        }
+        pb ^= 1;
+    }
+    cp_async_wait<0>();
+    for (int o = TS; o < 32; o <<= 1)
+#pragma unroll
+        for (int r = 0; r < RB; r++) tot[r] += __shfl_xor_sync(0xffffffffu, tot[r], o);
+    if (g == 0 && ti < t1) {
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            if (r0 + r < R) out[(size_t)ti * R + r0 + r] += tot[r];
+    }
+}
+
+// TI = targets per thread.  MIXED: a tile of at most 32 targets runs a one-target form, which does half the work (the
+// pipelined one for small boxes); the host picks this variant only when such tiles exist.
 template <int D, int RB, int POLY, int PNUM, int PDEN, bool MIXED>
-__global__ void __launch_bounds__(NT2, 32) near_kernel_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x,
+__global__ void __launch_bounds__(NT2, RB == 1 ? 32 : (RB <= 4 ? 20 : 12)) near_kernel_x2(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x,
                                                      int nbx, const int *__restrict__ tile_off,
                                                      const int *__restrict__ ptr, const int *__restrict__ idx,
                                                      const int *__restrict__ off_y, const float *__restrict__ ctr_y,
                                                      const float *__restrict__ packed, float scale, int R, int r0,
-                                                     float *out, ExpCoef pc, int row_begin, int row_end) {
+                                                     float *out, float pc0, float pc1, float pc2, float pc3, int row_begin,
+                                                     int row_end) {
     constexpr int W = row_width(D, RB);
-    __shared__ __align__(16) float smem[SP2 * 2 * W];
+    __shared__ __align__(16) float smem[sp2_of<RB>() * 2 * W];
+    if ((int)blockIdx.x >= tile_off[nbx]) return;
     int box, t0, t1;
     item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1, MIXED ? NT2 * TI2 : 0);
     if (MIXED && t1 - t0 <= NT2) {
-        near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc, smem, box, t0, t1);
+        // a box of at most 32 points has neighbours of its own kind (same level, same local density): short source boxes,
+        // where the pipelined form pays; the last tile of a large box meets large source boxes and keeps the plain loop
+        if (RB >= 4 && off_x[box + 1] - off_x[box] <= NT2)   // one column: measured slower than the plain loop on clustered data
+            near_tile_x2_small<D, RB, POLY, PNUM, PDEN>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2,
+                                                        pc3, smem, box, t0, t1);
+        else
+            near_tile_x2<D, RB, POLY, PNUM, PDEN, 1>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3,
+                                                     smem, box, t0, t1);
     } else
-        near_tile_x2<D, RB, POLY, PNUM, PDEN, TI2>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc, smem, box, t0, t1);
+        near_tile_x2<D, RB, POLY, PNUM, PDEN, TI2>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2, pc3, smem,
+                                                   box, t0, t1);
 }
 
 #include "near_mma.cuh"
@@ -421,14 +564,14 @@ __global__ void __launch_bounds__(256) near_tiles_per_box(int nbx, const int *__
     tiles[b] = t;
 }
 
-// Polynomial of degree deg (<= 5) through the Chebyshev points of [tlo, thi] for 2^t, as monomial coefficients.
+// Polynomial of degree deg (<= 3) through the Chebyshev points of [tlo, thi] for 2^t, as monomial coefficients.
 // Its error is at most h^(deg+1) / (2^deg (deg+1)!) with h = ln2 (thi - tlo) / 2.
-static void exp2_poly_fit(double tlo, double thi, int deg, double (&cf)[6]) {
-    for (int i = 0; i < 6; i++) cf[i] = 0.0;
+static void exp2_poly_fit(double tlo, double thi, int deg, double (&cf)[4]) {
+    for (int i = 0; i < 4; i++) cf[i] = 0.0;
     cf[0] = 1.0;
     if (deg <= 0) return;
     const int m = deg + 1;
-    double tn[6], dd[6];
+    double tn[4], dd[4];
     for (int i = 0; i < m; i++) {
         tn[i] = 0.5 * (thi + tlo) + 0.5 * (thi - tlo) * cos((2 * i + 1) * 3.14159265358979323846 / (2.0 * m));
         dd[i] = exp2(tn[i]);
@@ -471,6 +614,8 @@ static double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
 // could overflow while the first underflows, so such lists use the direct form
 constexpr double TMAX_EXPANDED = 64.0;
 
+constexpr int MAX_UNREAD_TILES = 8192;
+
 // one list, one block of RB columns starting at r0
 template <int D, int RB>
 static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, int r0, float *out,
@@ -494,11 +639,18 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
                                                                            tile_pts, tiles.p, n_small);
     F3M_LAUNCH_CHECK();
     exclusive_scan_i32(tiles.p, tiles.p, (int64_t)lx.nb + 1, s);
-    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, tiles.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
-    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + 1, n_small, sizeof(int), cudaMemcpyDeviceToHost, s));
-    F3M_CUDA(cudaStreamSynchronize(s));
-    const int items = pl->h_pinned[0];
-    const bool small_tiles = pl->h_pinned[1] > 0;   // some tiles hold at most 32 targets: use the kernel that halves their work
+    // Small calls launch a bound on the tiles (CTAs beyond the last tile leave at once: less than 2 us for the limit below) and
+    // the kernel that halves the work of short tiles; larger ones read the number of tiles and whether there are short ones.
+    const int64_t bound = (int64_t)(row_end - row_begin) / tile_pts + lx.nb;
+    int items = (int)std::min<int64_t>(bound, MAX_UNREAD_TILES);
+    bool small_tiles = true;
+    if (use_mma || bound > MAX_UNREAD_TILES) {
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, tiles.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + 1, n_small, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaStreamSynchronize(s));
+        items = pl->h_pinned[0];
+        small_tiles = pl->h_pinned[1] > 0;   // some tiles hold at most 32 targets
+    }
     if (items <= 0) return;
     // Packed sources are kept for the lists of one level that share (column block, form): the "small" list of the last
     // level and the final near list read the same boxes' rows.
@@ -528,7 +680,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         const double se = (double)scale * ly.edge;
         const double thi = D * se * se * reach, tlo = -D * se * se * (reach + 0.25);
         const int deg = exp2_poly_degree(0.5 * (thi - tlo));
-        double cf[6];
+        double cf[4];
         exp2_poly_fit(tlo, thi, deg, cf);
         int dev = 0, nsm = 0;
         F3M_CUDA(cudaGetDevice(&dev));
@@ -572,15 +724,12 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     if (expanded) {
         const int poly = exp2_poly_degree(tmax);
         pl->last.direct_variants[poly == 2 ? DV_POLY2 : (poly == 3 ? DV_POLY3 : DV_MUFU)]++;
-        double cf[6];
-        if (poly) exp2_poly_fit(-tmax, tmax, poly, cf);
-        else exp2_poly_fit(-0.5, 0.5, 5, cf);
-        ExpCoef pc{};
-        for (int k = 0; k < 6; k++) pc.c[k] = (float)cf[k];
+        double cf[4];
+        exp2_poly_fit(-tmax, tmax, poly, cf);
 #define F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, MIXED_)                                                                                       \
     near_kernel_x2<D, RB, POLY_, PNUM_, PDEN_, MIXED_><<<items, NT2, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, \
                                                                             csr.idx.p, ly.off.p, ly.ctr.p, packed.p, scale, R, r0, out, \
-                                                                            pc, row_begin, row_end)
+                                                                            (float)cf[0], (float)cf[1], (float)cf[2], (float)cf[3], row_begin, row_end)
 #define F3M_NEAR_EXP(POLY_, PNUM_, PDEN_)                         \
     {                                                             \
         if (small_tiles) F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, true); \
@@ -588,7 +737,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     }
         if (poly == 2) F3M_NEAR_EXP(2, 2, 5)
         else if (poly == 3) F3M_NEAR_EXP(3, 1, 3)
-        else F3M_NEAR_EXP(5, 1, 4)
+        else F3M_NEAR_EXP(0, 0, 1)
 #undef F3M_NEAR_EXP2
 #undef F3M_NEAR_EXP
     }
@@ -602,12 +751,24 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     F3M_LAUNCH_CHECK();
 }
 
+// Five to eight columns: tensor cores or CUDA cores?
+template <int D>
+static bool columns_on_tensor_cores(const f3m_plan *pl, int level, const PairCSR &csr) {
+    const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
+    return D >= 4 && (level == 0 || exp2_poly_degree(D * list_reach(pl, level, csr) * se * se) == 0);
+}
+
 template <int D>
 static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out, int rb, int re,
                      cudaStream_t s) {
     const bool expanded = level > 0 && near_scale(pl->lcs) * pl->tx.levels[level].edge <= 1.0f;   // near_cols.cu
     for (int r0 = 0; r0 < R;) {
-        if (R - r0 >= 2) { column_sums(pl, level, csr, expanded, bs, R, r0, out, rb, re, s); r0 += 8; }
+        const int left = R - r0;
+        if (left >= 5) {
+            if (columns_on_tensor_cores<D>(pl, level, csr)) column_sums(pl, level, csr, expanded, bs, R, r0, out, rb, re, s);
+            else direct_impl<D, 8>(pl, level, csr, bs, R, r0, out, rb, re, s);
+            r0 += 8;
+        } else if (left >= 2) { direct_impl<D, 4>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 4; }
         else { direct_impl<D, 1>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 1; }
     }
 }

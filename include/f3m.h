@@ -294,8 +294,8 @@ int f3m_plan_last_timings(const f3m_plan *plan, float ms[8]);
  * library since it was loaded (all entry points). */
 int f3m_plan_last_direct_launches(const f3m_plan *plan);
 /* Which form of the direct-sum kernel those launches took (the host picks it per list from a bound on the
- * exponent, see near_field_run n_tree.cu:831-902 for the sums themselves): counts[0] expanded form for any exponent
- * (one pair in four on the FMA pipe for one column), [1] expanded form with 2/5 of the pairs on a degree-2 polynomial,
+ * exponent, see near_field_run n_tree.cu:831-902 for the sums themselves): counts[0] expanded form with every
+ * exponential on the special-function unit, [1] expanded form with 2/5 of the pairs on a degree-2 polynomial,
  * [2] with 1/3 on a degree-3 polynomial, [3] direct form (differences, wide boxes), [4] moment form (of degree 2 and 3 it
  * counts in [1] and [2] too: every exponent of the list is in that polynomial), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES). */
 int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]);
