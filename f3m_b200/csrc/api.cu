@@ -290,15 +290,7 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
     // root pair list (n_tree.cu:1071)
     pl->lists.clear();
     pl->lists.emplace_back();
-    {
-        PairCSR &k = pl->lists[0].keep;
-        k.ptr.alloc(2, s); k.idx.alloc(1, s);
-        int h[2] = {0, 1};
-        F3M_CUDA(cudaMemcpyAsync(k.ptr.p, h, sizeof(h), cudaMemcpyHostToDevice, s));
-        F3M_CUDA(cudaMemsetAsync(k.idx.p, 0, 4, s));
-        F3M_CUDA(cudaStreamSynchronize(s));
-        k.count = 1;
-    }
+    build_root_list(pl->lists[0].keep, s);
     pl->stats = f3m_plan_stats{};
     int level = 0;
     auto go_on = [&]() {

@@ -317,6 +317,7 @@ void scatter_rows_nonzero(const float *src, const int *perm, float *dst, int64_t
 
 // ---- tree.cu ---------------------------------------------------------------------------------
 void build_root(Tree &t, cudaStream_t s);
+void build_root_list(PairCSR &k, cudaStream_t s);   // the one pair of roots (n_tree.cu:1071)
 void build_levels(Tree &t, int l_last, f3m_plan *pl, cudaStream_t s);   // appends levels up to l_last (<= sorted_depth)
 void build_level_lists(f3m_plan *pl, int level, cudaStream_t s);     // uses lists[level-1].keep
 void accumulate_pair_work(f3m_plan *pl, int level, int slot, const PairCSR &csr, cudaStream_t s);   // FL_PAIRWORK (device)

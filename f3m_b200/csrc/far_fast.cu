@@ -90,6 +90,15 @@ static void make_shift_tables(const NodeTab2 &nt, std::vector<float> &A, std::ve
         }
 }
 
+// both tables in one kernel parameter: no copies from pageable host memory and no wait for them
+struct ShiftTables { float a[2 * mat_stride(PMAX_FAST)], at[2 * mat_stride(PMAX_FAST)]; };
+__global__ void shift_tables_kernel(ShiftTables t, int n, float *A, float *AT) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        A[i] = t.a[i];
+        AT[i] = t.at[i];
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // warp-level "apply d matrices along the d axes"
 // Array layout: index = m*RB + r, m = sum_k m_k p^k (dimension 0 fastest), r the column.
@@ -1424,9 +1433,11 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     make_shift_tables(nt, hA, hAT);
     DevBuf<float> A, AT;
     A.alloc(hA.size(), s); AT.alloc(hAT.size(), s);
-    F3M_CUDA(cudaMemcpyAsync(A.p, hA.data(), hA.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-    F3M_CUDA(cudaMemcpyAsync(AT.p, hAT.data(), hAT.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-    F3M_CUDA(cudaStreamSynchronize(s));   // hA / hAT are pageable host vectors
+    ShiftTables st{};
+    std::copy(hA.begin(), hA.end(), st.a);
+    std::copy(hAT.begin(), hAT.end(), st.at);
+    shift_tables_kernel<<<1, 128, 0, s>>>(st, (int)hA.size(), A.p, AT.p);
+    F3M_LAUNCH_CHECK();
 
     // warps per CTA of the translation kernels, limited by shared memory
     const size_t per_warp = (size_t)3 * PR * sizeof(float);

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) bbox_kernel(const float *__restrict__ X, 
     if ((threadIdx.x & 31) == 0) {
 #pragma unroll
         for (int k = 0; k < D; k++) {
-            atomicMin(&mm[k], enc_f32(lo[k]));
+            atomicMax(&mm[k], ~enc_f32(lo[k]));   // complemented, so that zero is the start of either extreme
             atomicMax(&mm[MAXD + k], enc_f32(hi[k]));
         }
     }
@@ -153,9 +153,8 @@ __global__ void __launch_bounds__(256) bbox_kernel(const float *__restrict__ X, 
 
 void bounding_box(const float *X, int64_t n, int d, float *h_min, float *h_max, f3m_plan *pl, cudaStream_t s) {
     unsigned *mm = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX;   // 2*MAXD words
-    unsigned init[2 * MAXD];
-    for (int k = 0; k < MAXD; k++) { init[k] = 0xffffffffu; init[MAXD + k] = 0u; }
-    F3M_CUDA(cudaMemcpyAsync(mm, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    constexpr size_t mm_bytes = 2 * MAXD * sizeof(unsigned);
+    F3M_CUDA(cudaMemsetAsync(mm, 0, mm_bytes, s));
     int grid = (int)std::min<int64_t>((n + 255) / 256, NUM_SMS_HINT * 8);
     switch (d) {
         case 1: bbox_kernel<1><<<grid, 256, 0, s>>>(X, n, mm); break;
@@ -166,10 +165,10 @@ void bounding_box(const float *X, int64_t n, int d, float *h_min, float *h_max, 
     }
     F3M_LAUNCH_CHECK();
     unsigned *h = reinterpret_cast<unsigned *>(pl->h_pinned);
-    F3M_CUDA(cudaMemcpyAsync(h, mm, sizeof(init), cudaMemcpyDeviceToHost, s));
+    F3M_CUDA(cudaMemcpyAsync(h, mm, mm_bytes, cudaMemcpyDeviceToHost, s));
     F3M_CUDA(cudaStreamSynchronize(s));
     for (int k = 0; k < d; k++) {
-        h_min[k] = dec_f32(h[k]);
+        h_min[k] = dec_f32(~h[k]);
         h_max[k] = dec_f32(h[MAXD + k]);
     }
 }

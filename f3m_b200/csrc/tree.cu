@@ -188,6 +188,27 @@ __global__ void __launch_bounds__(256) child_starts(int nbp, const int *__restri
     child_start[p] = lo;
 }
 
+// The root's arrays come from kernel parameters: copies from host arrays would need a wait before those go out of scope.
+struct RootValues { int n, d; float c[MAXD]; };
+__global__ void root_kernel(RootValues v, int *off, uint32_t *code, int *parent, float *ctr) {
+    off[0] = 0;
+    off[1] = v.n;
+    code[0] = 0;
+    parent[0] = 0;
+    for (int k = 0; k < v.d; k++) ctr[k] = v.c[k];
+}
+__global__ void root_list_kernel(int *ptr, int *idx) {
+    ptr[0] = 0;
+    ptr[1] = 1;
+    idx[0] = 0;
+}
+void build_root_list(PairCSR &k, cudaStream_t s) {
+    k.ptr.alloc(2, s); k.idx.alloc(1, s);
+    root_list_kernel<<<1, 1, 0, s>>>(k.ptr.p, k.idx.p);
+    F3M_LAUNCH_CHECK();
+    k.count = 1;
+}
+
 void build_root(Tree &t, cudaStream_t s) {
     t.levels.clear();
     t.levels.emplace_back();
@@ -196,15 +217,11 @@ void build_root(Tree &t, cudaStream_t s) {
     L.edge = t.edge0;
     L.max_count = (int)t.n;
     L.off.alloc(2, s); L.code.alloc(1, s); L.parent.alloc(1, s); L.ctr.alloc(t.d, s);
-    int off[2] = {0, (int)t.n};
-    float c[MAXD];
+    RootValues v{(int)t.n, t.d, {0}};
     float half = 0.5f * t.edge0;                       // exact
-    for (int k = 0; k < t.d; k++) c[k] = t.origin[k] + half;   // n_tree.cu:93, float32 add
-    F3M_CUDA(cudaMemcpyAsync(L.off.p, off, sizeof(off), cudaMemcpyHostToDevice, s));
-    F3M_CUDA(cudaMemsetAsync(L.code.p, 0, 4, s));
-    F3M_CUDA(cudaMemsetAsync(L.parent.p, 0, 4, s));
-    F3M_CUDA(cudaMemcpyAsync(L.ctr.p, c, sizeof(float) * t.d, cudaMemcpyHostToDevice, s));
-    F3M_CUDA(cudaStreamSynchronize(s));   // host arrays above go out of scope
+    for (int k = 0; k < t.d; k++) v.c[k] = t.origin[k] + half;   // n_tree.cu:93, float32 add
+    root_kernel<<<1, 1, 0, s>>>(v, L.off.p, L.code.p, L.parent.p, L.ctr.p);
+    F3M_LAUNCH_CHECK();
 }
 
 // Appends the levels after the last one built, up to l_last, in batches of HB levels: two host synchronisations
