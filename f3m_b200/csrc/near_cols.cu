@@ -1,12 +1,13 @@
 // Direct sums of the near / small field with several right-hand sides (near_field_run, F3M_src/n_tree.cu:831-902).
 //
-// A pair costs its exponent (d multiply-adds in the expanded form, 2 d in the difference form), one exponential and R
-// multiply-adds into the columns.  On the CUDA cores the last part dominates at R = 8, and every source row of d + R
-// floats has to be broadcast out of shared memory to all 32 lanes for two targets each.  Here that part is the
-// contraction it is, C(16 targets x 8 columns) += E(16 x 8 sources) B(8 x 8), on mma.m16n8k8.tf32: a lane of the A
-// fragment owns the exponentials of two targets (g, g+8) and two sources (t, t+4), so no value is computed twice and a
-// source row is loaded once per four lanes.  The tile is too narrow for tcgen05 (N = 8 columns, E made in registers), and
-// mma.sync keeps up: the exponentials stay the limit.
+// Boxes of a few to some forty points (near.cu has the rule).  A pair costs its exponent (d multiply-adds in the expanded form,
+// 2 d in the difference form), one exponential and R multiply-adds into the columns.  The CUDA-core kernels lose their time there
+// on every source box: its rows through shared memory, target coordinates and factors anew, tiles and row pairs half empty.  Here the
+// sources of a tile are one stream, and the sum over columns is the contraction C(16 targets x 8 columns) += E(16 x 8
+// sources) B(8 x 8) on mma.m16n8k8.tf32: a lane of the A fragment owns the exponentials of two targets (g, g+8) and two
+// sources (t, t+4), so no value is computed twice and a source is loaded once per four lanes.  The tile is too narrow for
+// tcgen05 (N = 8 columns, E made in registers).  What bounds it: the three mma.sync per 128 pairs, 0.9e12 pairs/s at any
+// occupancy (1e6 points N(0,I), 8 columns: d = 4 35.5 -> 27.6 ms, d = 5 178 -> 166 ms; 3e5 points, d = 5: 33.6 -> 15.3 ms).
 //
 // Precision: E and B are split into two TF32 numbers each (hi rounded to 11 bits, lo = the exact remainder), and hi hi + hi lo +
 // lo hi is accumulated in FP32; what is dropped is below 2^-22 of a term.  The tensor core's own accumulator, which
