@@ -533,6 +533,27 @@ __global__ void __launch_bounds__(256) scatter_rows_kernel(const float *__restri
     int c = (int)(e - i * cols);
     dst[(int64_t)perm[i] * cols + c] = src[e];
 }
+// One column, destination larger than the L2: a random 4-byte write costs a 32-byte sector each way when its line has left the
+// cache before the neighbours come (1e8 rows: 3.82 ms; by windows 1.27 ms).  The destination is therefore filled window by window, each small enough to
+// stay in L2 until its lines are complete; the permutation is read once per window, in streams, and a value when its row falls
+// into the window.  blockIdx.y counts the windows, so blocks of one window are issued before those of the next.
+constexpr int64_t SCATTER_WINDOW = (int64_t)16 << 20;   // rows: 64 MB of the 126 MB L2
+__global__ void __launch_bounds__(256) scatter_window_kernel(const float *__restrict__ src, const int *__restrict__ perm, float *dst,
+                                                            int64_t n) {
+    const int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const int64_t lo = (int64_t)blockIdx.y * SCATTER_WINDOW, hi = lo + SCATTER_WINDOW;
+    if (i + 4 <= n) {
+        const int4 p = __ldcs(reinterpret_cast<const int4 *>(perm + i));
+        const int row[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (row[k] >= lo && row[k] < hi) dst[row[k]] = __ldcs(src + i + k);
+    } else {
+        for (int64_t k = i; k < n; k++)
+            if (perm[k] >= lo && perm[k] < hi) dst[perm[k]] = src[k];
+    }
+}
 // rows that are entirely zero are skipped (dst must be zero-filled): used when only a slice of the sorted
 // rows was computed, so that the random writes are paid for that slice only
 __global__ void __launch_bounds__(256) scatter_rows_nonzero_kernel(const float *__restrict__ src, const int *__restrict__ perm,
@@ -560,6 +581,12 @@ void gather_rows(const float *src, const int *perm, float *dst, int64_t n, int c
 void scatter_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s) {
     int64_t tot = n * cols;
     if (tot == 0) return;
+    if (cols == 1 && n > 2 * SCATTER_WINDOW) {
+        const dim3 grid((unsigned)((n + 1023) / 1024), (unsigned)((n + SCATTER_WINDOW - 1) / SCATTER_WINDOW));
+        scatter_window_kernel<<<grid, 256, 0, s>>>(src, perm, dst, n);
+        F3M_LAUNCH_CHECK();
+        return;
+    }
     scatter_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(src, perm, dst, n, cols);
     F3M_LAUNCH_CHECK();
 }

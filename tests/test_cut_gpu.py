@@ -53,3 +53,17 @@ def test_no_cut_where_the_interpolation_is_not_exact(cuda):
         plan = engine.Plan(X, None, engine.make_params(ls, 300.0, p ** 3, False, 0.15, p ** 3))
         plan.apply(b)
         assert plan.timings()["direct_launches"] > 0
+
+
+def test_result_larger_than_the_cache(cuda):
+    """More rows than two windows of the result's permutation, the last window and the last rows ragged."""
+    from f3m_b200 import engine
+    n = 2 * (16 << 20) + 4099
+    g = torch.Generator(device=cuda).manual_seed(9)
+    X = torch.rand(n, 3, device=cuda, generator=g)
+    b = torch.rand(n, 1, device=cuda, generator=g) + 0.5
+    out = engine.kmvm(X, None, b, engine.make_params(1.0, 1000.0, 216, False, 0.15, 216))
+    rows = torch.tensor([0, 1, 2, (16 << 20) - 1, 16 << 20, (32 << 20) - 1, 32 << 20, n - 4, n - 3, n - 2, n - 1], device=cuda)
+    exact = engine.rbf_dense(X[rows].double(), X.double(), b.double(), 1.0)
+    assert ((out[rows].double() - exact).abs() / exact).max().item() <= 2e-6
+    assert torch.isfinite(out).all() and (out > 0).all()
