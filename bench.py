@@ -396,11 +396,12 @@ def main():
                 "hbm_peak_gbs": hbm_gbs, "hbm_peak": hbm_src,
                 "tree+lists": stage_roof(tm["build"], N * (2 * 4 * d + 2 * 4 * R + 8), 0),   # sort traffic: 40 B/point at d=3, R=1
                 "p2m": stage_roof(tm["p2m"], N * (4 * d + 4 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
-                "m2l": stage_roof(tm["m2l"], 2 * nb_leaf * Pn * R * 4, st["far_box_pairs"] * d * pd * Pn * R),
+                "m2l": (stage_roof(tm["m2l"], 2 * nb_leaf * Pn * R * 4, st["far_box_pairs"] * d * pd * Pn * R) if direct_ms > 0
+                        else {"ms": round(tm["m2l"], 3), "note": "ends above the last level"}),
                 "l2p": stage_roof(tm["l2p"], N * (4 * d + 8 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
                 "direct": {"ms": round(direct_ms, 3), "frac": round(achieved_pairs / peak_pairs, 3) if pairs_summed else None},
                 "note": "m2l multiply-adds counted in the per-pair form (d axis transforms per far pair of all levels); the nested kernel does "
-                        "fewer, and a product that ends above the last level visits only the lists down to there"}
+                        "fewer"}
         line["work"] = {"levels": st["levels"], "direct_pairs": st["direct_pairs"], "far_box_pairs": st["far_box_pairs"],
                         "node_pairs_reference_form": st["node_pairs"]}
         rows = torch.randperm(N, device=dev, generator=g)[:a.check_rows]

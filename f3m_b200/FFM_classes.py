@@ -29,7 +29,7 @@ class FFM:
                  var_compression=False, small_field_points=1000, device="cuda:0", math_mode=MATH_FASTMATH,
                  near_moments=False):
         # math_mode and near_moments are additions to the reference's arguments: the numeric flavour of the box
-        # index / far test, and the optional evaluation of near sums by box moments (see include/f3m.h)
+        # index / far test, and a looser bound for evaluating near sums by box moments (see include/f3m.h)
         self.X = X.float().to(device)
         if torch.is_tensor(Y):
             self.Y = Y.float().to(device)

@@ -17,6 +17,8 @@ namespace f3m {
 //   * A CTA takes DTILE = 256 targets and one SLICE of the sources, straight from the caller's rows.  With one CTA per
 //     target tile a call of 2e4 points ran 157 four-warp CTAs on 148 SMs: most of the chip idle, then a second, nearly empty wave.
 //     The slices' partial sums are added in a fixed order by dense_combine, so results do not depend on scheduling.
+// Measured, product + gradient of 2e4 points, d = 3, 3 columns: 1280 -> 358 us on the device (171 + 181, floor 87 + 98 at nine and ten
+// FP32 lanes a pair); error against float64 5.4e-7 -> 3.1e-7.
 constexpr int DNT = 128, DT = 2, DTILE = DNT * DT;
 constexpr int DST = 256;   // sources per shared-memory tile; also the length of the blocked partial sums
 

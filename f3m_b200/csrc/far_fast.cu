@@ -1646,6 +1646,9 @@ int64_t far_moments_size(const f3m_plan *pl, int R) {
 // first it reproduces the kernel to rounding for EVERY pair of boxes, neighbours and the box itself included: there the
 // split into far, small and kept pairs no longer matters, and all child pairs of the kept parents are taken through M2L at
 // once.  That level (the cut) ends the product: no direct sums, no deeper lists, no translations below it.
+// Measured with box moments / with the cut too: 1e8 points in [0, sqrt12]^3, l = 1, 216 nodes 44.3 -> 18.5 ms (cut at level 4 of 6, M2L
+// 13.5 -> 0.24 ms), 1e7 points from host tensors 8.8 -> 5.5 ms, a mixture of 1e7 points, l = 0.5 50.8 -> 22.8 ms (level 7 of 8).  Error
+// against float64 unchanged or smaller (1e6 points, l = 4, positive weights 1.5e-7 -> 1.3e-7).
 //
 // Bound.  The kernel is a product over the axes, so the relative error of a pair is the sum over the axes of that of one axis.
 // There g(u) = exp(-u^2 / 2 l^2) is interpolated in x and in y over an edge e: error <= (1 + Lambda_p) E, with E =
