@@ -13,7 +13,7 @@
 //
 // Measured (near sums of one product, pair form -> this form): 1e8 points in [0, sqrt12]^3, l = 1, K = 3, 381 points per
 // box 223.7 -> 10.0 ms; 1e7 points 19.9 -> 1.6 ms (K = 4); 1e5 points in the unit cube (K = 3) 0.187 -> 0.029 ms; 2e4 points
-// (K = 5) 0.176 -> 0.048 ms; the two lists of a mixture of 1e7 points whose boxes are narrow enough 56.4 -> 35.4 ms of all
+// (K = 6) 0.176 -> 0.025 ms; the two lists of a mixture of 1e7 points whose boxes are narrow enough 56.4 -> 35.4 ms of all
 // lists.  near_moments_eval is bound by issue slots (about 37 per target and box at K = 3), near_moments_build by HBM.
 #include <math.h>
 #include <algorithm>
@@ -179,21 +179,24 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
 
 // One thread per target row.  Rows are in box order, so the lanes of a warp read the same record (a broadcast) except
 // where it straddles two boxes; no tiles, no scan and no host read-back are needed.  Two lists of the level (small and
-// near) are walked one after the other and written once.
-template <int D, int K, int RB>
+// near) are walked one after the other and written once.  G lanes share a row (every G-th box of its lists each): calls
+// whose rows do not fill the SMs would wait out the boxes one after the other (2e4 rows, K = 6: 29.2 -> 14.1 us; 1e5 rows, K = 3, the lanes' shorter
+// runs and wider gathers cost more than they hide: 16.1 -> 20.4 us).
+template <int D, int K, int RB, int G>
 __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x, int nbx,
                                                         int row_begin, int row_end, const int *__restrict__ ptr1,
                                                         const int *__restrict__ idx1, const int *__restrict__ ptr2,
                                                         const int *__restrict__ idx2, const float *__restrict__ rec, float s2, int R,
                                                         int r0, float *out) {
     constexpr int REC = mom_record(D, K, RB);
-    const int i0 = row_begin + blockIdx.x * 128 + (threadIdx.x & ~31), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int i0 = row_begin + (int)((blockIdx.x * 128 + (threadIdx.x & ~31)) / G);
     if (i0 >= row_end) return;
     // boxes of the warp's first and last row by two lanes, then each lane searches between them
-    int box = box_of_row(off_x, nbx, lane == 31 ? min(i0 + 31, row_end - 1) : i0);
+    int box = box_of_row(off_x, nbx, lane == 31 ? min(i0 + 32 / G - 1, row_end - 1) : i0);
     const int b_lo = __shfl_sync(0xffffffffu, box, 0), b_hi = __shfl_sync(0xffffffffu, box, 31);
-    const int i = i0 + lane;
-    if (i >= row_end) return;
+    const bool mine = i0 + lane / G < row_end;
+    const int i = mine ? i0 + lane / G : row_end - 1;
     box = b_lo + (b_hi > b_lo ? box_of_row(off_x + b_lo, b_hi - b_lo + 1, i) : 0);
     float x[D], tot[RB];
 #pragma unroll
@@ -207,10 +210,10 @@ __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict
         if (!ptr) continue;
         const int e0 = ptr[box], e1 = ptr[box + 1];
         any = any || e1 > e0;
-        int by = e0 < e1 ? idx[e0] : 0;
-        for (int e = e0; e < e1; e++) {
+        int by = e0 + sub < e1 ? idx[e0 + sub] : 0;
+        for (int e = e0 + sub; e < e1; e += G) {
             const float *m = rec + (size_t)by * REC;
-            if (e + 1 < e1) by = idx[e + 1];
+            if (e + G < e1) by = idx[e + G];
             if constexpr (RB == 1) {
                 float mr[REC];
 #pragma unroll
@@ -244,7 +247,11 @@ __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict
             }
         }
     }
-    if (!any) return;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+        for (int r = 0; r < RB; r++) tot[r] += __shfl_xor_sync(0xffffffffu, tot[r], o);
+    if (!any || !mine || sub) return;
 #pragma unroll
     for (int r = 0; r < RB; r++)
         if (r0 + r < R) out[(size_t)i * R + r0 + r] += tot[r];
@@ -348,16 +355,22 @@ static void moment_impl(f3m_plan *pl, int level, const PairCSR *l1, const PairCS
     if (nsplit > 1) rec.zero();
     const unsigned char *need = pl->shard.active && !pl->shard.all_sources ? pl->shard.need[level].p : nullptr;
     const int64_t groups = (int64_t)ly.nb * RB;
-    if (ly.max_count <= 1024)
+    // a warp per box, unless the boxes are long or too few to fill the SMs (64 boxes of 312 points, K = 6: 13.5 -> 5.2 us with
+    // a CTA per box; 512 boxes of 195 points, K = 3: 5.5 -> 6.8 us)
+    if (ly.max_count <= 1024 && (groups >= 2 * NUM_SMS_HINT || ly.max_count <= 64))
         near_moments_build<D, K, RB, 32><<<dim3((unsigned)((groups + 7) / 8), 1), 256, 0, s>>>(
             ty.pts.p, (int)ty.n, bs, R, r0, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, 1, rec.p);
     else
         near_moments_build<D, K, RB, 256><<<dim3((unsigned)groups, nsplit), 256, 0, s>>>(
             ty.pts.p, (int)ty.n, bs, R, r0, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, nsplit, rec.p);
     F3M_LAUNCH_CHECK();
-    near_moments_eval<D, K, RB><<<(unsigned)((re - rb + 127) / 128), 128, 0, s>>>(
-        tx.pts.p, (int)tx.n, lx.off.p, lx.nb, rb, re, l1->ptr.p, l1->idx.p, l2 ? l2->ptr.p : nullptr, l2 ? l2->idx.p : nullptr, rec.p, s2, R,
-        r0, out);
+    auto eval = [&](auto kernel, int G) {
+        kernel<<<(unsigned)(((int64_t)(re - rb) * G + 127) / 128), 128, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, rb, re, l1->ptr.p, l1->idx.p,
+                                                                               l2 ? l2->ptr.p : nullptr, l2 ? l2->idx.p : nullptr, rec.p, s2, R,
+                                                                               r0, out);
+    };
+    if ((int64_t)(re - rb) >= 256 * NUM_SMS_HINT) eval(near_moments_eval<D, K, RB, 1>, 1);
+    else eval(near_moments_eval<D, K, RB, 4>, 4);
     pl->last.end(s);
     F3M_LAUNCH_CHECK();
     pl->last.direct_launches++;
