@@ -1362,9 +1362,12 @@ static int box_parts(int max_count, int64_t n, int nb, int64_t part) {
 static int target_parts(int max_count, int64_t n, int nb) {
     return box_parts(max_count, n, nb, std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT))));
 }
-// Source boxes: at most 1024 points, so that no running sum is longer than some fifty terms (its rounding grows with the
-// square root); the box level is chosen so that few parts are added up (SRC_LEAF).
-static int source_parts(int max_count, int64_t n, int nb) { return box_parts(max_count, n, nb, 1024); }
+// Source boxes: 512 to 1024 points for p2m_leaf3, so that no running sum is longer than some fifty terms (its rounding grows with
+// the square root); the box level is chosen so that few parts are added up (SRC_LEAF).  p2m_leaf sums in blocks of 128 points
+// anyway and takes the parts that fill the SMs.
+static int source_parts(int max_count, int64_t n, int nb, bool blocked) {
+    return blocked ? target_parts(max_count, n, nb) : box_parts(max_count, n, nb, std::max<int64_t>(512, std::min<int64_t>(1024, n / (4 * NUM_SMS_HINT))));
+}
 // Sources are interpolated at the first level from L on whose boxes hold at most this many points on average, and moved up by
 // M2M, which adds in a tree: with 375 000 sources per box summed at the cut, 3e6 points and l = 10 were 8.4e-7 from float64,
 // the finest level's 5.6e-7.
@@ -1453,7 +1456,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         Level &ly = ty.levels[Ls];
         const float factor = 2.f / ly.edge;          // 1_d_conv.cu:473
         if (!pl->ext_mom) {
-            const int nsplit = source_parts(ly.max_count, ty.n, ly.nb);
+            const int nsplit = source_parts(ly.max_count, ty.n, ly.nb, !(RB == 1 && d == 3));
             if (nsplit > 1) mom[Ls].zero();
             size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
             F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
