@@ -754,7 +754,8 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 // Several columns: near_columns (near_cols.cu, split TF32) or the CUDA cores?  near_columns runs 0.9e12 pairs/s whatever the boxes hold:
 // mma.sync is its limit.  The CUDA-core kernels fall from 1.6e12 (boxes of 300 points, 4 columns) to 0.2e12 (boxes of ten points in
 // five dimensions) as rows per source box shorten.  Measured direct sums in ms, CUDA cores / near_columns, with f the root of the
-// pairs per box pair: eight columns, d = 5: f = 10 33.6 / 15.3, f = 28 52.7 / 40.2, f = 45 178 / 165, f = 297 5.6 / 7.8; d = 4: f = 25
+// pairs per box pair: eight columns, d = 5: f = 10 33.6 / 15.3, f = 28 52.7 / 40.2, f = 36 5 % slower, f = 45 with 18
+// points per box on average 178 / 165, f = 297 5.6 / 7.8; d = 4: f = 25
 // 33.5 / 26.1, f = 39 8.4 / 8.0, f = 72 10.0 / 11.5; d = 3: f = 12 2.4 / 1.5, f = 27 2.3 / 2.2.  Four columns (cheaper rows), d = 5: f = 10
 // 27.1 / 16.4, f = 17 47.3 / 40.9, f = 28 41.9 / 43.2; d = 4: f = 25 22.8 / 27.2.  Lists with polynomial exponentials stay on the CUDA cores.
 template <int D>
@@ -762,7 +763,10 @@ static bool columns_on_tensor_cores(const f3m_plan *pl, int level, const PairCSR
     if (level < 1 || D < 3) return false;
     const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
     if (exp2_poly_degree(D * list_reach(pl, level, csr) * se * se) != 0) return false;
-    const double limit = cols >= 5 ? (D == 5 ? 48.0 : D == 4 ? 36.0 : 20.0) : (D == 5 ? 20.0 : 0.0);
+    double limit = cols >= 5 ? (D == 5 ? 32.0 : D == 4 ? 36.0 : 20.0) : (D == 5 ? 20.0 : 0.0);
+    // uneven trees: f is carried by the few full boxes, most rows are short
+    const Level &lx = pl->tx.levels[level];
+    if (cols >= 5 && D == 5 && pl->tx.n <= 20 * (int64_t)lx.nb) limit = 48.0;
     return (double)csr.pairs <= limit * limit * (double)csr.count;
 }
 
