@@ -766,6 +766,7 @@ static bool columns_on_tensor_cores(const f3m_plan *pl, int level, const PairCSR
     double limit = cols >= 5 ? (D == 5 ? 32.0 : D == 4 ? 36.0 : 20.0) : (D == 5 ? 20.0 : 0.0);
     // uneven trees: f is carried by the few full boxes, most rows are short
     const Level &lx = pl->tx.levels[level];
+    if (lx.nb < 16 * NUM_SMS_HINT) return false;   // a warp per tile: fewer do not fill the SMs (1024 boxes of 36 points: 4 % slower)
     if (cols >= 5 && D == 5 && pl->tx.n <= 20 * (int64_t)lx.nb) limit = 48.0;
     return (double)csr.pairs <= limit * limit * (double)csr.count;
 }
