@@ -1353,9 +1353,10 @@ static void ensure_leaf_split(f3m_plan *pl, int which, int level, cudaStream_t s
 // Parts the boxes of a level are cut into (every box into the same number): `part` points in the longest box.  Levels of
 // uneven occupancy would launch a part for each of a million short boxes because one is long: the number of CTAs is held to the
 // boxes plus four times the parts that an even level would have, but parts never grow beyond what 64 parts of 8192 points give.
+// The parts are the second dimension of a grid: at most 65535.
 static int box_parts(int max_count, int64_t n, int nb, int64_t part) {
     const int64_t want = (max_count + part - 1) / part, even = 1 + 4 * n / (part * nb), at_least = std::min(64, (max_count + 8191) / 8192);
-    return (int)std::max<int64_t>(1, std::max<int64_t>(at_least, std::min<int64_t>(want, even)));
+    return (int)std::min<int64_t>(65535, std::max<int64_t>(1, std::max<int64_t>(at_least, std::min<int64_t>(want, even))));
 }
 // Target boxes: at most 8192 points, and short enough that the parts of all boxes fill the SMs four times over (a cut at
 // level 1 or 2 leaves 8 or 64 boxes), but not below 512 points.

@@ -67,3 +67,19 @@ def test_result_larger_than_the_cache(cuda):
     exact = engine.rbf_dense(X[rows].double(), X.double(), b.double(), 1.0)
     assert ((out[rows].double() - exact).abs() / exact).max().item() <= 2e-6
     assert torch.isfinite(out).all() and (out > 0).all()
+
+
+def test_more_source_parts_than_a_grid_dimension(cuda):
+    """Half of 1.4e8 sources in one octant of a tree that its few targets keep to one level: 68 000 parts of a box."""
+    from f3m_b200 import engine
+    g = torch.Generator(device=cuda).manual_seed(12)
+    m = 140_000_000
+    Y = torch.rand(m, 3, device=cuda, generator=g)
+    Y[: m // 2] *= 0.5
+    X = torch.rand(2000, 3, device=cuda, generator=g)
+    b = torch.rand(m, 1, device=cuda, generator=g) + 0.5
+    plan = engine.Plan(X, Y, engine.make_params(1.0, 1000.0, 512, False, 0.15, 512))   # too narrow for moments, exact on eight nodes
+    out = plan.apply(b)
+    assert plan.stats()["levels"] == 1 and plan.timings()["direct_launches"] == 0
+    exact = engine.rbf_dense(X[:64].double(), Y.double(), b.double(), 1.0)
+    assert rel_l2(out[:64].cpu(), exact.cpu()) <= TOL
