@@ -379,8 +379,7 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     row_end = std::min<int64_t>(N, row_end);
     for (float &m : pl->last.ms) m = 0.f;
     pl->last.ms[ST_BUILD] = pl->stats.build_ms;
-    pl->last.direct_launches = 0;
-    for (int &v : pl->last.direct_variants) v = 0;
+    pl->last.clear_counts();
     pl->last.begin(ST_TOTAL, s);
     pl->pack_cache.reset();
     struct DropPacked { f3m_plan *p; ~DropPacked() { p->pack_cache.reset(); } } drop_packed{pl};
@@ -395,6 +394,7 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
 
     // A product over all rows may end at a level whose interpolation is exact for all its pairs (far_cut_level)
     const int cut = row_begin <= 0 && row_end >= N && !pl->ext_mom && !pl->shard.active ? far_cut_level(pl, R) : 0;
+    pl->last.cut = cut;
     const int L = pl->levels;
     if (L == 0) {
         // largest box already small enough: one direct product over the root pair
@@ -607,8 +607,7 @@ int f3m_plan_shard_begin(f3m_plan *plan, const float *b, int32_t R, int64_t row_
         sh.row_end = std::min<int64_t>(tx.n, row_end);
         for (float &m : plan->last.ms) m = 0.f;
         plan->last.ms[ST_BUILD] = plan->stats.build_ms;
-        plan->last.direct_launches = 0;
-        for (int &v : plan->last.direct_variants) v = 0;
+        plan->last.clear_counts();
         const int64_t msize = far_moments_size(plan, R);
         const bool exchange = msize > 0 && mom_slice != nullptr;
         const int nby = ty.levels[L].nb;
@@ -960,6 +959,15 @@ int f3m_plan_last_direct_launches(const f3m_plan *plan) { return plan ? plan->la
 int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]) {
     if (!plan || !counts) return F3M_ERR_ARG;
     for (int i = 0; i < 6; i++) counts[i] = plan->last.direct_variants[i];
+    return F3M_OK;
+}
+
+int f3m_plan_last_work(const f3m_plan *plan, int64_t work[4]) {
+    if (!plan || !work) return F3M_ERR_ARG;
+    work[0] = plan->last.pairs;
+    work[1] = plan->last.box_pairs;
+    work[2] = plan->last.cut;
+    work[3] = plan->last.column_launches;
     return F3M_OK;
 }
 

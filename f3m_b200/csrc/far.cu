@@ -399,6 +399,7 @@ static void far_level_d(f3m_plan *pl, int level, const float *bs, int R, float *
 void far_field_level(f3m_plan *pl, int level, const float *b_sorted, int R, float *out_sorted, int64_t row_begin,
                      int64_t row_end, cudaStream_t s) {
     if (pl->lists[level].far.count == 0) return;
+    pl->last.box_pairs += pl->lists[level].far.count;
     F3M_REQUIRE(pl->lists[level].p <= MAXP, F3M_ERR_UNSUPPORTED, "%d nodes per dimension exceed the limit of %d",
                 pl->lists[level].p, MAXP);
     switch (pl->d) {

@@ -1513,6 +1513,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
             LevelLists &level_lists = pl->lists[l];
             LevelLists &ll = at_cut ? pl->cut_lists : level_lists;
             if (ll.far.count == 0) continue;
+            if (r0 == 0) pl->last.box_pairs += ll.far.count;
             Level &lx = tx.levels[l], &ly = ty.levels[l];
             const ListSet ls{{level_lists.far.ptr.p, level_lists.small.ptr.p, level_lists.keep.ptr.p},
                              {level_lists.far.idx.p, level_lists.small.idx.p, level_lists.keep.idx.p}, at_cut ? 3 : 1};

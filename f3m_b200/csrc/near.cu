@@ -703,6 +703,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         pl->last.end(s);
         pl->last.direct_launches++;
         pl->last.direct_variants[DV_TENSOR]++;
+        if (r0 == 0) pl->last.pairs += csr.pairs;
         F3M_LAUNCH_CHECK();
         return;
     }
@@ -748,6 +749,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     }
     pl->last.end(s);
     pl->last.direct_launches++;
+    if (r0 == 0) pl->last.pairs += level > 0 ? csr.pairs : tx.n * ty.n;
     F3M_LAUNCH_CHECK();
 }
 

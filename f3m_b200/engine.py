@@ -280,6 +280,12 @@ class Plan:
         check(_lib.lib().f3m_plan_last_direct_variants(self._h, c), "f3m_plan_last_direct_variants")
         return dict(zip(("mufu", "poly2", "poly3", "direct", "moments", "tensor"), (int(v) for v in c)))
 
+    def last_work(self) -> Dict:
+        """What the last apply() visited (f3m_plan_last_work)."""
+        w = (C.c_int64 * 4)()
+        check(_lib.lib().f3m_plan_last_work(self._h, w), "f3m_plan_last_work")
+        return dict(zip(("pairs", "box_pairs", "cut_level", "column_launches"), (int(v) for v in w)))
+
     def array(self, level: int, tree: int, what: int) -> np.ndarray:
         info = self.level(level) if level >= 1 else None
         nb = (info["boxes_x"] if tree == 0 else info["boxes_y"]) if info else 1

@@ -299,6 +299,11 @@ int f3m_plan_last_direct_launches(const f3m_plan *plan);
  * [2] with 1/3 on a degree-3 polynomial, [3] direct form (differences, wide boxes), [4] moment form (of degree 2 and 3 it
  * counts in [1] and [2] too: every exponent of the list is in that polynomial), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES). */
 int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]);
+/* What the last f3m_plan_apply visited: work[0] = pairs of points in the direct lists it summed pair by pair (whole lists, also
+ * when a slice of the rows was asked for), [1] = box pairs of its far field, [2] = the level it ended at before the tree's last
+ * one (0: none), [3] = direct-sum launches that took the kernel for several columns and short boxes (they count in counts[0] or
+ * counts[3] above too). */
+int f3m_plan_last_work(const f3m_plan *plan, int64_t work[4]);
 long long f3m_launch_count(void);
 
 #ifdef __cplusplus

@@ -1,4 +1,4 @@
-"""Direct sums with several columns (split TF32 contraction) against float64 and against single columns."""
+"""Direct sums with several columns against float64 and against single columns."""
 import pytest
 import torch
 
@@ -23,7 +23,7 @@ def test_columns_against_float64(d, n, m, R, ls, cuda):
     exact = engine.rbf_dense(X.double(), (X if Y is None else Y).double(), b.double(), ls)
     # positive terms; exponent of the expanded form: d + 1 roundings of a number below 2 d (side / ls)^2 in the worst pair
     assert rel_l2(out.cpu(), exact.cpu()) <= 5e-6
-    # and no further off than the single-column kernel, which splits nothing
+    # and no further off than the single-column kernel
     one = torch.cat([plan.apply(b[:, r:r + 1].contiguous()) for r in range(R)], 1)
     e_one, e_all = rel_l2(one.cpu(), exact.cpu()), rel_l2(out.cpu(), exact.cpu())
     print(f"columns {e_all:.2e}, one by one {e_one:.2e}")
@@ -45,3 +45,47 @@ def test_columns_of_trees_with_short_boxes(d, ls, leaf, dist, cuda):
     cuts = (0, 5, 1000, 1017, n)
     parts = sum(plan.apply(b, row_range=(lo, hi)) for lo, hi in zip(cuts, cuts[1:]))
     assert rel_l2(parts.cpu(), out.cpu()) <= 1e-6
+
+
+# short boxes at the last levels of a tree: narrow ones in the expanded form, wide ones (short lengthscale) in the difference form; columns
+# that fill a block of eight, parts of one, and a block and a single column; two point sets; slices that cut boxes
+@pytest.mark.parametrize("d,n,m,R,ls,leaf", [(3, 60000, 0, 8, 0.1, 20.0), (3, 60000, 0, 5, 0.01, 20.0), (3, 50021, 40009, 9, 0.02, 20.0), (4, 50021, 0, 8, 0.5, 20.0),
+                                             (4, 50021, 0, 7, 0.05, 20.0), (4, 40009, 50021, 6, 0.1, 20.0), (5, 60000, 0, 8, 0.5, 20.0), (5, 60000, 0, 2, 0.5, 20.0),
+                                             (5, 60000, 0, 3, 0.1, 20.0), (5, 50021, 60000, 8, 0.1, 20.0), (5, 50021, 60000, 4, 0.1, 20.0)])
+def test_columns_of_many_short_boxes(d, n, m, R, ls, leaf, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(31 + d + R)
+    X = torch.rand(n, d, generator=g).to(cuda)
+    Y = (torch.rand(m, d, generator=g) * 0.97 + 0.011).to(cuda) if m else None
+    b = (torch.rand(m or n, R, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, Y, engine.make_params(ls, leaf, 2 ** d, False, 0.15, 2 ** d))
+    cuts = (0, 5, 1000, 1017, n)
+    parts = sum(plan.apply(b, row_range=(lo, hi)) for lo, hi in zip(cuts, cuts[1:]))
+    assert plan.last_work()["column_launches"] > 0
+    wide = plan.direct_variants()["direct"] > 0
+    assert wide == (ls <= 0.1 and (d, ls) != (3, 0.1)), plan.direct_variants()
+    one = torch.cat([sum(plan.apply(b[:, r:r + 1].contiguous(), row_range=(lo, hi)) for lo, hi in ((0, 7), (7, n))) for r in range(R)], 1)
+    assert plan.last_work()["column_launches"] == 0
+    assert rel_l2(parts.cpu(), one.cpu()) <= 2e-6
+    whole = plan.apply(b)
+    assert rel_l2(whole.cpu(), one.cpu()) <= 2e-6
+
+
+# NaN as arithmetic on the GPU makes it (all mantissa bits set) and as the host writes it, and infinities
+@pytest.mark.parametrize("bits", [0x7fffffff, 0x7fc00000, 0x7f800000, -0x00800000])
+@pytest.mark.parametrize("d,n,ls,leaf,dist", [(4, 20011, 1.0, 60.0, "normal"), (3, 60000, 0.05, 20.0, "uniform")])
+def test_columns_keep_non_finite_weights(bits, d, n, ls, leaf, dist, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(7 + d)
+    X = (torch.randn(n, d, generator=g) if dist == "normal" else torch.rand(n, d, generator=g)).to(cuda)
+    b = torch.zeros(n, 8, dtype=torch.int32)
+    b[4321, 3] = bits
+    b = b.view(torch.float32).to(cuda)
+    plan = engine.Plan(X, None, engine.make_params(ls, leaf, 3 ** d, False, 0.15, 3 ** d))
+    out = plan.apply(b)
+    assert plan.last_work()["column_launches"] > 0
+    one = plan.apply(b[:, 3:4].contiguous())[:, 0]
+    assert not one.isfinite().all()
+    assert torch.equal(out[:, 3].isnan(), one.isnan()) and torch.equal(out[:, 3].isinf(), one.isinf())
+    others = out[:, [0, 1, 2, 4, 5, 6, 7]]
+    assert torch.equal(others, torch.zeros_like(others))
