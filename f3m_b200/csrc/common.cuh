@@ -357,7 +357,8 @@ void shard_rows_to_input_order(const f3m_plan *pl, const float *acc_sorted, int 
 // ---- near.cu ---------------------------------------------------------------------------------
 void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted,
                  int64_t row_begin, int64_t row_end, cudaStream_t s);
-// near_cols.cu: up to eight columns of a direct list, starting at r0
+double pair_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate
+// near_cols.cu: up to eight columns of a direct list, starting at r0 (two dimensions and more)
 void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, const float *b_sorted, int R, int r0, float *out_sorted,
                  int row_begin, int row_end, cudaStream_t s);
 // near_moments.cu: sums a direct list through box moments when its geometry allows; false: sum the pairs

@@ -753,24 +753,44 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     F3M_LAUNCH_CHECK();
 }
 
-// Several columns: near_columns (near_cols.cu, split TF32) or the CUDA cores?  near_columns runs 0.9e12 pairs/s whatever the boxes hold:
-// mma.sync is its limit.  The CUDA-core kernels fall from 1.6e12 (boxes of 300 points, 4 columns) to 0.2e12 (boxes of ten points in
-// five dimensions) as rows per source box shorten.  Measured direct sums in ms, CUDA cores / near_columns, with f the root of the
-// pairs per box pair: eight columns, d = 5: f = 10 33.6 / 15.3, f = 28 52.7 / 40.2, f = 36 5 % slower, f = 45 with 18
-// points per box on average 178 / 165, f = 297 5.6 / 7.8; d = 4: f = 25
-// 33.5 / 26.1, f = 39 8.4 / 8.0, f = 72 10.0 / 11.5; d = 3: f = 12 2.4 / 1.5, f = 27 2.3 / 2.2.  Four columns (cheaper rows), d = 5: f = 10
-// 27.1 / 16.4, f = 17 47.3 / 40.9, f = 28 41.9 / 43.2; d = 4: f = 25 22.8 / 27.2.  Lists with polynomial exponentials stay on the CUDA cores.
-template <int D>
-static bool columns_on_tensor_cores(const f3m_plan *pl, int level, const PairCSR &csr, int cols) {
-    if (level < 1 || D < 3) return false;
+// Several columns: the stream of sources (near_columns, near_cols.cu) or the tiles of this file?  Seconds per pair over the whole chip, from
+// direct sums of 280 trees (d = 1..5, uniform and normal, 5e3 to 1e6 points, boxes of 3 to 600 points, 2 to 8 columns).  The
+// stream always carries eight columns; a tile pays its coordinates and columns again on every source box, so it falls behind as the
+// rows per source box shorten, most in the difference form, which does not pack its operands.  Tile / stream time by sources per row
+// and source box, 8 columns: d = 2 16: 1.5, 62: 1.1, 247: 0.93; d = 3 9: 2.5, 74: 1.03, 247: 0.80; d = 4 15: 2.1, 72: 1.07, 247: 0.86;
+// d = 5 9: 2.7, 156: 1.3, 297: 0.94.  Four columns: d = 2 16: 1.1, 62: 0.68; d = 3 9: 1.8, 74: 0.75; d = 4 15: 1.5, 72: 0.8; d = 5
+// 9: 2.3, 297: 0.73.  Difference form, d = 3, 8 / 4 columns: 7: 6.4 / 5.1, 74: 1.8 / 1.3, 591: 1.3 / 0.88.
+// One dimension stays with the tiles: its lists name three boxes, too short for the stream's set-up (1e6 points, 4 columns 0.85).
+static double stream_seconds(int d, bool narrow, double row) {
+    return narrow ? 6.5e-14 * (d + 8) + 1e-11 / row : 6.1e-14 * (2 * d + 8) + 1.8e-11 / row;
+}
+static double tile_seconds(int d, bool expanded, int cols, double row) {
+    const int RB = cols >= 5 ? 8 : 4;
+    return expanded ? 4.3e-14 * (d + RB) + (7e-12 * d + 2e-12 * (RB - 4)) / row : 6.1e-14 * (1.5 * d + RB) + 1.1e-10 / row;
+}
+
+// seconds per pair for `cols` (2 or more) columns of a list, and whether the stream takes them
+static double column_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int cols, bool &stream) {
+    const int d = pl->d;
     const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
-    if (exp2_poly_degree(D * list_reach(pl, level, csr) * se * se) != 0) return false;
-    double limit = cols >= 5 ? (D == 5 ? 32.0 : D == 4 ? 36.0 : 20.0) : (D == 5 ? 20.0 : 0.0);
-    // uneven trees: f is carried by the few full boxes, most rows are short
-    const Level &lx = pl->tx.levels[level];
-    if (lx.nb < 16 * NUM_SMS_HINT) return false;   // a warp per tile: fewer do not fill the SMs (1024 boxes of 36 points: 4 % slower)
-    if (cols >= 5 && D == 5 && pl->tx.n <= 20 * (int64_t)lx.nb) limit = 48.0;
-    return (double)csr.pairs <= limit * limit * (double)csr.count;
+    const bool narrow = se <= 1.0, expanded = narrow && d * list_reach(pl, level, csr) * se * se <= TMAX_EXPANDED;
+    const double row = (double)csr.pairs / (double)std::max<int64_t>(1, csr.row_boxes);
+    const double st = stream_seconds(d, narrow, row), ti = tile_seconds(d, expanded, cols, row);
+    stream = d >= 2 && st <= ti;
+    return stream ? st : ti;
+}
+
+// Estimated device time of a list that is summed pair by pair (level >= 1); one column measured at 4e12 pairs/s.
+double pair_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R) {
+    double t = 0.0;
+    for (int r0 = 0; r0 < R;) {
+        const int left = R - r0;
+        if (left == 1) { t += (double)csr.pairs / 4e12; break; }
+        bool stream;
+        t += (double)csr.pairs * column_seconds(pl, level, csr, left, stream);
+        r0 += stream || left >= 5 ? 8 : 4;
+    }
+    return t;
 }
 
 template <int D>
@@ -779,10 +799,10 @@ static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *b
     const bool narrow = level > 0 && near_scale(pl->lcs) * pl->tx.levels[level].edge <= 1.0f;   // expanded form of near_cols.cu
     for (int r0 = 0; r0 < R;) {
         const int left = R - r0;
-        if (left >= 2 && columns_on_tensor_cores<D>(pl, level, csr, left)) {
-            column_sums(pl, level, csr, narrow, bs, R, r0, out, rb, re, s);
-            r0 += 8;
-        } else if (left >= 5) { direct_impl<D, 8>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 8; }
+        bool stream = false;
+        if (left >= 2 && level > 0) column_seconds(pl, level, csr, left, stream);
+        if (stream) { column_sums(pl, level, csr, narrow, bs, R, r0, out, rb, re, s); r0 += 8; }
+        else if (left >= 5) { direct_impl<D, 8>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 8; }
         else if (left >= 2) { direct_impl<D, 4>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 4; }
         else { direct_impl<D, 1>(pl, level, csr, bs, R, r0, out, rb, re, s); r0 += 1; }
     }

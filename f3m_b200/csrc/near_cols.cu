@@ -335,7 +335,6 @@ void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, con
         else columns_impl<D_, true>(pl, level, csr, bs, R, r0, out, row_begin, row_end, s);           \
         break;
     switch (pl->d) {
-        F3M_COLS(1)
         F3M_COLS(2)
         F3M_COLS(3)
         F3M_COLS(4)

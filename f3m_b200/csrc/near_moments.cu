@@ -327,12 +327,12 @@ static int list_moment_degree(const f3m_plan *pl, int level, bool keep) {
 }
 
 // Estimated device time of a direct list.  Measured: 3.2e-12 s per (target, box) evaluation of 20 terms + 17 other issue slots, so
-// 8.6e-14 s per slot (two columns share one); 4e12 pairs/s for one column, 0.9e12 to 1.6e12 for two to eight.
+// 8.6e-14 s per slot (two columns share one); pairs see pair_list_seconds.
 double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R) {
     if (csr.count == 0) return 0.0;
     const int K = list_moment_degree(pl, level, &csr == &pl->lists[level].keep);
     if (K) return (double)csr.row_boxes * (mom_count(pl->d, K) * (R == 1 ? 1.0 : 2.0 * ((R + 3) / 4)) + 17.0) * 8.6e-14;
-    return R == 1 ? (double)csr.pairs / 4e12 : (double)csr.pairs * ((R + 7) / 8) / 1.2e12;
+    return pair_list_seconds(pl, level, csr, R);
 }
 
 template <int D, int K, int RB>

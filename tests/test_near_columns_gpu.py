@@ -89,3 +89,58 @@ def test_columns_keep_non_finite_weights(bits, d, n, ls, leaf, dist, cuda):
     assert torch.equal(out[:, 3].isnan(), one.isnan()) and torch.equal(out[:, 3].isinf(), one.isinf())
     others = out[:, [0, 1, 2, 4, 5, 6, 7]]
     assert torch.equal(others, torch.zeros_like(others))
+
+
+def _one_level(n, d, g):
+    """Points whose boxes at level 1 are all neighbours (in the first three dimensions; four offsets of one box would be far)."""
+    X = torch.rand(n, d, generator=g)
+    X[:, 3:] *= 0.4
+    return X
+
+
+# every pair in the boxes of one level, so that the sums are exact: two to nine columns, boxes of one to 600 points, the lists that the
+# costs send to the stream of sources (expanded form up to some fifty sources per box, difference form)
+@pytest.mark.parametrize("d,n,m,R,ls", [(2, 200, 0, 8, 0.6), (2, 63, 30, 3, 0.6), (2, 1537, 900, 8, 0.1), (3, 400, 0, 7, 0.7), (3, 130, 0, 2, 0.7), (3, 5000, 0, 9, 0.05),
+                                        (3, 1200, 900, 4, 0.1), (4, 400, 0, 8, 0.9), (4, 200, 0, 5, 0.2), (5, 500, 0, 8, 1.0), (5, 500, 1999, 6, 0.3),
+                                        (5, 300, 250, 3, 1.0), (3, 12, 11, 2, 0.5), (3, 1700, 0, 8, 0.3)])
+def test_stream_of_sources_against_float64(d, n, m, R, ls, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(d * n + R)
+    X = _one_level(n, d, g).to(cuda)
+    Y = _one_level(m, d, g).to(cuda) if m else None
+    b = (torch.rand(m or n, R, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, Y, engine.make_params(ls, 5.0, 2 ** d, False, 0.15, 10 ** 6))
+    out = plan.apply(b)
+    assert plan.last_work()["column_launches"] > 0
+    assert plan.stats()["direct_pairs"] == n * (m or n) == plan.last_work()["pairs"]
+    exact = engine.rbf_dense(X.double(), (X if Y is None else Y).double(), b.double(), ls)
+    one = torch.cat([plan.apply(b[:, r:r + 1].contiguous()) for r in range(R)], 1)
+    e_one, e_all = rel_l2(one.cpu(), exact.cpu()), rel_l2(out.cpu(), exact.cpu())
+    print(f"columns {e_all:.2e}, one by one {e_one:.2e}")
+    assert e_all <= 5e-6 and e_all <= 1.2 * e_one + 2e-7, (e_all, e_one)    # bounds of test_columns_against_float64
+
+
+@pytest.mark.parametrize("value", [8e37, 2.0 ** -120])
+def test_stream_of_sources_at_the_ends_of_the_exponent_range(value, cuda):
+    """Neither a huge value nor a tiny one loses digits on its way through the columns (the expanded form holds terms of up to
+    2^(d/4) times a value)."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(19)
+    X = _one_level(400, 5, g).to(cuda)
+    b = torch.zeros(400, 8, device=cuda)
+    b[77, 5] = value * (1.0 if value > 1 else 1.2345678)
+    plan = engine.Plan(X, None, engine.make_params(1.0, 5.0, 32, False, 0.15, 10 ** 6))
+    out = plan.apply(b)
+    assert plan.last_work()["column_launches"] > 0 and plan.stats()["far_box_pairs"] == 0
+    exact = engine.rbf_dense(X.double(), X.double(), b.double(), 1.0)
+    assert ((out[:, 5].double() - exact[:, 5]).abs() <= 2e-6 * exact[:, 5]).all()
+
+
+def test_long_boxes_stay_with_the_tiles(cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(20)
+    for d, R, ls in ((3, 8, 1.0), (3, 3, 1.0), (1, 8, 0.01)):
+        X = torch.rand(4000, d, generator=g).to(cuda)
+        plan = engine.Plan(X, None, engine.make_params(ls, 5.0, 2 ** d, False, 0.15, 10 ** 6, flags=2))
+        plan.apply(torch.rand(4000, R, device=cuda))
+        assert plan.last_work()["column_launches"] == 0 and plan.last_work()["pairs"] == 4000 ** 2
