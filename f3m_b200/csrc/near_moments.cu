@@ -305,9 +305,20 @@ static double list_exponent_bound(const f3m_plan *pl, int level, bool keep) {
     return 1.01 * bound * e * e * 2.0 * (double)pl->lcs;   // 1 / l^2 = 2 lcs; 1 % for the rounding of centres and far test
 }
 
+// Estimated device time of a list's moments: evaluations, and what every block of columns pays once.  Measured: one column 3.2e-12 s per
+// (target, box) of 20 terms + 17 other issue slots, so 8.6e-14 s per slot; a block of four columns, whose records come through
+// L1, 1.2e-11 s at 10 terms, 2.1e-11 at 35, 3.2e-11 at 84.  A block builds the records of all boxes and looks up every row.
+struct MomentSeconds { double eval, fixed; };
+static MomentSeconds moment_seconds(const f3m_plan *pl, const PairCSR &csr, int K, int R) {
+    const double nm = mom_count(pl->d, K), build = (double)pl->ty->n * (nm + 20.0) * 8.6e-14, rows = (double)pl->tx.n * 1e-11;
+    const int fours = R % 4 == 1 ? R / 4 : (R + 3) / 4, ones = R % 4 == 1;
+    return {(double)csr.row_boxes * (fours * (8e-12 + 3.5e-13 * nm) + ones * (nm + 17.0) * 8.6e-14),
+            fours * (4.0 * build + rows) + ones * (build + rows)};
+}
+
 // Degree for one list, 0 when its pairs are summed one by one.  The Chebyshev interpolation error is at most
 // e^h h^(K+1) / (2^K (K+1)!), and exp(t) >= e^-h.
-static int list_moment_degree(const f3m_plan *pl, int level, bool keep) {
+static int list_moment_degree(const f3m_plan *pl, int level, bool keep, int R) {
     const PairCSR &csr = keep ? pl->lists[level].keep : pl->lists[level].small;
     const bool flag = pl->prm.flags & F3M_FLAG_NEAR_MOMENTS;
     if (level < 1 || csr.count == 0) return 0;
@@ -317,22 +328,28 @@ static int list_moment_degree(const f3m_plan *pl, int level, bool keep) {
     for (int K = 2; K <= mom_kmax(pl->d); K++) {
         term *= h / K;
         if (exp(2.0 * h) * term * h / (K + 1) * ldexp(1.0, -K) <= eps) {
-            // One (target, box) evaluation of 20 terms measured 3.2e11 /s, the pair form 5.2e12 pairs/s (3.5e12 without
-            // polynomial pairs): about one term per 0.5 to 0.8 pairs.  Lists whose boxes hold fewer sources on average, weighted
-            // by targets, stay with the pairs.
-            return flag || (double)csr.pairs >= 0.5 * mom_count(pl->d, K) * (double)csr.row_boxes ? K : 0;
+            if (flag) return K;
+            // Moments where they take less time than the pairs.  Either form also launches a few kernels per block of columns, 10 us
+            // for tiles, scan, packing and sums.  One column: an evaluation of 20 terms at 3.2e11 /s against pairs at 5.2e12 /s (3.5e12
+            // without polynomial pairs) is about one term per 0.5 to 0.8 pairs.  Two columns and more, eight columns measured,
+            // moments / pairs: d = 1, 1e6 normal points, lists of a few pairs on eight levels 0.72 / 0.56 ms; d = 3, l = 0.3, 1e6 normal
+            // points, boxes of twelve 10.1 / 4.3 ms; d = 2, 1e6 uniform points 0.25 / 0.59 ms.
+            const MomentSeconds t = moment_seconds(pl, csr, K, R);
+            const double pairs = pair_list_seconds(pl, level, csr, R) + 1e-5 * ((R + 7) / 8);
+            if (R == 1) return (double)csr.pairs >= 0.5 * mom_count(pl->d, K) * (double)csr.row_boxes && t.fixed <= pairs ? K : 0;
+            return t.eval + t.fixed <= pairs ? K : 0;
         }
     }
     return 0;
 }
 
-// Estimated device time of a direct list.  Measured: 3.2e-12 s per (target, box) evaluation of 20 terms + 17 other issue slots, so
-// 8.6e-14 s per slot (two columns share one); pairs see pair_list_seconds.
+// Estimated device time of a direct list.
 double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R) {
     if (csr.count == 0) return 0.0;
-    const int K = list_moment_degree(pl, level, &csr == &pl->lists[level].keep);
-    if (K) return (double)csr.row_boxes * (mom_count(pl->d, K) * (R == 1 ? 1.0 : 2.0 * ((R + 3) / 4)) + 17.0) * 8.6e-14;
-    return pair_list_seconds(pl, level, csr, R);
+    const int K = list_moment_degree(pl, level, &csr == &pl->lists[level].keep, R);
+    if (!K) return pair_list_seconds(pl, level, csr, R);
+    const MomentSeconds t = moment_seconds(pl, csr, K, R);
+    return t.eval + t.fixed;
 }
 
 template <int D, int K, int RB>
@@ -406,12 +423,12 @@ bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, i
     if (level < 1) return false;
     LevelLists &ll = pl->lists[level];
     const bool keep = &csr == &ll.keep;
-    int K = list_moment_degree(pl, level, keep);
+    int K = list_moment_degree(pl, level, keep, R);
     if (K == 0) return false;
     double h = list_exponent_bound(pl, level, keep);
     const PairCSR *other = nullptr;
     if (level == pl->levels) {
-        const int Ko = list_moment_degree(pl, level, !keep);
+        const int Ko = list_moment_degree(pl, level, !keep, R);
         if (Ko) {
             if (!keep) return true;   // summed with the near list
             other = &ll.small;

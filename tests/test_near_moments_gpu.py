@@ -78,3 +78,20 @@ def test_moments_of_a_slice_and_short_boxes(cuda):
     (a, p), forms, plan = _both(X, None, b, 6.0, 20.0, 32, cuda)
     assert forms["moments"] == 0 and forms["poly2"] + forms["poly3"] > 0, forms
     assert rel_l2(a, p) <= TOL
+
+
+def test_moments_only_where_they_take_less_time(cuda):
+    """Lists of a few pairs on upper levels and short boxes with several columns stay with the pairs; long boxes take moments whatever the
+    number of columns."""
+    from f3m_b200 import engine
+    g = torch.Generator(device=cuda).manual_seed(5)
+    for d, n, ls, leaf, R, most in ((1, 1000000, 0.3, 200.0, 8, 2), (1, 1000000, 0.3, 200.0, 1, 7), (3, 1000000, 0.3, 200.0, 8, 0), (3, 1000000, 0.3, 200.0, 4, 0)):
+        X = torch.randn(n, d, device=cuda, generator=g)
+        plan = engine.Plan(X, None, engine.make_params(ls, leaf, 3 ** d, False, 0.15, 3 ** d))
+        plan.apply(torch.randn(n, R, device=cuda, generator=g), row_range=(0, n - 1))
+        assert plan.direct_variants()["moments"] <= most, (d, R, plan.direct_variants())
+    X = torch.rand(300000, 2, device=cuda, generator=g)
+    plan = engine.Plan(X, None, engine.make_params(1.0, 200.0, 9, False, 0.15, 9))
+    for R in (1, 4, 8):
+        plan.apply(torch.randn(300000, R, device=cuda, generator=g), row_range=(0, 299999))
+        assert plan.direct_variants()["moments"] > 0 and plan.last_work()["pairs"] == 0
