@@ -119,7 +119,7 @@ __device__ __forceinline__ float mom_ex2(float x) {
 // very long boxes, whose parts are added atomically into zeroed records.
 template <int D, int K, int RB, int T>
 __global__ void __launch_bounds__(256) near_moments_build(const float *__restrict__ pts, int n, const float *__restrict__ bs, int R,
-                                                         int r0, float s2, const int *__restrict__ off_y, int nby,
+                                                         int r0, float unit, float s2, const int *__restrict__ off_y, int nby,
                                                          const float *__restrict__ ctr_y, const unsigned char *__restrict__ need,
                                                          MomFactors fac, int nsplit, float *rec) {
     constexpr int NM = mom_count(D, K), REC = mom_record(D, K, RB);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
             float y[D], n2 = 0.f;
 #pragma unroll
             for (int k = 0; k < D; k++) {
-                const float v = pts[(size_t)k * n + j] - c[k];
+                const float v = unit * (pts[(size_t)k * n + j] - c[k]);
                 n2 = fmaf(v, v, n2);
                 y[k] = 2.f * s2 * v;
             }
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
             put(q, v);
         }
     }
-    if (r == 0 && blockIdx.y == 0 && (int)(threadIdx.x % T) < D) dst[threadIdx.x % T] = ctr_y[by * D + threadIdx.x % T];
+    if (r == 0 && blockIdx.y == 0 && (int)(threadIdx.x % T) < D) dst[threadIdx.x % T] = unit * ctr_y[by * D + threadIdx.x % T];
 }
 
 // One thread per target row.  Rows are in box order, so the lanes of a warp read the same record (a broadcast) except
@@ -186,8 +186,8 @@ template <int D, int K, int RB, int G>
 __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x, int nbx,
                                                         int row_begin, int row_end, const int *__restrict__ ptr1,
                                                         const int *__restrict__ idx1, const int *__restrict__ ptr2,
-                                                        const int *__restrict__ idx2, const float *__restrict__ rec, float s2, int R,
-                                                        int r0, float *out) {
+                                                        const int *__restrict__ idx2, const float *__restrict__ rec, float unit, float s2,
+                                                        int R, int r0, float *out) {
     constexpr int REC = mom_record(D, K, RB);
     const int lane = threadIdx.x & 31, sub = lane % G;
     const int i0 = row_begin + (int)((blockIdx.x * 128 + (threadIdx.x & ~31)) / G);
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict
     box = b_lo + (b_hi > b_lo ? box_of_row(off_x + b_lo, b_hi - b_lo + 1, i) : 0);
     float x[D], tot[RB];
 #pragma unroll
-    for (int k = 0; k < D; k++) x[k] = xpts[(size_t)k * n_x + i];
+    for (int k = 0; k < D; k++) x[k] = unit * xpts[(size_t)k * n_x + i];
 #pragma unroll
     for (int r = 0; r < RB; r++) tot[r] = 0.f;
     bool any = false;
@@ -357,12 +357,17 @@ static void moment_impl(f3m_plan *pl, int level, const PairCSR *l1, const PairCS
                         int rb, int re, cudaStream_t s) {
     Tree &tx = pl->tx, &ty = *pl->ty;
     Level &lx = tx.levels[level], &ly = ty.levels[level];
-    const float s2 = (float)((double)pl->lcs * 1.4426950408889634);   // exp(-lcs v) = 2^(-s2 v)
+    // exp(-lcs v) = 2^(-s2 v).  Lengths are taken in a power of two near 1 / sqrt(s2), which rounds nothing, so that powers of
+    // them up to the sixth neither overflow nor vanish whatever the caller's unit.
+    const double s2_input = (double)pl->lcs * 1.4426950408889634;
+    int ex;
+    frexp(sqrt(s2_input), &ex);
+    const float unit = (float)ldexp(1.0, ex), s2 = (float)ldexp(s2_input, -2 * ex);
     double cf[MOM_KMAX + 1];
     exp_poly_fit(h, K, cf);
     const double ln2 = 0.6931471805599453;
     double pw = 1.0;
-    for (int k = 0; k <= K; k++) { cf[k] *= pw; pw *= ln2; }          // the records hold y 2 s2 = y / (l^2 ln 2)
+    for (int k = 0; k <= K; k++) { cf[k] *= pw; pw *= ln2; }          // the records hold y 2 s2 = y / (l^2 ln 2) (l, y in that unit)
     MomFactors fac{};
     MomTree<D, K, 0, 0, 0>::factors(cf, 1.0, 0, fac.f);
     const int nsplit = std::max(1, std::min(64, (ly.max_count + 16383) / 16384));
@@ -376,14 +381,14 @@ static void moment_impl(f3m_plan *pl, int level, const PairCSR *l1, const PairCS
     // a CTA per box; 512 boxes of 195 points, K = 3: 5.5 -> 6.8 us)
     if (ly.max_count <= 1024 && (groups >= 2 * NUM_SMS_HINT || ly.max_count <= 64))
         near_moments_build<D, K, RB, 32><<<dim3((unsigned)((groups + 7) / 8), 1), 256, 0, s>>>(
-            ty.pts.p, (int)ty.n, bs, R, r0, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, 1, rec.p);
+            ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, 1, rec.p);
     else
         near_moments_build<D, K, RB, 256><<<dim3((unsigned)groups, nsplit), 256, 0, s>>>(
-            ty.pts.p, (int)ty.n, bs, R, r0, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, nsplit, rec.p);
+            ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, nsplit, rec.p);
     F3M_LAUNCH_CHECK();
     auto eval = [&](auto kernel, int G) {
         kernel<<<(unsigned)(((int64_t)(re - rb) * G + 127) / 128), 128, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, rb, re, l1->ptr.p, l1->idx.p,
-                                                                               l2 ? l2->ptr.p : nullptr, l2 ? l2->idx.p : nullptr, rec.p, s2, R,
+                                                                               l2 ? l2->ptr.p : nullptr, l2 ? l2->idx.p : nullptr, rec.p, unit, s2, R,
                                                                                r0, out);
     };
     if ((int64_t)(re - rb) >= 256 * NUM_SMS_HINT) eval(near_moments_eval<D, K, RB, 1>, 1);

@@ -95,3 +95,17 @@ def test_moments_only_where_they_take_less_time(cuda):
     for R in (1, 4, 8):
         plan.apply(torch.randn(300000, R, device=cuda, generator=g), row_range=(0, 299999))
         assert plan.direct_variants()["moments"] > 0 and plan.last_work()["pairs"] == 0
+
+
+@pytest.mark.parametrize("ls", [0.42, 0.9, 4.0])
+@pytest.mark.parametrize("exponent", [-30, 30])
+def test_moments_do_not_depend_on_the_unit_of_length(ls, exponent, cuda):
+    """Points and lengthscale in another unit (a power of two, so that every rounding is the same)."""
+    g = torch.Generator().manual_seed(17)
+    X = torch.rand(30011, 3, generator=g)
+    b = _weights(30011, 1, g)
+    unit = 2.0 ** exponent
+    (a, _), forms, _ = _both(X, None, b, ls, 300.0, 64, cuda)
+    (c, p), scaled, _ = _both(X * unit, None, b, ls * unit, 300.0, 64, cuda)
+    assert forms == scaled and forms["moments"] > 0, (forms, scaled)
+    assert rel_l2(c, p) <= TOL and rel_l2(c, a) <= 1e-7
