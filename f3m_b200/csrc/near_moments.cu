@@ -158,20 +158,26 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
         if (nsplit == 1) *p = v * fac.f[q];
         else atomicAdd(p, v * fac.f[q]);
     };
+    // Where the sum of the weights is not finite, it alone stays: the pairs' terms are positive, so their sum is that value too, while
+    // the other moments would carry it with either sign.
     if (T == 32) {
+        const bool bad = !isfinite(acc[0]);
 #pragma unroll
         for (int q = 0; q < NM; q++)
-            if (lane == (q & 31)) put(q, acc[q]);
+            if (lane == (q & 31)) put(q, q && bad ? 0.f : acc[q]);
     } else {
 #pragma unroll
         for (int q = 0; q < NM; q++)
             if (lane == (q & 31)) part[T == 32 ? 0 : warp][q] = acc[q];
         __syncthreads();
         for (int q = threadIdx.x; q < NM; q += T) {
-            float v = 0.f;
+            float v = 0.f, v0 = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; w++) v += part[T == 32 ? 0 : w][q];
-            put(q, v);
+            for (int w = 0; w < 8; w++) {
+                v += part[T == 32 ? 0 : w][q];
+                v0 += part[T == 32 ? 0 : w][0];
+            }
+            put(q, q && !isfinite(v0) ? 0.f : v);
         }
     }
     if (r == 0 && blockIdx.y == 0 && (int)(threadIdx.x % T) < D) dst[threadIdx.x % T] = unit * ctr_y[by * D + threadIdx.x % T];

@@ -109,3 +109,21 @@ def test_moments_do_not_depend_on_the_unit_of_length(ls, exponent, cuda):
     (c, p), scaled, _ = _both(X * unit, None, b, ls * unit, 300.0, 64, cuda)
     assert forms == scaled and forms["moments"] > 0, (forms, scaled)
     assert rel_l2(c, p) <= TOL and rel_l2(c, a) <= 1e-7
+
+
+def test_moments_of_an_infinite_weight(cuda):
+    """Every pair is summed directly and every term of the kernel is positive: the sums over an infinite weight are infinite, those
+    over a NaN are NaN, and the other columns do not notice."""
+    g = torch.Generator().manual_seed(18)
+    X = torch.rand(3000, 3, generator=g)
+    for R in (1, 3):
+        b = _weights(3000, R, g)
+        ref, forms, plan = _both(X, None, b, 1.6, 1000.0, 27, cuda)
+        assert forms["moments"] > 0 and plan.stats()["far_box_pairs"] == 0
+        for bad in (float("inf"), float("-inf"), float("nan")):
+            c = b.clone()
+            c[1234, R - 1] = bad
+            (a, p), _, _ = _both(X, None, c, 1.6, 1000.0, 27, cuda)
+            want = torch.full((3000,), bad)
+            assert torch.equal(torch.nan_to_num(a[:, -1], 7.0), torch.nan_to_num(want, 7.0))
+            assert torch.equal(a[:, :-1], ref[0][:, :-1])
