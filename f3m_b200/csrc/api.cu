@@ -773,7 +773,8 @@ size_t f3m_workspace_bytes(int64_t N, int64_t M, int32_t R, int32_t d, const f3m
     const double boxes = std::max(1.0, pts * pow(2.0, d) / std::max(1.0f, prm->min_points));
     const double sort_peak = pts * (12.0 + 4.0 * d + 8.0 + 8.0 * RW);                       // keys, records (twice), planes
     const double tree = pts * (8.0 + 4.0 * d) + boxes * (pow(6.0, d) + 2.0 * pow(3.0, d)) * 12.0 + 64.0 * boxes;
-    const double product = 4.0 * R * (n + m) + 4.0 * W * (m + boxes) + 2.3 * boxes * P * RB * 4.0 + 8.0 * boxes;
+    const double parts = std::min(m / 128.0, 32.0 * NUM_SMS_HINT + m / 4096.0) * P * RB * 4.0;   // sums over parts of long boxes (p2m_level)
+    const double product = 4.0 * R * (n + m) + 4.0 * W * (m + boxes) + 2.3 * boxes * P * RB * 4.0 + 8.0 * boxes + parts;
     return (size_t)(1.15 * std::max(sort_peak + pts * (8.0 + 4.0 * d), tree + product)) + ((size_t)64 << 20);
 }
 

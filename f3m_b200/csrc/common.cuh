@@ -127,6 +127,52 @@ __device__ __forceinline__ int box_of_row(const int *__restrict__ off, int nb, i
     return lo;
 }
 
+// The same by a whole warp, every lane of it with the same i: 32 probes a round
+__device__ __forceinline__ int box_of_row_warp(const int *__restrict__ off, int nb, int i) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = nb;   // the box lies in [lo, hi)
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5, probe = lo + (lane + 1) * step;
+        const int below = __popc(__ballot_sync(0xffffffffu, probe < hi && off[probe] <= i));
+        lo += below * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// Sums over long boxes (more than `chunk` rows) are cut where a multiple of chunk rows falls, and the parts' sums are added in
+// the order of the rows: results do not depend on which part ends first.  Chunk k has two slots: (k, 0) belongs to a long box
+// that holds the chunk's first row, (k, 1) to one that starts behind it and goes on in the next chunk.  Every part of every long box
+// has a slot of its own, and 2 * chunks of them are enough whatever the boxes hold.
+__host__ __device__ inline int64_t part_slots(int64_t n, int chunk) { return 2 * ((n + chunk - 1) / chunk); }
+struct BoxPart { int box, begin, end; };
+// rows of a slot, begin == end when it has no part (all lanes of the warp call it with the same slot)
+__device__ __forceinline__ BoxPart part_of_slot(const int *__restrict__ off, int nb, int n, int chunk, int64_t slot) {
+    const int64_t first = (slot >> 1) * chunk, probe = first + (slot & 1) * chunk;
+    BoxPart p{0, 0, 0};
+    if (probe >= n) return p;
+    p.box = box_of_row_warp(off, nb, (int)probe);
+    const int a = off[p.box], e = off[p.box + 1];
+    if (e - a <= chunk || ((slot & 1) && a <= first)) return p;
+    p.begin = (int)(a > first ? a : first);
+    p.end = (int)(e < first + chunk ? e : first + chunk);
+    return p;
+}
+// the long box that starts in chunk k and its slots [s0, then 2 (k + 1), 2 (k + 2), .. last]; box < 0: none
+struct LongBox { int box; int64_t first_slot, last_slot; };
+__device__ __forceinline__ LongBox long_box_of_chunk(const int *__restrict__ off, int nb, int n, int chunk, int64_t k) {
+    LongBox l{-1, 0, 0};
+    const int64_t next = (k + 1) * chunk;
+    if (next > n) return l;                       // it would have to go on in the next chunk
+    const int box = box_of_row_warp(off, nb, (int)(next - 1));
+    const int a = off[box], e = off[box + 1];
+    if (a < k * chunk || e - a <= chunk) return l;
+    l.box = box;
+    l.first_slot = 2 * k + (a > k * chunk);
+    l.last_slot = 2 * ((int64_t)(e - 1) / chunk);
+    return l;
+}
+
 // chebyshev_nodes_1D / get_w_j_first_kind (F3M_src/n_tree.cu:265-285): first-kind Chebyshev nodes and barycentric
 // weights with the reference's float32 expression (PI as a float, arguments rounded to float before cos / sin).
 inline void cheb_nodes_weights(int p, float *node, float *w) {

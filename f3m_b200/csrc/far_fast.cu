@@ -919,6 +919,27 @@ __device__ __forceinline__ void lagrange_pp(float t, const NodeTab2 &nt, float *
     }
 }
 
+// What a CTA of the P2M kernels sums: the first nlist take a box each (all its rows, unless the box is long), the others a slot of
+// the long boxes' parts.  Boxes that start outside [src_begin, src_end) belong to another slice of the sorted sources.
+struct LeafWork { int box, s0, s1; int64_t slot; };
+__device__ __forceinline__ LeafWork leaf_work(const int *__restrict__ off, int nb, int n, const int *__restrict__ box_list, int nlist, int chunk,
+                                              int src_begin, int src_end) {
+    LeafWork w{0, 0, 0, -1};
+    if ((int)blockIdx.x < nlist) {
+        w.box = box_list ? box_list[blockIdx.x] : (int)blockIdx.x;
+        w.s0 = off[w.box];
+        w.s1 = off[w.box + 1];
+        if (chunk && w.s1 - w.s0 > chunk) w.s1 = w.s0;
+    } else {
+        w.slot = blockIdx.x - nlist;
+        const BoxPart p = part_of_slot(off, nb, n, chunk, w.slot);
+        w.box = p.box; w.s0 = p.begin; w.s1 = p.end;
+    }
+    const int a = off[w.box];
+    if (a < src_begin || a >= src_end) w.s1 = w.s0;
+    return w;
+}
+
 // P2M.  A thread owns one combination (m_1 .. m_{d-1}) of the slower node indices and all p values of
 // the fastest one: per point it forms w = b * prod_{k>=1} L_k[m_k] once and adds w * L_0[i] to p
 // accumulators, so a (point, node) pair costs about one shared-memory read and one multiply-add.
@@ -926,18 +947,15 @@ __device__ __forceinline__ void lagrange_pp(float t, const NodeTab2 &nt, float *
 template <int PP, int RB>
 __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, int n, int d, const float *__restrict__ bs, int R,
                                                int r0, const int *__restrict__ off, const float *__restrict__ ctr,
-                                               float factor, NodeTab2 nt, int P, int nsplit, int src_begin, int src_end,
-                                               float *mom) {
+                                               float factor, NodeTab2 nt, int P, int nb, int chunk, int src_begin, int src_end,
+                                               float *mom, float *part) {
     extern __shared__ __align__(16) float sm[];
     constexpr int TP = 128, NTH = 256, LS = TP + 1;
     float *Ls = sm;                                   // [d*PP][TP+1]
     float *bsm = Ls + (size_t)d * PP * LS;            // [TP][RB]
     float *accsm = bsm + (size_t)TP * RB;             // [P][RB]
-    const int box = blockIdx.x;
-    const int a = off[box], b = off[box + 1];
-    if (a < src_begin || a >= src_end) return;      // only the boxes of this slice of the sorted sources
-    const int len = b - a;
-    const int s0 = a + (int)(((long long)len * blockIdx.y) / nsplit), s1 = a + (int)(((long long)len * (blockIdx.y + 1)) / nsplit);
+    const LeafWork lw = leaf_work(off, nb, n, nullptr, nb, chunk, src_begin, src_end);
+    const int box = lw.box, s0 = lw.s0, s1 = lw.s1;
     if (s0 >= s1) return;
     const int PR = P * RB, C = P / PP;
     // the PP x RB block of one combination starts an odd number of floats after the previous one: the lanes of a
@@ -1000,10 +1018,21 @@ __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, i
         }
     }
     __syncthreads();
-    float *dst = mom + (size_t)box * PR;
+    float *dst = lw.slot < 0 ? mom + (size_t)box * PR : part + lw.slot * PR;
     constexpr int BLK = PP * RB;
-    if (nsplit == 1) for (int q = threadIdx.x; q < PR; q += NTH) dst[q] = accsm[q + (q / BLK) * (CS - BLK)];
-    else for (int q = threadIdx.x; q < PR; q += NTH) atomicAdd(dst + q, accsm[q + (q / BLK) * (CS - BLK)]);
+    for (int q = threadIdx.x; q < PR; q += NTH) dst[q] = accsm[q + (q / BLK) * (CS - BLK)];
+}
+
+// moments of the long boxes: the sums of their parts, in the order of the rows
+__global__ void __launch_bounds__(128) p2m_combine(const int *__restrict__ off, int nb, int n, int chunk, int PR, int src_begin, int src_end,
+                                                  const float *__restrict__ part, float *mom) {
+    const LongBox l = long_box_of_chunk(off, nb, n, chunk, blockIdx.x);
+    if (l.box < 0 || off[l.box] < src_begin || off[l.box] >= src_end) return;
+    for (int q = threadIdx.x; q < PR; q += 128) {
+        float v = part[l.first_slot * PR + q];
+        for (int64_t t = (l.first_slot | 1) + 1; t <= l.last_slot; t += 2) v += part[t * PR + q];
+        mom[(size_t)l.box * PR + q] = v;
+    }
 }
 
 template <int PP, int RB>
@@ -1107,29 +1136,27 @@ __device__ __forceinline__ void leaf3_rows_xyz(const float (&x)[3], const float 
 template <int PP>
 __global__ void __launch_bounds__(128) p2m_leaf3(const float *__restrict__ pts, int n, const float *__restrict__ bs, int R, int r0,
                                                 const int *__restrict__ off, const float *__restrict__ ctr, float factor,
-                                                NodeTab2 nt, int nsplit, int src_begin, int src_end, float *mom,
-                                                const int *__restrict__ box_list) {
+                                                NodeTab2 nt, int nb, int chunk, int src_begin, int src_end, float *mom, float *part,
+                                                const int *__restrict__ box_list, int nlist) {
     using G = Leaf3<PP>;
     constexpr int P = PP * PP * PP;
     // the Lagrange rows of a chunk; after the last chunk the same memory holds one partial moment array per stream
     constexpr int NSCR = (G::TP * L3_RS > G::NSTREAM * P) ? G::TP * L3_RS : G::NSTREAM * P;
     __shared__ __align__(16) float rows[NSCR];
-    const int box = box_list ? box_list[blockIdx.x] : (int)blockIdx.x;
-    const int a = off[box], b = off[box + 1];
-    if (a < src_begin || a >= src_end) return;      // only the boxes of this slice of the sorted sources
-    const int len = b - a;
-    const int s0 = a + (int)(((long long)len * blockIdx.y) / nsplit), s1 = a + (int)(((long long)len * (blockIdx.y + 1)) / nsplit);
+    const LeafWork lw = leaf_work(off, nb, n, box_list, nlist, chunk, src_begin, src_end);
+    const int box = lw.box, s0 = lw.s0, s1 = lw.s1;
     if (s0 >= s1) return;
     const float c[3] = {ctr[box * 3], ctr[box * 3 + 1], ctr[box * 3 + 2]};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / PP, m2 = lane - sub * PP;
     const bool active = sub < G::SUB;
     const int stream = warp * G::SUB + sub;
-    float acc[PP][PP];
+    // Running sums grow inaccurate with the square root of their length: after some fifty terms per stream (BLOCK points) they are
+    // added up over the streams and kept by the threads that write the moments.
+    constexpr int BLOCK = 1024 / G::TP * G::TP;
+    float tot[(P + 127) / 128];
 #pragma unroll
-    for (int i = 0; i < PP; i++)
-#pragma unroll
-        for (int j = 0; j < PP; j++) acc[i][j] = 0.f;
+    for (int t = 0; t < (P + 127) / 128; t++) tot[t] = 0.f;
     // the point of the next chunk is fetched while the streams consume the current one
     float px[3] = {0.f, 0.f, 0.f}, pb = 0.f;
     auto fetch = [&](int base) {
@@ -1140,46 +1167,59 @@ __global__ void __launch_bounds__(128) p2m_leaf3(const float *__restrict__ pts, 
         }
     };
     fetch(s0);
-    for (int base = s0; base < s1; base += G::TP) {
-        const int cnt = min(G::TP, s1 - base);
-        __syncthreads();
-        if ((int)threadIdx.x < cnt)   // the column value rides on the L2 row
-            leaf3_rows_xyz<PP>(px, c, factor, nt, pb, rows + threadIdx.x * L3_RS);
-        fetch(base + G::TP);
-        __syncthreads();
-        if (active)
-            for (int j = stream; j < cnt; j += G::NSTREAM) {
-                const float *row = rows + j * L3_RS;
-                const float4 a0 = *reinterpret_cast<const float4 *>(row), a1 = *reinterpret_cast<const float4 *>(row + 4);
-                const float4 b0 = *reinterpret_cast<const float4 *>(row + 8), b1 = *reinterpret_cast<const float4 *>(row + 12);
-                const float l0[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const float l1[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                const float w2 = row[16 + m2];
+    for (int block = s0; block < s1; block += BLOCK) {
+        float acc[PP][PP];
 #pragma unroll
-                for (int i1 = 0; i1 < PP; i1++) {
-                    const float u = w2 * l1[i1];
+        for (int i = 0; i < PP; i++)
 #pragma unroll
-                    for (int i0 = 0; i0 < PP; i0++) acc[i1][i0] = fmaf(u, l0[i0], acc[i1][i0]);
+            for (int j = 0; j < PP; j++) acc[i][j] = 0.f;
+        for (int base = block; base < min(block + BLOCK, s1); base += G::TP) {
+            const int cnt = min(G::TP, s1 - base);
+            __syncthreads();
+            if ((int)threadIdx.x < cnt)   // the column value rides on the L2 row
+                leaf3_rows_xyz<PP>(px, c, factor, nt, pb, rows + threadIdx.x * L3_RS);
+            fetch(base + G::TP);
+            __syncthreads();
+            if (active)
+                for (int j = stream; j < cnt; j += G::NSTREAM) {
+                    const float *row = rows + j * L3_RS;
+                    const float4 a0 = *reinterpret_cast<const float4 *>(row), a1 = *reinterpret_cast<const float4 *>(row + 4);
+                    const float4 b0 = *reinterpret_cast<const float4 *>(row + 8), b1 = *reinterpret_cast<const float4 *>(row + 12);
+                    const float l0[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                    const float l1[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                    const float w2 = row[16 + m2];
+#pragma unroll
+                    for (int i1 = 0; i1 < PP; i1++) {
+                        const float u = w2 * l1[i1];
+#pragma unroll
+                        for (int i0 = 0; i0 < PP; i0++) acc[i1][i0] = fmaf(u, l0[i0], acc[i1][i0]);
+                    }
                 }
+        }
+        __syncthreads();
+        if (active) {
+            float *mine = rows + stream * P + PP * PP * m2;
+#pragma unroll
+            for (int i1 = 0; i1 < PP; i1++)
+#pragma unroll
+                for (int i0 = 0; i0 < PP; i0++) mine[i0 + PP * i1] = acc[i1][i0];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < (P + 127) / 128; t++) {
+            const int q = threadIdx.x + 128 * t;
+            float v = 0.f;
+            if (q < P) {
+#pragma unroll
+                for (int st = 0; st < G::NSTREAM; st++) v += rows[st * P + q];
             }
+            tot[t] += v;
+        }
     }
-    __syncthreads();
-    if (active) {
-        float *mine = rows + stream * P + PP * PP * m2;
+    float *dst = lw.slot < 0 ? mom + (size_t)box * P : part + lw.slot * P;
 #pragma unroll
-        for (int i1 = 0; i1 < PP; i1++)
-#pragma unroll
-            for (int i0 = 0; i0 < PP; i0++) mine[i0 + PP * i1] = acc[i1][i0];
-    }
-    __syncthreads();
-    float *dst = mom + (size_t)box * P;
-    for (int q = threadIdx.x; q < P; q += 128) {
-        float v = 0.f;
-#pragma unroll
-        for (int st = 0; st < G::NSTREAM; st++) v += rows[st * P + q];
-        if (nsplit == 1) dst[q] = v;
-        else atomicAdd(dst + q, v);
-    }
+    for (int t = 0; t < (P + 127) / 128; t++)
+        if ((int)threadIdx.x + 128 * t < P) dst[threadIdx.x + 128 * t] = tot[t];
 }
 
 template <int PP>
@@ -1350,25 +1390,55 @@ static void ensure_leaf_split(f3m_plan *pl, int which, int level, cudaStream_t s
 // ---------------------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------------------
-// Parts the boxes of a level are cut into (every box into the same number): `part` points in the longest box.  Levels of
-// uneven occupancy would launch a part for each of a million short boxes because one is long: the number of CTAs is held to the
-// boxes plus four times the parts that an even level would have, but parts never grow beyond what 64 parts of 8192 points give.
-// The parts are the second dimension of a grid: at most 65535.
-static int box_parts(int max_count, int64_t n, int nb, int64_t part) {
+// Parts the target boxes of a level are cut into (every box into the same number): at most 8192 points in the longest box, and short
+// enough that the parts of all boxes fill the SMs four times over (a cut at level 1 or 2 leaves 8 or 64 boxes), but not below
+// 512 points.  Levels of uneven occupancy would launch a part for each of a million short boxes because one is long: the number of CTAs
+// is held to the boxes plus four times the parts that an even level would have, but parts never grow beyond what 64 parts of
+// 8192 points give.  The parts are the second dimension of a grid: at most 65535.
+static int target_parts(int max_count, int64_t n, int nb) {
+    const int64_t part = std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT)));
     const int64_t want = (max_count + part - 1) / part, even = 1 + 4 * n / (part * nb), at_least = std::min(64, (max_count + 8191) / 8192);
     return (int)std::min<int64_t>(65535, std::max<int64_t>(1, std::max<int64_t>(at_least, std::min<int64_t>(want, even))));
 }
-// Target boxes: at most 8192 points, and short enough that the parts of all boxes fill the SMs four times over (a cut at
-// level 1 or 2 leaves 8 or 64 boxes), but not below 512 points.
-static int target_parts(int max_count, int64_t n, int nb) {
-    return box_parts(max_count, n, nb, std::max<int64_t>(512, std::min<int64_t>(8192, n / (4 * NUM_SMS_HINT))));
+// Rows from which a source box is summed in parts; 0: no box of the level is that long.  A CTA works through its rows one chunk of
+// 128 after the other, so a box that is much longer than the SMs' even share ends last.  Whole calls in us, parts per SM 4 / 8 / 12:
+// two trees in 2-D, 60 007 sources, 3 columns (p2m_leaf) 856 / 817 / -; FALKON, 2e6 sources (p2m_leaf3) 454 / 443 / 441, 1024 rows 433.
+static int source_chunk(int max_count, int64_t n, bool blocked) {
+    const int64_t share = n / ((blocked ? 8 : 16) * NUM_SMS_HINT);
+    const int chunk = (int)std::max<int64_t>(blocked ? 256 : 512, std::min<int64_t>(8192, share));
+    return max_count > chunk ? chunk : 0;
 }
-// Source boxes: 512 to 1024 points for p2m_leaf3, so that no running sum is longer than some fifty terms (its rounding grows with
-// the square root); the box level is chosen so that few parts are added up (SRC_LEAF).  p2m_leaf sums in blocks of 128 points
-// anyway and takes the parts that fill the SMs.
-static int source_parts(int max_count, int64_t n, int nb, bool blocked) {
-    return blocked ? target_parts(max_count, n, nb) : box_parts(max_count, n, nb, std::max<int64_t>(512, std::min<int64_t>(1024, n / (4 * NUM_SMS_HINT))));
+// P2M of one level: boxes of the list (or all), the parts of the long ones, and their sums
+template <int PP, int RB>
+static void p2m_level(f3m_plan *pl, Level &ly, int which, const float *bs, int R, int r0, const NodeTab2 &nt, int P, int chunk, int src_begin,
+                      int src_end, float *mom, cudaStream_t s) {
+    Tree &ty = *pl->ty;
+    const int d = pl->d, n = (int)ty.n, PR = P * RB;
+    const float factor = 2.f / ly.edge;          // 1_d_conv.cu:473
+    const int64_t slots = chunk ? part_slots(n, chunk) : 0;
+    DevBuf<float> part;
+    if (chunk) part.alloc((size_t)slots * PR, s);
+    if (RB == 1 && d == 3) {
+        const int64_t big = pl->n_leaf_big[which];
+        if (big + slots)
+            p2m_leaf3<PP><<<(unsigned)(big + slots), 128, 0, s>>>(ty.pts.p, n, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, ly.nb, chunk, src_begin,
+                                                                 src_end, mom, part.p, pl->leaf_big[which].p, (int)big);
+        if (pl->n_leaf_small[which])
+            p2m_small3<PP><<<(pl->n_leaf_small[which] + 3) / 4, 128, 0, s>>>(ty.pts.p, n, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, src_begin,
+                                                                            src_end, mom, pl->leaf_small[which].p, pl->n_leaf_small[which]);
+    } else {
+        const size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
+        F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        p2m_leaf<PP, RB><<<(unsigned)(ly.nb + slots), 256, smem, s>>>(ty.pts.p, n, d, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, P, ly.nb, chunk,
+                                                                     src_begin, src_end, mom, part.p);
+    }
+    F3M_LAUNCH_CHECK();
+    if (chunk) {
+        p2m_combine<<<(unsigned)(slots / 2), 128, 0, s>>>(ly.off.p, ly.nb, n, chunk, PR, src_begin, src_end, part.p, mom);
+        F3M_LAUNCH_CHECK();
+    }
 }
+
 // Sources are interpolated at the first level from L on whose boxes hold at most this many points on average, and moved up by
 // M2M, which adds in a tree: with 375 000 sources per box summed at the cut, 3e6 points and l = 10 were 8.4e-7 from float64,
 // the finest level's 5.6e-7.
@@ -1387,7 +1457,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     constexpr int MS = mat_stride(PP);
     NodeTab2 nt = make_nodes2(PP);
     const KronCfg cfg = make_kron_cfg(d, PP, RB);
-    const int n_x = (int)tx.n, n_y = (int)ty.n;
+    const int n_x = (int)tx.n;
     if (RB == 1 && d == 3) {
         ensure_leaf_split(pl, 0, L, s);
         if (!pl->same || Ls != L) ensure_leaf_split(pl, 1, Ls, s);
@@ -1401,26 +1471,10 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                                      (size_t)(pl->mom_box_end - pl->mom_box_begin) * PR * sizeof(float), s));
         else
             F3M_CUDA(cudaMemsetAsync(pl->moments_out, 0, (size_t)ly.nb * PR * sizeof(float), s));
-        int nsplit = std::max(1, std::min(64, (ly.max_count + 8191) / 8192));
-        size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
-        F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         pl->last.begin(ST_P2M, s);
-        if (RB == 1 && d == 3) {
-            const int wy = pl->same ? 0 : 1;
-            if (pl->n_leaf_big[wy])
-                p2m_leaf3<PP><<<dim3(pl->n_leaf_big[wy], nsplit), 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, 2.f / ly.edge, nt,
-                                                                             nsplit > 1 ? nsplit : 1, (int)pl->mom_begin, (int)pl->mom_end,
-                                                                             pl->moments_out, pl->leaf_big[wy].p);
-            if (pl->n_leaf_small[wy])
-                p2m_small3<PP><<<(pl->n_leaf_small[wy] + 3) / 4, 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, 2.f / ly.edge, nt,
-                                                                            (int)pl->mom_begin, (int)pl->mom_end, pl->moments_out,
-                                                                            pl->leaf_small[wy].p, pl->n_leaf_small[wy]);
-        } else
-        p2m_leaf<PP, RB><<<dim3(ly.nb, nsplit), 256, smem, s>>>(ty.pts.p, n_y, d, bs, R, r0, ly.off.p, ly.ctr.p, 2.f / ly.edge, nt, P,
-                                                              nsplit > 1 ? nsplit : 1, (int)pl->mom_begin, (int)pl->mom_end,
-                                                              pl->moments_out);
+        p2m_level<PP, RB>(pl, ly, pl->same ? 0 : 1, bs, R, r0, nt, P, ly.max_count > 8192 ? 8192 : 0, (int)pl->mom_begin, (int)pl->mom_end,
+                          pl->moments_out, s);
         pl->last.end(s);
-        F3M_LAUNCH_CHECK();
         return;
     }
     std::vector<DevBuf<float>> mom(Ls + 1), loc(L + 1);
@@ -1454,25 +1508,10 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     // ---- P2M at level Ls, M2M upwards ------------------------------------------------------------
     pl->last.begin(ST_P2M, s);
     {
-        Level &ly = ty.levels[Ls];
-        const float factor = 2.f / ly.edge;          // 1_d_conv.cu:473
         if (!pl->ext_mom) {
-            const int nsplit = source_parts(ly.max_count, ty.n, ly.nb, !(RB == 1 && d == 3));
-            if (nsplit > 1) mom[Ls].zero();
-            size_t smem = ((size_t)d * PP * 129 + (size_t)128 * RB + (size_t)PR + (size_t)(P / PP)) * sizeof(float);
-            F3M_CUDA(cudaFuncSetAttribute(p2m_leaf<PP, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            if (RB == 1 && d == 3) {
-                const int wy = pl->same && Ls == L ? 0 : 1;
-                if (pl->n_leaf_big[wy])
-                    p2m_leaf3<PP><<<dim3(pl->n_leaf_big[wy], nsplit), 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt,
-                                                                                 nsplit, 0, n_y, mom[Ls].p, pl->leaf_big[wy].p);
-                if (pl->n_leaf_small[wy])
-                    p2m_small3<PP><<<(pl->n_leaf_small[wy] + 3) / 4, 128, 0, s>>>(ty.pts.p, n_y, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, 0,
-                                                                                n_y, mom[Ls].p, pl->leaf_small[wy].p, pl->n_leaf_small[wy]);
-            } else
-            p2m_leaf<PP, RB><<<dim3(ly.nb, nsplit), 256, smem, s>>>(ty.pts.p, n_y, d, bs, R, r0, ly.off.p, ly.ctr.p, factor, nt, P,
-                                                                  nsplit, 0, n_y, mom[Ls].p);
-            F3M_LAUNCH_CHECK();
+            Level &ly = ty.levels[Ls];
+            p2m_level<PP, RB>(pl, ly, pl->same && Ls == L ? 0 : 1, bs, R, r0, nt, P, source_chunk(ly.max_count, ty.n, !(RB == 1 && d == 3)), 0,
+                              (int)ty.n, mom[Ls].p, s);
         }
         const int nw = warps_for(2 * MS * sizeof(float));
         size_t sm2 = (size_t)2 * MS * sizeof(float) + nw * per_warp;

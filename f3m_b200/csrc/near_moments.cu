@@ -115,19 +115,27 @@ __device__ __forceinline__ float mom_ex2(float x) {
     return r;
 }
 
-// A group of T threads (one warp, or a CTA of 256 when the boxes are long) per (source box, column); blockIdx.y splits
-// very long boxes, whose parts are added atomically into zeroed records.
+// A group of T threads (one warp, or a CTA of 256 when the boxes are long) per (source box, column).  Boxes of more than `chunk`
+// rows (0: there are none) are summed in parts by the groups behind, a group per (slot, column); near_moments_combine adds
+// them up.
 template <int D, int K, int RB, int T>
 __global__ void __launch_bounds__(256) near_moments_build(const float *__restrict__ pts, int n, const float *__restrict__ bs, int R,
                                                          int r0, float unit, float s2, const int *__restrict__ off_y, int nby,
                                                          const float *__restrict__ ctr_y, const unsigned char *__restrict__ need,
-                                                         MomFactors fac, int nsplit, float *rec) {
+                                                         MomFactors fac, int chunk, float *rec, float *parts) {
     constexpr int NM = mom_count(D, K), REC = mom_record(D, K, RB);
     __shared__ float part[T == 32 ? 1 : 8][NM];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t g = ((int64_t)blockIdx.x * 256 + threadIdx.x) / T;
-    if (g >= (int64_t)nby * RB) return;      // whole groups leave: T = 256 is the whole CTA
-    const int by = (int)(g / RB), r = (int)(g - (int64_t)by * RB);
+    const int64_t g = ((int64_t)blockIdx.x * 256 + threadIdx.x) / T, boxes = (int64_t)nby * RB;
+    const bool in_part = g >= boxes;
+    if (in_part && (T == 32 || !chunk)) return;      // whole groups leave: T = 256 is the whole CTA
+    const int64_t item = (in_part ? g - boxes : g) / RB;
+    const int r = (int)((in_part ? g - boxes : g) - item * RB);
+    BoxPart bp{(int)item, 0, 0};
+    if (T == 256 && in_part) bp = part_of_slot(off_y, nby, n, chunk, item);
+    else { bp.begin = off_y[item]; bp.end = off_y[item + 1]; }
+    const int by = bp.box, a = bp.begin, b = bp.end;
+    if (in_part ? a == b : (chunk && b - a > chunk)) return;
     if (need && !need[by]) return;           // a slice of the targets names only some source boxes
     float c[D];
 #pragma unroll
@@ -135,8 +143,6 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
     float acc[NM];
 #pragma unroll
     for (int q = 0; q < NM; q++) acc[q] = 0.f;
-    const int o0 = off_y[by], len = off_y[by + 1] - o0;
-    const int a = o0 + (int)(((long long)len * blockIdx.y) / nsplit), b = o0 + (int)(((long long)len * (blockIdx.y + 1)) / nsplit);
     if (r0 + r < R)
         for (int j = a + (int)(threadIdx.x % T); j < b; j += T) {
             float y[D], n2 = 0.f;
@@ -154,9 +160,7 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
         for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
     float *dst = rec + (size_t)by * REC;
     auto put = [&](int q, float v) {
-        float *p = dst + mom_first(D, RB) + q * RB + r;
-        if (nsplit == 1) *p = v * fac.f[q];
-        else atomicAdd(p, v * fac.f[q]);
+        dst[mom_first(D, RB) + q * RB + r] = v * fac.f[q];
     };
     // Where the sum of the weights is not finite, it alone stays: the pairs' terms are positive, so their sum is that value too, while
     // the other moments would carry it with either sign.
@@ -177,10 +181,33 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
                 v += part[T == 32 ? 0 : w][q];
                 v0 += part[T == 32 ? 0 : w][0];
             }
-            put(q, q && !isfinite(v0) ? 0.f : v);
+            if (in_part) parts[((size_t)item * RB + r) * NM + q] = v;
+            else put(q, q && !isfinite(v0) ? 0.f : v);
         }
     }
-    if (r == 0 && blockIdx.y == 0 && (int)(threadIdx.x % T) < D) dst[threadIdx.x % T] = unit * ctr_y[by * D + threadIdx.x % T];
+    if (r == 0 && !in_part && (int)(threadIdx.x % T) < D) dst[threadIdx.x % T] = unit * ctr_y[by * D + threadIdx.x % T];
+}
+
+// records of the long boxes: their parts added in the order of the rows, a CTA per chunk of rows
+template <int D, int K, int RB>
+__global__ void __launch_bounds__(128) near_moments_combine(float unit, const int *__restrict__ off_y, int nby, int n,
+                                                           const float *__restrict__ ctr_y, const unsigned char *__restrict__ need,
+                                                           MomFactors fac, int chunk, const float *__restrict__ parts, float *rec) {
+    constexpr int NM = mom_count(D, K);
+    const LongBox l = long_box_of_chunk(off_y, nby, n, chunk, blockIdx.x);
+    if (l.box < 0 || (need && !need[l.box])) return;
+    float *dst = rec + (size_t)l.box * mom_record(D, K, RB);
+    auto sum = [&](int q, int r) {
+        float v = parts[((size_t)l.first_slot * RB + r) * NM + q];
+        for (int64_t t = (l.first_slot | 1) + 1; t <= l.last_slot; t += 2) v += parts[((size_t)t * RB + r) * NM + q];
+        return v;
+    };
+    for (int i = threadIdx.x; i < NM * RB; i += 128) {
+        const int q = i / RB, r = i - q * RB;
+        const float v = sum(q, r);
+        dst[mom_first(D, RB) + q * RB + r] = (q && !isfinite(sum(0, r)) ? 0.f : v) * fac.f[q];
+    }
+    if (threadIdx.x < D) dst[threadIdx.x] = unit * ctr_y[l.box * D + threadIdx.x];
 }
 
 // One thread per target row.  Rows are in box order, so the lanes of a warp read the same record (a broadcast) except
@@ -376,22 +403,28 @@ static void moment_impl(f3m_plan *pl, int level, const PairCSR *l1, const PairCS
     for (int k = 0; k <= K; k++) { cf[k] *= pw; pw *= ln2; }          // the records hold y 2 s2 = y / (l^2 ln 2) (l, y in that unit)
     MomFactors fac{};
     MomTree<D, K, 0, 0, 0>::factors(cf, 1.0, 0, fac.f);
-    const int nsplit = std::max(1, std::min(64, (ly.max_count + 16383) / 16384));
-    DevBuf<float> rec;
+    constexpr int CHUNK = 16384;
+    const int chunk = ly.max_count > CHUNK ? CHUNK : 0;
+    const int64_t groups = (int64_t)ly.nb * RB, slots = chunk ? part_slots(ty.n, chunk) : 0;
+    DevBuf<float> rec, parts;
     rec.alloc((size_t)ly.nb * mom_record(D, K, RB), s);
+    if (chunk) parts.alloc((size_t)slots * RB * mom_count(D, K), s);
     pl->last.begin(ST_DIRECT, s);
-    if (nsplit > 1) rec.zero();
     const unsigned char *need = pl->shard.active && !pl->shard.all_sources ? pl->shard.need[level].p : nullptr;
-    const int64_t groups = (int64_t)ly.nb * RB;
     // a warp per box, unless the boxes are long or too few to fill the SMs (64 boxes of 312 points, K = 6: 13.5 -> 5.2 us with
     // a CTA per box; 512 boxes of 195 points, K = 3: 5.5 -> 6.8 us)
     if (ly.max_count <= 1024 && (groups >= 2 * NUM_SMS_HINT || ly.max_count <= 64))
-        near_moments_build<D, K, RB, 32><<<dim3((unsigned)((groups + 7) / 8), 1), 256, 0, s>>>(
-            ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, 1, rec.p);
+        near_moments_build<D, K, RB, 32><<<(unsigned)((groups + 7) / 8), 256, 0, s>>>(ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb,
+                                                                                      ly.ctr.p, need, fac, 0, rec.p, nullptr);
     else
-        near_moments_build<D, K, RB, 256><<<dim3((unsigned)groups, nsplit), 256, 0, s>>>(
-            ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb, ly.ctr.p, need, fac, nsplit, rec.p);
+        near_moments_build<D, K, RB, 256><<<(unsigned)(groups + slots * RB), 256, 0, s>>>(ty.pts.p, (int)ty.n, bs, R, r0, unit, s2, ly.off.p, ly.nb,
+                                                                                         ly.ctr.p, need, fac, chunk, rec.p, parts.p);
     F3M_LAUNCH_CHECK();
+    if (chunk) {
+        near_moments_combine<D, K, RB><<<(unsigned)(slots / 2), 128, 0, s>>>(unit, ly.off.p, ly.nb, (int)ty.n, ly.ctr.p, need, fac, chunk, parts.p,
+                                                                            rec.p);
+        F3M_LAUNCH_CHECK();
+    }
     auto eval = [&](auto kernel, int G) {
         kernel<<<(unsigned)(((int64_t)(re - rb) * G + 127) / 128), 128, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, rb, re, l1->ptr.p, l1->idx.p,
                                                                                l2 ? l2->ptr.p : nullptr, l2 ? l2->idx.p : nullptr, rec.p, unit, s2, R,
