@@ -156,8 +156,12 @@ __global__ void __launch_bounds__(256) dense_combine(const float *__restrict__ p
 
 // Slices of the sources.  An SM works through ceil(CTAs / SMs) CTAs of slice + DENSE_FIXED source rows each (DENSE_FIXED: what
 // a CTA spends outside the pair loop, in rows); below four resident CTAs it waits for latencies, so fewer count as four.  The
-// smallest product wins, and the fewest slices among equals.  max_floats bounds the partial sums (a static scratch array).
+// smallest product wins, and the fewest slices among equals -- among partial sums of at most DENSE_FREE_FLOATS; larger ones have to
+// gain DENSE_GAIN: a product of many targets gains nothing from slices that take memory (1.8e6 targets, 8 columns: 510 MB for
+// 0.5 %).  max_floats bounds the partial sums.
 constexpr int64_t DENSE_FIXED = 48, DENSE_MAX_SLICES = 64;
+constexpr int64_t DENSE_FREE_FLOATS = (int64_t)1 << 22;   // 16 MB
+constexpr double DENSE_GAIN = 1.02;
 static int dense_slices(int64_t n, int64_t m, int RB, int64_t max_floats) {
     const int64_t tiles = (n + DTILE - 1) / DTILE;
     int best = 1;
@@ -166,7 +170,8 @@ static int dense_slices(int64_t n, int64_t m, int RB, int64_t max_floats) {
         if (s > 1 && (m / s < 32 || s * n * RB > max_floats)) break;
         const int64_t len = (((m + s - 1) / s) + 1) & ~(int64_t)1;
         const double cost = (double)std::max<int64_t>((tiles * s + NUM_SMS_HINT - 1) / NUM_SMS_HINT, 4) * (double)(len + DENSE_FIXED);
-        if (s == 1 || cost < best_cost) { best = (int)s; best_cost = cost; }
+        const double gain = s * n * RB <= DENSE_FREE_FLOATS ? 1.0 : DENSE_GAIN;
+        if (s == 1 || cost * gain < best_cost) { best = (int)s; best_cost = cost; }
     }
     return best;
 }
@@ -175,12 +180,18 @@ template <int D, int RB, bool GRAD>
 static void dense_block(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int r0, float scale, float post, float *out,
                         float *scratch, int64_t max_floats, cudaStream_t s) {
     const int want = dense_slices(N, M, RB, max_floats);
-    const int64_t slice = (((M + want - 1) / want) + 1) & ~(int64_t)1;
-    const int ns = (int)((M + slice - 1) / slice);
+    int64_t slice = (((M + want - 1) / want) + 1) & ~(int64_t)1;
+    int ns = (int)((M + slice - 1) / slice);
     DevBuf<float> part;
     if (ns > 1 && !scratch) {
-        part.alloc((size_t)ns * N * RB, s);
-        scratch = part.p;
+        try {
+            part.alloc((size_t)ns * N * RB, s);
+            scratch = part.p;
+        } catch (const Fail &) {   // no memory left for partial sums: the product does without
+            (void)cudaGetLastError();
+            slice = (M + 1) & ~(int64_t)1;
+            ns = 1;
+        }
     }
     const dim3 grid((unsigned)((N + DTILE - 1) / DTILE), (unsigned)ns);
     dense_kernel<D, RB, GRAD><<<grid, DNT, 0, s>>>(X, N, Y, b, M, slice, scale, post, R, r0, ns > 1 ? scratch : out);

@@ -34,3 +34,18 @@ def test_dense_extreme_values(cuda):
     Y = torch.tensor([[0.0, 0.0], [0.5, 0.0], [1.0, 0.0]], device=cuda)
     out = engine.rbf_dense(X, Y, torch.ones(3, 1, device=cuda), 1.0).cpu()
     assert abs(float(out[0, 0]) - 2.489027668) <= 1e-5 and float(out[1, 0]) == 0.0 and float(out[2, 0]) == 0.0
+
+
+@pytest.mark.parametrize("n,R,most", [(300_000, 8, 0), (100_000, 8, 3)])
+def test_dense_scratch_pays(n, R, most, cuda):
+    """Partial sums are kept only where slices shorten the call: enough targets fill the GPU without them."""
+    from f3m_b200 import engine
+    X = torch.rand(n, 3, device=cuda)
+    b = torch.rand(n, R, device=cuda)
+    torch.cuda.synchronize()
+    engine.release_cached_memory()
+    before = torch.cuda.mem_get_info()[0]
+    out = engine.rbf_dense(X, X, b, 0.6)
+    torch.cuda.synchronize()
+    held = before - torch.cuda.mem_get_info()[0] - out.numel() * 4
+    assert held <= most * n * R * 4 + (8 << 20), held
