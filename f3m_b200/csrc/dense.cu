@@ -78,10 +78,11 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
     for (int64_t base = m0; base < m1; base += DST) {
         const int cnt = (int)min((int64_t)DST, m1 - base), np = (cnt + 1) >> 1;
         __syncthreads();
-        // row j of the tile -> half (j & 1) of pair j / 2; an odd tile's partner has weight 0
+        // row j of the tile -> half (j & 1) of pair j / 2; an odd tile's partner has weight 0 and the last source's place, so that
+        // its distances are no larger than the sources' own
         for (int q = threadIdx.x; q < 2 * np * D; q += DNT) {
             const int j = q / D, k = q - j * D;
-            smem[(j >> 1) * 2 * W + 2 * k + (j & 1)] = j < cnt ? -scale * Y[base * D + q] : 0.f;
+            smem[(j >> 1) * 2 * W + 2 * k + (j & 1)] = -scale * Y[base * D + (j < cnt ? q : q - D)];
         }
         for (int q = threadIdx.x; q < 2 * np * (W - D); q += DNT) {
             const int j = q / (W - D), r = q - j * (W - D);

@@ -49,3 +49,12 @@ def test_dense_scratch_pays(n, R, most, cuda):
     torch.cuda.synchronize()
     held = before - torch.cuda.mem_get_info()[0] - out.numel() * 4
     assert held <= most * n * R * 4 + (8 << 20), held
+
+
+def test_dense_gradient_of_an_odd_count_far_from_the_origin(cuda):
+    """The partner of the last source weighs nothing, wherever the points lie."""
+    from f3m_b200 import engine
+    X = torch.full((3, 2), 1e20, device=cuda)
+    b = torch.ones(3, 1, device=cuda)
+    assert torch.equal(engine.rbf_dense(X, X, b, 1.0, grad=True), torch.zeros(3, 1, device=cuda))
+    assert torch.equal(engine.rbf_dense(X, X, b, 1.0), torch.full((3, 1), 3.0, device=cuda))
