@@ -347,15 +347,21 @@ def main():
         variants = plan.direct_variants()
         peaks = engine.measure_peaks(dev)
         flop_per_pair = 3 * d + 2 * R                      # 3d + 2R
-        # Where lists are summed pair by pair the direct-sum kernel (near_kernel_x2) spends per pair d multiply-adds on the inner
-        # product, R on the accumulation and one exponential, a quarter of them as degree-5 polynomials on the FMA pipe.  A
-        # product that ends at a level whose interpolation is exact, or whose lists go through box moments, visits no pairs:
-        # its longest stage is the tree (sort), bound by memory.
+        # Where lists are summed pair by pair, a pair costs multiply-adds for its exponent and its R columns and one exponential, by the
+        # form the host picked for its list: expanded (d + R), expanded with 2/5 or 1/3 of the exponentials as polynomials of degree
+        # 2 or 3 on the FMA pipe, differences (2 d + R).  Only the lists that the product visited count: one that ends at a level whose
+        # interpolation is exact, or whose lists go through box moments, visits few pairs or none; its longest stage is then the
+        # tree (sort), bound by memory.
         Lv = st["levels"]
-        pairs_summed = direct_ms > 0 and variants["moments"] == 0
-        fma_per_pair, exp_per_pair = d + R + 0.25 * 8, 0.75
-        peak_pairs = min(peaks["gfma_per_s"] / fma_per_pair, peaks["gexp_per_s"] / exp_per_pair) * 1e9
-        achieved_pairs = st["direct_pairs"] / (direct_ms * 1e-3) if pairs_summed else None
+        work, by_form = plan.last_work(), plan.last_pairs_by_form()
+        pairs_summed = work["pairs"] > 0
+        per_pair = {"mufu": (d + R, 1.0), "poly2": (d + R + 0.4 * 2, 0.6), "poly3": (d + R + 3 / 3.0, 2 / 3.0), "direct": (2 * d + R, 1.0),
+                    "tensor": (d + R, 1.0)}
+        exp_blocks = 1 if R <= 8 else (R + 7) // 8         # the exponential of a pair is shared by up to eight columns
+        roof_s = sum(n * max(per_pair[f][0] / (peaks["gfma_per_s"] * 1e9), exp_blocks * per_pair[f][1] / (peaks["gexp_per_s"] * 1e9))
+                     for f, n in by_form.items() if n)
+        achieved_pairs = work["pairs"] / (direct_ms * 1e-3) if pairs_summed else None
+        peak_pairs = work["pairs"] / roof_s if pairs_summed else None
         try:
             with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as fh:
                 hbm_gbs, hbm_src = float(json.load(fh)["hbm_gbs"]), "of measured"
@@ -365,10 +371,12 @@ def main():
             roof = {"bound": "fp32-fma+sfu", "bound_note": "inner product + exponential per pair; a source row is reused by every target of a tile",
                     "achieved": achieved_pairs * flop_per_pair / 1e12, "peak": peak_pairs * flop_per_pair / 1e12,
                     "unit": "TFLOP/s", "frac": achieved_pairs / peak_pairs,
-                    "kernel": f"direct sums ({'near_kernel_x2' if R == 1 else 'near_columns'}, all launches of one product)",
-                    "pairs": st["direct_pairs"], "ms": direct_ms, "launches": tm["direct_launches"], "kernel_forms": variants,
+                    "kernel": "direct sums (near_kernel_x2, near_kernel; near_columns: "
+                              f"{work['column_launches']} launches; all launches of one product, box moments included)",
+                    "pairs": work["pairs"], "pairs_by_form": {f: n for f, n in by_form.items() if n}, "ms": direct_ms,
+                    "launches": tm["direct_launches"], "kernel_forms": variants,
                     "peak_source": f"measured in this run by register-only probes: {peaks['gexp_per_s']:.0f} Gexp/s, "
-                                   f"{peaks['gfma_per_s']:.0f} Gfma/s; peak = min(fma/{fma_per_pair:.2f}, exp/{exp_per_pair:.2f}) pairs/s x {flop_per_pair} flop",
+                                   f"{peaks['gfma_per_s']:.0f} Gfma/s; per form the slower of its multiply-adds and exponentials, x {flop_per_pair} flop",
                     "traffic": None}
         else:
             build_ms = statistics.median(t["build"] for t in tms)
@@ -396,14 +404,13 @@ def main():
                 "hbm_peak_gbs": hbm_gbs, "hbm_peak": hbm_src,
                 "tree+lists": stage_roof(tm["build"], N * (2 * 4 * d + 2 * 4 * R + 8), 0),   # sort traffic: 40 B/point at d=3, R=1
                 "p2m": stage_roof(tm["p2m"], N * (4 * d + 4 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
-                "m2l": (stage_roof(tm["m2l"], 2 * nb_leaf * Pn * R * 4, st["far_box_pairs"] * d * pd * Pn * R) if direct_ms > 0
-                        else {"ms": round(tm["m2l"], 3), "note": "ends above the last level"}),
+                "m2l": stage_roof(tm["m2l"], 2 * plan.level(work["cut_level"] or Lv)["boxes_x"] * Pn * R * 4, work["box_pairs"] * d * pd * Pn * R),
                 "l2p": stage_roof(tm["l2p"], N * (4 * d + 8 * R) + nb_leaf * Pn * R * 4, N * Pn * R),
                 "direct": {"ms": round(direct_ms, 3), "frac": round(achieved_pairs / peak_pairs, 3) if pairs_summed else None},
-                "note": "m2l multiply-adds counted in the per-pair form (d axis transforms per far pair of all levels); the nested kernel does "
-                        "fewer"}
+                "note": "m2l multiply-adds counted in the per-pair form (d axis transforms per box pair of the levels visited); the nested kernel "
+                        "does fewer"}
         line["work"] = {"levels": st["levels"], "direct_pairs": st["direct_pairs"], "far_box_pairs": st["far_box_pairs"],
-                        "node_pairs_reference_form": st["node_pairs"]}
+                        "node_pairs_reference_form": st["node_pairs"], "visited": work}
         rows = torch.randperm(N, device=dev, generator=g)[:a.check_rows]
         num, den = rel_l2_on_sample(out[rows], Xs[rows], Xs, bs, a.ls, engine)
         line["rel_l2_vs_f64"] = math.sqrt(num / den)
@@ -428,7 +435,8 @@ def main():
             # ---- the same product with the optional forms of the near field (not the headline: `value` above is the
             # default path) ---------------------------------------------------------------------------------------------
             line["near_moments_mode"] = dict(mode_run(f3m_lib.FLAG_NEAR_MOMENTS),
-                                             note="F3M_FLAG_NEAR_MOMENTS: all levels, near sums from box moments to 1e-6; optional, off by default")
+                                             note="F3M_FLAG_NEAR_MOMENTS: box moments to 1e-6 where a list is summed at all (this product ends at a level whose "
+                                                  "interpolation is exact, like the default); optional, off by default")
             line["near_tensor_cores_mode"] = dict(mode_run(f3m_lib.FLAG_NEAR_TENSOR_CORES),
                                                   note="F3M_FLAG_NEAR_TENSOR_CORES: exponent tiles as TF32 tcgen05 products of split operands "
                                                        "(TMEM accumulators, bulk copies, mbarrier pipeline); optional, off by default")

@@ -95,6 +95,7 @@ SIGNATURES = {
     "f3m_plan_last_direct_launches": (C.c_int, [_P]),
     "f3m_plan_last_direct_variants": (C.c_int, [_P, C.POINTER(_I32)]),
     "f3m_plan_last_work": (C.c_int, [_P, C.POINTER(_I64)]),
+    "f3m_plan_last_pairs_by_form": (C.c_int, [_P, C.POINTER(_I64)]),
     "f3m_launch_count": (C.c_longlong, []),
 }
 

@@ -963,9 +963,16 @@ int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]) {
     return F3M_OK;
 }
 
+int f3m_plan_last_pairs_by_form(const f3m_plan *plan, int64_t pairs[6]) {
+    if (!plan || !pairs) return F3M_ERR_ARG;
+    for (int i = 0; i < 6; i++) pairs[i] = plan->last.pairs[i];
+    return F3M_OK;
+}
+
 int f3m_plan_last_work(const f3m_plan *plan, int64_t work[4]) {
     if (!plan || !work) return F3M_ERR_ARG;
-    work[0] = plan->last.pairs;
+    work[0] = 0;
+    for (int64_t v : plan->last.pairs) work[0] += v;
     work[1] = plan->last.box_pairs;
     work[2] = plan->last.cut;
     work[3] = plan->last.column_launches;

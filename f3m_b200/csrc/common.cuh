@@ -263,12 +263,14 @@ struct Timings {
     int direct_launches = 0;
     int direct_variants[DV_COUNT] = {0};
     int column_launches = 0;           // of those, launches of the several-column kernel (near_cols.cu)
-    int64_t pairs = 0, box_pairs = 0;  // pairs of points in the lists summed pair by pair, box pairs of the far field
+    int64_t pairs[DV_COUNT] = {0};     // pairs of points in the lists summed pair by pair, by the form of the sum
+    int64_t box_pairs = 0;             // box pairs of the far field
     int cut = 0;                       // level the product ended at before the last one, 0: none
     void clear_counts() {
         direct_launches = column_launches = cut = 0;
-        pairs = box_pairs = 0;
+        box_pairs = 0;
         for (int &v : direct_variants) v = 0;
+        for (int64_t &v : pairs) v = 0;
     }
     struct Span { int stage; cudaEvent_t a, b; bool closed; };
     std::vector<Span> spans;

@@ -5,6 +5,7 @@
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace f3m {
 
@@ -21,34 +22,6 @@ namespace f3m {
 // FP32 lanes a pair); error against float64 5.4e-7 -> 3.1e-7.
 constexpr int DNT = 128, DT = 2, DTILE = DNT * DT;
 constexpr int DST = 256;   // sources per shared-memory tile; also the length of the blocked partial sums
-
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 d_pack(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void d_unpack(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 d_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 d_mul(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 d_add(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ float d_ex2(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 
 // columns of a source pair in shared memory: minus the scaled coordinates, then the RB values; even, for 16-byte loads
 __host__ __device__ constexpr int dense_width(int D, int RB) { return (D + RB + 1) / 2 * 2; }
@@ -70,7 +43,7 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
 #pragma unroll
         for (int k = 0; k < D; k++) {
             const float v = scale * X[ii * D + k];
-            x[u][k] = d_pack(v, v);
+            x[u][k] = pack2(v, v);
         }
 #pragma unroll
         for (int r = 0; r < RB; r++) tot[u][r] = 0.f;
@@ -93,7 +66,7 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
 #pragma unroll
         for (int u = 0; u < DT; u++)
 #pragma unroll
-            for (int r = 0; r < RB; r++) acc[u][r] = d_pack(0.f, 0.f);
+            for (int r = 0; r < RB; r++) acc[u][r] = pack2(0.f, 0.f);
 #pragma unroll 2
         for (int p = 0; p < np; p++) {
             f32x2 col[W];
@@ -106,19 +79,19 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
             }
 #pragma unroll
             for (int u = 0; u < DT; u++) {
-                f32x2 df = d_add(x[u][0], col[0]);
-                f32x2 r2 = d_mul(df, df);
+                f32x2 df = add2(x[u][0], col[0]);
+                f32x2 r2 = mul2(df, df);
 #pragma unroll
                 for (int k = 1; k < D; k++) {
-                    df = d_add(x[u][k], col[k]);
-                    r2 = d_fma(df, df, r2);
+                    df = add2(x[u][k], col[k]);
+                    r2 = fma2(df, df, r2);
                 }
                 float ra, rb;
-                d_unpack(r2, ra, rb);
-                f32x2 e = d_pack(d_ex2(-ra), d_ex2(-rb));
-                if (GRAD) e = d_mul(e, r2);
+                unpack2(r2, ra, rb);
+                f32x2 e = pack2(ex2_approx(-ra), ex2_approx(-rb));
+                if (GRAD) e = mul2(e, r2);
 #pragma unroll
-                for (int r = 0; r < RB; r++) acc[u][r] = d_fma(e, col[D + r], acc[u][r]);
+                for (int r = 0; r < RB; r++) acc[u][r] = fma2(e, col[D + r], acc[u][r]);
             }
         }
 #pragma unroll
@@ -126,7 +99,7 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
 #pragma unroll
             for (int r = 0; r < RB; r++) {   // blocked accumulation: one partial sum per tile
                 float lo, hi;
-                d_unpack(acc[u][r], lo, hi);
+                unpack2(acc[u][r], lo, hi);
                 tot[u][r] += lo + hi;
             }
     }

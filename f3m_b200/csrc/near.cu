@@ -13,6 +13,7 @@
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace f3m {
 
@@ -20,12 +21,6 @@ constexpr int NT = 128;        // threads per CTA
 constexpr int ST = 512;        // source rows per shared-memory tile
 
 __host__ __device__ constexpr int row_width(int D, int RB) { return (D + RB + 3) / 4 * 4; }
-
-__device__ __forceinline__ float ex2_approx(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 
 template <int D, int RB>
 __global__ void __launch_bounds__(256) pack_sources(const float *__restrict__ pts, int64_t n, const float *__restrict__ bs,
@@ -179,23 +174,6 @@ constexpr int TI2 = 2;      // targets per thread
 // 16-byte shared-memory load yields two aligned register pairs.  Box b starts at the even row
 // (off[b] + b + 1) & ~1 of the packed array; an odd box gets a zero-weight partner for its last source.
 // ---------------------------------------------------------------------------------------------
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __host__ __device__ __forceinline__ int pair_row_start(int off, int box) { return (off + box + 1) & ~1; }
 
 // Packing with one warp per source box (and per part of a long box): boxes no list of this product names
@@ -703,7 +681,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         pl->last.end(s);
         pl->last.direct_launches++;
         pl->last.direct_variants[DV_TENSOR]++;
-        if (r0 == 0) pl->last.pairs += csr.pairs;
+        if (r0 == 0) pl->last.pairs[DV_TENSOR] += csr.pairs;
         F3M_LAUNCH_CHECK();
         return;
     }
@@ -721,10 +699,11 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         pl->last.end(s);
         F3M_LAUNCH_CHECK();
     }
+    int form = DV_DIRECT;
     pl->last.begin(ST_DIRECT, s);
     if (expanded) {
         const int poly = exp2_poly_degree(tmax);
-        pl->last.direct_variants[poly == 2 ? DV_POLY2 : (poly == 3 ? DV_POLY3 : DV_MUFU)]++;
+        form = poly == 2 ? DV_POLY2 : (poly == 3 ? DV_POLY3 : DV_MUFU);
         double cf[4];
         exp2_poly_fit(-tmax, tmax, poly, cf);
 #define F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, MIXED_)                                                                                       \
@@ -743,13 +722,13 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 #undef F3M_NEAR_EXP
     }
     else {
-        pl->last.direct_variants[DV_DIRECT]++;
         near_kernel<D, RB, 1><<<items, NT, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, csr.idx.p, ly.off.p,
                                                    packed.p, scale, R, r0, out, row_begin, row_end);
     }
     pl->last.end(s);
     pl->last.direct_launches++;
-    if (r0 == 0) pl->last.pairs += level > 0 ? csr.pairs : tx.n * ty.n;
+    pl->last.direct_variants[form]++;
+    if (r0 == 0) pl->last.pairs[form] += level > 0 ? csr.pairs : tx.n * ty.n;
     F3M_LAUNCH_CHECK();
 }
 

@@ -15,6 +15,7 @@
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace f3m {
 
@@ -22,33 +23,6 @@ constexpr int CM = 4;        // target rows per lane
 constexpr int CT = 8 * CM;   // targets per tile
 constexpr int CR = 8;        // columns
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 c_pack(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void c_unpack(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 c_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 c_mul(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 c_add(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ float c_ex2(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 // asynchronous copies into shared memory
 __device__ __forceinline__ void c_copy4(float *dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -134,7 +108,7 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
             xr[m][k] = DIFF ? x : 2.f * x;
         }
 #pragma unroll
-        for (int r = 0; r < CR / 2; r++) acc[m][r] = tot[m][r] = c_pack(0.f, 0.f);
+        for (int r = 0; r < CR / 2; r++) acc[m][r] = tot[m][r] = pack2(0.f, 0.f);
     }
     if (r0 + CR > R)   // columns that do not exist are never copied
         for (int q = S::COORDS * CST + lane; q < S::FLOATS; q += 32) stage[q] = 0.f;
@@ -221,12 +195,12 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
 #pragma unroll
                         for (int k = 1; k < D; k++) v = fmaf(xr[m][k], y[k][q], v);
                     }
-                    const float ev = c_ex2(v);
-                    const f32x2 e2 = c_pack(ev, ev);
-                    acc[m][0] = c_fma(e2, b01.x, acc[m][0]);
-                    acc[m][1] = c_fma(e2, b01.y, acc[m][1]);
-                    acc[m][2] = c_fma(e2, b23.x, acc[m][2]);
-                    acc[m][3] = c_fma(e2, b23.y, acc[m][3]);
+                    const float ev = ex2_approx(v);
+                    const f32x2 e2 = pack2(ev, ev);
+                    acc[m][0] = fma2(e2, b01.x, acc[m][0]);
+                    acc[m][1] = fma2(e2, b01.y, acc[m][1]);
+                    acc[m][2] = fma2(e2, b23.x, acc[m][2]);
+                    acc[m][3] = fma2(e2, b23.y, acc[m][3]);
                 }
             }
         }
@@ -235,8 +209,8 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
         for (int m = 0; m < MT; m++)
 #pragma unroll
             for (int r = 0; r < CR / 2; r++) {
-                tot[m][r] = c_add(tot[m][r], acc[m][r]);
-                acc[m][r] = c_pack(0.f, 0.f);
+                tot[m][r] = add2(tot[m][r], acc[m][r]);
+                acc[m][r] = pack2(0.f, 0.f);
             }
         if (last) break;
         fill = 0;
@@ -247,7 +221,7 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
         // the four lanes of a target add up their sources: columns 2t, 2t + 1 end in lane t
         float v[CR], half[CR / 2], sum[2];
 #pragma unroll
-        for (int r = 0; r < CR / 2; r++) c_unpack(tot[m][r], v[2 * r], v[2 * r + 1]);
+        for (int r = 0; r < CR / 2; r++) unpack2(tot[m][r], v[2 * r], v[2 * r + 1]);
 #pragma unroll
         for (int r = 0; r < CR / 2; r++)
             half[r] = ((t & 2) ? v[r + 4] : v[r]) + __shfl_xor_sync(0xffffffffu, (t & 2) ? v[r] : v[r + 4], 2);
@@ -259,7 +233,7 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
             float n2 = 0.f;
 #pragma unroll
             for (int k = 0; k < D; k++) n2 = fmaf(xr[m][k], xr[m][k], n2);
-            f = c_ex2(-0.25f * n2);
+            f = ex2_approx(-0.25f * n2);
         }
         const int i = 8 * m + g, r = r0 + 2 * t;
         if (i >= nt) continue;
@@ -321,7 +295,7 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
     pl->last.direct_launches++;
     pl->last.direct_variants[DIFF ? DV_DIRECT : DV_MUFU]++;
     pl->last.column_launches++;
-    if (r0 == 0) pl->last.pairs += csr.pairs;
+    if (r0 == 0) pl->last.pairs[DIFF ? DV_DIRECT : DV_MUFU] += csr.pairs;
     F3M_LAUNCH_CHECK();
 }
 

@@ -18,6 +18,7 @@
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace f3m {
 
@@ -95,25 +96,14 @@ struct Val1 {   // one column; the record already lies in registers
     static __device__ __forceinline__ Val1 fma(float x, Val1 a, Val1 c) { return Val1{fmaf(x, a.v, c.v)}; }
 };
 struct Val4 {   // four columns of one moment: one 16-byte load, two packed multiply-adds
-    typedef unsigned long long X;
-    unsigned long long lo, hi;
+    typedef f32x2 X;
+    f32x2 lo, hi;
     static __device__ __forceinline__ Val4 load(const float *m, int q) {
         const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2 *>(m + 4 * q));
         return Val4{w.x, w.y};
     }
-    static __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-        unsigned long long d;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-        return d;
-    }
     static __device__ __forceinline__ Val4 fma(X x, Val4 a, Val4 c) { return Val4{fma2(x, a.lo, c.lo), fma2(x, a.hi, c.hi)}; }
 };
-
-__device__ __forceinline__ float mom_ex2(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 
 // A group of T threads (one warp, or a CTA of 256 when the boxes are long) per (source box, column).  Boxes of more than `chunk`
 // rows (0: there are none) are summed in parts by the groups behind, a group per (slot, column); near_moments_combine adds
@@ -152,7 +142,7 @@ __global__ void __launch_bounds__(256) near_moments_build(const float *__restric
                 n2 = fmaf(v, v, n2);
                 y[k] = 2.f * s2 * v;
             }
-            MomTree<D, K, 0, 0, 0>::build(bs[(size_t)j * R + r0 + r] * mom_ex2(-s2 * n2), y, acc);
+            MomTree<D, K, 0, 0, 0>::build(bs[(size_t)j * R + r0 + r] * ex2_approx(-s2 * n2), y, acc);
         }
 #pragma unroll
     for (int q = 0; q < NM; q++)
@@ -260,21 +250,21 @@ __global__ void __launch_bounds__(128) near_moments_eval(const float *__restrict
                     xr[k] = x[k] - mr[k];
                     n2 = fmaf(xr[k], xr[k], n2);
                 }
-                tot[0] = fmaf(mom_ex2(-s2 * n2), MomTree<D, K, 0, 0, 0>::template eval<Val1>(xr, mr + mom_first(D, RB)).v, tot[0]);
+                tot[0] = fmaf(ex2_approx(-s2 * n2), MomTree<D, K, 0, 0, 0>::template eval<Val1>(xr, mr + mom_first(D, RB)).v, tot[0]);
             } else {
-                unsigned long long xr[D];
+                f32x2 xr[D];
                 float n2 = 0.f;
 #pragma unroll
                 for (int k = 0; k < D; k++) {
                     const float v = x[k] - __ldg(m + k);
                     n2 = fmaf(v, v, n2);
-                    asm("mov.b64 %0, {%1, %1};" : "=l"(xr[k]) : "f"(v));
+                    xr[k] = pack2(v, v);
                 }
                 const Val4 p = MomTree<D, K, 0, 0, 0>::template eval<Val4>(xr, m + mom_first(D, RB));
-                const float fx = mom_ex2(-s2 * n2);
+                const float fx = ex2_approx(-s2 * n2);
                 float pv[4];
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(pv[0]), "=f"(pv[1]) : "l"(p.lo));
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(pv[2]), "=f"(pv[3]) : "l"(p.hi));
+                unpack2(p.lo, pv[0], pv[1]);
+                unpack2(p.hi, pv[2], pv[3]);
 #pragma unroll
                 for (int r = 0; r < RB; r++) tot[r] = fmaf(fx, pv[r], tot[r]);
             }

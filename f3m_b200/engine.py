@@ -286,6 +286,12 @@ class Plan:
         check(_lib.lib().f3m_plan_last_work(self._h, w), "f3m_plan_last_work")
         return dict(zip(("pairs", "box_pairs", "cut_level", "column_launches"), (int(v) for v in w)))
 
+    def last_pairs_by_form(self) -> Dict:
+        """Pairs the last apply() summed one by one, by kernel form (f3m_plan_last_pairs_by_form)."""
+        w = (C.c_int64 * 6)()
+        check(_lib.lib().f3m_plan_last_pairs_by_form(self._h, w), "f3m_plan_last_pairs_by_form")
+        return dict(zip(("mufu", "poly2", "poly3", "direct", "moments", "tensor"), (int(v) for v in w)))
+
     def array(self, level: int, tree: int, what: int) -> np.ndarray:
         info = self.level(level) if level >= 1 else None
         nb = (info["boxes_x"] if tree == 0 else info["boxes_y"]) if info else 1

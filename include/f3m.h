@@ -125,7 +125,8 @@ int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, 
  * row_begin/row_end restrict the product to the target boxes whose sorted point range starts
  * inside [row_begin,row_end) (a slice of the sorted target order, used to shard target boxes
  * over GPUs); rows outside the slice are written as 0.  Use 0, N for the whole product, which may end at the level whose
- * interpolation is exact for every pair (relative bound 1.2e-7); slices visit all levels. */
+ * interpolation is exact for every pair (relative bound 1.2e-7); slices visit all levels.
+ * A NaN in b makes every row it reaches NaN.  An infinity reaches rows through direct sums as infinity, through interpolation as NaN. */
 int f3m_plan_apply(f3m_plan *plan, const float *b, int32_t R, float *out, void *stream);
 int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, int64_t row_begin,
                          int64_t row_end, void *stream);
@@ -271,11 +272,11 @@ int f3m_rbf_dense_grad_f32(const float *X, int64_t N, const float *Y, int64_t M,
 
 /* The same product as f3m_rbf_dense_f32 for hosts that must not allocate device memory while they run
  * (all memory pre-reserved by the host's own pool, or a no-allocation-after-start-up rule because an
- * allocation can stall the device).  It has no counterpart in the reference.  Its scratch -- the packed
- * source rows -- lives in a fixed 16 MiB array inside the library image (F3M_STATIC_SCRATCH_FLOATS floats,
+ * allocation can stall the device).  It has no counterpart in the reference.  Its scratch -- partial
+ * sums of the source slices -- lives in a fixed 16 MiB array inside the library image (F3M_STATIC_SCRATCH_FLOATS floats,
  * held by every GPU that loads the library), so it calls no cudaMalloc, cudaFree or pool routine.
  * Limit: M * w <= F3M_STATIC_SCRATCH_FLOATS with w = 4 floats per source for d <= 3 and one column
- * (in general d + min(R,4) rounded up to a multiple of 4); larger inputs return F3M_ERR_TOO_LARGE.
+ * (in general d + 1 for one column, d + 4 for more, rounded up to a multiple of 4); larger inputs return F3M_ERR_TOO_LARGE.
  * The first call on a device looks up the array's device address; make it before any stream capture.
  * Calls share the array: calls that overlap on the GPU (other streams or host threads) race. */
 #define F3M_STATIC_SCRATCH_FLOATS (4 * 1024 * 1024)
@@ -304,6 +305,8 @@ int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]);
  * one (0: none), [3] = direct-sum launches that took the kernel for several columns and short boxes (they count in counts[0] or
  * counts[3] above too). */
 int f3m_plan_last_work(const f3m_plan *plan, int64_t work[4]);
+/* work[0] by the form that summed the pairs, in the order of f3m_plan_last_direct_variants (moments visit no pairs: pairs[4] = 0). */
+int f3m_plan_last_pairs_by_form(const f3m_plan *plan, int64_t pairs[6]);
 long long f3m_launch_count(void);
 
 #ifdef __cplusplus

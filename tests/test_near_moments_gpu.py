@@ -50,14 +50,18 @@ def test_moments_at_the_corners_of_the_boxes(cuda):
     assert rel_l2(a, b) <= TOL
 
 
-@pytest.mark.parametrize("n,m", [(1, 70000), (31, 40000), (129, 3000), (40000, 1500), (70001, 33)])
+@pytest.mark.parametrize("n,m", [(1, 70000), (31, 40000), (129, 3000), (40000, 1500), (70001, 33), (31, 400_000), (200, 1_000_003)])
 def test_moments_of_two_point_sets(n, m, cuda):
-    """Source boxes of very different length (blocks of 256 threads, parts of a box added atomically) and few targets."""
+    """Source boxes of very different length (a warp, 256 threads, parts of more than 16 384 rows) and few targets."""
     g = torch.Generator().manual_seed(n + m)
     X, Y = torch.rand(n, 3, generator=g), torch.rand(m, 3, generator=g)
+    if m >= 400_000:
+        Y[: m // 3] *= 0.5     # one octant holds several times the others' sources
     if n == 1:
         X = torch.cat([X, X + 0.2])
-    (a, b), _, _ = _both(X, Y, _weights(m, 1, g), 2.0, 20.0 if min(n, m) > 20 else 1.0, 27, cuda)
+    (a, b), forms, plan = _both(X, Y, _weights(m, 1, g), 2.0, 20.0 if min(n, m) > 20 else 1.0, 27, cuda)
+    if m >= 400_000:
+        assert forms["moments"] > 0 and plan.level(1)["max_count_y"] > 2 * 16384, forms
     assert torch.isfinite(a).all()
     assert rel_l2(a, b) <= TOL
 

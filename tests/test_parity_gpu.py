@@ -198,11 +198,15 @@ def test_near_moments_flag(d, ls, R, cuda):
     b = torch.randn(40000, R, generator=g)
     P = {2: 36, 3: 64, 4: 81}[d]
     outs = {}
-    for flags in (0, _lib.FLAG_NEAR_MOMENTS):
+    # the reference sums its pairs one by one: the tensor-core flag keeps moments and the cut out
+    for flags in (_lib.FLAG_NEAR_TENSOR_CORES, _lib.FLAG_NEAR_MOMENTS):
         prm = engine.make_params(ls, 300.0, P, False, 0.15, P, flags=flags)
         plan = engine.Plan(X.to(cuda), None, prm)
-        outs[flags] = plan.apply(b.to(cuda)).cpu()
-        assert plan.stats()["direct_pairs"] > 0
+        outs[flags if flags == _lib.FLAG_NEAR_MOMENTS else 0] = plan.apply(b.to(cuda)).cpu()
+        if flags == _lib.FLAG_NEAR_TENSOR_CORES:
+            assert plan.last_work()["pairs"] == plan.stats()["direct_pairs"] > 0 and plan.direct_variants()["moments"] == 0
+        else:
+            assert plan.last_work()["pairs"] == 0
     assert rel_l2(outs[_lib.FLAG_NEAR_MOMENTS], outs[0]) <= 3e-6
     rows = torch.arange(2000)
     exact = dense_kmvm_f64(X, X, b, ls, rows=rows)
