@@ -739,13 +739,19 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 // and source box, 8 columns: d = 2 16: 1.5, 62: 1.1, 247: 0.93; d = 3 9: 2.5, 74: 1.03, 247: 0.80; d = 4 15: 2.1, 72: 1.07, 247: 0.86;
 // d = 5 9: 2.7, 156: 1.3, 297: 0.94.  Four columns: d = 2 16: 1.1, 62: 0.68; d = 3 9: 1.8, 74: 0.75; d = 4 15: 1.5, 72: 0.8; d = 5
 // 9: 2.3, 297: 0.73.  Difference form, d = 3, 8 / 4 columns: 7: 6.4 / 5.1, 74: 1.8 / 1.3, 591: 1.3 / 0.88.
+// Fewer targets than fill the SMs with tiles of 64 (a CTA each, 20 per SM) make the tiles up to 1.6 times slower than that, the stream's shorter
+// and more numerous ones less (d = 3, 3e4 points, 4 columns, 59 sources 1.2; d = 5, 65 sources 1.7).
+// With four columns the constants lean to the tiles where rows hold some 15 to 30 sources: uneven trees lose there (d = 4, 4.8e5 normal
+// points, 2 columns, whole call 20.2 -> 22.6 ms on the stream).
 // One dimension stays with the tiles: its lists name three boxes, too short for the stream's set-up (1e6 points, 4 columns 0.85).
 static double stream_seconds(int d, bool narrow, double row) {
     return narrow ? 6.5e-14 * (d + 8) + 1e-11 / row : 6.1e-14 * (2 * d + 8) + 1.8e-11 / row;
 }
-static double tile_seconds(int d, bool expanded, int cols, double row) {
+static double tile_seconds(int d, bool expanded, int cols, double row, int64_t targets) {
     const int RB = cols >= 5 ? 8 : 4;
-    return expanded ? 4.3e-14 * (d + RB) + (7e-12 * d + 2e-12 * (RB - 4)) / row : 6.1e-14 * (1.5 * d + RB) + 1.1e-10 / row;
+    const double idle = 1.0 + 0.6 * std::max(0.0, 1.0 - (double)targets / (64.0 * 20 * NUM_SMS_HINT));
+    if (!expanded) return (6.1e-14 * (1.5 * d + RB) + 1.1e-10 / row) * idle;
+    return (4.3e-14 * (d + RB) + (RB == 8 ? 7e-12 * d + 8e-12 : 4.3e-12 * d) / row) * idle;
 }
 
 // seconds per pair for `cols` (2 or more) columns of a list, and whether the stream takes them
@@ -754,7 +760,7 @@ static double column_seconds(const f3m_plan *pl, int level, const PairCSR &csr, 
     const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
     const bool narrow = se <= 1.0, expanded = narrow && d * list_reach(pl, level, csr) * se * se <= TMAX_EXPANDED;
     const double row = (double)csr.pairs / (double)std::max<int64_t>(1, csr.row_boxes);
-    const double st = stream_seconds(d, narrow, row), ti = tile_seconds(d, expanded, cols, row);
+    const double st = stream_seconds(d, narrow, row), ti = tile_seconds(d, expanded, cols, row, pl->tx.n);
     stream = d >= 2 && st <= ti;
     return stream ? st : ti;
 }

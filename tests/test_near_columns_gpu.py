@@ -140,7 +140,7 @@ def test_long_boxes_stay_with_the_tiles(cuda):
     from f3m_b200 import engine
     g = torch.Generator().manual_seed(20)
     for d, R, ls in ((3, 8, 1.0), (3, 3, 1.0), (1, 8, 0.01)):
-        X = torch.rand(4000, d, generator=g).to(cuda)
+        X = torch.rand(200_000, d, generator=g).to(cuda)     # enough targets for tiles on every SM
         plan = engine.Plan(X, None, engine.make_params(ls, 5.0, 2 ** d, False, 0.15, 10 ** 6, flags=2))
-        plan.apply(torch.rand(4000, R, device=cuda))
-        assert plan.last_work()["column_launches"] == 0 and plan.last_work()["pairs"] == 4000 ** 2
+        plan.apply(torch.rand(200_000, R, device=cuda))
+        assert plan.last_work()["column_launches"] == 0 and plan.last_work()["pairs"] == 200_000 ** 2
