@@ -354,12 +354,14 @@ static int list_moment_degree(const f3m_plan *pl, int level, bool keep, int R) {
             if (flag) return K;
             // Moments where they take less time than the pairs.  Either form also launches a few kernels per block of columns, 10 us
             // for tiles, scan, packing and sums.  One column: an evaluation of 20 terms at 3.2e11 /s against pairs at 5.2e12 /s (3.5e12
-            // without polynomial pairs) is about one term per 0.5 to 0.8 pairs.  Two columns and more, eight columns measured,
+            // without polynomial pairs) is about one term per 0.5 to 0.8 pairs;
+            // the pair form's own preparation (flags, packing, read-backs) costs lists of a few pairs no less than the records do (mixture of
+            // 1.4e7 points, l = 5.5: 24.8 ms with moments, 25.4 with pairs).  Two columns and more, eight columns measured,
             // moments / pairs: d = 1, 1e6 normal points, lists of a few pairs on eight levels 0.72 / 0.56 ms; d = 3, l = 0.3, 1e6 normal
             // points, boxes of twelve 10.1 / 4.3 ms; d = 2, 1e6 uniform points 0.25 / 0.59 ms.
+            if (R == 1) return (double)csr.pairs >= 0.5 * mom_count(pl->d, K) * (double)csr.row_boxes ? K : 0;
             const MomentSeconds t = moment_seconds(pl, csr, K, R);
             const double pairs = pair_list_seconds(pl, level, csr, R) + 1e-5 * ((R + 7) / 8);
-            if (R == 1) return (double)csr.pairs >= 0.5 * mom_count(pl->d, K) * (double)csr.row_boxes && t.fixed <= pairs ? K : 0;
             return t.eval + t.fixed <= pairs ? K : 0;
         }
     }
