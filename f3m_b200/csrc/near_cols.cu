@@ -10,8 +10,8 @@
 //
 // What bounds it: FMA lanes (57 % busy at boxes of 246 points, d = 4) and the shared-memory pipe (70 %), which carries a source
 // to every tile that reads it; with short boxes the latter, as a source then serves few rows.  Direct sums of 8 columns, all lists on
-// the kernels of near.cu / short boxes as split TF32 / short boxes here: 1e6 points N(0,I), d = 5 60.7 / 36.0 / 32.9 ms, d = 4 33.5 /
-// 26.5 / 22.9 ms; 3e5 points U[0,1]^5 in boxes of nine 40.3 / 17.9 / 14.4 ms.  All lists here: 1e6 points in boxes of 246, d = 4 8.0 -> 9.1 ms.
+// the kernels of near.cu / short boxes as split TF32 / short boxes here: 1e6 points N(0,I), d = 5 60.7 / 36.0 / 31.7 ms, d = 4 33.5 /
+// 26.5 / 22.6 ms; 3e5 points U[0,1]^5 in boxes of nine 40.3 / 17.9 / 14.4 ms.  All lists here: 1e6 points in boxes of 246, d = 4 8.0 -> 9.1 ms.
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
