@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <vector>
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace f3m {
 
@@ -34,7 +35,7 @@ constexpr int PMAX_FAST = 8;  // nodes per dimension handled by this path
 struct NodeTab2 {
     int p;
     float node[PMAX_FAST];
-    float w[PMAX_FAST];
+    float c[PMAX_FAST];   // 1 / prod_{l != i} (node_i - node_l)
 };
 
 struct Geom2 {
@@ -47,7 +48,14 @@ __host__ __device__ constexpr int mat_stride(int p) { return (p * p + 3) / 4 * 4
 static NodeTab2 make_nodes2(int p) {
     NodeTab2 t{};
     t.p = p;
-    cheb_nodes_weights(p, t.node, t.w);
+    float w[PMAX_FAST];   // barycentric weights: the reference's form, not used here
+    cheb_nodes_weights(p, t.node, w);
+    for (int i = 0; i < p; i++) {
+        double v = 1.0;
+        for (int l = 0; l < p; l++)
+            if (l != i) v *= (double)t.node[i] - (double)t.node[l];
+        t.c[i] = (float)(1.0 / v);
+    }
     return t;
 }
 
@@ -894,28 +902,24 @@ __global__ void __launch_bounds__(128) l2l_fast(int nbc, int d, const int *__res
 // ---------------------------------------------------------------------------------------------
 // P2M / L2P at the finest level: one CTA per (box, split)
 // ---------------------------------------------------------------------------------------------
-// Barycentric Lagrange basis (lagrange_data_load + calculate_barycentric_lagrange, 1_d_conv.cu:217-238, 418-448)
+// Lagrange basis at t (lagrange_data_load + calculate_barycentric_lagrange, 1_d_conv.cu:217-238, 418-448), as products of the
+// differences t - t_l before and after node i: 5 p multiplications and additions and no division; a point on a node
+// needs no case of its own.  The barycentric form cost a reciprocal, a comparison and a select per node: half of all instructions
+// of the leaf kernels.
 template <int PP>
 __device__ __forceinline__ void lagrange_pp(float t, const NodeTab2 &nt, float *L) {
-    // q_i = w_i / (t - t_i) with the fast reciprocal (2 ulp): L_i = q_i / sum_l q_l.  The reference's kernels are
-    // built with --use_fast_math, so their divisions are the approximate ones too.
-    int hit = -1;
-    float sum = 0.f;
-    float q[PP];
+    float diff[PP], after[PP];
+#pragma unroll
+    for (int i = 0; i < PP; i++) diff[i] = t - nt.node[i];
+    after[PP - 1] = 1.f;
+#pragma unroll
+    for (int i = PP - 2; i >= 0; i--) after[i] = (i == PP - 2) ? diff[PP - 1] : after[i + 1] * diff[i + 1];
+    float before = 1.f;
 #pragma unroll
     for (int i = 0; i < PP; i++) {
-        const float diff = t - nt.node[i];
-        if (diff == 0.f) hit = i;
-        q[i] = __fdividef(nt.w[i], diff);
-        sum += q[i];
-    }
-    if (hit >= 0) {
-#pragma unroll
-        for (int i = 0; i < PP; i++) L[i] = (i == hit) ? 1.f : 0.f;
-    } else {
-        const float lx = __fdividef(1.f, sum);
-#pragma unroll
-        for (int i = 0; i < PP; i++) L[i] = lx * q[i];
+        const float cb = i == 0 ? nt.c[0] : nt.c[i] * before;
+        L[i] = i == PP - 1 ? cb : cb * after[i];
+        before = i == 0 ? diff[0] : before * diff[i];
     }
 }
 
@@ -1093,19 +1097,24 @@ __global__ void __launch_bounds__(128) l2p_leaf(const float *__restrict__ pts, i
 }
 
 // ---------------------------------------------------------------------------------------------
-// P2M / L2P for d = 3 and one column, register-tiled.  A lane is (point stream, m2): it keeps the PP x PP block
-// (m0, m1) of the box's moments (or local expansion) for its m2 in registers, so a point costs the lane PP
-// multiplies and PP^2 multiply-adds against 4 broadcast 16-byte loads and one 4-byte load of the point's Lagrange
-// rows -- the multiply-add rate, not shared memory, is the limit.  32 / PP streams per warp, 4 warps per CTA, one box
-// per CTA (blockIdx.y splits very large boxes).  The rows [L0 (8) | L1 (8) | L2 (8) | pad (4)] are 28 floats apart,
-// which puts the rows of the streams of one warp on different banks.
+// P2M / L2P for d = 3 and one column, register-tiled.  A lane is (stream, m2): it keeps the PP x PP block (m0, m1) of the
+// box's moments (or local expansion) for its m2 in registers and takes two points at a time, one in either half of every
+// packed instruction, so that nothing has to be duplicated: PP multiplications and PP^2 multiply-adds per two points against
+// 16-byte loads of their Lagrange rows.  A warp works alone: its lanes first build the rows of two points each (coordinates
+// of the next ones are on their way meanwhile), then 32 / PP streams share them; CTAs meet only to add up.  Bound: FP32 lanes, PP^2 + PP
+// of them per point and m2 besides some 30 per axis for the rows.  1e8 points, 216 nodes, against one point at
+// a time, barycentric rows and CTA-wide chunks: p2m_leaf3 2.11 -> 1.61 ms, l2p_leaf3 2.46 -> 1.56 ms (0.62 at the FMA rate).
+// A row [L0 | L1 | L2] holds its two points alternating; rows are RS floats apart, an odd number of 16-byte groups, which puts
+// the streams of a warp on different banks.
 // ---------------------------------------------------------------------------------------------
-constexpr int L3_RS = 28;
 template <int PP>
 struct Leaf3 {
-    static constexpr int SUB = 32 / PP;              // point streams per warp
+    static constexpr int SUB = 32 / PP;              // streams per warp
+    static constexpr int ROWS = 32 / SUB * SUB;      // rows (pairs of points) per warp and chunk
+    static constexpr int WP = 2 * ROWS;              // points per warp and chunk
     static constexpr int NSTREAM = 4 * SUB;          // per CTA
-    static constexpr int TP = NSTREAM * (128 / NSTREAM);   // points per chunk
+    static constexpr int AX = (2 * PP + 3) / 4 * 4;  // floats per axis
+    static constexpr int RS = 3 * AX % 8 == 4 ? 3 * AX : 3 * AX + 4;
 };
 
 template <int PP>
@@ -1120,17 +1129,42 @@ __device__ __forceinline__ void leaf3_rows(const float *__restrict__ pts, int n,
     }
 }
 
-// the same from coordinates already in registers (the loads of a chunk are issued while the previous chunk is consumed)
+// rows of two points at once, xa and xb; the third axis carries the factors f
 template <int PP>
-__device__ __forceinline__ void leaf3_rows_xyz(const float (&x)[3], const float (&c)[3], float factor, const NodeTab2 &nt,
-                                               float scale2, float *row) {
-    float L[PP];
+__device__ __forceinline__ void leaf3_row_pair(const float (&xa)[3], const float (&xb)[3], const float (&c)[3], float factor,
+                                               const NodeTab2 &nt, f32x2 f, float *row) {
+    using G = Leaf3<PP>;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        lagrange_pp<PP>(factor * (x[k] - c[k]), nt, L);
+        const f32x2 t = pack2(factor * (xa[k] - c[k]), factor * (xb[k] - c[k]));
+        f32x2 diff[PP], after[PP], L[PP];
 #pragma unroll
-        for (int q = 0; q < PP; q++) row[8 * k + q] = (k == 2) ? scale2 * L[q] : L[q];
+        for (int i = 0; i < PP; i++) diff[i] = add2(t, pack2(-nt.node[i], -nt.node[i]));
+#pragma unroll
+        for (int i = PP - 2; i >= 0; i--) after[i] = (i == PP - 2) ? diff[PP - 1] : mul2(after[i + 1], diff[i + 1]);
+        f32x2 before = diff[0];
+#pragma unroll
+        for (int i = 0; i < PP; i++) {
+            f32x2 cb = pack2(nt.c[i], nt.c[i]);
+            if (k == 2) cb = mul2(cb, f);
+            if (i > 0) cb = mul2(cb, before);
+            L[i] = i == PP - 1 ? cb : mul2(cb, after[i]);
+            if (i > 0) before = mul2(before, diff[i]);
+        }
+        ulonglong2 *dst = reinterpret_cast<ulonglong2 *>(row + k * G::AX);
+#pragma unroll
+        for (int q = 0; q < G::AX / 4; q++) dst[q] = make_ulonglong2(L[2 * q], 2 * q + 1 < PP ? L[2 * q + 1] : 0ull);
     }
+}
+template <int PP>
+__device__ __forceinline__ void leaf3_load_axis(const float *axis, f32x2 (&l)[PP]) {
+#pragma unroll
+    for (int q = 0; q < PP / 2; q++) {
+        const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(axis)[q];
+        l[2 * q] = v.x;
+        l[2 * q + 1] = v.y;
+    }
+    if (PP & 1) l[PP - 1] = *reinterpret_cast<const f32x2 *>(axis + 2 * PP - 2);
 }
 
 template <int PP>
@@ -1140,9 +1174,9 @@ __global__ void __launch_bounds__(128) p2m_leaf3(const float *__restrict__ pts, 
                                                 const int *__restrict__ box_list, int nlist) {
     using G = Leaf3<PP>;
     constexpr int P = PP * PP * PP;
-    // the Lagrange rows of a chunk; after the last chunk the same memory holds one partial moment array per stream
-    constexpr int NSCR = (G::TP * L3_RS > G::NSTREAM * P) ? G::TP * L3_RS : G::NSTREAM * P;
-    __shared__ __align__(16) float rows[NSCR];
+    // the warps' rows; at the end of a block of points the same memory holds one partial moment array per stream
+    constexpr int NSCR = (4 * G::ROWS * G::RS > G::NSTREAM * P) ? 4 * G::ROWS * G::RS : G::NSTREAM * P;
+    __shared__ __align__(16) float scr[NSCR];
     const LeafWork lw = leaf_work(off, nb, n, box_list, nlist, chunk, src_begin, src_end);
     const int box = lw.box, s0 = lw.s0, s1 = lw.s1;
     if (s0 >= s1) return;
@@ -1151,58 +1185,67 @@ __global__ void __launch_bounds__(128) p2m_leaf3(const float *__restrict__ pts, 
     const int sub = lane / PP, m2 = lane - sub * PP;
     const bool active = sub < G::SUB;
     const int stream = warp * G::SUB + sub;
-    // Running sums grow inaccurate with the square root of their length: after some fifty terms per stream (BLOCK points) they are
-    // added up over the streams and kept by the threads that write the moments.
-    constexpr int BLOCK = 1024 / G::TP * G::TP;
+    float *rows = scr + warp * G::ROWS * G::RS;
+    // Running sums grow inaccurate with the square root of their length: after some fifty terms in either half of a stream (BLOCK
+    // points) they are added up over the streams and kept by the threads that write the moments.
+    constexpr int BLOCK = 2048 / (4 * G::WP) * (4 * G::WP);
     float tot[(P + 127) / 128];
 #pragma unroll
     for (int t = 0; t < (P + 127) / 128; t++) tot[t] = 0.f;
-    // the point of the next chunk is fetched while the streams consume the current one
-    float px[3] = {0.f, 0.f, 0.f}, pb = 0.f;
+    // the next two points of the lane are fetched while the streams consume the current ones; points past the end weigh nothing
+    float xa[3], xb[3], ba, bb;
     auto fetch = [&](int base) {
-        const int i = base + (int)threadIdx.x;
-        if (i < s1) {
-            px[0] = pts[i]; px[1] = pts[(size_t)n + i]; px[2] = pts[(size_t)2 * n + i];
-            pb = bs[(size_t)i * R + r0];
+        const int ia = base + lane, ib = ia + G::ROWS;
+        const bool ha = ia < s1, hb = ib < s1;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            xa[k] = ha ? pts[(size_t)k * n + ia] : c[k];
+            xb[k] = hb ? pts[(size_t)k * n + ib] : c[k];
         }
+        ba = ha ? bs[(size_t)ia * R + r0] : 0.f;
+        bb = hb ? bs[(size_t)ib * R + r0] : 0.f;
     };
-    fetch(s0);
+    fetch(s0 + warp * G::WP);
     for (int block = s0; block < s1; block += BLOCK) {
-        float acc[PP][PP];
+        f32x2 acc[PP][PP];
 #pragma unroll
         for (int i = 0; i < PP; i++)
 #pragma unroll
-            for (int j = 0; j < PP; j++) acc[i][j] = 0.f;
-        for (int base = block; base < min(block + BLOCK, s1); base += G::TP) {
-            const int cnt = min(G::TP, s1 - base);
-            __syncthreads();
-            if ((int)threadIdx.x < cnt)   // the column value rides on the L2 row
-                leaf3_rows_xyz<PP>(px, c, factor, nt, pb, rows + threadIdx.x * L3_RS);
-            fetch(base + G::TP);
-            __syncthreads();
+            for (int j = 0; j < PP; j++) acc[i][j] = 0ull;
+        const int bend = min(block + BLOCK, s1);
+        for (int base = block + warp * G::WP; base < bend; base += 4 * G::WP) {
+            __syncwarp();
+            if (lane < G::ROWS) leaf3_row_pair<PP>(xa, xb, c, factor, nt, pack2(ba, bb), rows + lane * G::RS);
+            fetch(base + 4 * G::WP);
+            __syncwarp();
+            const int cnt = min(G::ROWS, s1 - base);
             if (active)
-                for (int j = stream; j < cnt; j += G::NSTREAM) {
-                    const float *row = rows + j * L3_RS;
-                    const float4 a0 = *reinterpret_cast<const float4 *>(row), a1 = *reinterpret_cast<const float4 *>(row + 4);
-                    const float4 b0 = *reinterpret_cast<const float4 *>(row + 8), b1 = *reinterpret_cast<const float4 *>(row + 12);
-                    const float l0[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                    const float l1[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                    const float w2 = row[16 + m2];
+#pragma unroll 1
+                for (int j = sub; j < cnt; j += G::SUB) {
+                    const float *row = rows + j * G::RS;
+                    f32x2 l0[PP], l1[PP];
+                    leaf3_load_axis<PP>(row, l0);
+                    leaf3_load_axis<PP>(row + G::AX, l1);
+                    const f32x2 w2 = *reinterpret_cast<const f32x2 *>(row + 2 * G::AX + 2 * m2);
 #pragma unroll
                     for (int i1 = 0; i1 < PP; i1++) {
-                        const float u = w2 * l1[i1];
+                        const f32x2 u = mul2(w2, l1[i1]);
 #pragma unroll
-                        for (int i0 = 0; i0 < PP; i0++) acc[i1][i0] = fmaf(u, l0[i0], acc[i1][i0]);
+                        for (int i0 = 0; i0 < PP; i0++) acc[i1][i0] = fma2(u, l0[i0], acc[i1][i0]);
                     }
                 }
         }
         __syncthreads();
         if (active) {
-            float *mine = rows + stream * P + PP * PP * m2;
+            float *mine = scr + stream * P + PP * PP * m2;
 #pragma unroll
             for (int i1 = 0; i1 < PP; i1++)
 #pragma unroll
-                for (int i0 = 0; i0 < PP; i0++) mine[i0 + PP * i1] = acc[i1][i0];
+                for (int i0 = 0; i0 < PP; i0++) {
+                    float a, b;
+                    unpack2(acc[i1][i0], a, b);
+                    mine[i0 + PP * i1] = a + b;
+                }
         }
         __syncthreads();
 #pragma unroll
@@ -1211,10 +1254,11 @@ __global__ void __launch_bounds__(128) p2m_leaf3(const float *__restrict__ pts, 
             float v = 0.f;
             if (q < P) {
 #pragma unroll
-                for (int st = 0; st < G::NSTREAM; st++) v += rows[st * P + q];
+                for (int st = 0; st < G::NSTREAM; st++) v += scr[st * P + q];
             }
             tot[t] += v;
         }
+        __syncthreads();
     }
     float *dst = lw.slot < 0 ? mom + (size_t)box * P : part + lw.slot * P;
 #pragma unroll
@@ -1229,59 +1273,76 @@ __global__ void __launch_bounds__(128) l2p_leaf3(const float *__restrict__ pts, 
                                                 float *out, const int *__restrict__ box_list) {
     using G = Leaf3<PP>;
     constexpr int P = PP * PP * PP;
-    __shared__ __align__(16) float rows[G::TP * L3_RS];
-    __shared__ float part[G::TP * 8];   // per point: the PP partial sums over m2
+    __shared__ __align__(16) float scr[4 * G::ROWS * G::RS];
     const int box = box_list ? box_list[blockIdx.x] : (int)blockIdx.x;
     const int a = off[box], b = off[box + 1];
     if (a < row_begin || a >= row_end) return;    // finest-level boxes belong to the slice their first point is in
     const int len = b - a;
     const int s0 = a + (int)(((long long)len * blockIdx.y) / nsplit), s1 = a + (int)(((long long)len * (blockIdx.y + 1)) / nsplit);
-    if (s0 >= s1) return;
-    const float c[3] = {ctr[box * 3], ctr[box * 3 + 1], ctr[box * 3 + 2]};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (s0 + warp * G::WP >= s1) return;          // warps do not meet
+    const float c[3] = {ctr[box * 3], ctr[box * 3 + 1], ctr[box * 3 + 2]};
     const int sub = lane / PP, m2 = lane - sub * PP;
     const bool active = sub < G::SUB;
-    const int stream = warp * G::SUB + sub;
-    float lc[PP][PP];   // loc[m0][m1][m2] of this lane's m2
+    float *rows = scr + warp * G::ROWS * G::RS;
+    f32x2 lc[PP][PP];   // loc[m0][m1][m2] of this lane's m2, twice
 #pragma unroll
     for (int i1 = 0; i1 < PP; i1++)
 #pragma unroll
-        for (int i0 = 0; i0 < PP; i0++) lc[i1][i0] = active ? __ldg(loc + (size_t)box * P + i0 + PP * i1 + PP * PP * m2) : 0.f;
-    float px[3] = {0.f, 0.f, 0.f};
+        for (int i0 = 0; i0 < PP; i0++) {
+            const float v = active ? __ldg(loc + (size_t)box * P + i0 + PP * i1 + PP * PP * m2) : 0.f;
+            lc[i1][i0] = pack2(v, v);
+        }
+    float xa[3], xb[3], oa, ob;
     auto fetch = [&](int base) {
-        const int i = base + (int)threadIdx.x;
-        if (i < s1) { px[0] = pts[i]; px[1] = pts[(size_t)n + i]; px[2] = pts[(size_t)2 * n + i]; }
+        const int ia = base + lane, ib = ia + G::ROWS;
+        const bool mine = lane < G::ROWS, ha = mine && ia < s1, hb = mine && ib < s1;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            xa[k] = ha ? pts[(size_t)k * n + ia] : c[k];
+            xb[k] = hb ? pts[(size_t)k * n + ib] : c[k];
+        }
+        oa = ha ? out[(size_t)ia * R + r0] : 0.f;
+        ob = hb ? out[(size_t)ib * R + r0] : 0.f;
     };
-    fetch(s0);
-    for (int base = s0; base < s1; base += G::TP) {
-        const int cnt = min(G::TP, s1 - base);
-        __syncthreads();
-        if ((int)threadIdx.x < cnt) leaf3_rows_xyz<PP>(px, c, factor, nt, 1.f, rows + threadIdx.x * L3_RS);
-        fetch(base + G::TP);   // the next chunk's point, while the streams consume this one
-        __syncthreads();
+    fetch(s0 + warp * G::WP);
+    for (int base = s0 + warp * G::WP; base < s1; base += 4 * G::WP) {
+        __syncwarp();
+        if (lane < G::ROWS) leaf3_row_pair<PP>(xa, xb, c, factor, nt, pack2(1.f, 1.f), rows + lane * G::RS);
+        const float pa = oa, pb = ob;
+        fetch(base + 4 * G::WP);   // the next points and their sums so far, while the streams consume these
+        __syncwarp();
+        const int cnt = min(G::ROWS, s1 - base);
         if (active)
-            for (int j = stream; j < cnt; j += G::NSTREAM) {
-                const float *row = rows + j * L3_RS;
-                const float4 a0 = *reinterpret_cast<const float4 *>(row), a1 = *reinterpret_cast<const float4 *>(row + 4);
-                const float4 b0 = *reinterpret_cast<const float4 *>(row + 8), b1 = *reinterpret_cast<const float4 *>(row + 12);
-                const float l0[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const float l1[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                float sacc = 0.f;
+#pragma unroll 1
+            for (int j = sub; j < cnt; j += G::SUB) {
+                float *row = rows + j * G::RS;
+                f32x2 l0[PP], l1[PP];
+                leaf3_load_axis<PP>(row, l0);
+                leaf3_load_axis<PP>(row + G::AX, l1);
+                f32x2 *w2 = reinterpret_cast<f32x2 *>(row + 2 * G::AX + 2 * m2);
+                f32x2 sum = 0ull;
 #pragma unroll
                 for (int i1 = 0; i1 < PP; i1++) {
-                    float t = 0.f;
+                    f32x2 t = mul2(l0[0], lc[i1][0]);
 #pragma unroll
-                    for (int i0 = 0; i0 < PP; i0++) t = fmaf(l0[i0], lc[i1][i0], t);
-                    sacc = fmaf(l1[i1], t, sacc);
+                    for (int i0 = 1; i0 < PP; i0++) t = fma2(l0[i0], lc[i1][i0], t);
+                    sum = fma2(l1[i1], t, sum);
                 }
-                part[j * 8 + m2] = row[16 + m2] * sacc;
+                *w2 = mul2(*w2, sum);   // only this lane reads the entry: the partial sums over m2 take its place
             }
-        __syncthreads();
-        if ((int)threadIdx.x < cnt) {
-            float v = 0.f;
+        __syncwarp();
+        if (lane < cnt) {
+            f32x2 l2[PP];
+            leaf3_load_axis<PP>(rows + lane * G::RS + 2 * G::AX, l2);
+            f32x2 v = l2[0];
 #pragma unroll
-            for (int q = 0; q < PP; q++) v += part[threadIdx.x * 8 + q];
-            out[(size_t)(base + threadIdx.x) * R + r0] += v;
+            for (int q = 1; q < PP; q++) v = add2(v, l2[q]);
+            float va, vb;
+            unpack2(v, va, vb);
+            const int ia = base + lane, ib = ia + G::ROWS;
+            out[(size_t)ia * R + r0] = pa + va;
+            if (ib < s1) out[(size_t)ib * R + r0] = pb + vb;
         }
     }
 }
@@ -1289,6 +1350,7 @@ __global__ void __launch_bounds__(128) l2p_leaf3(const float *__restrict__ pts, 
 // Small finest-level boxes (clustered data leaves millions of boxes with a handful of points): one warp per box, so
 // that a box costs a few hundred instructions instead of a CTA's launch, barriers and reductions.
 constexpr int LEAF_SMALL = 32;
+constexpr int SMALL_RS = 28;   // floats between their rows [L0 (8) | L1 (8) | L2 (8) | pad (4)]
 
 __global__ void __launch_bounds__(256) split_leaf_boxes(int nb, const int *__restrict__ off, int *small_list, int *big_list, int *counts) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1305,7 +1367,7 @@ __global__ void __launch_bounds__(128) p2m_small3(const float *__restrict__ pts,
                                                  NodeTab2 nt, int src_begin, int src_end, float *mom,
                                                  const int *__restrict__ box_list, int nlist) {
     constexpr int P = PP * PP * PP, NPL = (P + 31) / 32;
-    __shared__ __align__(16) float rows_s[4][LEAF_SMALL * L3_RS];
+    __shared__ __align__(16) float rows_s[4][LEAF_SMALL * SMALL_RS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int li = blockIdx.x * 4 + warp;
     if (li >= nlist) return;
@@ -1314,7 +1376,7 @@ __global__ void __launch_bounds__(128) p2m_small3(const float *__restrict__ pts,
     if (a < src_begin || a >= src_end) return;
     const float c[3] = {ctr[box * 3], ctr[box * 3 + 1], ctr[box * 3 + 2]};
     float *rows = rows_s[warp];
-    if (lane < len) leaf3_rows<PP>(pts, n, a + lane, c, factor, nt, bs[(size_t)(a + lane) * R + r0], rows + lane * L3_RS);
+    if (lane < len) leaf3_rows<PP>(pts, n, a + lane, c, factor, nt, bs[(size_t)(a + lane) * R + r0], rows + lane * SMALL_RS);
     __syncwarp();
     float acc[NPL];
     int o0[NPL], o1[NPL], o2[NPL];
@@ -1325,7 +1387,7 @@ __global__ void __launch_bounds__(128) p2m_small3(const float *__restrict__ pts,
         o0[q] = m % PP; o1[q] = 8 + (m / PP) % PP; o2[q] = 16 + m / (PP * PP);
     }
     for (int j = 0; j < len; j++) {
-        const float *row = rows + j * L3_RS;
+        const float *row = rows + j * SMALL_RS;
 #pragma unroll
         for (int q = 0; q < NPL; q++) acc[q] = fmaf(row[o2[q]] * row[o1[q]], row[o0[q]], acc[q]);
     }
