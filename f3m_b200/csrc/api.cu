@@ -380,6 +380,7 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     for (float &m : pl->last.ms) m = 0.f;
     pl->last.ms[ST_BUILD] = pl->stats.build_ms;
     pl->last.clear_counts();
+    pl->weights_ok = -1;
     pl->last.begin(ST_TOTAL, s);
     pl->pack_cache.reset();
     struct DropPacked { f3m_plan *p; ~DropPacked() { p->pack_cache.reset(); } } drop_packed{pl};

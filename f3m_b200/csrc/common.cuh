@@ -193,6 +193,7 @@ enum FlagSlot {
     FL_MMA_COUNTER = 32, // tile cursor of the tensor-core near kernel
     FL_LEAF = 40,        // 2 words: small / big finest-level boxes
     FL_NSMALL = 42,      // target tiles of at most 32 points
+    FL_WEIGHTS = 43,     // a weight is not finite, or near the largest float
     FL_LVTOT = 64,       // boxes per level of the batch being built (F3M_MAX_LEVELS words)
     FL_LVMAX = 96,       // largest box per level (F3M_MAX_LEVELS words)
     FL_PAIRWORK = 128    // 4 words per direct list (PAIRWORK_LISTS of them): 64-bit sums of n_x * n_y and of n_x over its box pairs
@@ -256,8 +257,8 @@ struct LevelLists {
 // Device time per stage, from CUDA events recorded on the product's stream and read after its
 // final synchronisation (no extra synchronisation inside the product).
 enum Stage { ST_PERMUTE = 0, ST_DIRECT = 1, ST_P2M = 2, ST_M2L = 3, ST_L2P = 4, ST_UNPERMUTE = 5, ST_TOTAL = 6, ST_BUILD = 7 };
-// forms of the direct-sum kernels (counted per launch, see f3m_plan_last_direct_variants)
-enum DirectVariant { DV_MUFU = 0, DV_POLY2 = 1, DV_POLY3 = 2, DV_DIRECT = 3, DV_MOMENTS = 4, DV_TENSOR = 5, DV_COUNT = 6 };
+// forms of the direct-sum kernels (counted per launch; the first six by f3m_plan_last_direct_variants)
+enum DirectVariant { DV_MUFU = 0, DV_POLY2 = 1, DV_POLY3 = 2, DV_DIRECT = 3, DV_MOMENTS = 4, DV_TENSOR = 5, DV_NODES = 6, DV_COUNT = 7 };
 struct Timings {
     float ms[8] = {0};
     int direct_launches = 0;
@@ -338,6 +339,14 @@ struct f3m_plan {
         f3m::DevBuf<float> buf;
         void reset() { level = -1; buf.release(); }
     } pack_cache;
+    // direct lists taken through nodes (near_nodes.cu): a level's rows in the order of the box offsets, built on first use
+    struct NodeRows {
+        bool ready = false, small = false, keep = false;   // which lists the rows hold
+        f3m::DevBuf<int> ptr, oidx;
+        f3m::DevBuf<uint32_t> okey;
+    };
+    std::vector<NodeRows> node_rows;
+    int weights_ok = -1;                  // of the product under way: all weights finite (-1: not looked at yet)
     // a product shared by several GPUs, in phases (f3m_plan_shard_begin / _near / _far): state kept between the calls
     struct Shard {
         bool active = false;
@@ -412,7 +421,15 @@ void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, con
 // near_moments.cu: sums a direct list through box moments when its geometry allows; false: sum the pairs
 bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted, int row_begin,
                  int row_end, cudaStream_t s);
-double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate
+double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate, pairs or moments
+// near_nodes.cu: the direct lists of a level through interpolation nodes (whole products of one column)
+struct NodeChoice {
+    int p = 0;                          // nodes per axis, 0: no list of the level takes this form
+    bool small = false, keep = false;   // the lists that do (near list: last level only)
+    double seconds = 0.0;               // estimated time of the level's direct lists with this choice
+};
+NodeChoice node_choice(const f3m_plan *pl, int level, int R);
+bool node_sums(f3m_plan *pl, int level, const NodeChoice &choice, const float *b_sorted, float *out_sorted, cudaStream_t s);
 template <bool GRAD>
 void dense_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,
                cudaStream_t s);

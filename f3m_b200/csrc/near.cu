@@ -793,9 +793,8 @@ static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *b
     }
 }
 
-void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out_sorted, int64_t row_begin,
+static void direct_sums_plain(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out_sorted, int64_t row_begin,
                  int64_t row_end, cudaStream_t s) {
-    if (csr.count == 0) return;
     const int rb = (int)row_begin, re = (int)row_end;
     if (moment_sums(pl, level, csr, bs, R, out_sorted, rb, re, s)) return;
     switch (pl->d) {
@@ -805,6 +804,20 @@ void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, i
         case 4: direct_d<4>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
         default: direct_d<5>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
     }
+}
+
+void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out_sorted, int64_t row_begin,
+                 int64_t row_end, cudaStream_t s) {
+    if (csr.count == 0) return;
+    LevelLists &ll = pl->lists[level];
+    const bool keep = &csr == &ll.keep, whole = row_begin <= 0 && row_end >= pl->tx.n && !pl->shard.active && !pl->ext_mom;
+    const NodeChoice c = whole && R == 1 && level > 0 ? node_choice(pl, level, R) : NodeChoice{};
+    if (c.p && (keep ? c.keep : c.small)) {
+        if (!keep && c.keep) return;   // summed with the near list
+        if (node_sums(pl, level, c, bs, out_sorted, s)) return;
+        if (keep && c.small) direct_sums_plain(pl, level, ll.small, bs, R, out_sorted, row_begin, row_end, s);
+    }
+    direct_sums_plain(pl, level, csr, bs, R, out_sorted, row_begin, row_end, s);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,101 @@
+"""Direct lists through interpolation nodes (near_nodes.cu) against float64, over the node counts and the shapes of boxes."""
+import pytest
+import torch
+
+from cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# Relative to the 2-norm of the product, normal weights: a fifth of the interpolation bound 4e-7, and roundings of 6e-8 in moments and
+# expansions that Lagrange weights of either sign enlarge (12 for nine nodes in three dimensions) and random signs keep to a few.
+TOL = 1.2e-6
+
+
+def _used(plan):
+    return plan.timings()["direct_launches"] > 0 and plan.last_work()["pairs"] == 0 and not any(plan.direct_variants().values())
+
+
+def _plan(X, ls, leaf, nodes, cuda):
+    from f3m_b200 import engine
+    return engine.Plan(X.to(cuda), None, engine.make_params(ls, leaf, nodes, False, 0.15, nodes))
+
+
+# edge over lengthscale -> nodes per axis 7, 8, 9, 10, 11, 12, 13; far fields stay empty: every pair of boxes holds fewer than 2 P points
+@pytest.mark.parametrize("edge", [0.5, 0.7, 1.0, 1.3, 1.6, 1.95, 2.3])
+@pytest.mark.parametrize("shape", ["long", "short"])
+def test_against_float64(edge, shape, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(int(100 * edge))
+    level = 1 if shape == "long" else 2     # boxes of 4000 points (summed in parts) or of 480
+    X = torch.rand(32003 if shape == "long" else 30707, 3, generator=g) + 1.3   # coordinates that are large against the boxes
+    n = X.shape[0]
+    side = float((X.max(0).values - X.min(0).values).max()) * 1.01
+    ls = side / 2 ** level / edge
+    b = torch.randn(n, 1, generator=g)
+    plan = _plan(X, ls, 2000.0 if shape == "long" else 300.0, 5000 if shape == "long" else 1000, cuda)
+    out = plan.apply(b.to(cuda))
+    assert plan.stats()["levels"] == level and plan.stats()["far_box_pairs"] == 0
+    assert _used(plan)
+    Xd = X.to(cuda).double()
+    exact = engine.rbf_dense(Xd, Xd, b.to(cuda).double(), ls)
+    assert rel_l2(out.cpu(), exact.cpu()) <= TOL
+    again = plan.apply(b.to(cuda))          # the ordered rows are kept in the plan
+    assert torch.equal(out, again)
+    half = n // 2 + 3
+    parts = plan.apply(b.to(cuda), row_range=(0, half)) + plan.apply(b.to(cuda), row_range=(half, n))   # slices sum the pairs
+    assert rel_l2(out.cpu(), parts.cpu()) <= TOL + rel_l2(parts.cpu(), exact.cpu())
+
+
+@pytest.mark.parametrize("edge", [0.5, 0.7, 1.0, 1.3, 1.6, 1.95, 2.3])
+def test_uneven_boxes(edge, cuda):
+    """Boxes of some tens to four thousand points, far pairs beside the direct ones: against the same lists summed pair by pair."""
+    g = torch.Generator().manual_seed(int(100 * edge))
+    n = 1500011
+    X = torch.rand(n, 3, generator=g) ** 1.4 + 1.3
+    b = torch.rand(n, 1, generator=g) + 0.5
+    plan = _plan(X, 1.01 / 16 / edge, 6000.0, 216, cuda)
+    assert plan.stats()["levels"] == 4
+    out = plan.apply(b.to(cuda))
+    assert plan.timings()["direct_launches"] > 0 and plan.last_work()["pairs"] < plan.stats()["direct_pairs"] // 2
+    assert torch.equal(plan.apply(b.to(cuda)), out)
+    parts = plan.apply(b.to(cuda), row_range=(0, 700001)) + plan.apply(b.to(cuda), row_range=(700001, n))
+    assert plan.last_work()["pairs"] > 0
+    assert rel_l2(out.cpu(), parts.cpu()) <= 2 * TOL
+
+
+def test_weights_that_are_not_finite(cuda):
+    """An infinite weight gives what the pairs give: infinity, and NaN rows for a NaN weight."""
+    g = torch.Generator().manual_seed(3)
+    X = torch.rand(30707, 3, generator=g)
+    plan = _plan(X, 0.25, 300.0, 1000, cuda)
+    b = torch.rand(30707, 1, generator=g) + 0.5
+    plan.apply(b.to(cuda))
+    assert _used(plan)
+    for value in (float("inf"), float("nan"), 3e38):
+        c = b.clone()
+        c[777] = value
+        out = plan.apply(c.to(cuda))
+        half = 15000
+        parts = plan.apply(c.to(cuda), row_range=(0, half)) + plan.apply(c.to(cuda), row_range=(half, 30707))
+        assert torch.equal(torch.isnan(out), torch.isnan(parts)) and torch.equal(torch.isinf(out), torch.isinf(parts))
+        assert not torch.isfinite(out).all() or value == 3e38
+    plan.apply(b.to(cuda))
+    assert _used(plan)
+
+
+def test_small_workspace_sums_the_pairs(cuda):
+    """A workspace without room for the moments: the product is there all the same."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(4)
+    X = torch.rand(32003, 3, generator=g).to(cuda)
+    b = torch.rand(32003, 1, generator=g).to(cuda)
+    prm = engine.make_params(0.22, 2000.0, 5000, False, 0.15, 5000)
+    want = engine.kmvm(X, None, b, prm)
+    for mb in (64, 8, 6, 5, 4):
+        ws = torch.empty(mb << 20, dtype=torch.uint8, device=cuda)
+        try:
+            out = engine.kmvm_ws(X, None, b, prm, ws)
+        except RuntimeError as e:
+            assert "workspace" in str(e)
+            continue
+        assert rel_l2(out.cpu(), want.cpu()) <= TOL
