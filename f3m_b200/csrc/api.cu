@@ -382,8 +382,8 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     pl->last.clear_counts();
     pl->weights_ok = -1;
     pl->last.begin(ST_TOTAL, s);
-    pl->pack_cache.reset();
-    struct DropPacked { f3m_plan *p; ~DropPacked() { p->pack_cache.reset(); } } drop_packed{pl};
+    struct DropPacked { f3m_plan *p; void drop() { p->pack_cache.reset(); p->column_rows.reset(); } ~DropPacked() { drop(); } } drop_packed{pl};
+    drop_packed.drop();
 
     pl->last.begin(ST_PERMUTE, s);
     DevBuf<float> bs, outs;
@@ -650,8 +650,8 @@ int f3m_plan_shard_near(f3m_plan *plan, float *acc_sorted, void *stream) {
         F3M_REQUIRE(sh.active, F3M_ERR_ARG, "f3m_plan_shard_near without f3m_plan_shard_begin");
         const int L = plan->levels, R = sh.R;
         const int64_t rb = sh.row_begin, re = sh.row_end;
-        plan->pack_cache.reset();
-        struct DropPacked { f3m_plan *p; ~DropPacked() { p->pack_cache.reset(); } } drop_packed{plan};
+        struct DropPacked { f3m_plan *p; void drop() { p->pack_cache.reset(); p->column_rows.reset(); } ~DropPacked() { drop(); } } drop_packed{plan};
+        drop_packed.drop();
         if (re > rb) F3M_CUDA(cudaMemsetAsync(acc_sorted + rb * R, 0, (size_t)(re - rb) * R * sizeof(float), s));
         if (L == 0) direct_sums(plan, 0, plan->lists[0].keep, sh.bs.p, R, acc_sorted, rb, re, s);
         for (int level = 1; level <= L; level++) direct_sums(plan, level, plan->lists[level].small, sh.bs.p, R, acc_sorted, rb, re, s);

@@ -347,6 +347,12 @@ struct f3m_plan {
     };
     std::vector<NodeRows> node_rows;
     int weights_ok = -1;                  // of the product under way: all weights finite (-1: not looked at yet)
+    // source rows of the several-column kernel (near_cols.cu; valid inside one product)
+    struct ColumnRows {
+        int r0 = -1;
+        f3m::DevBuf<float> buf;
+        void reset() { r0 = -1; buf.release(); }
+    } column_rows;
     // a product shared by several GPUs, in phases (f3m_plan_shard_begin / _near / _far): state kept between the calls
     struct Shard {
         bool active = false;

@@ -733,19 +733,19 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 }
 
 // Several columns: the stream of sources (near_columns, near_cols.cu) or the tiles of this file?  Seconds per pair over the whole chip, from
-// direct sums of 280 trees (d = 1..5, uniform and normal, 5e3 to 1e6 points, boxes of 3 to 600 points, 2 to 8 columns).  The
-// stream always carries eight columns; a tile pays its coordinates and columns again on every source box, so it falls behind as the
-// rows per source box shorten, most in the difference form, which does not pack its operands.  Tile / stream time by sources per row
-// and source box, 8 columns: d = 2 16: 1.5, 62: 1.1, 247: 0.93; d = 3 9: 2.5, 74: 1.03, 247: 0.80; d = 4 15: 2.1, 72: 1.07, 247: 0.86;
-// d = 5 9: 2.7, 156: 1.3, 297: 0.94.  Four columns: d = 2 16: 1.1, 62: 0.68; d = 3 9: 1.8, 74: 0.75; d = 4 15: 1.5, 72: 0.8; d = 5
-// 9: 2.3, 297: 0.73.  Difference form, d = 3, 8 / 4 columns: 7: 6.4 / 5.1, 74: 1.8 / 1.3, 591: 1.3 / 0.88.
-// Fewer targets than fill the SMs with tiles of 64 (a CTA each, 20 per SM) make the tiles up to 1.6 times slower than that, the stream's shorter
-// and more numerous ones less (d = 3, 3e4 points, 4 columns, 59 sources 1.2; d = 5, 65 sources 1.7).
-// With four columns the constants lean to the tiles where rows hold some 15 to 30 sources: uneven trees lose there (d = 4, 4.8e5 normal
-// points, 2 columns, whole call 20.2 -> 22.6 ms on the stream).
+// direct sums of some 100 trees (d = 2..5, uniform and normal, 3e4 to 6e5 points, boxes of 3 to 940 points, 2, 4 and 8 columns).  A
+// tile pays its coordinates and columns again on every source box, so it falls behind as the rows per source box shorten, most in the
+// difference form, which does not pack its operands; the stream pays a fetch per source and tile of up to 64 rows.  Tile / stream time by
+// sources per row and source box, 8 columns: d = 2 460: 1.35, 790: 1.18; d = 3 19: 1.65, 45: 1.33, 148: 1.01; d = 4 9: 4.7, 49: 1.36, 148:
+// 1.05, 790: 1.45; d = 5 28: 2.8, 197: 1.31, 940: 1.39.  Two and four columns (half the multiply-adds in either kernel): d = 2 790: 0.97; d = 3
+// 19: 1.5, 45: 1.24, 148: 0.95; d = 4 9: 4.3, 49: 1.28, 148: 0.95, 790: 1.16; d = 5 28: 3.5, 197: 1.31.  Difference form, d = 3, 8 / 4 columns:
+// 47: 2.05 / 1.95, 124: 1.7 / 1.6, 390: 1.8 / 1.8; d = 4 157: 1.8 / 1.7; d = 5 24: 5.1 / 5.4, 197: 1.8 / 1.75.  What is left to the tiles are
+// boxes of hundreds of points and more in the expanded form of two and three dimensions.
+// Fewer targets than fill the SMs with tiles of 64 (a CTA each, 20 per SM) make the tiles up to 1.6 times slower than that.
 // One dimension stays with the tiles: its lists name three boxes, too short for the stream's set-up (1e6 points, 4 columns 0.85).
-static double stream_seconds(int d, bool narrow, double row) {
-    return narrow ? 6.5e-14 * (d + 8) + 1e-11 / row : 6.1e-14 * (2 * d + 8) + 1.8e-11 / row;
+static double stream_seconds(int d, bool narrow, int cols, double row) {
+    const int c = cols > 4 ? 8 : narrow ? 5 : 4;
+    return narrow ? 5.0e-14 * (d + c) + 1.2e-11 / std::max(row, 12.0) : 5.0e-14 * (2 * d + c) + 1.5e-11 / row;
 }
 static double tile_seconds(int d, bool expanded, int cols, double row, int64_t targets) {
     const int RB = cols >= 5 ? 8 : 4;
@@ -760,7 +760,7 @@ static double column_seconds(const f3m_plan *pl, int level, const PairCSR &csr, 
     const double se = (double)near_scale(pl->lcs) * pl->ty->levels[level].edge;
     const bool narrow = se <= 1.0, expanded = narrow && d * list_reach(pl, level, csr) * se * se <= TMAX_EXPANDED;
     const double row = (double)csr.pairs / (double)std::max<int64_t>(1, csr.row_boxes);
-    const double st = stream_seconds(d, narrow, row), ti = tile_seconds(d, expanded, cols, row, pl->tx.n);
+    const double st = stream_seconds(d, narrow, cols, row), ti = tile_seconds(d, expanded, cols, row, pl->tx.n);
     stream = d >= 2 && st <= ti;
     return stream ? st : ti;
 }

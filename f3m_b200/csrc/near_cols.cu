@@ -1,17 +1,18 @@
 // Direct sums of the near / small field with several right-hand sides (near_field_run, F3M_src/n_tree.cu:831-902).
 //
-// Boxes of a few to some forty points (near.cu has the rule).  A pair costs its exponent (d multiply-adds in the expanded form,
-// 2 d in the difference form), one exponential and 8 multiply-adds into the columns.  The kernels of near.cu lose their time
-// there on every source box: its rows through shared memory, target coordinates and factors anew, tiles and row pairs half empty.
-// Here the sources of a tile are ONE stream, box borders left out, and a warp takes 8 MT targets and 16 sources at a time: lane
-// (g, t) owns the targets g, g + 8, .. and the sources 4t .. 4t + 3 of the 16.  Two columns share an instruction (f32x2).  All
-// in FP32: the columns as split TF32 products on mma.sync lost what the split's parts cannot hold (the NaN of GPU arithmetic,
-// values near either end of the exponent range) and were no faster.
+// A pair costs its exponent (d multiply-adds in the expanded form, 2 d in the difference form), one exponential and 8 (or 4)
+// multiply-adds into the columns.  The kernels of near.cu lose their time on every source box: its rows through shared memory,
+// target coordinates and factors anew, tiles and row pairs half empty.  Here the sources of a tile are ONE stream, box borders left out,
+// and the targets of sibling boxes with equal lists are one box (near.cu has the rule when which kernel runs).  A warp takes up
+// to 64 targets: a lane owns four of them and every second quadruple of sources (smaller tiles: every fourth), so that a source's row
+// is read by half-warps at one address each.  Sources are rows of 64 bytes, copied 64 at a time with cp.async while the 64 before
+// them are summed.  Two columns share an instruction (f32x2).  All in FP32: the columns as split TF32 products on mma.sync lost
+// what the split's parts cannot hold (the NaN of GPU arithmetic, values near either end of the exponent range) and were no faster.
 //
-// What bounds it: FMA lanes (57 % busy at boxes of 246 points, d = 4) and the shared-memory pipe (70 %), which carries a source
-// to every tile that reads it; with short boxes the latter, as a source then serves few rows.  Direct sums of 8 columns, all lists on
-// the kernels of near.cu / short boxes as split TF32 / short boxes here: 1e6 points N(0,I), d = 5 60.7 / 36.0 / 31.7 ms, d = 4 33.5 /
-// 26.5 / 22.6 ms; 3e5 points U[0,1]^5 in boxes of nine 40.3 / 17.9 / 14.4 ms.  All lists here: 1e6 points in boxes of 246, d = 4 8.0 -> 9.1 ms.
+// What bounds it: FMA lanes and the issue slots of the pairs.  8 columns, d = 5: 16.7 cycles per 32 pairs and SM quarter with everything in
+// registers, 25 here (FMA pipe 61 % busy, 13.5 instructions of the ideal 11).  Before, tiles of 32 targets each box by itself, sources
+// gathered float by float and no overlap of copies and sums took 34 to 50.  Direct sums of 8 columns, then / now: 1e6 points N(0,I), d = 5 (boxes
+// of 18 points on average, 139 weighted by pairs) 119.5 / 87.4 ms, d = 4 21.8 / 15.3 ms; 3e5 points, d = 5 22.1 / 10.9 ms.
 #include <math.h>
 #include <algorithm>
 #include "common.cuh"
@@ -19,190 +20,216 @@
 
 namespace f3m {
 
-constexpr int CM = 4;        // target rows per lane
-constexpr int CT = 8 * CM;   // targets per tile
-constexpr int CR = 8;        // columns
+constexpr int CT = 64;       // targets per tile
 
-// asynchronous copies into shared memory
-__device__ __forceinline__ void c_copy4(float *dst, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void c_copy16(float *dst, const float *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void c_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void c_copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void c_copy_wait_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-constexpr int CST = 128;     // sources staged before they are summed: their copies are in flight together
-// Staged sources: a plane per coordinate (in the expanded form one more for minus the squared length), read four sources at a
-// time, then the rows of b; every four rows are followed by four floats, so that the lanes' 16-byte accesses meet no bank twice.
-template <int D, bool DIFF> struct ColStage {
-    static constexpr int COORDS = DIFF ? D : D + 1;
-    static constexpr int FLOATS = COORDS * CST + CST / 4 * (4 * CR + 4);
-    static __device__ __forceinline__ int b_row(int q) { return COORDS * CST + q * CR + (q >> 2) * 4; }
-};
+// A source is a row of 16 floats: its coordinates (in shared memory scaled and, in the expanded form, followed by minus their
+// squared length), at CB the columns of b.  Staged rows are 20 floats apart: the lanes' 16-byte accesses to eight rows meet no bank twice.
+constexpr int CROW = 16, CB = 8, CSTRIDE = 20;
+constexpr int CST = 64;      // sources staged at a time; the next ones are copied while these are summed
 
-// tiles[b] = tiles of the rows of target box b inside [row_begin, row_end)
-__global__ void __launch_bounds__(256) col_tiles_per_box(int nbx, const int *__restrict__ off_x, const int *__restrict__ ptr, int row_begin,
-                                                        int row_end, int *tiles) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+// Siblings whose rows of the list are equal -- most of them, where all boxes around are small: the classes depend on the two boxes' sizes
+// first -- are summed as one target box, around their parent's centre: tiles fill up, and a source is fetched once for all of
+// them.  first[b] = 1 where a new group begins (always at a new parent); a warp per box.
+__global__ void __launch_bounds__(256) col_groups(int nbx, const int *__restrict__ parent, const int *__restrict__ ptr, const int *__restrict__ idx,
+                                                 int group, int *first) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (b > nbx) return;
+    bool same = group && b > 0 && b < nbx && parent[b] == parent[b - 1];
+    if (same) {
+        const int p0 = ptr[b - 1], p1 = ptr[b], len = p1 - p0;
+        same = ptr[b + 1] - p1 == len;
+        for (int e = lane; same && e - lane < len; e += 32) same = !__any_sync(0xffffffffu, e < len && idx[p0 + e] != idx[p1 + e]);
+    }
+    if (lane == 0) first[b] = !same;
+}
+
+// items[b] = tiles of the rows of the group that begins with target box b inside [row_begin, row_end), times the parts its list is cut
+// into (chunk sources each, 0: not cut); a warp per box
+struct ColGroup { int boxes, parts; };
+__global__ void __launch_bounds__(256) col_items(int nbx, const int *__restrict__ off_x, const int *__restrict__ ptr, const int *__restrict__ idx,
+                                                const int *__restrict__ off_y, const int *__restrict__ first, int chunk, int row_begin,
+                                                int row_end, int *items, ColGroup *groups) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b > nbx) return;
     int t = 0;
-    if (b < nbx && ptr[b + 1] > ptr[b]) t = (max(0, min(off_x[b + 1], row_end) - max(off_x[b], row_begin)) + CT - 1) / CT;
-    tiles[b] = t;
-}
-
-// how the rows of b are copied: eight columns in two 16-byte copies, or four in one
-enum ColCopy { COPY_8, COPY_4 };
-
-// Rows of eight columns, from r0 on, zeros where b has none: other row lengths than multiples of four would be copied float by
-// float, which meets the same banks (direct sums of 2 columns, 1e6 normal points, d = 5: 37.6 ms, with padded rows 28.0).
-__global__ void __launch_bounds__(256) pad_columns(const float *__restrict__ bs, int64_t n, int R, int r0, float *dst) {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n * CR) return;
-    const int r = r0 + (int)(i % CR);
-    dst[i] = r < R ? bs[i / CR * R + r] : 0.f;
-}
-
-// stream positions pos .. pos + take of the loaded entries -> staged sources fill .. fill + take
-template <int D, bool DIFF, int COPY>
-__device__ __forceinline__ void col_gather(float *stage, const int *entries, int pos, int fill, int take, const float *__restrict__ ypts,
-                                           int n_y, const float *__restrict__ bs, int bw) {
-    using S = ColStage<D, DIFF>;
-    const int lane = threadIdx.x;
+    ColGroup g{1, 1};
+    if (b < nbx && first[b] && ptr[b + 1] > ptr[b]) {
+        while (!first[b + g.boxes]) g.boxes++;      // first[nbx] = 1
+        t = (max(0, min(off_x[b + g.boxes], row_end) - max(off_x[b], row_begin)) + CT - 1) / CT;
+        if (chunk && t) {
+            int64_t sum = 0;
+            for (int e = ptr[b] + lane; e < ptr[b + 1]; e += 32) { const int by = idx[e]; sum += off_y[by + 1] - off_y[by]; }
 #pragma unroll
-    for (int u = 0; u < CST / 32; u++) {
-        if (lane + 32 * u >= take) continue;
-        const int p = pos + lane + 32 * u;
-        int lo = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (entries[lo + step] <= p) lo += step;
-        const int j = p + entries[32 + lo];
-        const int q = fill + lane + 32 * u;
-#pragma unroll
-        for (int k = 0; k < D; k++) c_copy4(stage + k * CST + q, ypts + (size_t)k * n_y + j);
-        float *dst = stage + S::b_row(q);
-        const float *b = bs + (size_t)j * bw;
-        c_copy16(dst, b);
-        if (COPY == COPY_8) c_copy16(dst + 4, b + 4);
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            g.parts = (int)min((int64_t)(ptr[b + 1] - ptr[b]), max((int64_t)1, (sum + chunk - 1) / chunk));
+        }
+    }
+    if (lane == 0) {
+        items[b] = t * g.parts;
+        if (b < nbx) groups[b] = g;
     }
 }
 
-// The list arrives 32 entries at a time (lane = entry): they are prefix-summed, and a lane finds the source of its stream position
-// by bisection.  All coordinates are relative to the centre c of the TARGET box, which keeps them for the whole list: with
-// X = s (x-c), Y = s (y-c) the exponent -|X-Y|^2 is, in the expanded form, (2 X.Y - |Y|^2) - |X|^2, whose last part leaves the
-// sum; |X|^2 is at most d/4 there (boxes up to one scaled unit), so the terms of the bracket cancel by no more than that and no
-// factor overflows.  Wide boxes take the differences.
-template <int D, bool DIFF, int MT>
-__device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int n_x, float *stage, int *entries,
-                                            const int *__restrict__ idx, int e0, int e1, const int *__restrict__ off_y,
-                                            const float *__restrict__ ypts, int n_y, const float *__restrict__ bs, const float (&c)[D],
-                                            float scale, int bw, int copy, int R, int r0, float *out, int t0, int nt) {
-    using S = ColStage<D, DIFF>;
-    const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+template <int D>
+__global__ void __launch_bounds__(256) pack_column_rows(const float *__restrict__ pts, int64_t n, const float *__restrict__ bs, int R, int r0,
+                                                       float *rows) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j = i / CROW;
+    if (j >= n) return;
+    const int c = (int)(i % CROW), r = r0 + c - CB;
+    rows[i] = c < D ? pts[(size_t)c * n + j] : (c >= CB && r < R) ? bs[j * R + r] : 0.f;
+}
+
+// The list arrives 32 entries at a time (lane = entry; the next 32 are read ahead) and is prefix-summed; 32 stream positions at a
+// time, a lane counts the entries that start up to its own.  All coordinates are relative to the centre c of the TARGET box, which keeps them for the
+// whole list: with X = s (x-c), Y = s (y-c) the exponent -|X-Y|^2 is, in the expanded form, (2 X.Y - |Y|^2) - |X|^2, whose last part
+// leaves the sum; |X|^2 is at most d/4 there (boxes up to one scaled unit), so the terms of the bracket cancel by no more than that and
+// no factor overflows.  Wide boxes take the differences.
+// A lane owns MT target rows, TR = 32 / G of them apart, and every G-th quadruple of sources; NC = 8 or 4 columns.
+template <int D, bool DIFF, int NC, int G, int MT>
+__device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int n_x, float *stages, const int *__restrict__ idx, int e0,
+                                            int e1, const int *__restrict__ off_y, const float *__restrict__ rows, const float (&c)[D],
+                                            float scale, int R, int r0, float *out, int t0, int nt, bool shared) {
+    constexpr int TR = 32 / G, STEP = 4 * G;
+    const int lane = threadIdx.x, g = lane % TR, h = lane / TR;
     float xr[MT][D];
-    f32x2 acc[MT][CR / 2], tot[MT][CR / 2];
+    f32x2 acc[MT][NC / 2], tot[MT][NC / 2];
 #pragma unroll
     for (int m = 0; m < MT; m++) {
-        const int i = t0 + min(8 * m + g, nt - 1);
+        const int i = t0 + min(TR * m + g, nt - 1);
 #pragma unroll
         for (int k = 0; k < D; k++) {
             const float x = scale * (xpts[(size_t)k * n_x + i] - c[k]);
             xr[m][k] = DIFF ? x : 2.f * x;
         }
 #pragma unroll
-        for (int r = 0; r < CR / 2; r++) acc[m][r] = tot[m][r] = pack2(0.f, 0.f);
+        for (int r = 0; r < NC / 2; r++) acc[m][r] = tot[m][r] = pack2(0.f, 0.f);
     }
-    if (copy == COPY_4)   // the other four columns are never copied
-        for (int q = S::COORDS * CST + lane; q < S::FLOATS; q += 32) stage[q] = 0.f;
-    int e = e0, total = 0, pos = 0;   // entries not loaded yet, stream positions loaded and used
-    int fill = 0;                     // staged sources
-    while (true) {
-        if (pos == total && e < e1) {
-            int len = 0, s0 = 0;
-            if (e + lane < e1) {
-                const int by = idx[e + lane];
-                s0 = off_y[by];
-                len = off_y[by + 1] - s0;
-            }
-            int inc = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
-            }
-            total = __shfl_sync(0xffffffffu, inc, 31);
-            __syncwarp();
-            entries[lane] = inc - len;               // first stream position of the entry
-            entries[32 + lane] = s0 - (inc - len);   // sorted row of stream position p: p + this
-            __syncwarp();
-            pos = 0;
-            e = min(e + 32, e1);
+    int e = e0, total = 0, pos = 0;    // entries not loaded yet, stream positions loaded and used
+    int start = 0, shift = 0;          // the lane's entry: its first stream position (past all for none), sorted row of position p: p + shift
+    int nlen = 0, nrow = 0;            // the lane's entry among the next 32
+    auto read_ahead = [&]() {
+        nlen = nrow = 0;
+        if (e + lane < e1) {
+            const int by = idx[e + lane];
+            nrow = off_y[by];
+            nlen = off_y[by + 1] - nrow;
         }
-        const int take = min(CST - fill, total - pos);
-        // one loop per kind of copy: the four gathers of a lane stay together only without branches inside
-        if (copy == COPY_8) col_gather<D, DIFF, COPY_8>(stage, entries, pos, fill, take, ypts, n_y, bs, bw);
-        else col_gather<D, DIFF, COPY_4>(stage, entries, pos, fill, take, ypts, n_y, bs, bw);
-        pos += take;
-        fill += take;
-        const bool last = pos == total && e >= e1;
-        if (fill < CST && !last) continue;
-        c_copy_wait();
+    };
+    read_ahead();
+    // copies the next sources of the stream into a stage, as many as fit; how many they are
+    auto fetch = [&](float *stage) {
+        int fill = 0;
+        while (fill < CST) {
+            if (pos == total) {
+                if (e >= e1) break;
+                const int len = nlen, s0 = nrow;
+                e = min(e + 32, e1);
+                read_ahead();
+                int inc = len;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                total = __shfl_sync(0xffffffffu, inc, 31);
+                start = len ? inc - len : 0x7fffffff;
+                shift = s0 - (inc - len);
+                pos = 0;
+            }
+            const int take = min(32, min(CST - fill, total - pos));
+            const int before = __popc(__ballot_sync(0xffffffffu, start < pos)), rel = start - pos;
+            const unsigned starts = __reduce_or_sync(0xffffffffu, (unsigned)rel < 32u ? 1u << rel : 0u);
+            const int entry = before + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
+            const int j = pos + lane + __shfl_sync(0xffffffffu, shift, entry & 31);
+            if (lane < take) {
+                const float *src = rows + (size_t)j * CROW;
+                float *dst = stage + (fill + lane) * CSTRIDE;
+#pragma unroll
+                for (int q = 0; q < CROW; q += 4)
+                    if (q < D || (q >= CB && q < CB + NC)) c_copy16(dst + q, src + q);
+            }
+            pos += take;
+            fill += take;
+        }
+        return fill;
+    };
+    int fill = fetch(stages), cur = 0;
+    c_copy_commit();
+    while (fill > 0) {
+        float *stage = stages + cur * (CST * CSTRIDE);
+        const int next = fetch(stages + (cur ^ 1) * (CST * CSTRIDE));
+        c_copy_commit();
+        c_copy_wait_but_last();
         __syncwarp();
-        const int ngr = (fill + 15) >> 4;
-        for (int q = lane; q < 16 * ngr; q += 32) {
+        const int ngr = (fill + STEP - 1) / STEP;
+        for (int q = lane; q < STEP * ngr; q += 32) {
+            float4 *row = reinterpret_cast<float4 *>(stage + q * CSTRIDE);
             if (q < fill) {
+                float y[8];
+#pragma unroll
+                for (int k = 0; k < (D > 4 ? 8 : 4); k += 4) {
+                    const float4 v = row[k / 4];
+                    y[k] = v.x; y[k + 1] = v.y; y[k + 2] = v.z; y[k + 3] = v.w;
+                }
                 float n2 = 0.f;
 #pragma unroll
                 for (int k = 0; k < D; k++) {
-                    const float v = scale * (stage[k * CST + q] - c[k]);
-                    n2 = fmaf(-v, v, n2);
-                    stage[k * CST + q] = v;
+                    y[k] = scale * (y[k] - c[k]);
+                    n2 = fmaf(-y[k], y[k], n2);
                 }
-                if (!DIFF) stage[D * CST + q] = n2;
+                if (!DIFF) y[D] = n2;
+                row[0] = make_float4(y[0], y[1], y[2], y[3]);
+                if (D + !DIFF > 4) *reinterpret_cast<float2 *>(row + 1) = make_float2(y[4], y[5]);
             } else {   // the sources that fill the last group weigh nothing
 #pragma unroll
-                for (int k = 0; k < S::COORDS; k++) stage[k * CST + q] = 0.f;
-#pragma unroll
-                for (int r = 0; r < CR; r++) stage[S::b_row(q) + r] = 0.f;
+                for (int k = 0; k < CROW / 4; k++) row[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         __syncwarp();
 #pragma unroll 1
         for (int gr = 0; gr < ngr; gr++) {
-            const float *p = stage + 16 * gr + 4 * t;
-            float y[S::COORDS][4];
-#pragma unroll
-            for (int k = 0; k < S::COORDS; k++) {
-                const float4 v = *reinterpret_cast<const float4 *>(p + k * CST);
-                y[k][0] = v.x; y[k][1] = v.y; y[k][2] = v.z; y[k][3] = v.w;
-            }
-            const ulonglong2 *pb = reinterpret_cast<const ulonglong2 *>(stage + S::b_row(16 * gr + 4 * t));
+            const float *p = stage + (STEP * gr + 4 * h) * CSTRIDE;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const ulonglong2 b01 = pb[2 * q], b23 = pb[2 * q + 1];
+                float y[6];
+                const float4 y0 = *reinterpret_cast<const float4 *>(p + q * CSTRIDE);
+                y[0] = y0.x; y[1] = y0.y; y[2] = y0.z; y[3] = y0.w;
+                if (D + !DIFF > 4) {
+                    const float2 y4 = *reinterpret_cast<const float2 *>(p + q * CSTRIDE + 4);
+                    y[4] = y4.x; y[5] = y4.y;
+                }
+                const ulonglong2 b01 = *reinterpret_cast<const ulonglong2 *>(p + q * CSTRIDE + CB);
+                const ulonglong2 b23 = NC > 4 ? *reinterpret_cast<const ulonglong2 *>(p + q * CSTRIDE + CB + 4) : b01;
 #pragma unroll
                 for (int m = 0; m < MT; m++) {
                     float v;
                     if (DIFF) {
-                        float df = xr[m][0] - y[0][q];
+                        float df = xr[m][0] - y[0];
                         v = -df * df;
 #pragma unroll
                         for (int k = 1; k < D; k++) {
-                            df = xr[m][k] - y[k][q];
+                            df = xr[m][k] - y[k];
                             v = fmaf(-df, df, v);
                         }
                     } else {
-                        v = fmaf(xr[m][0], y[0][q], y[S::COORDS - 1][q]);
+                        v = fmaf(xr[m][0], y[0], y[D]);
 #pragma unroll
-                        for (int k = 1; k < D; k++) v = fmaf(xr[m][k], y[k][q], v);
+                        for (int k = 1; k < D; k++) v = fmaf(xr[m][k], y[k], v);
                     }
                     const float ev = ex2_approx(v);
                     const f32x2 e2 = pack2(ev, ev);
                     acc[m][0] = fma2(e2, b01.x, acc[m][0]);
                     acc[m][1] = fma2(e2, b01.y, acc[m][1]);
-                    acc[m][2] = fma2(e2, b23.x, acc[m][2]);
-                    acc[m][3] = fma2(e2, b23.y, acc[m][3]);
+                    if (NC > 4) {
+                        acc[m][NC / 2 - 2] = fma2(e2, b23.x, acc[m][NC / 2 - 2]);
+                        acc[m][NC / 2 - 1] = fma2(e2, b23.y, acc[m][NC / 2 - 1]);
+                    }
                 }
             }
         }
@@ -210,26 +237,29 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
 #pragma unroll
         for (int m = 0; m < MT; m++)
 #pragma unroll
-            for (int r = 0; r < CR / 2; r++) {
+            for (int r = 0; r < NC / 2; r++) {
                 tot[m][r] = add2(tot[m][r], acc[m][r]);
                 acc[m][r] = pack2(0.f, 0.f);
             }
-        if (last) break;
-        fill = 0;
         __syncwarp();
+        fill = next;
+        cur ^= 1;
     }
 #pragma unroll
     for (int m = 0; m < MT; m++) {
-        // the four lanes of a target add up their sources: columns 2t, 2t + 1 end in lane t
-        float v[CR], half[CR / 2], sum[2];
+        // the G lanes of a target add up their sources: columns CPL h .. CPL h + CPL - 1 end in lane h
+        constexpr int CPL = NC / G;
+        float v[NC], half[NC / 2], sum[CPL];
 #pragma unroll
-        for (int r = 0; r < CR / 2; r++) unpack2(tot[m][r], v[2 * r], v[2 * r + 1]);
+        for (int r = 0; r < NC / 2; r++) unpack2(tot[m][r], v[2 * r], v[2 * r + 1]);
+        const bool up = h >= G / 2, odd = h & 1;
 #pragma unroll
-        for (int r = 0; r < CR / 2; r++)
-            half[r] = ((t & 2) ? v[r + 4] : v[r]) + __shfl_xor_sync(0xffffffffu, (t & 2) ? v[r] : v[r + 4], 2);
+        for (int r = 0; r < NC / 2; r++) half[r] = (up ? v[r + NC / 2] : v[r]) + __shfl_xor_sync(0xffffffffu, up ? v[r] : v[r + NC / 2], 16);
 #pragma unroll
-        for (int r = 0; r < 2; r++)
-            sum[r] = ((t & 1) ? half[r + 2] : half[r]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? half[r] : half[r + 2], 1);
+        for (int r = 0; r < CPL; r++) {
+            const float other = half[(r + CPL) % (NC / 2)];
+            sum[r] = G == 2 ? half[r] : (odd ? other : half[r]) + __shfl_xor_sync(0xffffffffu, odd ? half[r] : other, TR);
+        }
         float f = 1.f;
         if (!DIFF) {   // 2^(-|X|^2); xr holds 2 X
             float n2 = 0.f;
@@ -237,41 +267,50 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
             for (int k = 0; k < D; k++) n2 = fmaf(xr[m][k], xr[m][k], n2);
             f = ex2_approx(-0.25f * n2);
         }
-        const int i = 8 * m + g, r = r0 + 2 * t;
+        const int i = TR * m + g, r = r0 + CPL * h;
         if (i >= nt) continue;
         float *o = out + (size_t)(t0 + i) * R + r;
-        if (r < R) o[0] += f * sum[0];
-        if (r + 1 < R) o[1] += f * sum[1];
+#pragma unroll
+        for (int q = 0; q < CPL; q++)
+            if (r + q < R) {
+                if (shared) atomicAdd(o + q, f * sum[q]);   // the parts of a long list
+                else o[q] += f * sum[q];
+            }
     }
 }
 
-template <int D, bool DIFF>
+template <int D, bool DIFF, int NC>
 __global__ void __launch_bounds__(32, 16) near_columns(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x, int nbx,
-                                                       const float *__restrict__ ctr_x, const int *__restrict__ tile_off,
-                                                       const int *__restrict__ ptr, const int *__restrict__ idx,
-                                                       const int *__restrict__ off_y, const float *__restrict__ ypts, int n_y,
-                                                       const float *__restrict__ bs, float scale, int bw, int copy, int R, int r0, float *out,
-                                                       int row_begin, int row_end) {
-    __shared__ __align__(16) float stage[ColStage<D, DIFF>::FLOATS];
-    __shared__ int entries[64];
+                                                       const float *__restrict__ ctr_x, const int *__restrict__ parent,
+                                                       const float *__restrict__ parent_ctr, const int *__restrict__ item_off,
+                                                       const ColGroup *__restrict__ groups, const int *__restrict__ ptr, const int *__restrict__ idx,
+                                                       const int *__restrict__ off_y, const float *__restrict__ rows, float scale, int R,
+                                                       int r0, float *out, int row_begin, int row_end) {
+    __shared__ __align__(16) float stage[2 * CST * CSTRIDE];
     const int item = blockIdx.x;
-    if (item >= tile_off[nbx]) return;      // the grid is sized by a bound on the tiles, no read-back
-    const int box = box_of_row(tile_off, nbx, item);
-    // the box's groups of 8 rows are dealt out evenly over its tiles
-    const int a = max(off_x[box], row_begin), len = min(off_x[box + 1], row_end) - a;
-    const int tile = item - tile_off[box], ntiles = tile_off[box + 1] - tile_off[box], units = (len + 7) >> 3;
-    const int t0 = a + 8 * (int)(((long long)units * tile) / ntiles);
-    const int nt = min(a + 8 * (int)(((long long)units * (tile + 1)) / ntiles), a + len) - t0;
+    if (item >= item_off[nbx]) return;      // the grid may be sized by a bound
+    const int box = box_of_row(item_off, nbx, item);
+    const ColGroup group = groups[box];
+    const int np = group.parts, part = (item - item_off[box]) % np, tile = (item - item_off[box]) / np;
+    // the group's rows are dealt out evenly over its tiles, 16 at a time
+    const int a = max(off_x[box], row_begin), len = min(off_x[box + group.boxes], row_end) - a;
+    const int ntiles = (item_off[box + 1] - item_off[box]) / np, units = (len + 15) >> 4;
+    const int t0 = a + 16 * (int)(((long long)units * tile) / ntiles);
+    const int nt = min(a + 16 * (int)(((long long)units * (tile + 1)) / ntiles), a + len) - t0;
     float c[D];
+    const float *centre = group.boxes > 1 ? parent_ctr + parent[box] * D : ctr_x + box * D;
 #pragma unroll
-    for (int k = 0; k < D; k++) c[k] = ctr_x[box * D + k];
-    const int mt = (nt + 7) >> 3;
-    const int e0 = ptr[box], e1 = ptr[box + 1];
-#define F3M_TILE(MT_) column_tile<D, DIFF, MT_>(xpts, n_x, stage, entries, idx, e0, e1, off_y, ypts, n_y, bs, c, scale, bw, copy, R, r0, out, t0, nt)
-    if (mt == 4) F3M_TILE(4);
-    else if (mt == 3) F3M_TILE(3);
-    else if (mt == 2) F3M_TILE(2);
-    else F3M_TILE(1);
+    for (int k = 0; k < D; k++) c[k] = centre[k];
+    const int p0 = ptr[box], n_entries = ptr[box + 1] - p0;
+    const int e0 = p0 + (int)(((long long)n_entries * part) / np), e1 = p0 + (int)(((long long)n_entries * (part + 1)) / np);
+#define F3M_TILE(G_, MT_) \
+    column_tile<D, DIFF, NC, G_, MT_>(xpts, n_x, stage, idx, e0, e1, off_y, rows, c, scale, R, r0, out, t0, nt, np > 1)
+    if (nt > 48) F3M_TILE(2, 4);
+    else if (nt > 32) F3M_TILE(2, 3);
+    else if (nt > 24) F3M_TILE(4, 4);
+    else if (nt > 16) F3M_TILE(4, 3);
+    else if (nt > 8) F3M_TILE(4, 2);
+    else F3M_TILE(4, 1);
 #undef F3M_TILE
 }
 
@@ -281,27 +320,47 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
     Tree &tx = pl->tx, &ty = *pl->ty;
     Level &lx = tx.levels[level], &ly = ty.levels[level];
     const float scale = sqrtf(pl->lcs * 1.4426950408889634f);
-    DevBuf<int> tiles;
-    tiles.alloc((size_t)lx.nb + 1, s);
-    col_tiles_per_box<<<(unsigned)((lx.nb + 1 + 255) / 256), 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, row_begin, row_end, tiles.p);
+    // Boxes in the middle of a cloud have lists a hundred times as long as the average: such a list, summed by one warp, outlasts all others.
+    // Lists of large calls are cut into parts (chunk sources or so each, some ten thousand items in all), and the host reads how
+    // many items there are; small calls launch a bound.
+    const int chunk = csr.pairs >= 100000000 ? (int)std::min<int64_t>(32768, std::max<int64_t>(1024, csr.pairs / 600000)) : 0;
+    // Groups of the expanded form: |X|^2 stays below d/4 times 1.25^2 around a parent's centre.
+    const bool grouped = DIFF || scale * tx.levels[level - 1].edge <= 1.25f;
+    DevBuf<int> items, first;
+    DevBuf<ColGroup> groups;
+    items.alloc((size_t)lx.nb + 1, s);
+    first.alloc((size_t)lx.nb + 1, s);
+    groups.alloc((size_t)lx.nb, s);
+    const unsigned box_warps = (unsigned)(((int64_t)(lx.nb + 1) * 32 + 255) / 256);
+    col_groups<<<box_warps, 256, 0, s>>>(lx.nb, lx.parent.p, csr.ptr.p, csr.idx.p, grouped, first.p);
     F3M_LAUNCH_CHECK();
-    exclusive_scan_i32(tiles.p, tiles.p, (int64_t)lx.nb + 1, s);
-    const int64_t max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1;
-    // rows of b start on 16 bytes: bs starts on 256 bytes, and so does the padded copy that other row lengths get
-    DevBuf<float> padded;
-    if (R % 4) {
-        padded.alloc((size_t)ty.n * CR, s);
+    col_items<<<box_warps, 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, csr.idx.p, ly.off.p, first.p, chunk, row_begin, row_end, items.p, groups.p);
+    F3M_LAUNCH_CHECK();
+    exclusive_scan_i32(items.p, items.p, (int64_t)lx.nb + 1, s);
+    int64_t max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1;
+    if (chunk) {
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, items.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaStreamSynchronize(s));
+        max_items = pl->h_pinned[0];
+        if (max_items <= 0) return;
+    }
+    // one set of rows serves every list of the product
+    f3m_plan::ColumnRows &cr = pl->column_rows;
+    if (cr.r0 != r0) {
+        cr.buf.alloc((size_t)ty.n * CROW, s);
+        cr.r0 = r0;
         pl->last.begin(ST_PERMUTE, s);
-        pad_columns<<<(unsigned)((ty.n * CR + 255) / 256), 256, 0, s>>>(bs, ty.n, R, r0, padded.p);
+        pack_column_rows<D><<<(unsigned)((ty.n * CROW + 255) / 256), 256, 0, s>>>(ty.pts.p, ty.n, bs, R, r0, cr.buf.p);
         pl->last.end(s);
         F3M_LAUNCH_CHECK();
     }
-    const float *b = R % 4 ? padded.p : bs + r0;
-    const int bw = R % 4 ? CR : R, copy = R % 4 || R - r0 >= CR ? COPY_8 : COPY_4;
     pl->last.begin(ST_DIRECT, s);
-    near_columns<D, DIFF><<<(unsigned)max_items, 32, 0, s>>>(
-        tx.pts.p, (int)tx.n, lx.off.p, lx.nb, lx.ctr.p, tiles.p, csr.ptr.p, csr.idx.p, ly.off.p, ty.pts.p, (int)ty.n, b, scale, bw, copy, R, r0, out,
-        row_begin, row_end);
+    auto launch = [&](auto kernel) {
+        kernel<<<(unsigned)max_items, 32, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, lx.ctr.p, lx.parent.p, tx.levels[level - 1].ctr.p, items.p,
+                                                 groups.p, csr.ptr.p, csr.idx.p, ly.off.p, cr.buf.p, scale, R, r0, out, row_begin, row_end);
+    };
+    if (R - r0 <= 4) launch(near_columns<D, DIFF, 4>);
+    else launch(near_columns<D, DIFF, 8>);
     pl->last.end(s);
     pl->last.direct_launches++;
     pl->last.direct_variants[DIFF ? DV_DIRECT : DV_MUFU]++;

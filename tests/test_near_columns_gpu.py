@@ -144,3 +144,23 @@ def test_long_boxes_stay_with_the_tiles(cuda):
         plan = engine.Plan(X, None, engine.make_params(ls, 5.0, 2 ** d, False, 0.15, 10 ** 6, flags=2))
         plan.apply(torch.rand(200_000, R, device=cuda))
         assert plan.last_work()["column_launches"] == 0 and plan.last_work()["pairs"] == 200_000 ** 2
+
+
+# lists of more than 1e8 pairs are cut into parts; siblings whose rows are equal are summed as one box (nodes large: all of them) or keep
+# their own rows (normal points, few nodes: rows differ); tiles of every number of rows; four columns and eight
+@pytest.mark.parametrize("d,n,R,ls,leaf,nodes,dist", [(2, 60011, 8, 0.05, 300.0, 1000, "normal"), (3, 90011, 4, 0.7, 60.0, 64, "normal"),
+                                                      (4, 70003, 8, 1.0, 60.0, 81, "normal"), (4, 70003, 3, 0.1, 60.0, 16, "uniform"),
+                                                      (5, 90001, 2, 1.0, 200.0, 243, "normal"), (5, 60001, 7, 0.5, 40.0, 32, "normal")])
+def test_groups_and_parts_of_long_lists(d, n, R, ls, leaf, nodes, dist, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(41 + d + R)
+    X = (torch.randn(n, d, generator=g) if dist == "normal" else torch.rand(n, d, generator=g)).to(cuda)
+    b = (torch.rand(n, R, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, None, engine.make_params(ls, leaf, nodes, False, 0.15, nodes))
+    assert plan.stats()["direct_pairs"] > 2e8
+    cuts = (0, 5, 1000, 1017, n // 2 + 3, n)
+    parts = sum(plan.apply(b, row_range=(lo, hi)) for lo, hi in zip(cuts, cuts[1:]))
+    assert plan.last_work()["column_launches"] > 0
+    one = torch.cat([sum(plan.apply(b[:, r:r + 1].contiguous(), row_range=(lo, hi)) for lo, hi in ((0, 7), (7, n))) for r in range(R)], 1)
+    assert rel_l2(parts.cpu(), one.cpu()) <= 2e-6    # as in test_columns_of_many_short_boxes
+    assert rel_l2(plan.apply(b).cpu(), one.cpu()) <= 2e-6
