@@ -88,7 +88,8 @@ thread_local Arena *g_arena = nullptr;
 thread_local size_t g_last_ws_peak = 0;
 }  // namespace
 
-void *dev_alloc(size_t bytes, size_t *granted) {
+void *dev_alloc(size_t bytes, size_t *granted, int *device) {
+    *device = -1;
     if (g_arena) {
         void *p = g_arena->take(bytes ? bytes : 1, granted);
         if (!p) {
@@ -101,6 +102,7 @@ void *dev_alloc(size_t bytes, size_t *granted) {
     const size_t need = round_request(bytes);
     int dev = 0;
     F3M_CUDA(cudaGetDevice(&dev));
+    *device = dev;
     {
         std::lock_guard<std::mutex> lk(g_mem_mu);
         int best = -1;
@@ -137,14 +139,13 @@ void *dev_alloc(size_t bytes, size_t *granted) {
     return p;
 }
 
-void dev_free(void *p, size_t granted) {
-    if (g_arena && g_arena->owns(p)) { g_arena->give(p, granted); return; }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, p) == cudaSuccess) dev = attr.device;
+void dev_free(void *p, size_t granted, int device) {
+    if (device < 0) {   // out of a caller's workspace: gone with it, unless the call that was given it is still running
+        if (g_arena && g_arena->owns(p)) g_arena->give(p, granted);
+        return;
+    }
     std::lock_guard<std::mutex> lk(g_mem_mu);
-    g_free_blocks.push_back(FreeBlock{p, granted, dev});
+    g_free_blocks.push_back(FreeBlock{p, granted, device});
 }
 
 }  // namespace f3m
@@ -155,7 +156,7 @@ using namespace f3m;
 // cudaHostAlloc / cudaMalloc / cudaFree serialise the device, so slots are created once and recycled:
 // a plan takes a slot of its device from a free list and gives it back when it is destroyed.
 namespace {
-struct ScratchSlot { int device; int *h_pinned; int *d_flags; };
+struct ScratchSlot { int device; int *h_pinned; int *d_flags; std::vector<cudaEvent_t> *events; };
 std::mutex g_slot_mu;
 std::vector<ScratchSlot> g_free_slots;
 
@@ -169,9 +170,10 @@ ScratchSlot take_slot(int device) {
                 return sl;
             }
     }
-    ScratchSlot sl{device, nullptr, nullptr};
+    ScratchSlot sl{device, nullptr, nullptr, nullptr};
     F3M_CUDA(cudaHostAlloc((void **)&sl.h_pinned, FLAG_WORDS * sizeof(int), cudaHostAllocDefault));
     F3M_CUDA(cudaMalloc((void **)&sl.d_flags, FLAG_WORDS * sizeof(int)));
+    sl.events = new std::vector<cudaEvent_t>();
     return sl;
 }
 void give_slot(const ScratchSlot &sl) {
@@ -180,9 +182,16 @@ void give_slot(const ScratchSlot &sl) {
 }
 }  // namespace
 
+static void plan_take_slot(f3m_plan *pl) {
+    F3M_CUDA(cudaGetDevice(&pl->device));
+    const ScratchSlot sl = take_slot(pl->device);
+    pl->h_pinned = sl.h_pinned;
+    pl->d_flags = sl.d_flags;
+    pl->events = pl->last.events = sl.events;
+}
+
 f3m_plan::~f3m_plan() {
-    last.resolve();
-    if (h_pinned && d_flags) give_slot(ScratchSlot{device, h_pinned, d_flags});
+    if (h_pinned && d_flags) give_slot(ScratchSlot{device, h_pinned, d_flags, events});
 }
 
 template <typename F>
@@ -223,16 +232,11 @@ static int estimate_depth(int64_t n, int d, float min_points) {
 }
 
 static void plan_begin(f3m_plan *pl, int d, const f3m_params *prm, bool same, cudaStream_t s) {
-    F3M_CUDA(cudaGetDevice(&pl->device));
     pl->d = d;
     pl->prm = *prm;
     pl->same = same;
     pl->lcs = 1 / (2 * prm->ls * prm->ls);                // n_tree.cu:1060
-    {
-        ScratchSlot sl = take_slot(pl->device);
-        pl->h_pinned = sl.h_pinned;
-        pl->d_flags = sl.d_flags;
-    }
+    plan_take_slot(pl);
     F3M_CUDA(cudaMemsetAsync(pl->d_flags, 0, FLAG_WORDS * sizeof(int), s));
     pl->last.begin(ST_BUILD, s);
 }
@@ -361,9 +365,6 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
     };
     for (int l = 1; l <= level; l++) take_work(pl->lists[l].small, l);
     if (level > 0) take_work(pl->lists[level].keep, PAIRWORK_LISTS - 1);
-    pl->last.ms[ST_BUILD] = 0.f;
-    pl->last.resolve();
-    pl->stats.build_ms = pl->last.ms[ST_BUILD];
 }
 
 static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t row_begin, int64_t row_end,
@@ -377,10 +378,10 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     const int64_t N = tx.n, M = ty.n;
     row_begin = std::max<int64_t>(0, row_begin);
     row_end = std::min<int64_t>(N, row_end);
-    for (float &m : pl->last.ms) m = 0.f;
-    pl->last.ms[ST_BUILD] = pl->stats.build_ms;
+    pl->last.start_product();
     pl->last.clear_counts();
     pl->weights_ok = -1;
+    const size_t total = pl->last.spans.size();
     pl->last.begin(ST_TOTAL, s);
     struct DropPacked { f3m_plan *p; void drop() { p->pack_cache.reset(); p->column_rows.reset(); } ~DropPacked() { drop(); } } drop_packed{pl};
     drop_packed.drop();
@@ -388,9 +389,8 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     pl->last.begin(ST_PERMUTE, s);
     DevBuf<float> bs, outs;
     bs.alloc((size_t)M * R, s);
-    gather_rows(b, ty.perm.p, bs.p, M, R, s);
     outs.alloc((size_t)N * R, s);
-    outs.zero();
+    gather_rows(b, ty.perm.p, bs.p, M, R, s, outs.p, N * R);
     pl->last.end(s);
 
     // A product over all rows may end at a level whose interpolation is exact for all its pairs (far_cut_level)
@@ -412,11 +412,9 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     if (row_begin <= 0 && row_end >= N) scatter_rows(outs.p, tx.perm.p, out, N, R, s);
     else scatter_rows_nonzero(outs.p, tx.perm.p, out, N, R, s);   // a slice: most rows are zero
     pl->last.end(s);
-    F3M_CUDA(cudaEventRecord(pl->last.spans[0].b, s));   // closes the ST_TOTAL span opened first
-    pl->last.spans[0].closed = true;
+    pl->last.spans[total].b = pl->last.last_end;
     F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, pl->d_flags, sizeof(int), cudaMemcpyDeviceToHost, s));
     F3M_CUDA(cudaStreamSynchronize(s));
-    pl->last.resolve();
     F3M_REQUIRE(pl->h_pinned[0] == 0, F3M_ERR_INTERNAL, "device-side consistency check failed (code %d)", pl->h_pinned[0]);
 }
 
@@ -463,7 +461,7 @@ int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, 
                          void *stream) {
     if (!plan) return F3M_ERR_ARG;
     int st = guarded([&] { plan_apply(plan, b, R, out, row_begin, row_end, (cudaStream_t)stream); });
-    if (st != F3M_OK) { cudaStreamSynchronize((cudaStream_t)stream); plan->last.resolve(); }
+    if (st != F3M_OK) cudaStreamSynchronize((cudaStream_t)stream);
     return st;
 }
 
@@ -522,10 +520,7 @@ int f3m_bounding_box_f32(const float *X, int64_t n, int32_t d, float *min_out, f
     if (!X || !min_out || !max_out || n < 1 || d < 1 || d > F3M_MAX_DIM) return F3M_ERR_ARG;
     return guarded([&] {
         f3m_plan tmp;   // only its scratch words are used
-        F3M_CUDA(cudaGetDevice(&tmp.device));
-        ScratchSlot sl = take_slot(tmp.device);
-        tmp.h_pinned = sl.h_pinned;
-        tmp.d_flags = sl.d_flags;
+        plan_take_slot(&tmp);
         bounding_box(X, n, d, min_out, max_out, &tmp, (cudaStream_t)stream);
     });
 }
@@ -606,8 +601,7 @@ int f3m_plan_shard_begin(f3m_plan *plan, const float *b, int32_t R, int64_t row_
         sh.R = R;
         sh.row_begin = std::max<int64_t>(0, row_begin);
         sh.row_end = std::min<int64_t>(tx.n, row_end);
-        for (float &m : plan->last.ms) m = 0.f;
-        plan->last.ms[ST_BUILD] = plan->stats.build_ms;
+        plan->last.start_product();
         plan->last.clear_counts();
         const int64_t msize = far_moments_size(plan, R);
         const bool exchange = msize > 0 && mom_slice != nullptr;
@@ -846,7 +840,10 @@ int f3m_kmvm_host_f32(const float *X, int64_t N, const float *Y, int64_t M, cons
 
 int f3m_plan_get_stats(const f3m_plan *plan, f3m_plan_stats *stats) {
     if (!plan || !stats) return F3M_ERR_ARG;
+    Timings &t = const_cast<f3m_plan *>(plan)->last;   // events that nobody has read yet
+    t.resolve();
     *stats = plan->stats;
+    stats->build_ms = t.build_ms;
     return F3M_OK;
 }
 
@@ -952,6 +949,7 @@ int f3m_release_cached_memory(void) {
 
 int f3m_plan_last_timings(const f3m_plan *plan, float ms[8]) {
     if (!plan || !ms) return F3M_ERR_ARG;
+    const_cast<f3m_plan *>(plan)->last.resolve();
     for (int i = 0; i < 8; i++) ms[i] = plan->last.ms[i];
     return F3M_OK;
 }

@@ -51,23 +51,24 @@ extern std::atomic<long long> g_launches;   // kernels launched by this library 
 // unpredictable times, 200 ms at a time.)  A released block may be reused immediately by work that is
 // enqueued later on the same stream; every entry point synchronises its stream before it returns, so
 // blocks never cross streams while in use.  f3m_release_cached_memory() returns the free list to the driver.
-void *dev_alloc(size_t bytes, size_t *granted);
-void dev_free(void *p, size_t granted);
+void *dev_alloc(size_t bytes, size_t *granted, int *device);
+void dev_free(void *p, size_t granted, int device);
 
 template <typename T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     size_t granted = 0;
+    int device = 0;
     cudaStream_t s = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), granted(o.granted), s(o.s) { o.p = nullptr; o.n = 0; }
+    DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), granted(o.granted), device(o.device), s(o.s) { o.p = nullptr; o.n = 0; }
     DevBuf &operator=(DevBuf &&o) noexcept {
         if (this != &o) {
             release();
-            p = o.p; n = o.n; granted = o.granted; s = o.s;
+            p = o.p; n = o.n; granted = o.granted; device = o.device; s = o.s;
             o.p = nullptr; o.n = 0;
         }
         return *this;
@@ -77,11 +78,11 @@ struct DevBuf {
         s = stream;
         n = count;
         if (count == 0) count = 1;
-        p = static_cast<T *>(dev_alloc(count * sizeof(T), &granted));
+        p = static_cast<T *>(dev_alloc(count * sizeof(T), &granted, &device));
     }
     void zero() { F3M_CUDA(cudaMemsetAsync(p, 0, (n ? n : 1) * sizeof(T), s)); }
     void release() {
-        if (p) dev_free(p, granted);
+        if (p) dev_free(p, granted, device);
         p = nullptr;
         n = 0;
     }
@@ -252,6 +253,7 @@ struct LevelLists {
     DevBuf<uint32_t> far_okey;
     DevBuf<int> far_oidx;
     bool far_ordered = false;
+    DevBuf<float> T;   // axis matrices of the level (far_fast.cu), built on first use
 };
 
 // Device time per stage, from CUDA events recorded on the product's stream and read after its
@@ -273,18 +275,40 @@ struct Timings {
         for (int &v : direct_variants) v = 0;
         for (int64_t &v : pairs) v = 0;
     }
-    struct Span { int stage; cudaEvent_t a, b; bool closed; };
+    // Events are created once and recycled with the plan's scratch slot (api.cu).  They are read when somebody asks (resolve), not by
+    // every product: a query costs as much as a launch.  A span that begins where the one before ended shares its event.
+    struct Span { int stage, a, b; };      // event numbers; b < 0: not closed
     std::vector<Span> spans;
-    void begin(int stage, cudaStream_t s) {
-        Span sp{stage, nullptr, nullptr, false};
-        F3M_CUDA(cudaEventCreate(&sp.a));
-        F3M_CUDA(cudaEventCreate(&sp.b));
-        F3M_CUDA(cudaEventRecord(sp.a, s));
-        spans.push_back(sp);
+    std::vector<cudaEvent_t> *events = nullptr;
+    int used = 0, last_end = -1;
+    long long launches_at_end = 0;
+    float build_ms = 0.f;
+    int record(cudaStream_t s) {
+        if (used == (int)events->size()) {
+            cudaEvent_t e;
+            F3M_CUDA(cudaEventCreate(&e));
+            events->push_back(e);
+        }
+        F3M_CUDA(cudaEventRecord((*events)[used], s));
+        return used++;
     }
-    void end(cudaStream_t s) {
-        F3M_CUDA(cudaEventRecord(spans.back().b, s));
-        spans.back().closed = true;
+    void begin(int stage, cudaStream_t s) {
+        const bool adjoins = last_end >= 0 && launches_at_end == g_launches.load(std::memory_order_relaxed);
+        spans.push_back(Span{stage, adjoins ? last_end : record(s), -1});
+        last_end = -1;
+    }
+    void end(cudaStream_t s) { close(spans.size() - 1, s); }
+    void close(size_t span, cudaStream_t s) {
+        spans[span].b = last_end = record(s);
+        launches_at_end = g_launches.load(std::memory_order_relaxed);
+    }
+    // a product begins: the spans of the one before are forgotten, the plan's own (the build, if nobody has read it yet) is kept
+    void start_product() {
+        const bool build = !spans.empty() && spans[0].stage == ST_BUILD && spans[0].b >= 0;
+        spans.resize(build ? 1 : 0);
+        used = build ? spans[0].b + 1 : 0;
+        last_end = -1;
+        for (float &m : ms) m = 0.f;
     }
     // Call after the stream has been synchronised.  A span that was never closed (the product failed in between)
     // is dropped; a failed query must not stay behind as the runtime's last error, or the next launch check of an
@@ -292,14 +316,15 @@ struct Timings {
     void resolve() {
         for (auto &sp : spans) {
             float t = 0.f;
-            if (sp.closed) {
-                if (cudaEventElapsedTime(&t, sp.a, sp.b) == cudaSuccess) ms[sp.stage] += t;
-                else (void)cudaGetLastError();
-            }
-            cudaEventDestroy(sp.a);
-            cudaEventDestroy(sp.b);
+            if (sp.b < 0) continue;
+            if (cudaEventElapsedTime(&t, (*events)[sp.a], (*events)[sp.b]) != cudaSuccess) (void)cudaGetLastError();
+            else if (sp.stage == ST_BUILD) build_ms = t;
+            else ms[sp.stage] += t;
         }
         spans.clear();
+        used = 0;
+        last_end = -1;
+        ms[ST_BUILD] = build_ms;
     }
 };
 
@@ -316,6 +341,8 @@ struct f3m_plan {
     std::vector<f3m::LevelLists> lists;   // lists[l] for level l (index 0 unused)
     f3m::LevelLists cut_lists;            // all pairs of the level a product is cut at (count, row pointers and the ordered rows)
     int cut_level = 0;
+    f3m::DevBuf<float> shift_a, shift_at; // matrices between a box and its children, for shift_p nodes; built on first use
+    int shift_p = 0;
     int levels = 0;
     f3m_plan_stats stats{};
     f3m::Timings last;
@@ -364,6 +391,7 @@ struct f3m_plan {
     } shard;
     int *h_pinned = nullptr;              // pinned host words for count read-back (FLAG_WORDS ints)
     int *d_flags = nullptr;               // device status / counters (FLAG_WORDS ints, see FlagSlot)
+    std::vector<cudaEvent_t> *events = nullptr;   // of the scratch slot, see Timings
     ~f3m_plan();
 };
 
@@ -382,7 +410,7 @@ void tree_attach_runs(Tree &t, const uint32_t *recs, int64_t stride, cudaStream_
 void exclusive_scan_i32(const int *in, int *out, int64_t n, cudaStream_t s);  // n values; out may alias in
 // up to four arrays of n values scanned in place by one set of launches; their sums as 64-bit numbers -> totals64 (device)
 void exclusive_scan_multi(int *const *arrays, int narr, int64_t n, long long *totals64, cudaStream_t s);
-void gather_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s);
+void gather_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s, float *zeroed = nullptr, int64_t nz = 0);
 void scatter_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s);
 void scatter_rows_nonzero(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s);
 

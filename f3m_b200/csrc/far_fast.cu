@@ -214,8 +214,11 @@ __global__ void __launch_bounds__(128, 5) m2l_fast(int nbx, int d, const int *__
     constexpr int MS = mat_stride(PP);
     const int bx = blockIdx.x;
     const int e0 = fptr[bx], e1 = fptr[bx + 1];
-    if (e0 == e1) return;
     if (off_x[bx + 1] <= row_begin || off_x[bx] >= row_end) return;   // box has no point in this rank's slice
+    if (e0 == e1) {
+        for (int q = threadIdx.x; q < cfg.P * cfg.RB; q += blockDim.x) loc[(size_t)bx * cfg.P * cfg.RB + q] = 0.f;
+        return;
+    }
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int PR = cfg.P * cfg.RB, ntab = d * NOFF2 * MS;
     float *Tsm = sm;
@@ -403,8 +406,11 @@ __global__ void __launch_bounds__(128, PP <= 6 ? 4 : 2) m2l_nested(int nbx, cons
     constexpr int KA = DD - 1;               // axis applied per pair
     const int bx = blockIdx.x;
     const int e0 = fptr[bx], e1 = fptr[bx + 1];
-    if (e0 == e1) return;
     if (off_x[bx + 1] <= row_begin || off_x[bx] >= row_end) return;
+    if (e0 == e1) {
+        for (int q = threadIdx.x; q < P; q += blockDim.x) loc[(size_t)bx * P + q] = 0.f;
+        return;
+    }
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int ntab = DD * NOFF2 * MS;
     float *Tsm = sm;
@@ -571,8 +577,11 @@ m2l_rows(int nbx, const int *__restrict__ fptr, const uint32_t *__restrict__ oke
     extern __shared__ __align__(16) float sm[];
     const int bx = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const int e0 = fptr[bx], e1 = fptr[bx + 1];
-    if (e0 == e1) return;
     if (off_x[bx + 1] <= row_begin || off_x[bx] >= row_end) return;
+    if (e0 == e1) {
+        for (int q = tid; q < PR; q += NT) loc[(size_t)bx * PR + q] = 0.f;
+        return;
+    }
     constexpr int ntab = DD * NOFF2 * MS;
     float *Tsm = sm, *buf = sm + ntab;
     for (int q = tid; q < ntab; q += NT) Tsm[q] = T[q];
@@ -1086,17 +1095,23 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     }
     for (int l = lmin; l <= L; l++) {
         loc[l].alloc((size_t)tx.levels[l].nb * PR, s);
-        loc[l].zero();
+        // the node-to-node kernels write every box of the levels they run on
+        if ((l == cut ? pl->cut_lists : pl->lists[l]).far.count == 0) loc[l].zero();
     }
-    std::vector<float> hA, hAT;
-    make_shift_tables(nt, hA, hAT);
-    DevBuf<float> A, AT;
-    A.alloc(hA.size(), s); AT.alloc(hAT.size(), s);
-    ShiftTables st{};
-    std::copy(hA.begin(), hA.end(), st.a);
-    std::copy(hAT.begin(), hAT.end(), st.at);
-    shift_tables_kernel<<<1, 128, 0, s>>>(st, (int)hA.size(), A.p, AT.p);
-    F3M_LAUNCH_CHECK();
+    if (pl->shift_p != PP) {
+        std::vector<float> hA, hAT;
+        make_shift_tables(nt, hA, hAT);
+        pl->shift_p = 0;
+        pl->shift_a.alloc(hA.size(), s);
+        pl->shift_at.alloc(hAT.size(), s);
+        ShiftTables st{};
+        std::copy(hA.begin(), hA.end(), st.a);
+        std::copy(hAT.begin(), hAT.end(), st.at);
+        shift_tables_kernel<<<1, 128, 0, s>>>(st, (int)hA.size(), pl->shift_a.p, pl->shift_at.p);
+        F3M_LAUNCH_CHECK();
+        pl->shift_p = PP;
+    }
+    const float *A = pl->shift_a.p, *AT = pl->shift_at.p;
 
     // warps per CTA of the translation kernels, limited by shared memory
     const size_t per_warp = (size_t)3 * PR * sizeof(float);
@@ -1119,7 +1134,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         F3M_CUDA(cudaFuncSetAttribute(m2m_fast<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
         for (int l = Ls - 1; l >= lmin; l--) {
             Level &lp = ty.levels[l], &lc = ty.levels[l + 1];
-            m2m_fast<PP><<<lp.nb, 32 * nw, sm2, s>>>(lp.nb, d, lp.child_start.p, lc.code.p, A.p, cfg, momp[l + 1], mom[l].p);
+            m2m_fast<PP><<<lp.nb, 32 * nw, sm2, s>>>(lp.nb, d, lp.child_start.p, lc.code.p, A, cfg, momp[l + 1], mom[l].p);
             F3M_LAUNCH_CHECK();
         }
     }
@@ -1127,19 +1142,17 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
     // ---- M2L at every level that has far pairs -------------------------------------------------
     pl->last.begin(ST_M2L, s);
     {
-        DevBuf<float> T;
-        T.alloc((size_t)d * NOFF2 * MS, s);
         const size_t tab = (size_t)d * NOFF2 * MS * sizeof(float);
         const int nw = warps_for(tab);
         size_t smem = tab + nw * per_warp;
         const bool acc_reg = cfg.nf <= 64;
         // launcher: static strides for d = 2, 3 with one column, runtime strides otherwise
         auto launch_m2l = [&](int nbx, const int *fptr, const int *fidx, const int *cx, const int *cy, const int *offx,
-                              const Geom2 &geo, const float *momL, float *locL) {
+                              const float *T, const Geom2 &geo, const float *momL, float *locL) {
 #define F3M_M2L_CALL(ACC_, DD_)                                                                                          \
     {                                                                                                                    \
         F3M_CUDA(cudaFuncSetAttribute(m2l_fast<PP, ACC_, DD_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        m2l_fast<PP, ACC_, DD_><<<nbx, 32 * nw, smem, s>>>(nbx, d, fptr, fidx, cx, cy, offx, rb, re, T.p, geo, cfg, momL,  \
+        m2l_fast<PP, ACC_, DD_><<<nbx, 32 * nw, smem, s>>>(nbx, d, fptr, fidx, cx, cy, offx, rb, re, T, geo, cfg, momL,  \
                                                           locL, pl->d_flags);                                            \
     }
             if (RB == 1 && d == 3) { if (acc_reg) F3M_M2L_CALL(true, 3) else F3M_M2L_CALL(false, 3) }
@@ -1170,20 +1183,27 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                 // within a few boxes of -shift/edge; level-1 pairs are children of the root pair: offsets -1, 0, 1
                 geo.dqmin[k] = (l == 1 ? 0 : (int)floor(-sh / (double)lx.edge)) - NOFF2 / 2 + 1;
             }
-            m2l_table2<<<8, 256, 0, s>>>(nt, d, (double)lx.edge, (double)pl->lcs, geo, T.p);
-            F3M_LAUNCH_CHECK();
-            cellx.alloc((size_t)lx.nb * d, s);
-            decode_cells_kernel<<<(lx.nb + 255) / 256, 256, 0, s>>>(lx.nb, l, d, lx.code.p, cellx.p);
-            F3M_LAUNCH_CHECK();
-            const int *cy = cellx.p;
-            if (!pl->same) {
-                celly.alloc((size_t)ly.nb * d, s);
-                decode_cells_kernel<<<(ly.nb + 255) / 256, 256, 0, s>>>(ly.nb, l, d, ly.code.p, celly.p);
+            if (!ll.T.p) {   // a constant of the plan: every product uses as many nodes on the level
+                ll.T.alloc((size_t)d * NOFF2 * MS, s);
+                m2l_table2<<<8, 256, 0, s>>>(nt, d, (double)lx.edge, (double)pl->lcs, geo, ll.T.p);
                 F3M_LAUNCH_CHECK();
-                cy = celly.p;
             }
+            const float *T = ll.T.p;
             const bool nested = RB == 1 && (d == 2 || d == 3) && cfg.nf <= 64;
             const bool rows = !nested && rows_form_available<PP, RB>(d);
+            const int *cy = nullptr;
+            if (!(nested || rows) || !ll.far_ordered) {   // the ordered rows hold the offsets
+                cellx.alloc((size_t)lx.nb * d, s);
+                decode_cells_kernel<<<(lx.nb + 255) / 256, 256, 0, s>>>(lx.nb, l, d, lx.code.p, cellx.p);
+                F3M_LAUNCH_CHECK();
+                cy = cellx.p;
+                if (!pl->same) {
+                    celly.alloc((size_t)ly.nb * d, s);
+                    decode_cells_kernel<<<(ly.nb + 255) / 256, 256, 0, s>>>(ly.nb, l, d, ly.code.p, celly.p);
+                    F3M_LAUNCH_CHECK();
+                    cy = celly.p;
+                }
+            }
             if (nested || rows) {
                 if (!ll.far_ordered) {
                     ll.far_okey.alloc((size_t)ll.far.count, s);
@@ -1200,20 +1220,20 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                 }
             }
             if (rows) {
-                launch_m2l_rows<PP, RB>(d, lx.nb, ll.far.ptr.p, ll.far_okey.p, ll.far_oidx.p, lx.off.p, rb, re, T.p, momp[l], loc[l].p, s);
+                launch_m2l_rows<PP, RB>(d, lx.nb, ll.far.ptr.p, ll.far_okey.p, ll.far_oidx.p, lx.off.p, rb, re, T, momp[l], loc[l].p, s);
             } else if (nested) {
                 const size_t smem_n = tab + (size_t)4 * P * sizeof(float);   // tables + one buffer per warp
                 if (d == 3) {
                     F3M_CUDA(cudaFuncSetAttribute(m2l_nested<PP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_n));
                     m2l_nested<PP, 3><<<lx.nb, 128, smem_n, s>>>(lx.nb, ll.far.ptr.p, ll.far_okey.p, ll.far_oidx.p, lx.off.p, rb, re,
-                                                                  T.p, momp[l], loc[l].p);
+                                                                  T, momp[l], loc[l].p);
                 } else {
                     F3M_CUDA(cudaFuncSetAttribute(m2l_nested<PP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_n));
                     m2l_nested<PP, 2><<<lx.nb, 128, smem_n, s>>>(lx.nb, ll.far.ptr.p, ll.far_okey.p, ll.far_oidx.p, lx.off.p, rb, re,
-                                                                  T.p, momp[l], loc[l].p);
+                                                                  T, momp[l], loc[l].p);
                 }
             } else
-                launch_m2l(lx.nb, ll.far.ptr.p, ll.far.idx.p, cellx.p, cy, lx.off.p, geo, momp[l], loc[l].p);
+                launch_m2l(lx.nb, ll.far.ptr.p, ll.far.idx.p, cellx.p, cy, lx.off.p, T, geo, momp[l], loc[l].p);
             F3M_LAUNCH_CHECK();
         }
     }
@@ -1226,7 +1246,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         F3M_CUDA(cudaFuncSetAttribute(l2l_fast<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
         for (int l = lmin; l < L; l++) {
             Level &lc = tx.levels[l + 1];
-            l2l_fast<PP><<<(lc.nb + nw - 1) / nw, 32 * nw, sm2, s>>>(lc.nb, d, lc.parent.p, lc.code.p, lc.off.p, rb, re, AT.p, cfg,
+            l2l_fast<PP><<<(lc.nb + nw - 1) / nw, 32 * nw, sm2, s>>>(lc.nb, d, lc.parent.p, lc.code.p, lc.off.p, rb, re, AT, cfg,
                                                                     loc[l].p, loc[l + 1].p);
             F3M_LAUNCH_CHECK();
         }
@@ -1367,6 +1387,7 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
     if (cut && pl->cut_level != cut) {   // the number of columns can move the cut
         LevelLists &ll = pl->lists[cut], &all = pl->cut_lists;
         all.far_ordered = false;
+        all.T.release();
         all.far.count = ll.far.count + ll.small.count + ll.keep.count;
         all.p = ll.p;
         pl->cut_level = cut;

@@ -650,8 +650,8 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         Gb.alloc(rows, s);
         pl->last.begin(ST_PERMUTE, s);
         pack_split_rows<D><<<g, 256, 0, s>>>(ty.pts.p, (int)ty.n, bs, R, r0, scale, ly.off.p, ly.nb, ly.ctr.p, Bc.p, rows, Gb.p);
-        pl->last.end(s);
         F3M_LAUNCH_CHECK();
+        pl->last.end(s);
         int *counter = pl->d_flags + FL_MMA_COUNTER;
         F3M_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), s));
         // range of t = 2 u.v - |v|^2 over the pairs of the list: |u| <= reach * se, |v| <= se / 2 per dimension
@@ -678,11 +678,11 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         else if (deg == 3) F3M_NEAR_MMA(3, 5)
         else F3M_NEAR_MMA(0, 0)
 #undef F3M_NEAR_MMA
+        F3M_LAUNCH_CHECK();
         pl->last.end(s);
         pl->last.direct_launches++;
         pl->last.direct_variants[DV_TENSOR]++;
         if (r0 == 0) pl->last.pairs[DV_TENSOR] += csr.pairs;
-        F3M_LAUNCH_CHECK();
         return;
     }
     if (!cached) {
@@ -696,8 +696,8 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
                 ty.pts.p, (int)ty.n, bs, R, r0, scale, ly.off.p, ly.nb, ly.ctr.p, need, nsplit, packed.p);
         } else
             pack_sources<D, RB><<<g, 256, 0, s>>>(ty.pts.p, ty.n, bs, R, r0, scale, packed.p);
-        pl->last.end(s);
         F3M_LAUNCH_CHECK();
+        pl->last.end(s);
     }
     int form = DV_DIRECT;
     pl->last.begin(ST_DIRECT, s);
@@ -725,11 +725,11 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         near_kernel<D, RB, 1><<<items, NT, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, csr.idx.p, ly.off.p,
                                                    packed.p, scale, R, r0, out, row_begin, row_end);
     }
+    F3M_LAUNCH_CHECK();
     pl->last.end(s);
     pl->last.direct_launches++;
     pl->last.direct_variants[form]++;
     if (r0 == 0) pl->last.pairs[form] += level > 0 ? csr.pairs : tx.n * ty.n;
-    F3M_LAUNCH_CHECK();
 }
 
 // Several columns: the stream of sources (near_columns, near_cols.cu) or the tiles of this file?  Seconds per pair over the whole chip, from

@@ -351,8 +351,8 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
         cr.r0 = r0;
         pl->last.begin(ST_PERMUTE, s);
         pack_column_rows<D><<<(unsigned)((ty.n * CROW + 255) / 256), 256, 0, s>>>(ty.pts.p, ty.n, bs, R, r0, cr.buf.p);
-        pl->last.end(s);
         F3M_LAUNCH_CHECK();
+        pl->last.end(s);
     }
     pl->last.begin(ST_DIRECT, s);
     auto launch = [&](auto kernel) {
@@ -361,12 +361,12 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
     };
     if (R - r0 <= 4) launch(near_columns<D, DIFF, 4>);
     else launch(near_columns<D, DIFF, 8>);
+    F3M_LAUNCH_CHECK();
     pl->last.end(s);
     pl->last.direct_launches++;
     pl->last.direct_variants[DIFF ? DV_DIRECT : DV_MUFU]++;
     pl->last.column_launches++;
     if (r0 == 0) pl->last.pairs[DIFF ? DV_DIRECT : DV_MUFU] += csr.pairs;
-    F3M_LAUNCH_CHECK();
 }
 
 // up to eight columns starting at r0; expanded: boxes at most one scaled unit wide

@@ -424,8 +424,8 @@ static void moment_impl(f3m_plan *pl, int level, const PairCSR *l1, const PairCS
     };
     if ((int64_t)(re - rb) >= 256 * NUM_SMS_HINT) eval(near_moments_eval<D, K, RB, 1>, 1);
     else eval(near_moments_eval<D, K, RB, 4>, 4);
-    pl->last.end(s);
     F3M_LAUNCH_CHECK();
+    pl->last.end(s);
     pl->last.direct_launches++;
     pl->last.direct_variants[DV_MOMENTS]++;
     if (K == 2) pl->last.direct_variants[DV_POLY2]++;

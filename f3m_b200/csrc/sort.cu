@@ -517,9 +517,11 @@ __global__ void __launch_bounds__(RS_T, 3) rs_scatter(SortIO io, int64_t n, int 
     }
 }
 
+// zeroed: nz values set to zero on the way (the sums of a product, which would be a launch of their own)
 __global__ void __launch_bounds__(256) gather_rows_kernel(const float *__restrict__ src, const int *__restrict__ perm,
-                                                         float *dst, int64_t n, int cols) {
+                                                         float *dst, int64_t n, int cols, float *zeroed, int64_t nz) {
     int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < nz) zeroed[e] = 0.f;
     if (e >= n * cols) return;
     int64_t i = e / cols;
     int c = (int)(e - i * cols);
@@ -572,10 +574,10 @@ void scatter_rows_nonzero(const float *src, const int *perm, float *dst, int64_t
     scatter_rows_nonzero_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, perm, dst, n, cols);
     F3M_LAUNCH_CHECK();
 }
-void gather_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s) {
-    int64_t tot = n * cols;
+void gather_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s, float *zeroed, int64_t nz) {
+    int64_t tot = std::max(n * cols, nz);
     if (tot == 0) return;
-    gather_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(src, perm, dst, n, cols);
+    gather_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(src, perm, dst, n, cols, zeroed, nz);
     F3M_LAUNCH_CHECK();
 }
 void scatter_rows(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s) {
