@@ -88,6 +88,8 @@ thread_local Arena *g_arena = nullptr;
 thread_local size_t g_last_ws_peak = 0;
 }  // namespace
 
+bool dev_in_workspace() { return g_arena != nullptr; }
+
 void *dev_alloc(size_t bytes, size_t *granted, int *device) {
     *device = -1;
     if (g_arena) {
@@ -216,8 +218,14 @@ static void check_common(const void *X, int64_t N, const void *Y, int64_t M, int
     F3M_REQUIRE(prm->nr_interpolation >= 1, F3M_ERR_ARG, "nr_interpolation must be >= 1");
 }
 
-static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const float *Y, int64_t M, const float *xmin, const float *ymin,
-                              float edge0, cudaStream_t s);
+static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool max_counts_pending, cudaStream_t s);
+
+// the plan's device words on the host; a negative check of the tree ends the build
+static void read_flags(f3m_plan *pl, cudaStream_t s) {
+    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, pl->d_flags, FLAG_WORDS * sizeof(int), cudaMemcpyDeviceToHost, s));
+    F3M_CUDA(cudaStreamSynchronize(s));
+    F3M_REQUIRE(pl->h_pinned[FL_ERR] == 0, F3M_ERR_INTERNAL, "a box has no parent one level up");
+}
 
 // levels the sort covers: the level loop stops at the first level whose largest box holds at most min_points points;
 // for evenly spread points that is the level where the mean occupancy falls below min_points (one more when the mean
@@ -247,9 +255,35 @@ static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, 
     // (smaller) point set, so the sizes must agree too
     plan_begin(pl, d, prm, X == Y && N == M, s);
 
+    // Only the key bits of the levels the loop below will visit are sorted.  If the loop does go deeper than estimated
+    // (clustered points), the trees are sorted again to the full key depth.
+    int depth = estimate_depth(N, d, prm->min_points);
+    if (!pl->same) depth = std::min(depth, estimate_depth(M, d, prm->min_points));
+    pl->ty = pl->same ? &pl->tx : &pl->ty_store;
+    Tree &tx = pl->tx, &ty = *pl->ty;
+
+    // The cube, the sort and the counts of the first levels' boxes follow one another on the device; the host waits once, for the
+    // counts.  A cube that turns out not to be finite has been clamped into by then and ends the build here.
+    unsigned *mx = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX, *my = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX_Y;
+    bounding_box(X, N, d, mx, s);
+    if (!pl->same) bounding_box(Y, M, d, my, s);
+    Cube cx, cy;
+    cx.own = cy.other = mx;
+    cx.other = cy.own = pl->same ? nullptr : my;
+    HeadsBatch hx, hy;
+    const int lmax = std::min(30 / d, 20), first = depth < lmax ? depth : std::min(lmax, 3);
+    build_sorted_tree(tx, X, N, d, cx, prm->math_mode, depth, s);
+    heads_begin(tx, hx, 1, std::min(first, HEADS_BATCH), pl->d_flags + FL_LVTOT, s);
+    if (!pl->same) {
+        build_sorted_tree(ty, Y, M, d, cy, prm->math_mode, depth, s);
+        heads_begin(ty, hy, 1, std::min(first, HEADS_BATCH), pl->d_flags + FL_LVTOT_Y, s);
+    }
+    read_flags(pl, s);
+
     // bounding cube: calculate_edge_X / calculate_edge (n_tree.cu:25-46), float32 throughout
+    const unsigned *words = reinterpret_cast<const unsigned *>(pl->h_pinned);
     float xmin[MAXD], xmax[MAXD], ymin[MAXD], ymax[MAXD];
-    bounding_box(X, N, d, xmin, xmax, pl, s);
+    bounding_box_values(words + FL_BBOX, d, xmin, xmax);
     float range = 0.f;
     bool finite = true;   // std::max drops a NaN operand, so non-finite extents are checked one by one
     for (int k = 0; k < d; k++) {
@@ -257,7 +291,7 @@ static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, 
         range = std::max(range, xmax[k] - xmin[k]);
     }
     if (!pl->same) {
-        bounding_box(Y, M, d, ymin, ymax, pl, s);
+        bounding_box_values(words + FL_BBOX_Y, d, ymin, ymax);
         float ry = 0.f;
         for (int k = 0; k < d; k++) {
             finite = finite && std::isfinite(ymin[k]) && std::isfinite(ymax[k]);
@@ -268,44 +302,89 @@ static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, 
     F3M_REQUIRE(finite, F3M_ERR_ARG, "degenerate or non-finite bounding cube (a coordinate is NaN or infinite)");
     float edge0 = range * 1.01f;
     F3M_REQUIRE(edge0 > 0.f && std::isfinite(edge0), F3M_ERR_ARG, "degenerate or non-finite bounding cube (edge %g)", edge0);
-
-    // Only the key bits of the levels the loop below will visit are sorted.  If the loop does go deeper than estimated
-    // (clustered points), the trees are sorted again to the full key depth.
-    int depth = estimate_depth(N, d, prm->min_points);
-    if (!pl->same) depth = std::min(depth, estimate_depth(M, d, prm->min_points));
-    build_sorted_tree(pl->tx, X, N, d, xmin, edge0, prm->math_mode, depth, s);
-    build_root(pl->tx, s);
-    if (pl->same) pl->ty = &pl->tx;
-    else {
-        build_sorted_tree(pl->ty_store, Y, M, d, ymin, edge0, prm->math_mode, depth, s);
-        build_root(pl->ty_store, s);
-        pl->ty = &pl->ty_store;
+    tx.edge0 = ty.edge0 = edge0;
+    for (int k = 0; k < d; k++) {
+        tx.origin[k] = xmin[k];
+        if (!pl->same) ty.origin[k] = ymin[k];
     }
-    plan_build_levels(pl, X, N, Y, M, xmin, ymin, edge0, s);
+    build_roots(pl, s);
+    heads_finish(tx, hx, pl->h_pinned + FL_LVTOT, pl->d_flags + FL_LVMAX, pl->d_flags + FL_ERR, s);
+    if (!pl->same) heads_finish(ty, hy, pl->h_pinned + FL_LVTOT_Y, pl->d_flags + FL_LVMAX_Y, pl->d_flags + FL_ERR, s);
+    plan_build_levels(pl, X, Y, true, s);
 }
 
-// second half of the plan: levels, interaction lists, work accounting (the trees hold sorted points)
-static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const float *Y, int64_t M, const float *xmin, const float *ymin,
-                              float edge0, cudaStream_t s) {
+// Entries a level's list can have: kept pairs of one tree are at most two boxes apart, 3^d offsets and the 2 d (and, in four dimensions,
+// 16) that lie on that distance; of two trees, whose boxes are shifted against each other, 4^d.  Every kept parent has 2^d children.
+static int64_t list_bound(const f3m_plan *pl, int level) {
+    const int d = pl->d;
+    const double parents = pl->same ? pow(3.0, d) + 2 * d : pow(4.0, d);
+    const int64_t row = std::min<int64_t>(pl->ty->levels[level].nb, (int64_t)(parents * pow(2.0, d)));
+    return row * pl->tx.levels[level].nb;
+}
+// Lists up to this bound are given the bound's memory and written without asking how long they are.
+constexpr int64_t LIST_BOUND = 1 << 21;
+
+// second half of the plan: levels, interaction lists, work accounting (the trees hold sorted points).  max_counts_pending: the largest
+// boxes of the levels built so far are still on the device.
+static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool max_counts_pending, cudaStream_t s) {
     const f3m_params *prm = &pl->prm;
     const int d = pl->d;
     Tree &tx = pl->tx, &ty = *pl->ty;
-
-    // root pair list (n_tree.cu:1071)
-    pl->lists.clear();
-    pl->lists.emplace_back();
-    build_root_list(pl->lists[0].keep, s);
+    const int64_t N = tx.n, M = ty.n;
+    const int first_batch = max_counts_pending ? (int)tx.levels.size() - 1 : 0;
     pl->stats = f3m_plan_stats{};
-    int level = 0;
-    auto go_on = [&]() {
+    bool bounds_allowed = !dev_in_workspace();   // a caller's workspace holds no more than the lists need
+    auto take_flags = [&]() {
+        read_flags(pl, s);
+        for (int l = 1; l <= first_batch && max_counts_pending; l++) {
+            tx.levels[l].max_count = pl->h_pinned[FL_LVMAX + l - 1];
+            if (!pl->same) ty.levels[l].max_count = pl->h_pinned[FL_LVMAX_Y + l - 1];
+        }
+        max_counts_pending = false;
+    };
+    auto take_counts = [&](int l) {
+        const long long *h = reinterpret_cast<const long long *>(pl->h_pinned + FL_LISTS) + 3 * l;
+        F3M_REQUIRE(h[0] <= 0x7fffffffLL && h[1] <= 0x7fffffffLL && h[2] <= 0x7fffffffLL, F3M_ERR_OVERFLOW,
+                    "interaction list of level %d exceeds 2^31 pairs (far %lld, small %lld, kept %lld)", l, h[0], h[1], h[2]);
+        LevelLists &ll = pl->lists[l];
+        ll.far.count = h[0]; ll.small.count = h[1]; ll.keep.count = h[2];
+    };
+    auto go_on = [&](int level) {
         if (pl->lists[level].keep.count == 0) return false;
         bool gx = (float)tx.levels[level].max_count > prm->min_points;     // n_tree.cu:1075
         if (pl->same) return gx;
         return gx && (float)ty.levels[level].max_count > prm->min_points;  // n_tree.cu:1099
     };
-    const int p_full = nodes_per_dim(d, prm->nr_interpolation);
-    int p_small = nodes_per_dim(d, std::min((int)lround(pow(3.0, d)), prm->nr_interpolation));
-    while (go_on()) {
+    // the mean box is above the limit, so the largest is
+    auto surely_on = [&](int level) {
+        auto over = [&](const Tree &t) { return (double)t.n > (double)prm->min_points * t.levels[level].nb; };
+        return over(tx) && (pl->same || over(ty));
+    };
+    // lists of one level; true: on a bound, the counts are still on the device
+    auto enqueue = [&](int l) {
+        pl->lists.resize(l + 1);
+        lists_count(pl, l, s);
+        const int64_t bound = list_bound(pl, l);
+        if (bounds_allowed && bound <= LIST_BOUND) {
+            const int64_t cap[3] = {bound, bound, bound};
+            lists_write(pl, l, cap, s);
+            return true;
+        }
+        take_flags();
+        take_counts(l);
+        const LevelLists &ll = pl->lists[l];
+        const int64_t cap[3] = {ll.far.count, ll.small.count, ll.keep.count};
+        lists_write(pl, l, cap, s);
+        return false;
+    };
+    int level = 0, listed = 0;   // levels accepted, levels whose lists are there
+    bool work_pending = false;   // the lists' work of some level has not been read
+    while (level < listed || go_on(level)) {
+        if (level < listed) {    // enqueued ahead
+            if (!go_on(level)) break;
+            level++;
+            continue;
+        }
         const int need = level + 1;
         F3M_REQUIRE(need <= tx.lmax, F3M_ERR_DEPTH,
                     "tree needs level %d but a 30-bit cell index holds %d levels in %d dimensions", need, tx.lmax, d);
@@ -314,8 +393,15 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
                         "the tree needs level %d but the runs it was merged from are sorted to level %d: build the plan from the points",
                         need, tx.sorted_depth);
             // deeper than estimated: sort to the full key depth (levels already built keep their boxes)
-            build_sorted_tree(tx, X, N, d, xmin, edge0, prm->math_mode, tx.lmax, s);
-            if (!pl->same) build_sorted_tree(ty, Y, M, d, ymin, edge0, prm->math_mode, ty.lmax, s);
+            Cube cx, cy;
+            float ox[MAXD], oy[MAXD];
+            std::copy(tx.origin, tx.origin + MAXD, ox);
+            std::copy(ty.origin, ty.origin + MAXD, oy);
+            cx.origin = ox;
+            cy.origin = oy;
+            cx.edge0 = cy.edge0 = tx.edge0;
+            build_sorted_tree(tx, X, N, d, cx, prm->math_mode, tx.lmax, s);
+            if (!pl->same) build_sorted_tree(ty, Y, M, d, cy, prm->math_mode, ty.lmax, s);
         }
         if ((int)tx.levels.size() <= need) {
             // a first batch up to the estimated depth, later batches three levels at a time
@@ -323,14 +409,38 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
             build_levels(tx, last, pl, s);
             if (!pl->same) build_levels(ty, last, pl, s);
         }
+        // this level, and those after it that are certain to follow, until one has to be waited for
+        bool on_bound = false;
+        int l = level;
+        do {
+            on_bound = enqueue(++l);
+        } while (on_bound && l + 1 < (int)tx.levels.size() && surely_on(l));
+        if (on_bound) take_flags();
+        work_pending = !on_bound;
+        for (int q = level + 1; q <= l; q++) take_counts(q);
+        if (pl->h_pinned[FL_LISTOVER]) {   // a bound was wrong (the lists after it are empty): start over, asking for every length
+            bounds_allowed = false;
+            pl->lists.resize(1);
+            level = listed = 0;
+            F3M_CUDA(cudaMemsetAsync(pl->d_flags + FL_LISTOVER, 0, sizeof(int), s));
+            F3M_CUDA(cudaMemsetAsync(pl->d_flags + FL_LISTS, 0, (FLAG_WORDS - FL_LISTS) * sizeof(int), s));
+            continue;
+        }
+        listed = l;
         level++;
-        pl->lists.emplace_back();
-        build_level_lists(pl, level, s);
-        LevelLists &ll = pl->lists[level];
+    }
+    pl->lists.resize(level + 1);
+    pl->last.end(s);
+    if (work_pending) take_flags();
+    const int p_full = nodes_per_dim(d, prm->nr_interpolation);
+    const int p_small = nodes_per_dim(d, std::min((int)lround(pow(3.0, d)), prm->nr_interpolation));
+    const long long *work = reinterpret_cast<const long long *>(pl->h_pinned + FL_PAIRWORK);
+    for (int l = 1; l <= level; l++) {
+        LevelLists &ll = pl->lists[l];
         // nodes for this level: get_interpolation_rule (n_tree.cu:971-978, 1022-1028)
         ll.p = p_full;
         if (prm->var_compression) {
-            float e = tx.levels[level].edge;
+            float e = tx.levels[l].edge;
             float eff = e * e * pl->lcs;
             if (eff < 0.01f) ll.p = p_small;
         }
@@ -338,33 +448,22 @@ static void plan_build_levels(f3m_plan *pl, const float *X, int64_t N, const flo
         for (int k = 0; k < d; k++) P *= ll.p;
         pl->stats.far_box_pairs += ll.far.count;
         pl->stats.node_pairs += ll.far.count * (int64_t)P * P;
-        pl->stats.near_box_pairs += ll.small.count;
-        accumulate_pair_work(pl, level, level, ll.small, s);
+        pl->stats.near_box_pairs += ll.small.count + (l == level ? ll.keep.count : 0);
+        ll.small.pairs = work[4 * l];
+        ll.small.row_boxes = work[4 * l + 1];
+        ll.keep.pairs = work[4 * l + 2];
+        ll.keep.row_boxes = work[4 * l + 3];
+        pl->stats.direct_pairs += ll.small.pairs + (l == level ? ll.keep.pairs : 0);
     }
     pl->levels = level;
-    if (level > 0) {
-        pl->stats.near_box_pairs += pl->lists[level].keep.count;
-        accumulate_pair_work(pl, level, PAIRWORK_LISTS - 1, pl->lists[level].keep, s);
-    } else {
+    if (level == 0) {
         // no level was built: the root pair is summed directly
         pl->stats.near_box_pairs = 1;
         pl->stats.direct_pairs = N * M;
     }
     pl->stats.levels = level;
     pl->stats.shared_tree = pl->same;
-    pl->stats.edge0 = edge0;
-    pl->last.end(s);
-    F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + FL_PAIRWORK, pl->d_flags + FL_PAIRWORK, 2 * PAIRWORK_LISTS * sizeof(long long),
-                             cudaMemcpyDeviceToHost, s));
-    F3M_CUDA(cudaStreamSynchronize(s));
-    const long long *work = reinterpret_cast<const long long *>(pl->h_pinned + FL_PAIRWORK);
-    auto take_work = [&](PairCSR &csr, int slot) {
-        csr.pairs = work[2 * slot];
-        csr.row_boxes = work[2 * slot + 1];
-        pl->stats.direct_pairs += csr.pairs;
-    };
-    for (int l = 1; l <= level; l++) take_work(pl->lists[l].small, l);
-    if (level > 0) take_work(pl->lists[level].keep, PAIRWORK_LISTS - 1);
+    pl->stats.edge0 = tx.edge0;
 }
 
 static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t row_begin, int64_t row_end,
@@ -521,7 +620,13 @@ int f3m_bounding_box_f32(const float *X, int64_t n, int32_t d, float *min_out, f
     return guarded([&] {
         f3m_plan tmp;   // only its scratch words are used
         plan_take_slot(&tmp);
-        bounding_box(X, n, d, min_out, max_out, &tmp, (cudaStream_t)stream);
+        cudaStream_t s = (cudaStream_t)stream;
+        unsigned *words = reinterpret_cast<unsigned *>(tmp.d_flags) + FL_BBOX;
+        F3M_CUDA(cudaMemsetAsync(words, 0, 2 * MAXD * sizeof(unsigned), s));
+        bounding_box(X, n, d, words, s);
+        F3M_CUDA(cudaMemcpyAsync(tmp.h_pinned + FL_BBOX, words, 2 * MAXD * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaStreamSynchronize(s));
+        bounding_box_values(reinterpret_cast<const unsigned *>(tmp.h_pinned) + FL_BBOX, d, min_out, max_out);
     });
 }
 
@@ -550,9 +655,9 @@ int f3m_plan_create_from_cell_counts(f3m_plan **plan, const int32_t *cell_counts
         pl = new f3m_plan();
         plan_begin(pl, d, prm, true, s);
         tree_from_cell_counts(pl->tx, cell_counts, nruns, d, origin, edge0, depth, pl, s);
-        build_root(pl->tx, s);
         pl->ty = &pl->tx;
-        plan_build_levels(pl, nullptr, pl->tx.n, nullptr, pl->tx.n, origin, origin, edge0, s);
+        build_roots(pl, s);
+        plan_build_levels(pl, nullptr, nullptr, false, s);
     });
     if (st != F3M_OK) {
         if (pl) { cudaStreamSynchronize(s); delete pl; }

@@ -51,6 +51,7 @@ extern std::atomic<long long> g_launches;   // kernels launched by this library 
 // unpredictable times, 200 ms at a time.)  A released block may be reused immediately by work that is
 // enqueued later on the same stream; every entry point synchronises its stream before it returns, so
 // blocks never cross streams while in use.  f3m_release_cached_memory() returns the free list to the driver.
+bool dev_in_workspace();   // this thread's buffers come out of a caller's workspace
 void *dev_alloc(size_t bytes, size_t *granted, int *device);
 void dev_free(void *p, size_t granted, int device);
 
@@ -186,20 +187,24 @@ inline void cheb_nodes_weights(int p, float *node, float *w) {
 }
 
 // ---- small per-plan device words (f3m_plan::d_flags) and their pinned host mirror ------------------
-constexpr int FLAG_WORDS = 256;
+constexpr int FLAG_WORDS = 640;
 enum FlagSlot {
     FL_ERR = 0,          // device-side consistency check failed
-    FL_LISTTOT = 8,      // 6 words: 64-bit far / small / keep pair counts of the level being built
+    FL_LISTOVER = 1,     // a list is longer than the memory it was given on a bound
+    FL_LISTTOT = 8,      // 4 words: 64-bit totals of a merged tree
     FL_BBOX = 16,        // 2 * MAXD words
     FL_MMA_COUNTER = 32, // tile cursor of the tensor-core near kernel
     FL_LEAF = 40,        // 2 words: small / big finest-level boxes
     FL_NSMALL = 42,      // target tiles of at most 32 points
     FL_WEIGHTS = 43,     // a weight is not finite, or near the largest float
+    FL_BBOX_Y = 48,      // 2 * MAXD words, the second point set
     FL_LVTOT = 64,       // boxes per level of the batch being built (F3M_MAX_LEVELS words)
     FL_LVMAX = 96,       // largest box per level (F3M_MAX_LEVELS words)
-    FL_PAIRWORK = 128    // 4 words per direct list (PAIRWORK_LISTS of them): 64-bit sums of n_x * n_y and of n_x over its box pairs
+    FL_LVTOT_Y = 128, FL_LVMAX_Y = 160,   // the same of the second tree
+    FL_LISTS = 192,      // 6 words per level: 64-bit far / small / keep pair counts
+    FL_PAIRWORK = 352    // 8 words per level: 64-bit sums of n_x * n_y and of n_x over the box pairs of the small list and of the kept one
 };
-constexpr int PAIRWORK_LISTS = 22;   // "small" lists of levels 1..20, the near list in slot 21
+static_assert(FL_LISTS + 6 * (F3M_MAX_LEVELS + 1) <= FL_PAIRWORK && FL_PAIRWORK + 8 * (F3M_MAX_LEVELS + 1) <= FLAG_WORDS, "flag words");
 
 // ---- tree ------------------------------------------------------------------------------------
 struct Level {
@@ -398,9 +403,15 @@ struct f3m_plan {
 namespace f3m {
 
 // ---- sort.cu ---------------------------------------------------------------------------------
-void bounding_box(const float *X, int64_t n, int d, float *h_min, float *h_max, f3m_plan *pl, cudaStream_t s);
-void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const float *origin, float edge0,
-                       int math_mode, int depth, cudaStream_t s);
+void bounding_box(const float *X, int64_t n, int d, unsigned *words, cudaStream_t s);   // 2 * MAXD device words, zero before
+void bounding_box_values(const unsigned *words, int d, float *h_min, float *h_max);     // the words on the host, decoded
+// The cube on the host, or still on the device: the words of bounding_box, of the set itself and of the one it shares the edge with
+struct Cube {
+    const float *origin = nullptr;
+    float edge0 = 0.f;
+    const unsigned *own = nullptr, *other = nullptr;
+};
+void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s);
 int record_words(int d);   // 32-bit words of the record [input row, coordinates] that travels with a key in the sort
 void sort_shard(const float *X, int64_t n, int64_t row0, int d, const float *origin, float edge0, int math_mode, int depth,
                 uint32_t *recs_out, int *cell_counts_out, cudaStream_t s);
@@ -415,11 +426,19 @@ void scatter_rows(const float *src, const int *perm, float *dst, int64_t n, int 
 void scatter_rows_nonzero(const float *src, const int *perm, float *dst, int64_t n, int cols, cudaStream_t s);
 
 // ---- tree.cu ---------------------------------------------------------------------------------
-void build_root(Tree &t, cudaStream_t s);
-void build_root_list(PairCSR &k, cudaStream_t s);   // the one pair of roots (n_tree.cu:1071)
+void build_roots(f3m_plan *pl, cudaStream_t s);   // of both trees, and the list of their one pair (n_tree.cu:1071)
+// box starts of the levels after the last one built, up to l_last (at most HEADS_BATCH of them): counted, then written
+constexpr int HEADS_BATCH = 8;
+struct HeadsBatch {
+    DevBuf<int> part;
+    int l_first = 0, nlev = 0, nt = 0;
+};
+void heads_begin(Tree &t, HeadsBatch &hb, int l_first, int l_last, int *d_tot, cudaStream_t s);
+void heads_finish(Tree &t, HeadsBatch &hb, const int *h_tot, int *d_max, int *d_err, cudaStream_t s);
 void build_levels(Tree &t, int l_last, f3m_plan *pl, cudaStream_t s);   // appends levels up to l_last (<= sorted_depth)
-void build_level_lists(f3m_plan *pl, int level, cudaStream_t s);     // uses lists[level-1].keep
-void accumulate_pair_work(f3m_plan *pl, int level, int slot, const PairCSR &csr, cudaStream_t s);   // FL_PAIRWORK (device)
+// interaction lists of a level from lists[level-1].keep: counted (FL_LISTS), then written; cap: entries each list has room for
+void lists_count(f3m_plan *pl, int level, cudaStream_t s);
+void lists_write(f3m_plan *pl, int level, const int64_t cap[3], cudaStream_t s);
 
 // ---- far.cu ----------------------------------------------------------------------------------
 int nodes_per_dim(int d, int nr_interpolation);   // get_node_list for perfect powers, floor otherwise

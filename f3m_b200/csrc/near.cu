@@ -503,16 +503,18 @@ __global__ void __launch_bounds__(NT2, RB == 1 ? 32 : (RB <= 4 ? 20 : 12)) near_
                                                      const int *__restrict__ off_y, const float *__restrict__ ctr_y,
                                                      const float *__restrict__ packed, float scale, int R, int r0,
                                                      float *out, float pc0, float pc1, float pc2, float pc3, int row_begin,
-                                                     int row_end) {
+                                                     int row_end, int full_tile) {
     constexpr int W = row_width(D, RB);
     __shared__ __align__(16) float smem[sp2_of<RB>() * 2 * W];
     if ((int)blockIdx.x >= tile_off[nbx]) return;
     int box, t0, t1;
-    item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1, MIXED ? NT2 * TI2 : 0);
+    item_to_tile(blockIdx.x, tile_off, nbx, off_x, row_begin, row_end, box, t0, t1, full_tile);
     if (MIXED && t1 - t0 <= NT2) {
         // a box of at most 32 points has neighbours of its own kind (same level, same local density): short source boxes,
         // where the pipelined form pays; the last tile of a large box meets large source boxes and keeps the plain loop
-        if (RB >= 4 && off_x[box + 1] - off_x[box] <= NT2)   // one column: measured slower than the plain loop on clustered data
+        // One column: measured slower than the plain loop on clustered data, but a call of short tiles (full_tile 0) has few warps to wait
+        // with.
+        if (full_tile == 0 || (RB >= 4 && off_x[box + 1] - off_x[box] <= NT2))
             near_tile_x2_small<D, RB, POLY, PNUM, PDEN>(xpts, n_x, ptr, idx, off_y, ctr_y, packed, scale, R, r0, out, pc0, pc1, pc2,
                                                         pc3, smem, box, t0, t1);
         else
@@ -593,6 +595,7 @@ static double list_reach(const f3m_plan *pl, int level, const PairCSR &csr) {
 constexpr double TMAX_EXPANDED = 64.0;
 
 constexpr int MAX_UNREAD_TILES = 8192;
+constexpr int64_t PACK_ALL = 1 << 16;   // so few sources are packed without asking which boxes a list names (two launches)
 
 // one list, one block of RB columns starting at r0
 template <int D, int RB>
@@ -608,26 +611,32 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
     // tensor-core form (on request): one column, boxes at most half a scaled unit wide, so that the split
     // operands keep the exponent at FP32 accuracy
     const bool use_mma = RB == 1 && expanded && scale * ly.edge <= 0.5f && (pl->prm.flags & F3M_FLAG_NEAR_TENSOR_CORES);
-    const int tile_pts = use_mma ? MM_M : (expanded ? NT2 * TI2 : NT);
+    // A tile is one warp's work.  Calls whose rows do not give every SM eight full tiles get shorter ones, down to four rows, whose
+    // sources the lanes share (2000 targets and sources, 32 full tiles: 42.6 us; 500 tiles of four rows, rows of the next box copied ahead: 16.8).
+    int short_tile = NT2;
+    while (short_tile > 4 && (row_end - row_begin) / short_tile < 8 * NUM_SMS_HINT) short_tile /= 2;
+    const bool short_tiles = expanded && !use_mma && (row_end - row_begin) / (NT2 * TI2) < 8 * NUM_SMS_HINT;
+    const int tile_pts = use_mma ? MM_M : short_tiles ? short_tile : (expanded ? NT2 * TI2 : NT);
     DevBuf<int> tiles;
     tiles.alloc((size_t)lx.nb + 1, s);
-    int *n_small = pl->d_flags + FL_NSMALL;
-    F3M_CUDA(cudaMemsetAsync(n_small, 0, sizeof(int), s));
-    near_tiles_per_box<<<(unsigned)((lx.nb + 1 + 255) / 256), 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, row_begin, row_end,
-                                                                           tile_pts, tiles.p, n_small);
-    F3M_LAUNCH_CHECK();
-    exclusive_scan_i32(tiles.p, tiles.p, (int64_t)lx.nb + 1, s);
     // Small calls launch a bound on the tiles (CTAs beyond the last tile leave at once: less than 2 us for the limit below) and
     // the kernel that halves the work of short tiles; larger ones read the number of tiles and whether there are short ones.
     const int64_t bound = (int64_t)(row_end - row_begin) / tile_pts + lx.nb;
+    const bool read_tiles = use_mma || bound > MAX_UNREAD_TILES;
+    int *n_small = pl->d_flags + FL_NSMALL;
+    if (read_tiles) F3M_CUDA(cudaMemsetAsync(n_small, 0, sizeof(int), s));
+    near_tiles_per_box<<<(unsigned)((lx.nb + 1 + 255) / 256), 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, row_begin, row_end,
+                                                                           tile_pts, tiles.p, read_tiles ? n_small : nullptr);
+    F3M_LAUNCH_CHECK();
+    exclusive_scan_i32(tiles.p, tiles.p, (int64_t)lx.nb + 1, s);
     int items = (int)std::min<int64_t>(bound, MAX_UNREAD_TILES);
-    bool small_tiles = true;
-    if (use_mma || bound > MAX_UNREAD_TILES) {
+    bool small_tiles = true;   // some tiles hold at most 32 targets
+    if (read_tiles) {
         F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, tiles.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
         F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + 1, n_small, sizeof(int), cudaMemcpyDeviceToHost, s));
         F3M_CUDA(cudaStreamSynchronize(s));
         items = pl->h_pinned[0];
-        small_tiles = pl->h_pinned[1] > 0;   // some tiles hold at most 32 targets
+        small_tiles = short_tiles || pl->h_pinned[1] > 0;
     }
     if (items <= 0) return;
     // Packed sources are kept for the lists of one level that share (column block, form): the "small" list of the last
@@ -690,7 +699,7 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
         if (expanded) {
             // only the boxes that a direct list of this level names (for this slice of the targets, when the product is
             // shared by several GPUs) are packed
-            const unsigned char *need = level_source_flags(pl, level, s);
+            const unsigned char *need = ty.n <= PACK_ALL && !pl->shard.active ? nullptr : level_source_flags(pl, level, s);
             const int nsplit = std::max(1, std::min(65535, (ly.max_count + 2047) / 2048));
             pack_pairs_box<D, RB><<<dim3((unsigned)(((int64_t)ly.nb * 32 + 255) / 256), nsplit), 256, 0, s>>>(
                 ty.pts.p, (int)ty.n, bs, R, r0, scale, ly.off.p, ly.nb, ly.ctr.p, need, nsplit, packed.p);
@@ -709,7 +718,8 @@ static void direct_impl(f3m_plan *pl, int level, const PairCSR &csr, const float
 #define F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, MIXED_)                                                                                       \
     near_kernel_x2<D, RB, POLY_, PNUM_, PDEN_, MIXED_><<<items, NT2, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, tiles.p, csr.ptr.p, \
                                                                             csr.idx.p, ly.off.p, ly.ctr.p, packed.p, scale, R, r0, out, \
-                                                                            (float)cf[0], (float)cf[1], (float)cf[2], (float)cf[3], row_begin, row_end)
+                                                                            (float)cf[0], (float)cf[1], (float)cf[2], (float)cf[3], row_begin, row_end, \
+                                                                            MIXED_ && !short_tiles ? NT2 * TI2 : 0)
 #define F3M_NEAR_EXP(POLY_, PNUM_, PDEN_)                         \
     {                                                             \
         if (small_tiles) F3M_NEAR_EXP2(POLY_, PNUM_, PDEN_, true); \

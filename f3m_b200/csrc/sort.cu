@@ -72,10 +72,44 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_tile_write(ScanArrays a, in
     }
 }
 
+// Short arrays: one block each, one launch (8193 values 3 us, against three launches of 2 us and their gaps)
+constexpr int64_t SCAN_ONE = 65536;
+__global__ void __launch_bounds__(1024) scan_one_block(ScanArrays a, int n, long long *totals64) {
+    __shared__ int sm[33];
+    const int *in = a.in[blockIdx.x];
+    int *out = a.out[blockIdx.x];
+    long long carry = 0;
+    for (int tile = 0; tile < n; tile += 1024 * SCAN_ITEMS) {
+        const int base = tile + threadIdx.x * SCAN_ITEMS;
+        int v[SCAN_ITEMS], s = 0;
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            v[k] = base + k < n ? in[base + k] : 0;
+            s += v[k];
+        }
+        int total;
+        int ex = block_exclusive_scan(s, &total, sm) + (int)carry;
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            if (base + k < n) out[base + k] = ex;
+            ex += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0 && totals64) totals64[blockIdx.x] = carry;
+}
+
 // arrays[k] is scanned in place, k < narr <= 4; totals64 (device, narr entries, may be null) receives the sums
 void exclusive_scan_multi(int *const *arrays, int narr, int64_t n, long long *totals64, cudaStream_t s) {
     if (n <= 0 || narr <= 0) return;
     F3M_REQUIRE(narr <= 4, F3M_ERR_INTERNAL, "exclusive_scan_multi takes at most four arrays");
+    if (n <= SCAN_ONE) {
+        ScanArrays o{};
+        for (int k = 0; k < narr; k++) o.in[k] = o.out[k] = arrays[k];
+        scan_one_block<<<narr, 1024, 0, s>>>(o, (int)n, totals64);
+        F3M_LAUNCH_CHECK();
+        return;
+    }
     const int nt = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     ScanArrays a{};
     for (int k = 0; k < narr; k++) { a.in[k] = arrays[k]; a.out[k] = arrays[k]; }
@@ -94,6 +128,11 @@ void exclusive_scan_i32(const int *in, int *out, int64_t n, cudaStream_t s) {
     const int nt = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     ScanArrays a{};
     a.in[0] = in; a.out[0] = out;
+    if (n <= SCAN_ONE) {
+        scan_one_block<<<1, 1024, 0, s>>>(a, (int)n, nullptr);
+        F3M_LAUNCH_CHECK();
+        return;
+    }
     DevBuf<int> part;
     part.alloc(nt, s);
     scan_tile_sums<<<dim3(nt, 1), SCAN_THREADS, 0, s>>>(a, n, nt, part.p);
@@ -111,7 +150,7 @@ __device__ __forceinline__ unsigned enc_f32(float f) {
     unsigned u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-static inline float dec_f32(unsigned u) {
+__host__ __device__ inline float dec_f32(unsigned u) {
     unsigned v = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
     float f;
     memcpy(&f, &v, 4);
@@ -142,19 +181,21 @@ __global__ void __launch_bounds__(256) bbox_kernel(const float *__restrict__ X, 
             hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
         }
     }
-    if ((threadIdx.x & 31) == 0) {
+    // one atomic per block and extreme: from every warp they queued up (1e5 points 14 -> 4 us)
+    __shared__ float block_lo[8][D], block_hi[8][D];
+    if ((threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int k = 0; k < D; k++) {
-            atomicMax(&mm[k], ~enc_f32(lo[k]));   // complemented, so that zero is the start of either extreme
-            atomicMax(&mm[MAXD + k], enc_f32(hi[k]));
-        }
+        for (int k = 0; k < D; k++) { block_lo[threadIdx.x >> 5][k] = lo[k]; block_hi[threadIdx.x >> 5][k] = hi[k]; }
+    __syncthreads();
+    if (threadIdx.x < D) {
+        float l = block_lo[0][threadIdx.x], h = block_hi[0][threadIdx.x];
+        for (int w = 1; w < 8; w++) { l = fminf(l, block_lo[w][threadIdx.x]); h = fmaxf(h, block_hi[w][threadIdx.x]); }
+        atomicMax(&mm[threadIdx.x], ~enc_f32(l));   // complemented, so that zero is the start of either extreme
+        atomicMax(&mm[MAXD + threadIdx.x], enc_f32(h));
     }
 }
 
-void bounding_box(const float *X, int64_t n, int d, float *h_min, float *h_max, f3m_plan *pl, cudaStream_t s) {
-    unsigned *mm = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX;   // 2*MAXD words
-    constexpr size_t mm_bytes = 2 * MAXD * sizeof(unsigned);
-    F3M_CUDA(cudaMemsetAsync(mm, 0, mm_bytes, s));
+void bounding_box(const float *X, int64_t n, int d, unsigned *mm, cudaStream_t s) {
     int grid = (int)std::min<int64_t>((n + 255) / 256, NUM_SMS_HINT * 8);
     switch (d) {
         case 1: bbox_kernel<1><<<grid, 256, 0, s>>>(X, n, mm); break;
@@ -164,9 +205,8 @@ void bounding_box(const float *X, int64_t n, int d, float *h_min, float *h_max, 
         default: bbox_kernel<5><<<grid, 256, 0, s>>>(X, n, mm); break;
     }
     F3M_LAUNCH_CHECK();
-    unsigned *h = reinterpret_cast<unsigned *>(pl->h_pinned);
-    F3M_CUDA(cudaMemcpyAsync(h, mm, mm_bytes, cudaMemcpyDeviceToHost, s));
-    F3M_CUDA(cudaStreamSynchronize(s));
+}
+void bounding_box_values(const unsigned *h, int d, float *h_min, float *h_max) {
     for (int k = 0; k < d; k++) {
         h_min[k] = dec_f32(~h[k]);
         h_max[k] = dec_f32(h[MAXD + k]);
@@ -212,7 +252,20 @@ struct MortonCfg {
     float org[MAXD];
     float side, edge0;
     int L, ieee;
+    const unsigned *own, *other;   // not null: origin and edge come from these words, as the host computes them (api.cu)
 };
+template <int D>
+__device__ __forceinline__ void resolve_cube(MortonCfg &cfg) {
+    if (!cfg.own) return;
+    float range = 0.f;
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        cfg.org[k] = dec_f32(~cfg.own[k]);
+        range = fmaxf(range, __fsub_rn(dec_f32(cfg.own[MAXD + k]), cfg.org[k]));
+        if (cfg.other) range = fmaxf(range, __fsub_rn(dec_f32(cfg.other[MAXD + k]), dec_f32(~cfg.other[k])));
+    }
+    cfg.edge0 = __fmul_rn(range, 1.01f);
+}
 
 // Morton key of one point; spread[v] moves bit j of the 5-bit value v to bit D*j (a 32-entry table in shared memory)
 template <int D>
@@ -248,6 +301,7 @@ __global__ void __launch_bounds__(512) morton_hist_kernel(const float *__restric
     __shared__ int hist[RS_MAXBINS];
     __shared__ uint32_t spread[32];   // bit j of a 5-bit value -> bit D*j
     for (int q = threadIdx.x; q < RS_MAXBINS; q += blockDim.x) hist[q] = 0;
+    resolve_cube<D>(cfg);
     fill_spread_table<D>(spread);
     __syncthreads();
     const uint32_t mask = (1u << dbits) - 1u;
@@ -678,12 +732,14 @@ static void sort_passes(Tree &t, const float *X, const MortonCfg &cfg, int shift
     F3M_LAUNCH_CHECK();
 }
 
-static MortonCfg morton_cfg(int d, const float *origin, float edge0, int math_mode) {
+static MortonCfg morton_cfg(int d, const Cube &cube, int math_mode) {
     MortonCfg cfg{};
-    for (int k = 0; k < d; k++) cfg.org[k] = origin[k];
+    cfg.own = cube.own;
+    cfg.other = cube.other;
+    for (int k = 0; k < d && cube.origin; k++) cfg.org[k] = cube.origin[k];
     cfg.L = std::min(30 / d, 20);
     cfg.side = (float)(1u << cfg.L);
-    cfg.edge0 = edge0;
+    cfg.edge0 = cube.edge0;
     cfg.ieee = math_mode == F3M_MATH_IEEE;
     return cfg;
 }
@@ -719,7 +775,10 @@ __global__ void __launch_bounds__(256) cell_counts_kernel(int ncells, const int 
 void sort_shard(const float *X, int64_t n, int64_t row0, int d, const float *origin, float edge0, int math_mode, int depth,
                 uint32_t *recs_out, int *cell_counts_out, cudaStream_t s) {
     F3M_REQUIRE(row0 + n < (int64_t)0x7fffffff, F3M_ERR_OVERFLOW, "row %lld does not fit a 31-bit index", (long long)(row0 + n));
-    const MortonCfg cfg = morton_cfg(d, origin, edge0, math_mode);
+    Cube cube;
+    cube.origin = origin;
+    cube.edge0 = edge0;
+    const MortonCfg cfg = morton_cfg(d, cube, math_mode);
     depth = std::max(1, std::min(depth, cfg.L));
     F3M_REQUIRE(d * depth <= 22, F3M_ERR_UNSUPPORTED, "shards sorted by %d key bits: the cell table holds at most 22", d * depth);
     const int shift0 = d * (cfg.L - depth), bits = d * depth, ncells = 1 << bits;
@@ -879,20 +938,19 @@ void tree_attach_runs(Tree &t, const uint32_t *recs, int64_t stride, cudaStream_
 
 // Sorts the points of one tree by the first `depth` levels of their Morton key (all later levels are read off the
 // sorted keys, tree.cu) and leaves keys, permutation and coordinate planes in the tree.
-void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const float *origin, float edge0, int math_mode, int depth,
-                       cudaStream_t s) {
+void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s) {
     F3M_REQUIRE(n < (int64_t)0x7fffffff, F3M_ERR_OVERFLOW, "point count %lld does not fit a 31-bit index", (long long)n);
     t.n = n;
     t.d = d;
     t.data = X;
-    t.edge0 = edge0;
-    for (int k = 0; k < d; k++) t.origin[k] = origin[k];
+    t.edge0 = cube.edge0;      // where the cube is still on the device, the caller sets both later
+    for (int k = 0; k < d && cube.origin; k++) t.origin[k] = cube.origin[k];
     // deepest level a 30-bit cell index holds (the reference's int cell index overflows beyond that)
     t.lmax = std::min(30 / d, 20);
     depth = std::max(1, std::min(depth, t.lmax));
     t.sorted_depth = depth;
     t.keys.release(); t.perm.release(); t.pts.release();   // a second sort (deeper) replaces the first
-    const MortonCfg cfg = morton_cfg(d, origin, edge0, math_mode);
+    const MortonCfg cfg = morton_cfg(d, cube, math_mode);
     const int shift0 = d * (t.lmax - depth), bits = d * depth;
     switch (d) {
         case 1: sort_passes<1>(t, X, cfg, shift0, bits, s); break;
