@@ -249,8 +249,13 @@ static void plan_begin(f3m_plan *pl, int d, const f3m_params *prm, bool same, cu
     pl->last.begin(ST_BUILD, s);
 }
 
-static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, int64_t M, int d, const f3m_params *prm,
-                       cudaStream_t s) {
+// Calls from this many points on may end their tree early and carry b through the sort: the wait for the cube (10 us) is nothing to
+// them, and a gather of b by a random permutation leaves the cache.
+constexpr int64_t ONE_PRODUCT_POINTS = 1 << 21;
+
+// R > 0: the plan serves one product of R columns; b: its right-hand side where that is on the device already, or null
+static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, int64_t M, int d, const f3m_params *prm, int R,
+                       const float *b, cudaStream_t s) {
     // n_tree.cu:1072 tests the address only; a leading slice of X starts at the same address but is another
     // (smaller) point set, so the sizes must agree too
     plan_begin(pl, d, prm, X == Y && N == M, s);
@@ -267,41 +272,53 @@ static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, 
     unsigned *mx = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX, *my = reinterpret_cast<unsigned *>(pl->d_flags) + FL_BBOX_Y;
     bounding_box(X, N, d, mx, s);
     if (!pl->same) bounding_box(Y, M, d, my, s);
+    float xmin[MAXD], xmax[MAXD], ymin[MAXD], ymax[MAXD];
+    // bounding cube: calculate_edge_X / calculate_edge (n_tree.cu:25-46), float32 throughout
+    auto cube_edge = [&]() {
+        const unsigned *words = reinterpret_cast<const unsigned *>(pl->h_pinned);
+        bounding_box_values(words + FL_BBOX, d, xmin, xmax);
+        float range = 0.f;
+        bool finite = true;   // std::max drops a NaN operand, so non-finite extents are checked one by one
+        for (int k = 0; k < d; k++) {
+            finite = finite && std::isfinite(xmin[k]) && std::isfinite(xmax[k]);
+            range = std::max(range, xmax[k] - xmin[k]);
+        }
+        if (!pl->same) {
+            bounding_box_values(words + FL_BBOX_Y, d, ymin, ymax);
+            float ry = 0.f;
+            for (int k = 0; k < d; k++) {
+                finite = finite && std::isfinite(ymin[k]) && std::isfinite(ymax[k]);
+                ry = std::max(ry, ymax[k] - ymin[k]);
+            }
+            range = std::max(range, ry);
+        }
+        F3M_REQUIRE(finite, F3M_ERR_ARG, "degenerate or non-finite bounding cube (a coordinate is NaN or infinite)");
+        const float edge = range * 1.01f;
+        F3M_REQUIRE(edge > 0.f && std::isfinite(edge), F3M_ERR_ARG, "degenerate or non-finite bounding cube (edge %g)", edge);
+        return edge;
+    };
+    const bool one_product = R > 0 && std::min(N, M) >= ONE_PRODUCT_POINTS;
+    if (one_product) {
+        read_flags(pl, s);
+        const int stop = far_stop_level(pl, R, cube_edge(), xmin, pl->same ? nullptr : ymin, std::min(N, M));
+        if (stop && stop <= depth) depth = pl->stop_level = stop;
+        // a tree that ends early is not sorted again; a caller's workspace holds no more than it did
+        if (pl->stop_level && R == 1 && b && sort_carries(d, depth) && !dev_in_workspace()) pl->carry_b = b;
+    }
+    const float *bx = pl->same ? pl->carry_b : nullptr, *by = pl->same ? nullptr : pl->carry_b;
     Cube cx, cy;
     cx.own = cy.other = mx;
     cx.other = cy.own = pl->same ? nullptr : my;
     HeadsBatch hx, hy;
     const int lmax = std::min(30 / d, 20), first = depth < lmax ? depth : std::min(lmax, 3);
-    build_sorted_tree(tx, X, N, d, cx, prm->math_mode, depth, s);
+    build_sorted_tree(tx, X, N, d, cx, prm->math_mode, depth, s, bx, &pl->carried_b);
     heads_begin(tx, hx, 1, std::min(first, HEADS_BATCH), pl->d_flags + FL_LVTOT, s);
     if (!pl->same) {
-        build_sorted_tree(ty, Y, M, d, cy, prm->math_mode, depth, s);
+        build_sorted_tree(ty, Y, M, d, cy, prm->math_mode, depth, s, by, &pl->carried_b);
         heads_begin(ty, hy, 1, std::min(first, HEADS_BATCH), pl->d_flags + FL_LVTOT_Y, s);
     }
     read_flags(pl, s);
-
-    // bounding cube: calculate_edge_X / calculate_edge (n_tree.cu:25-46), float32 throughout
-    const unsigned *words = reinterpret_cast<const unsigned *>(pl->h_pinned);
-    float xmin[MAXD], xmax[MAXD], ymin[MAXD], ymax[MAXD];
-    bounding_box_values(words + FL_BBOX, d, xmin, xmax);
-    float range = 0.f;
-    bool finite = true;   // std::max drops a NaN operand, so non-finite extents are checked one by one
-    for (int k = 0; k < d; k++) {
-        finite = finite && std::isfinite(xmin[k]) && std::isfinite(xmax[k]);
-        range = std::max(range, xmax[k] - xmin[k]);
-    }
-    if (!pl->same) {
-        bounding_box_values(words + FL_BBOX_Y, d, ymin, ymax);
-        float ry = 0.f;
-        for (int k = 0; k < d; k++) {
-            finite = finite && std::isfinite(ymin[k]) && std::isfinite(ymax[k]);
-            ry = std::max(ry, ymax[k] - ymin[k]);
-        }
-        range = std::max(range, ry);
-    }
-    F3M_REQUIRE(finite, F3M_ERR_ARG, "degenerate or non-finite bounding cube (a coordinate is NaN or infinite)");
-    float edge0 = range * 1.01f;
-    F3M_REQUIRE(edge0 > 0.f && std::isfinite(edge0), F3M_ERR_ARG, "degenerate or non-finite bounding cube (edge %g)", edge0);
+    const float edge0 = cube_edge();
     tx.edge0 = ty.edge0 = edge0;
     for (int k = 0; k < d; k++) {
         tx.origin[k] = xmin[k];
@@ -350,13 +367,14 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
         ll.far.count = h[0]; ll.small.count = h[1]; ll.keep.count = h[2];
     };
     auto go_on = [&](int level) {
-        if (pl->lists[level].keep.count == 0) return false;
+        if (pl->lists[level].keep.count == 0 || (pl->stop_level && level >= pl->stop_level)) return false;
         bool gx = (float)tx.levels[level].max_count > prm->min_points;     // n_tree.cu:1075
         if (pl->same) return gx;
         return gx && (float)ty.levels[level].max_count > prm->min_points;  // n_tree.cu:1099
     };
     // the mean box is above the limit, so the largest is
     auto surely_on = [&](int level) {
+        if (pl->stop_level && level >= pl->stop_level) return false;
         auto over = [&](const Tree &t) { return (double)t.n > (double)prm->min_points * t.levels[level].nb; };
         return over(tx) && (pl->same || over(ty));
     };
@@ -487,9 +505,14 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
 
     pl->last.begin(ST_PERMUTE, s);
     DevBuf<float> bs, outs;
-    bs.alloc((size_t)M * R, s);
     outs.alloc((size_t)N * R, s);
-    gather_rows(b, ty.perm.p, bs.p, M, R, s, outs.p, N * R);
+    if (pl->carried_b.p && R == 1 && b == pl->carry_b) {
+        bs = std::move(pl->carried_b);
+        outs.zero();
+    } else {
+        bs.alloc((size_t)M * R, s);
+        gather_rows(b, ty.perm.p, bs.p, M, R, s, outs.p, N * R);
+    }
     pl->last.end(s);
 
     // A product over all rows may end at a level whose interpolation is exact for all its pairs (far_cut_level)
@@ -538,15 +561,15 @@ const char *f3m_status_string(int st) {
 const char *f3m_last_error(void) { return g_err; }
 long long f3m_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
-int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, int64_t M, int32_t d,
-                    const f3m_params *prm, void *stream) {
+static int plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, int64_t M, int32_t d, const f3m_params *prm, int R,
+                       const float *b, void *stream) {
     if (!plan) return F3M_ERR_ARG;
     *plan = nullptr;
     f3m_plan *pl = nullptr;
     int st = guarded([&] {
         check_common(X, N, Y, M, d, prm);
         pl = new f3m_plan();
-        plan_build(pl, X, N, Y, M, d, prm, (cudaStream_t)stream);
+        plan_build(pl, X, N, Y, M, d, prm, R, b, (cudaStream_t)stream);
     });
     if (st != F3M_OK) {
         if (pl) { cudaStreamSynchronize((cudaStream_t)stream); delete pl; }
@@ -554,6 +577,11 @@ int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, 
     }
     *plan = pl;
     return F3M_OK;
+}
+
+int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, int64_t M, int32_t d,
+                    const f3m_params *prm, void *stream) {
+    return plan_create(plan, X, N, Y, M, d, prm, 0, nullptr, stream);
 }
 
 int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, int64_t row_begin, int64_t row_end,
@@ -855,7 +883,7 @@ int f3m_plan_destroy(f3m_plan *plan) {
 int f3m_kmvm_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int32_t R, int32_t d,
                  const f3m_params *prm, float *out, void *stream) {
     f3m_plan *pl = nullptr;
-    int st = f3m_plan_create(&pl, X, N, Y, M, d, prm, stream);
+    int st = plan_create(&pl, X, N, Y, M, d, prm, std::max(R, 0), b, stream);
     if (st != F3M_OK) return st;
     st = f3m_plan_apply(pl, b, R, out, stream);
     f3m_plan_destroy(pl);
@@ -932,7 +960,7 @@ int f3m_kmvm_host_f32(const float *X, int64_t N, const float *Y, int64_t M, cons
         F3M_CUDA(cudaMemcpyAsync(db.p, b, (size_t)M * R * sizeof(float), cudaMemcpyHostToDevice, sb));
         F3M_CUDA(cudaEventRecord(ev_b, sb));
         dout.alloc((size_t)N * R, s);
-        int st2 = f3m_plan_create(&pl, dX.p, N, same ? dX.p : dY.p, M, d, prm, s);
+        int st2 = plan_create(&pl, dX.p, N, same ? dX.p : dY.p, M, d, prm, R, nullptr, s);   // b is still on its way
         if (st2 != F3M_OK) throw Fail{st2};
         F3M_CUDA(cudaStreamWaitEvent(s, ev_b, 0));
         st2 = f3m_plan_apply(pl, db.p, R, dout.p, s);

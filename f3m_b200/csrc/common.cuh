@@ -394,6 +394,11 @@ struct f3m_plan {
         f3m::DevBuf<float> bs;                             // b in sorted order, filled for the boxes this rank reads
         std::vector<f3m::DevBuf<unsigned char>> need;      // per level: source boxes named by the rank's direct lists
     } shard;
+    // a plan for one product (f3m_kmvm_f32): it may end at the level where that product will (far_stop_level), and b may have been sorted
+    // with its points
+    int stop_level = 0;
+    const float *carry_b = nullptr;
+    f3m::DevBuf<float> carried_b;
     int *h_pinned = nullptr;              // pinned host words for count read-back (FLAG_WORDS ints)
     int *d_flags = nullptr;               // device status / counters (FLAG_WORDS ints, see FlagSlot)
     std::vector<cudaEvent_t> *events = nullptr;   // of the scratch slot, see Timings
@@ -411,7 +416,10 @@ struct Cube {
     float edge0 = 0.f;
     const unsigned *own = nullptr, *other = nullptr;
 };
-void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s);
+bool sort_carries(int d, int depth);   // a sort to this depth takes a value per point along at less cost than a gather
+// b (or null): a value per point that travels along, in sorted order at b_out
+void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s,
+                       const float *b = nullptr, DevBuf<float> *b_out = nullptr);
 int record_words(int d);   // 32-bit words of the record [input row, coordinates] that travels with a key in the sort
 void sort_shard(const float *X, int64_t n, int64_t row0, int d, const float *origin, float edge0, int math_mode, int depth,
                 uint32_t *recs_out, int *cell_counts_out, cudaStream_t s);
@@ -448,6 +456,7 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
                cudaStream_t s);                                               // whole product (far_fast.cu)
 int64_t far_moments_size(const f3m_plan *pl, int R);
 int far_cut_level(const f3m_plan *pl, int R);   // level at which a product over all rows may end, 0: none
+int far_stop_level(const f3m_plan *pl, int R, float edge0, const float *xmin, const float *ymin, int64_t n);   // before the tree is built
 
 // ---- shard.cu --------------------------------------------------------------------------------
 const unsigned char *level_source_flags(f3m_plan *pl, int level, cudaStream_t s);   // per source box of the level: named by a direct list?

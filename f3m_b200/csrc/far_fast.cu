@@ -1324,17 +1324,18 @@ int64_t far_moments_size(const f3m_plan *pl, int R) {
 // ---------------------------------------------------------------------------------------------
 constexpr double CUT_EPS = 1.2e-7;
 
-static bool cut_is_exact(const f3m_plan *pl, int level, int p) {
-    const int d = pl->d;
-    const double e = (double)pl->ty->levels[level].edge * sqrt(2.0 * (double)pl->lcs);   // edge / l
+// edge: of the level; offset: between the two trees' origins, null for one tree
+static bool cut_is_exact(int d, double edge, double lcs, const double *offset, int level, int p) {
+    const bool same = offset == nullptr;
+    const double e = edge * sqrt(2.0 * lcs);   // edge / l
     auto inv_g = [&](double r) { return exp(0.5 * r * r * e * e); };
     double sum;
     if (level == 1) {   // children of the root pair, which is kept without a distance test
         sum = 0.0;
         for (int k = 0; k < d; k++)
-            sum += inv_g(2.0 + (pl->same ? 0.0 : fabs((double)pl->tx.origin[k] - (double)pl->ty->origin[k]) / (double)pl->ty->levels[1].edge));
+            sum += inv_g(2.0 + (same ? 0.0 : fabs(offset[k]) / edge));
     } else
-        sum = pl->same ? std::max(d * inv_g(4.0), inv_g(6.0) + (d - 1) * inv_g(2.0)) : d * inv_g(6.0);
+        sum = same ? std::max(d * inv_g(4.0), inv_g(6.0) + (d - 1) * inv_g(2.0)) : d * inv_g(6.0);
     double fact = 1.0;
     for (int i = 2; i <= p; i++) fact *= i;
     const double E = 2.0 * 1.0865 * pow(e / 4.0, p) / sqrt(fact);
@@ -1345,18 +1346,43 @@ static bool cut_is_exact(const f3m_plan *pl, int level, int p) {
 // estimated time wins.  Measured rates behind the estimate: M2L 1.25e-12 s per pair, node and column (0.25 ns per pair at 216
 // nodes, 2.5 ns at 243 nodes and 8 columns), translations 8e-12 s per box, node and column, direct lists see
 // node_choice; a cut orders a list of its own and sets up the level (20 us), which small trees do not win back.
-int far_cut_level(const f3m_plan *pl, int R) {
-    const int L = pl->levels;
-    if (L < 1 || (pl->prm.flags & F3M_FLAG_NEAR_TENSOR_CORES) || pl->prm.var_compression) return 0;
-    const int p = pl->lists[1].p, d = pl->d;
-    if (p < 2 || p > PMAX_FAST || d < 2) return 0;
+static bool cut_kernels_fit(const f3m_plan *pl, int R, int p, bool &wide) {
+    const int d = pl->d;
+    if ((pl->prm.flags & F3M_FLAG_NEAR_TENSOR_CORES) || pl->prm.var_compression || p < 2 || p > PMAX_FAST || d < 2) return false;
     int P = 1;
     for (int k = 0; k < d; k++) P *= p;
     const size_t tab = (size_t)d * NOFF2 * mat_stride(p) * sizeof(float);
-    if ((size_t)3 * P * sizeof(float) + tab > 200 * 1024) return 0;
-    const bool wide = R > 1 && (size_t)3 * P * 8 * sizeof(float) + tab <= 200 * 1024;
+    if ((size_t)3 * P * sizeof(float) + tab > 200 * 1024) return false;
+    wide = R > 1 && (size_t)3 * P * 8 * sizeof(float) + tab <= 200 * 1024;
     // the combined list exists in ordered form only, which these kernels read
-    if (!(wide ? rows_form_for(p, d) : (d <= 3 && P / p <= 64))) return 0;
+    return wide ? rows_form_for(p, d) : (d <= 3 && P / p <= 64);
+}
+
+// The level at which a plan for one product can end, known before its points are sorted; 0: unknown.  It is the first level whose
+// interpolation is exact for all pairs, where its boxes hold STOP_POINTS points on average however they are spread: neither the pairs
+// nor the moments of so full boxes take less time than one node-to-node step, and the levels below have a multiple of its pairs.
+constexpr int64_t STOP_POINTS = 256;
+int far_stop_level(const f3m_plan *pl, int R, float edge0, const float *xmin, const float *ymin, int64_t n) {
+    const int d = pl->d, p = nodes_per_dim(d, pl->prm.nr_interpolation);
+    bool wide;
+    if (!cut_kernels_fit(pl, R, p, wide)) return 0;
+    double off[MAXD];
+    for (int k = 0; k < d && ymin; k++) off[k] = (double)xmin[k] - (double)ymin[k];
+    for (int l = 1; (n >> (d * l)) >= STOP_POINTS; l++)
+        if (cut_is_exact(d, ldexp((double)edge0, -l), (double)pl->lcs, ymin ? off : nullptr, l, p)) return l;
+    return 0;
+}
+
+int far_cut_level(const f3m_plan *pl, int R) {
+    const int L = pl->levels, d = pl->d;
+    if (L < 1) return 0;
+    const int p = pl->lists[1].p;
+    bool wide;
+    if (!cut_kernels_fit(pl, R, p, wide)) return 0;
+    int P = 1;
+    for (int k = 0; k < d; k++) P *= p;
+    double off[MAXD];
+    for (int k = 0; k < d; k++) off[k] = (double)pl->tx.origin[k] - (double)pl->ty->origin[k];
     const double cols = wide ? 8.0 * ((R + 7) / 8) : R;
     auto m2l = [&](const PairCSR &c) { return (double)c.count * P * cols * 1.25e-12; };
     auto shifts = [&](int l) { return ((double)pl->tx.levels[l].nb + pl->ty->levels[l].nb) * P * cols * 8e-12; };
@@ -1371,7 +1397,8 @@ int far_cut_level(const f3m_plan *pl, int R) {
     for (int l = 1; l <= L; l++) {
         const LevelLists &ll = pl->lists[l];
         const double t = head + m2l(ll.far) + m2l(ll.small) + m2l(ll.keep) + shifts(l);
-        if (t < best_t && ll.far.count + ll.small.count + ll.keep.count <= 0x7fffffffLL && cut_is_exact(pl, l, p)) { best = l; best_t = t; }
+        if (t < best_t && ll.far.count + ll.small.count + ll.keep.count <= 0x7fffffffLL && 
+            cut_is_exact(d, (double)pl->ty->levels[l].edge, (double)pl->lcs, pl->same ? nullptr : off, l, p)) { best = l; best_t = t; }
         head += direct[l] + m2l(ll.far) + shifts(l);
     }
     return best;

@@ -236,9 +236,13 @@ __device__ __forceinline__ float div_mode(float a, float b, int ieee) {
 //
 // A fixed grid of blocks (one wave: SM count x resident blocks) each owns a contiguous run of tiles.  Per pass:
 // digit histogram per block (the first one is taken while the keys are computed), one scan per digit over the
-// blocks, stable scatter.  The scatter ranks a tile's keys with warp-level match (warp-private counters), stages
+// blocks, stable scatter.  The scatter ranks a tile's keys with ballots (warp-private counters), stages
 // every array of the tile in shared memory in digit order and writes runs of consecutive addresses.
 // No block waits for another block.
+//
+// 1e8 points, d = 3: two passes of nine bits 4.65 ms, the records taken apart 0.50, b gathered 1.85; two passes of six bits (a tree that
+// ends at level 4) with planes from the last pass and b carried along 1.15 + 1.72.  b in passes of nine and ten bits, whose runs are four
+// words long: 1e7 points, five passes 1.03 -> 1.51 ms, so it is carried by short digits only.
 // ---------------------------------------------------------------------------------------------
 constexpr int RS_T = 256;                 // threads per block
 constexpr int RS_I = 8;                   // keys per thread and tile
@@ -373,20 +377,24 @@ struct SortIO {
     int row0;                  // first pass: the record's row is row0 + position
     const void *rin;           // later passes: records of the input order
     uint32_t *kout;
-    void *rout;                // records of the output order
+    void *rout;                // records of the output order, or (last pass)
+    int *perm;                 // their parts: permutation
+    float *pts;                // and coordinate planes
+    const float *bin;          // a value per point that travels along, or null
+    float *bout;
     int first;
 };
 
-__host__ __device__ constexpr size_t rs_smem_bytes(int nbins, int rec_words) {
-    // per-warp counters (u16), gofs + bbase (int), staged keys, staged records
-    return (size_t)RS_W * nbins * 2 + (size_t)2 * nbins * 4 + (size_t)RS_TILE * 4 + (size_t)RS_TILE * rec_words * 4;
+__host__ __device__ constexpr size_t rs_smem_bytes(int nbins, int rec_words, bool value) {
+    // per-warp counters (u16), gofs + bbase (int), staged keys, staged records, staged values
+    return (size_t)RS_W * nbins * 2 + (size_t)2 * nbins * 4 + (size_t)RS_TILE * 4 + (size_t)RS_TILE * rec_words * 4 + (value ? (size_t)RS_TILE * 4 : 0);
 }
 
-// STABLE = false ranks a key among the tile's keys of its digit in whatever order the shared-memory atomics grant.
-// That would do for a first pass on one GPU (points that agree in every sorted bit lie in one finest-level box), but
-// the order then differs from run to run, so the host uses the stable form for every pass.
-template <int D, bool STABLE>
-__global__ void __launch_bounds__(RS_T, 3) rs_scatter(SortIO io, int64_t n, int shift, int dbits, int64_t chunk,
+// The keys of a tile are ranked first; records (and values) are read when their slots are known, so that they occupy no registers
+// while the ballots run: four blocks per SM instead of three.  PLANES: the last pass writes permutation and planes instead of
+// records, where runs of equal digits are long enough for stores of single words.
+template <int D, bool PLANES, bool VALUE>
+__global__ void __launch_bounds__(RS_T, 4) rs_scatter(SortIO io, int64_t n, int shift, int dbits, int64_t chunk,
                                                   const int *__restrict__ rowex, const int *__restrict__ tot, int G) {
     constexpr int VW = Rec<D>::VW, RV = Rec<D>::RV, RW = VW * RV;
     typedef typename VecOf<VW>::type vec_t;
@@ -395,7 +403,8 @@ __global__ void __launch_bounds__(RS_T, 3) rs_scatter(SortIO io, int64_t n, int 
     const int nbins = 1 << dbits;
     vec_t *stage_rec = reinterpret_cast<vec_t *>(rs_smem);                                  // [RS_TILE][RV]
     uint32_t *stage_key = reinterpret_cast<uint32_t *>(rs_smem + (size_t)RS_TILE * RW * 4);   // [RS_TILE]
-    int *gofs = reinterpret_cast<int *>(stage_key + RS_TILE);   // global position of staged slot q of digit g: gofs[g] + q
+    float *stage_val = reinterpret_cast<float *>(stage_key + RS_TILE);                        // [RS_TILE] with VALUE
+    int *gofs = reinterpret_cast<int *>(stage_val + (VALUE ? RS_TILE : 0));   // global position of staged slot q of digit g: gofs[g] + q
     int *bbase = gofs + nbins;                                  // next global position per digit for this block
     unsigned short *wcnt = reinterpret_cast<unsigned short *>(bbase + nbins);   // [RS_W][nbins] counts, then start slots
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -419,95 +428,57 @@ __global__ void __launch_bounds__(RS_T, 3) rs_scatter(SortIO io, int64_t n, int 
                 bbase[d0 + q] = ex + rowex[(size_t)(d0 + q) * G + blockIdx.x];
                 ex += t[q];
                 for (int ww = 0; ww < RS_W; ww++) wcnt[(size_t)ww * nbins + d0 + q] = 0;
-                gofs[d0 + q] = 0;
             }
         }
     }
     __syncthreads();
     const int64_t beg = (int64_t)blockIdx.x * chunk, end = min(n, beg + chunk);
+    const int j0 = w * (32 * RS_I) + lane;   // item r of this lane: point tile + j0 + 32 r
+    uint32_t key[RS_I];
+    auto load_keys = [&](int64_t tile) {
+#pragma unroll
+        for (int r = 0; r < RS_I; r++) key[r] = tile + j0 + 32 * r < end ? io.kin[tile + j0 + 32 * r] : 0u;
+    };
+    load_keys(beg);
     for (int64_t tile = beg; tile < end; tile += RS_TILE) {
         const int tile_cnt = (int)min((int64_t)RS_TILE, end - tile);
-        const int j0 = w * (32 * RS_I) + lane;   // item r of this lane: point tile + j0 + 32 r
-        const uint32_t *__restrict__ kin = io.kin + tile;
-        uint32_t key[RS_I];
-        vec_t rec[RS_I][RV];
         int sp[RS_I];
+        // rank inside the warp: items in (r, lane) order = input order.  The lanes that hold the same digit are
+        // found with one ballot per digit bit (the match instruction costs a step per distinct value, and nearly
+        // all 32 digits of a warp are distinct).
 #pragma unroll
-        for (int r = 0; r < RS_I; r++) key[r] = (j0 + 32 * r < tile_cnt) ? kin[j0 + 32 * r] : 0u;
-        if (io.first) {
-            const float *__restrict__ xin = io.X + tile * D;
+        for (int r = 0; r < RS_I; r++) {
+            const bool valid = j0 + 32 * r < tile_cnt;
+            const int dg = (int)((key[r] >> shift) & mask);
+            unsigned m = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
-            for (int r = 0; r < RS_I; r++) {
-                const int j = j0 + 32 * r;
-                uint32_t wds[RW];
-#pragma unroll
-                for (int q = 0; q < RW; q++) wds[q] = 0u;
-                if (j < tile_cnt) {
-                    wds[0] = (uint32_t)(io.row0 + tile + j);
-#pragma unroll
-                    for (int k = 0; k < D; k++) wds[1 + k] = __float_as_uint(xin[j * D + k]);
-                }
-#pragma unroll
-                for (int v = 0; v < RV; v++) {
-                    if (VW == 4) rec[r][v] = *reinterpret_cast<vec_t *>(&wds[4 * v]);
-                    else { uint2 t2 = make_uint2(wds[2 * v], wds[2 * v + 1]); rec[r][v] = *reinterpret_cast<vec_t *>(&t2); }
+            for (int bit = 0; bit < RS_MAXBITS; bit++) {
+                if (bit < dbits) {
+                    const unsigned bal = __ballot_sync(0xffffffffu, (dg >> bit) & 1);
+                    m &= ((dg >> bit) & 1) ? bal : ~bal;
                 }
             }
-        } else {
-            const vec_t *__restrict__ rin = reinterpret_cast<const vec_t *>(io.rin) + tile * RV;
-#pragma unroll
-            for (int r = 0; r < RS_I; r++) {
-                const int j = j0 + 32 * r;
-#pragma unroll
-                for (int v = 0; v < RV; v++)
-                    if (j < tile_cnt) rec[r][v] = rin[j * RV + v];
+            // m: valid lanes with this lane's digit (meaningless on invalid lanes, which take no part)
+            const int leader = __ffs(m) - 1;
+            int old = 0;
+            if (valid && lane == leader) {
+                old = wrow[dg];
+                wrow[dg] = (unsigned short)(old + __popc(m));
             }
-        }
-        if (STABLE) {
-            // rank inside the warp: items in (r, lane) order = input order.  The lanes that hold the same digit are
-            // found with one ballot per digit bit (the match instruction costs a step per distinct value, and nearly
-            // all 32 digits of a warp are distinct).
-#pragma unroll
-            for (int r = 0; r < RS_I; r++) {
-                const bool valid = j0 + 32 * r < tile_cnt;
-                const int dg = (int)((key[r] >> shift) & mask);
-                unsigned m = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-                for (int bit = 0; bit < RS_MAXBITS; bit++) {
-                    if (bit < dbits) {
-                        const unsigned bal = __ballot_sync(0xffffffffu, (dg >> bit) & 1);
-                        m &= ((dg >> bit) & 1) ? bal : ~bal;
-                    }
-                }
-                // m: valid lanes with this lane's digit (meaningless on invalid lanes, which take no part)
-                const int leader = __ffs(m) - 1;
-                int old = 0;
-                if (valid && lane == leader) {
-                    old = wrow[dg];
-                    wrow[dg] = (unsigned short)(old + __popc(m));
-                }
-                old = __shfl_sync(0xffffffffu, old, valid ? leader : lane);
-                sp[r] = valid ? old + __popc(m & ((1u << lane) - 1u)) : -1;
-                __syncwarp();
-            }
-        } else {
-            // one counter per digit for the whole tile (kept in gofs until the scan below replaces it)
-#pragma unroll
-            for (int r = 0; r < RS_I; r++)
-                sp[r] = (j0 + 32 * r < tile_cnt) ? atomicAdd(&gofs[(key[r] >> shift) & mask], 1) : -1;
+            old = __shfl_sync(0xffffffffu, old, valid ? leader : lane);
+            sp[r] = valid ? old + __popc(m & ((1u << lane) - 1u)) : -1;
+            __syncwarp();
         }
         __syncthreads();
-        // per digit: start slot in the staged tile (per warp in the stable form), global position of slot 0
+        // per digit: start slot in the staged tile per warp, global position of slot 0
         int tsum[RS_DPT];
         {
             int sum = 0;
 #pragma unroll
             for (int q = 0; q < RS_DPT; q++) {
                 int run = 0;
-                if (q < dpt && owner) {
-                    if (STABLE) for (int ww = 0; ww < RS_W; ww++) run += wcnt[(size_t)ww * nbins + d0 + q];
-                    else run = gofs[d0 + q];
-                }
+                if (q < dpt && owner)
+                    for (int ww = 0; ww < RS_W; ww++) run += wcnt[(size_t)ww * nbins + d0 + q];
                 tsum[q] = run;
                 sum += run;
             }
@@ -516,55 +487,91 @@ __global__ void __launch_bounds__(RS_T, 3) rs_scatter(SortIO io, int64_t n, int 
             for (int q = 0; q < RS_DPT; q++) {
                 if (q < dpt && owner) {
                     gofs[d0 + q] = bbase[d0 + q] - ex;
-                    if (STABLE) {
-                        int run = ex;
-                        for (int ww = 0; ww < RS_W; ww++) {
-                            const int c = wcnt[(size_t)ww * nbins + d0 + q];
-                            wcnt[(size_t)ww * nbins + d0 + q] = (unsigned short)run;
-                            run += c;
-                        }
-                    } else
-                        wcnt[d0 + q] = (unsigned short)ex;   // row 0 holds the start slots
+                    int run = ex;
+                    for (int ww = 0; ww < RS_W; ww++) {
+                        const int c = wcnt[(size_t)ww * nbins + d0 + q];
+                        wcnt[(size_t)ww * nbins + d0 + q] = (unsigned short)run;
+                        run += c;
+                    }
                     ex += tsum[q];
                 }
             }
         }
         __syncthreads();
+        if (io.first) {
+            const float *__restrict__ xin = io.X + tile * D;
 #pragma unroll
-        for (int r = 0; r < RS_I; r++) {
-            if (sp[r] >= 0) {
-                const int slot = sp[r] + (STABLE ? wrow : wcnt)[(key[r] >> shift) & mask];
-                stage_key[slot] = key[r];
+            for (int r = 0; r < RS_I; r++) {
+                if (sp[r] < 0) continue;
+                const int j = j0 + 32 * r;
+                uint32_t wds[RW];
+                wds[0] = (uint32_t)(io.row0 + tile + j);
 #pragma unroll
-                for (int v = 0; v < RV; v++) stage_rec[slot * RV + v] = rec[r][v];
+                for (int k = 0; k < D; k++) wds[1 + k] = __float_as_uint(xin[j * D + k]);
+#pragma unroll
+                for (int q = D + 1; q < RW; q++) wds[q] = 0u;
+                const int slot = sp[r] + wrow[(key[r] >> shift) & mask];
+#pragma unroll
+                for (int v = 0; v < RV; v++) {
+                    if (VW == 4) stage_rec[slot * RV + v] = *reinterpret_cast<vec_t *>(&wds[4 * v]);
+                    else { uint2 t2 = make_uint2(wds[2 * v], wds[2 * v + 1]); stage_rec[slot * RV + v] = *reinterpret_cast<vec_t *>(&t2); }
+                }
+            }
+        } else {
+            const vec_t *__restrict__ rin = reinterpret_cast<const vec_t *>(io.rin) + tile * RV;
+#pragma unroll
+            for (int r = 0; r < RS_I; r++) {
+                if (sp[r] < 0) continue;
+                const int slot = sp[r] + wrow[(key[r] >> shift) & mask];
+#pragma unroll
+                for (int v = 0; v < RV; v++) stage_rec[slot * RV + v] = rin[(j0 + 32 * r) * RV + v];
             }
         }
+#pragma unroll
+        for (int r = 0; r < RS_I; r++) {
+            if (sp[r] < 0) continue;
+            const int slot = sp[r] + wrow[(key[r] >> shift) & mask];
+            stage_key[slot] = key[r];
+            if (VALUE) stage_val[slot] = io.bin[tile + j0 + 32 * r];
+        }
+        load_keys(tile + RS_TILE);   // on their way while this tile is written
         __syncthreads();
-        // positions of the staged slots (runs of consecutive global positions per digit); then the counters are
+        // positions of the staged slots (runs of consecutive global positions per digit); the counters are
         // cleared for the next tile and the block's positions advance
-        int pos[RS_I];
+        if (owner) {
+#pragma unroll
+            for (int q = 0; q < RS_DPT; q++) {
+                if (q < dpt) {
+                    bbase[d0 + q] += tsum[q];
+                    for (int ww = 0; ww < RS_W; ww++) wcnt[(size_t)ww * nbins + d0 + q] = 0;
+                }
+            }
+        }
 #pragma unroll
         for (int k = 0; k < RS_I; k++) {
             const int q = threadIdx.x + k * RS_T;
-            pos[k] = q < tile_cnt ? gofs[(stage_key[q] >> shift) & mask] + q : -1;
-        }
-        if (!STABLE) __syncthreads();   // gofs is cleared below: every thread must have read it
+            if (q < tile_cnt) {
+                const uint32_t ky = stage_key[q];
+                const int64_t pos = gofs[(ky >> shift) & mask] + q;
+                io.kout[pos] = ky;
+                if (PLANES) {
+                    uint32_t wds[RW];
 #pragma unroll
-        for (int q = 0; q < RS_DPT; q++) {
-            if (q < dpt && owner) {
-                bbase[d0 + q] += tsum[q];
-                if (STABLE) for (int ww = 0; ww < RS_W; ww++) wcnt[(size_t)ww * nbins + d0 + q] = 0;
-                else gofs[d0 + q] = 0;
-            }
-        }
+                    for (int v = 0; v < RV; v++) {
+                        const vec_t t = stage_rec[q * RV + v];
+                        const uint32_t *tw = reinterpret_cast<const uint32_t *>(&t);
 #pragma unroll
-        for (int k = 0; k < RS_I; k++) {
-            if (pos[k] >= 0) {
-                const int q = threadIdx.x + k * RS_T;
-                io.kout[pos[k]] = stage_key[q];
-                vec_t *rout = reinterpret_cast<vec_t *>(io.rout) + (size_t)pos[k] * RV;
+                        for (int c = 0; c < VW; c++) wds[VW * v + c] = tw[c];
+                    }
+                    io.perm[pos] = (int)wds[0];
 #pragma unroll
-                for (int v = 0; v < RV; v++) rout[v] = stage_rec[q * RV + v];
+                    for (int c = 0; c < D; c++) io.pts[(size_t)c * n + pos] = __uint_as_float(wds[1 + c]);
+                } else {
+                    vec_t *rout = reinterpret_cast<vec_t *>(io.rout) + (size_t)pos * RV;
+#pragma unroll
+                    for (int v = 0; v < RV; v++) rout[v] = stage_rec[q * RV + v];
+                }
+                if (VALUE) io.bout[pos] = stage_val[q];
             }
         }
         __syncthreads();
@@ -667,20 +674,29 @@ __global__ void __launch_bounds__(256) unpack_records(const void *__restrict__ r
     for (int c = 0; c < D; c++) pts[(size_t)c * n + i] = __uint_as_float(wds[1 + c]);
 }
 
-// keys and records [row0 + position, coordinates] of n points, sorted by the key bits [shift0, shift0 + bits)
-template <int D>
+// Stores of single words want runs: digits of at most PLANE_BITS bits, or arrays that stay in L2 until their lines are complete.
+constexpr int PLANE_BITS = 7;
+constexpr int64_t PLANE_POINTS = 1 << 21;
+static int sort_pass_count(int bits) { return (bits + RS_MAXBITS - 1) / RS_MAXBITS; }
+static int sort_digit_bits(int bits) { return (bits + sort_pass_count(bits) - 1) / sort_pass_count(bits); }
+bool sort_carries(int d, int depth) { return sort_digit_bits(d * depth) <= PLANE_BITS; }
+
+// Keys and records [row0 + position, coordinates] of n points, sorted by the key bits [shift0, shift0 + bits).  With a tree, its
+// permutation and planes instead of records; with b, the values b in sorted order.
+template <int D, bool VALUE>
 static void sort_records(const float *X, int64_t n, int row0, const MortonCfg &cfg, int shift0, int bits, DevBuf<uint32_t> &keys_out,
-                         DevBuf<uint32_t> &recs_out, cudaStream_t s) {
+                         DevBuf<uint32_t> &recs_out, Tree *tree, const float *b, DevBuf<float> *b_out, cudaStream_t s) {
     constexpr int RW = Rec<D>::VW * Rec<D>::RV;
-    const int passes = (bits + RS_MAXBITS - 1) / RS_MAXBITS;
-    const int dbits_all = (bits + passes - 1) / passes;
-    const size_t smem = rs_smem_bytes(1 << dbits_all, RW);
+    const int passes = sort_pass_count(bits), dbits_all = sort_digit_bits(bits);
+    const size_t smem = rs_smem_bytes(1 << dbits_all, RW, VALUE);
+    const bool planes = tree && (dbits_all <= PLANE_BITS || n <= PLANE_POINTS);
     // one wave of blocks, each with a contiguous run of whole tiles
     int dev = 0, sms = NUM_SMS_HINT, occ = 1;
     F3M_CUDA(cudaGetDevice(&dev));
     F3M_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    F3M_CUDA(cudaFuncSetAttribute(rs_scatter<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    F3M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rs_scatter<D, true>, RS_T, smem));
+    F3M_CUDA(cudaFuncSetAttribute(rs_scatter<D, false, VALUE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    F3M_CUDA(cudaFuncSetAttribute(rs_scatter<D, true, VALUE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    F3M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rs_scatter<D, false, VALUE>, RS_T, smem));
     const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
     const int64_t wave = (int64_t)sms * std::max(1, occ);
     const int64_t tpb = (ntiles + wave - 1) / wave;
@@ -688,17 +704,21 @@ static void sort_records(const float *X, int64_t n, int row0, const MortonCfg &c
     const int64_t chunk = tpb * RS_TILE;
 
     DevBuf<uint32_t> kA, kB, rA, rB;   // keys and records, ping-pong
+    DevBuf<float> bA, bB;
     DevBuf<int> counts, tot;
     kA.alloc(n, s); kB.alloc(n, s);
-    rB.alloc((size_t)n * RW, s);
-    if (passes > 1) rA.alloc((size_t)n * RW, s);
+    const bool last_to_b = passes % 2 == 1;
+    if (!(planes && last_to_b && passes == 1)) rB.alloc((size_t)n * RW, s);
+    if (passes > 2 || (passes == 2 && !planes)) rA.alloc((size_t)n * RW, s);
+    if (VALUE) { bB.alloc(n, s); if (passes > 1) bA.alloc(n, s); }
+    if (planes) { tree->perm.alloc(n, s); tree->pts.alloc((size_t)n * D, s); }
     counts.alloc((size_t)RS_MAXBINS * G, s);
     tot.alloc(RS_MAXBINS, s);
 
     for (int pass = 0; pass < passes; pass++) {
         const int shift = shift0 + pass * dbits_all;
         const int dbits = std::min(dbits_all, shift0 + bits - shift);
-        const bool to_b = (pass % 2) == 0;
+        const bool to_b = (pass % 2) == 0, last = pass == passes - 1;
         if (pass == 0) morton_hist_kernel<D><<<G, 512, 0, s>>>(X, n, cfg, shift, dbits, chunk, kA.p, counts.p, G);
         else rs_hist<<<G, 512, 0, s>>>(to_b ? kA.p : kB.p, n, shift, dbits, chunk, counts.p, G);
         F3M_LAUNCH_CHECK();
@@ -712,24 +732,33 @@ static void sort_records(const float *X, int64_t n, int row0, const MortonCfg &c
         io.X = X;
         io.rin = to_b ? rA.p : rB.p;
         io.rout = to_b ? rB.p : rA.p;
+        io.bin = pass == 0 ? b : to_b ? bA.p : bB.p;
+        io.bout = to_b ? bB.p : bA.p;
+        if (planes) { io.perm = tree->perm.p; io.pts = tree->pts.p; }
         // every pass stable, the first one too: ranks that build the same plan on different GPUs must end with the same
-        // permutation (their sorted slices are exchanged), and the form ranked by atomics measured no faster
-        rs_scatter<D, true><<<G, RS_T, rs_smem_bytes(1 << dbits, RW), s>>>(io, n, shift, dbits, chunk, counts.p, tot.p, G);
+        // permutation (their sorted slices are exchanged)
+        const size_t bytes = rs_smem_bytes(1 << dbits, RW, VALUE);
+        if (planes && last) rs_scatter<D, true, VALUE><<<G, RS_T, bytes, s>>>(io, n, shift, dbits, chunk, counts.p, tot.p, G);
+        else rs_scatter<D, false, VALUE><<<G, RS_T, bytes, s>>>(io, n, shift, dbits, chunk, counts.p, tot.p, G);
         F3M_LAUNCH_CHECK();
     }
-    keys_out = std::move(passes % 2 == 1 ? kB : kA);
-    recs_out = std::move(passes % 2 == 1 ? rB : rA);
+    keys_out = std::move(last_to_b ? kB : kA);
+    if (VALUE) *b_out = std::move(last_to_b ? bB : bA);
+    DevBuf<uint32_t> &recs = last_to_b ? rB : rA;
+    if (tree && !planes) {
+        tree->perm.alloc(n, s);
+        tree->pts.alloc((size_t)n * D, s);
+        unpack_records<D><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(recs.p, n, tree->perm.p, tree->pts.p);
+        F3M_LAUNCH_CHECK();
+    }
+    if (!tree) recs_out = std::move(recs);
 }
 
 template <int D>
-static void sort_passes(Tree &t, const float *X, const MortonCfg &cfg, int shift0, int bits, cudaStream_t s) {
-    const int64_t n = t.n;
-    DevBuf<uint32_t> recs;
-    sort_records<D>(X, n, 0, cfg, shift0, bits, t.keys, recs, s);
-    t.perm.alloc(n, s);
-    t.pts.alloc((size_t)n * D, s);
-    unpack_records<D><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(recs.p, n, t.perm.p, t.pts.p);
-    F3M_LAUNCH_CHECK();
+static void sort_passes(Tree &t, const float *X, const MortonCfg &cfg, int shift0, int bits, const float *b, DevBuf<float> *b_out, cudaStream_t s) {
+    DevBuf<uint32_t> none;
+    if (b) sort_records<D, true>(X, t.n, 0, cfg, shift0, bits, t.keys, none, &t, b, b_out, s);
+    else sort_records<D, false>(X, t.n, 0, cfg, shift0, bits, t.keys, none, &t, nullptr, nullptr, s);
 }
 
 static MortonCfg morton_cfg(int d, const Cube &cube, int math_mode) {
@@ -784,11 +813,11 @@ void sort_shard(const float *X, int64_t n, int64_t row0, int d, const float *ori
     const int shift0 = d * (cfg.L - depth), bits = d * depth, ncells = 1 << bits;
     DevBuf<uint32_t> keys, recs;
     switch (d) {
-        case 1: sort_records<1>(X, n, (int)row0, cfg, shift0, bits, keys, recs, s); break;
-        case 2: sort_records<2>(X, n, (int)row0, cfg, shift0, bits, keys, recs, s); break;
-        case 3: sort_records<3>(X, n, (int)row0, cfg, shift0, bits, keys, recs, s); break;
-        case 4: sort_records<4>(X, n, (int)row0, cfg, shift0, bits, keys, recs, s); break;
-        default: sort_records<5>(X, n, (int)row0, cfg, shift0, bits, keys, recs, s); break;
+        case 1: sort_records<1, false>(X, n, (int)row0, cfg, shift0, bits, keys, recs, nullptr, nullptr, nullptr, s); break;
+        case 2: sort_records<2, false>(X, n, (int)row0, cfg, shift0, bits, keys, recs, nullptr, nullptr, nullptr, s); break;
+        case 3: sort_records<3, false>(X, n, (int)row0, cfg, shift0, bits, keys, recs, nullptr, nullptr, nullptr, s); break;
+        case 4: sort_records<4, false>(X, n, (int)row0, cfg, shift0, bits, keys, recs, nullptr, nullptr, nullptr, s); break;
+        default: sort_records<5, false>(X, n, (int)row0, cfg, shift0, bits, keys, recs, nullptr, nullptr, nullptr, s); break;
     }
     F3M_CUDA(cudaMemcpyAsync(recs_out, recs.p, (size_t)n * record_words(d) * 4, cudaMemcpyDeviceToDevice, s));
     DevBuf<int> a, b;
@@ -938,7 +967,8 @@ void tree_attach_runs(Tree &t, const uint32_t *recs, int64_t stride, cudaStream_
 
 // Sorts the points of one tree by the first `depth` levels of their Morton key (all later levels are read off the
 // sorted keys, tree.cu) and leaves keys, permutation and coordinate planes in the tree.
-void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s) {
+void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s,
+                       const float *b, DevBuf<float> *b_out) {
     F3M_REQUIRE(n < (int64_t)0x7fffffff, F3M_ERR_OVERFLOW, "point count %lld does not fit a 31-bit index", (long long)n);
     t.n = n;
     t.d = d;
@@ -953,11 +983,11 @@ void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cu
     const MortonCfg cfg = morton_cfg(d, cube, math_mode);
     const int shift0 = d * (t.lmax - depth), bits = d * depth;
     switch (d) {
-        case 1: sort_passes<1>(t, X, cfg, shift0, bits, s); break;
-        case 2: sort_passes<2>(t, X, cfg, shift0, bits, s); break;
-        case 3: sort_passes<3>(t, X, cfg, shift0, bits, s); break;
-        case 4: sort_passes<4>(t, X, cfg, shift0, bits, s); break;
-        default: sort_passes<5>(t, X, cfg, shift0, bits, s); break;
+        case 1: sort_passes<1>(t, X, cfg, shift0, bits, b, b_out, s); break;
+        case 2: sort_passes<2>(t, X, cfg, shift0, bits, b, b_out, s); break;
+        case 3: sort_passes<3>(t, X, cfg, shift0, bits, b, b_out, s); break;
+        case 4: sort_passes<4>(t, X, cfg, shift0, bits, b, b_out, s); break;
+        default: sort_passes<5>(t, X, cfg, shift0, bits, b, b_out, s); break;
     }
 }
 
