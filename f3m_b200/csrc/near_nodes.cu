@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(128) l2p_wide3(const float *__restrict__ pts, 
 // Node-to-node step: one CTA per target box, its groups of WPG warps share the row, which is ordered by (o0, o1, o2).  A thread
 // owns FPT fibres (positions m0, m1) of the sums V over the pairs of one (o0, o1): per pair it reads their PP moments along the last
 // axis and applies that axis' matrix, whose columns come from shared memory as broadcasts -- FPT * PP multiply-adds per PP / 4 of
-// them.  When (o0, o1) changes V is laid out anew for the axis before, as in m2l_nested.  Bound: FP32 lanes (NF of FPT * 32 * WPG
+// them, two outputs per instruction (p = 9: 2.67 -> 2.28 ms; one by one the issue slots were 65 % busy, the FMA pipe 47 %).  When (o0, o1) changes V is laid out anew for the axis before, as in m2l_nested.  Bound: FP32 lanes (NF of FPT * 32 * WPG
 // busy), then the groups' ends.
 // ---------------------------------------------------------------------------------------------
 template <int PP>
@@ -288,23 +288,56 @@ __device__ __forceinline__ void group_sync(int group) {
     else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(32 * WPG) : "memory");
 }
 
-// acc[r][i] += sum_j M[j][i] v[r][j]
+// A thread's sums: PP values of each of its fibres, two to a register pair (the last one of an odd number by itself)
 template <int PP>
-__device__ __forceinline__ void column_apply(const float (&v)[ColCfg<PP>::FPT][PP], const float *M, float (&acc)[ColCfg<PP>::FPT][PP]) {
+struct ColAcc {
+    static constexpr int FPT = ColCfg<PP>::FPT, NP = PP / 2, ODD = PP & 1;
+    f32x2 p[FPT][NP];
+    float last[FPT];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int r = 0; r < FPT; r++) {
+#pragma unroll
+            for (int i = 0; i < NP; i++) p[r][i] = 0ull;
+            last[r] = 0.f;
+        }
+    }
+    // stores entry i of fibre r at dst[i * stride]
+    __device__ __forceinline__ void store(int r, float *dst, int stride) const {
+#pragma unroll
+        for (int i = 0; i < NP; i++) {
+            float lo, hi;
+            unpack2(p[r][i], lo, hi);
+            dst[2 * i * stride] = lo;
+            dst[(2 * i + 1) * stride] = hi;
+        }
+        if (ODD) dst[(PP - 1) * stride] = last[r];
+    }
+};
+// acc[r][i] += sum_j M[j][i] v[r][j]: two outputs per instruction, the column's entries come in pairs from shared memory
+template <int PP>
+__device__ __forceinline__ void column_apply(const float (&v)[ColCfg<PP>::FPT][PP], const float *M, ColAcc<PP> &acc) {
     using C = ColCfg<PP>;
+    using A = ColAcc<PP>;
 #pragma unroll
     for (int j = 0; j < PP; j++) {
-        float m[C::MSR];
-        const float4 *M4 = reinterpret_cast<const float4 *>(M + j * C::MSR);
+        f32x2 m[C::MSR / 2];
+        const ulonglong2 *M4 = reinterpret_cast<const ulonglong2 *>(M + j * C::MSR);
 #pragma unroll
         for (int q = 0; q < C::MSR / 4; q++) {
-            const float4 w = M4[q];
-            m[4 * q] = w.x; m[4 * q + 1] = w.y; m[4 * q + 2] = w.z; m[4 * q + 3] = w.w;
+            const ulonglong2 w = M4[q];
+            m[2 * q] = w.x;
+            m[2 * q + 1] = w.y;
         }
+        float m_last, unused;
+        unpack2(m[A::NP < C::MSR / 2 ? A::NP : 0], m_last, unused);
 #pragma unroll
-        for (int r = 0; r < C::FPT; r++)
+        for (int r = 0; r < C::FPT; r++) {
+            const f32x2 vv = pack2(v[r][j], v[r][j]);
 #pragma unroll
-            for (int i = 0; i < PP; i++) acc[r][i] = fmaf(m[i], v[r][j], acc[r][i]);
+            for (int i = 0; i < A::NP; i++) acc.p[r][i] = fma2(m[i], vv, acc.p[r][i]);
+            if (A::ODD) acc.last[r] = fmaf(m_last, v[r][j], acc.last[r]);
+        }
     }
 }
 
@@ -321,15 +354,9 @@ __global__ void __launch_bounds__(128) m2l_columns(const int *__restrict__ fptr,
     const int group = threadIdx.x / NT, t = threadIdx.x - group * NT, lane = threadIdx.x & 31;
     float *buf = sm + 3 * NOFF2 * C::MS + (size_t)group * P, *sum = buf + (size_t)C::NGRP * P;   // the group's transposes, its sums
     for (int q = t; q < P; q += NT) sum[q] = 0.f;
-    float V[FPT][PP], U[FPT][PP];
-    auto clear = [&](float (&a)[FPT][PP]) {
-#pragma unroll
-        for (int r = 0; r < FPT; r++)
-#pragma unroll
-            for (int i = 0; i < PP; i++) a[r][i] = 0.f;
-    };
-    clear(V);
-    clear(U);
+    ColAcc<PP> V, U;
+    V.clear();
+    U.clear();
     __syncthreads();
     // fibre f of the middle axis: m0 = f % PP, m2 = f / PP; of the first axis: m1 = f % PP, m2 = f / PP
     auto mid = [&](int f) { return f / PP * NF + f % PP; };
@@ -337,11 +364,9 @@ __global__ void __launch_bounds__(128) m2l_columns(const int *__restrict__ fptr,
 #pragma unroll
         for (int r = 0; r < FPT; r++) {
             const int f = t + r * NT;
-            if (f < NF)
-#pragma unroll
-                for (int i = 0; i < PP; i++) buf[f + NF * i] = V[r][i];
+            if (f < NF) V.store(r, buf + f, NF);
         }
-        clear(V);
+        V.clear();
         group_sync<C::WPG>(group);
         float v[FPT][PP];
 #pragma unroll
@@ -356,11 +381,9 @@ __global__ void __launch_bounds__(128) m2l_columns(const int *__restrict__ fptr,
 #pragma unroll
         for (int r = 0; r < FPT; r++) {
             const int f = t + r * NT;
-            if (f < NF)
-#pragma unroll
-                for (int i = 0; i < PP; i++) buf[mid(f) + PP * i] = U[r][i];
+            if (f < NF) U.store(r, buf + mid(f), PP);
         }
-        clear(U);
+        U.clear();
         group_sync<C::WPG>(group);
 #pragma unroll
         for (int r = 0; r < FPT; r++) {
@@ -369,14 +392,17 @@ __global__ void __launch_bounds__(128) m2l_columns(const int *__restrict__ fptr,
             for (int j = 0; j < PP; j++) v[r][j] = buf[PP * f + j];
         }
         column_apply<PP>(v, Tsm + ((key >> 8) & 15u) * C::MS, U);
+        group_sync<C::WPG>(group);
 #pragma unroll
         for (int r = 0; r < FPT; r++) {
             const int f = t + r * NT;
-            if (f < NF)
+            if (f < NF) {   // the fibre's own entries of buf were read by this thread only
+                U.store(r, buf + PP * f, 1);
 #pragma unroll
-                for (int i = 0; i < PP; i++) sum[PP * f + i] += U[r][i];
+                for (int i = 0; i < PP; i++) sum[PP * f + i] += buf[PP * f + i];
+            }
         }
-        clear(U);
+        U.clear();
         group_sync<C::WPG>(group);
     };
     const int len = e1 - e0;
@@ -423,8 +449,8 @@ static __global__ void __launch_bounds__(256) weights_check(const float *__restr
 // ---------------------------------------------------------------------------------------------
 // Rule.  Estimated seconds of the lists of one level through nodes: the points' two passes, the pairs of boxes, and what the form pays
 // once (launches, the order of the rows, the check of the weights with its read-back).  Measured: 1.8e-13 s per point and node for
-// both passes up to eight nodes, 2.3e-13 beyond; 1e-13 to 1.2e-13 per pair of boxes and p^4 (p = 9, 4.15e6 pairs in rows of 127:
-// 2.64 ms; p = 7, 3.7e6 in rows of 63: 1.08 ms).  Whole calls, lists summed directly / here: 4e6 uniform points, boxes of 122, 1.09
+// both passes up to eight nodes, 2.3e-13 beyond; 0.9e-13 to 1.2e-13 per pair of boxes and p^4 (p = 9, 4.15e6 pairs in rows of 127:
+// 2.28 ms; p = 7, 3.7e6 in rows of 63: 1.08 ms).  Whole calls, lists summed directly / here: 4e6 uniform points, boxes of 122, 1.09
 // lengthscales wide 18.2 / 5.4 ms; 2.9e7 points, l = 0.19 of sqrt12, 179 / 9.2 ms; 6e6 normal points 10.7 / 7.2 ms; 3.6e5 points 3.0 /
 // 0.87 ms; a mixture of 1e7 points 22.8 / 16.8 ms; 6e4 points, 1.5e8 to 7e8 pairs: even, so NODE_FIXED.
 // ---------------------------------------------------------------------------------------------
