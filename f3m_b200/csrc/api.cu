@@ -297,11 +297,16 @@ static void plan_build(f3m_plan *pl, const float *X, int64_t N, const float *Y, 
         F3M_REQUIRE(edge > 0.f && std::isfinite(edge), F3M_ERR_ARG, "degenerate or non-finite bounding cube (edge %g)", edge);
         return edge;
     };
-    const bool one_product = R > 0 && std::min(N, M) >= ONE_PRODUCT_POINTS;
-    if (one_product) {
+    if (R > 0 && std::min(N, M) >= ONE_PRODUCT_POINTS) {
+        pl->one_product = R == 1;
         read_flags(pl, s);
-        const int stop = far_stop_level(pl, R, cube_edge(), xmin, pl->same ? nullptr : ymin, std::min(N, M));
+        const float edge = cube_edge();
+        const int stop = far_stop_level(pl, R, edge, xmin, pl->same ? nullptr : ymin, std::min(N, M));
         if (stop && stop <= depth) depth = pl->stop_level = stop;
+        // uneven points take the tree below the estimate, but often no further than the level that can end it: sorted at once where that
+        // takes no more passes
+        const int node_end = pl->one_product && !pl->stop_level ? far_node_end_level(pl, edge, std::min(30 / d, 20)) : 0;
+        if (node_end > depth && sort_passes_for(d * node_end) == sort_passes_for(d * depth)) depth = node_end;
         // a tree that ends early is not sorted again; a caller's workspace holds no more than it did
         if (pl->stop_level && R == 1 && b && sort_carries(d, depth) && !dev_in_workspace()) pl->carry_b = b;
     }
@@ -366,6 +371,14 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
         LevelLists &ll = pl->lists[l];
         ll.far.count = h[0]; ll.small.count = h[1]; ll.keep.count = h[2];
     };
+    auto take_work = [&](int l) {
+        const long long *work = reinterpret_cast<const long long *>(pl->h_pinned + FL_PAIRWORK) + 4 * l;
+        LevelLists &ll = pl->lists[l];
+        ll.small.pairs = work[0];
+        ll.small.row_boxes = work[1];
+        ll.keep.pairs = work[2];
+        ll.keep.row_boxes = work[3];
+    };
     auto go_on = [&](int level) {
         if (pl->lists[level].keep.count == 0 || (pl->stop_level && level >= pl->stop_level)) return false;
         bool gx = (float)tx.levels[level].max_count > prm->min_points;     // n_tree.cu:1075
@@ -395,6 +408,8 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
         lists_write(pl, l, cap, s);
         return false;
     };
+    // plans for one product: from this level on it is asked whether the product can end there
+    const int end_from = pl->one_product ? far_node_end_level(pl, tx.edge0, tx.lmax) : 0;
     int level = 0, listed = 0;   // levels accepted, levels whose lists are there
     bool work_pending = false;   // the lists' work of some level has not been read
     while (level < listed || go_on(level)) {
@@ -402,6 +417,15 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
             if (!go_on(level)) break;
             level++;
             continue;
+        }
+        if (end_from && level >= end_from && !pl->stop_level) {
+            if (work_pending) take_flags();
+            work_pending = false;
+            take_work(level);
+            if (far_ends_with_nodes(pl, level)) {
+                pl->stop_level = level;
+                break;
+            }
         }
         const int need = level + 1;
         F3M_REQUIRE(need <= tx.lmax, F3M_ERR_DEPTH,
@@ -452,7 +476,6 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
     if (work_pending) take_flags();
     const int p_full = nodes_per_dim(d, prm->nr_interpolation);
     const int p_small = nodes_per_dim(d, std::min((int)lround(pow(3.0, d)), prm->nr_interpolation));
-    const long long *work = reinterpret_cast<const long long *>(pl->h_pinned + FL_PAIRWORK);
     for (int l = 1; l <= level; l++) {
         LevelLists &ll = pl->lists[l];
         // nodes for this level: get_interpolation_rule (n_tree.cu:971-978, 1022-1028)
@@ -467,10 +490,7 @@ static void plan_build_levels(f3m_plan *pl, const float *X, const float *Y, bool
         pl->stats.far_box_pairs += ll.far.count;
         pl->stats.node_pairs += ll.far.count * (int64_t)P * P;
         pl->stats.near_box_pairs += ll.small.count + (l == level ? ll.keep.count : 0);
-        ll.small.pairs = work[4 * l];
-        ll.small.row_boxes = work[4 * l + 1];
-        ll.keep.pairs = work[4 * l + 2];
-        ll.keep.row_boxes = work[4 * l + 3];
+        take_work(l);
         pl->stats.direct_pairs += ll.small.pairs + (l == level ? ll.keep.pairs : 0);
     }
     pl->levels = level;
@@ -515,20 +535,26 @@ static void plan_apply(f3m_plan *pl, const float *b, int R, float *out, int64_t 
     }
     pl->last.end(s);
 
-    // A product over all rows may end at a level whose interpolation is exact for all its pairs (far_cut_level)
-    const int cut = row_begin <= 0 && row_end >= N && !pl->ext_mom && !pl->shard.active ? far_cut_level(pl, R) : 0;
-    pl->last.cut = cut;
+    // A product over all rows may end before the last level (far_cut)
+    const bool whole = row_begin <= 0 && row_end >= N && !pl->ext_mom && !pl->shard.active;
     const int L = pl->levels;
+    CutChoice end = whole ? far_cut(pl, R) : CutChoice{};
+    if (end.level && end.nodes.p && (end.nodes.small || end.nodes.keep) && !node_sums(pl, end.level, end.nodes, bs.p, outs.p, s)) {
+        // no memory for the nodes' moments, or a weight that is not finite: the lists below, which a plan for one product may lack
+        end = far_cut(pl, R, false);
+    }
+    const int cut = end.nodes.p ? 0 : end.level;      // all pairs of the level through the far field's nodes
+    pl->last.cut = end.level;
     if (L == 0) {
         // largest box already small enough: one direct product over the root pair
         direct_sums(pl, 0, pl->lists[0].keep, bs.p, R, outs.p, row_begin, row_end, s);
     }
-    for (int level = 1; level <= (cut ? cut - 1 : L); level++) {
+    for (int level = 1; level <= (end.level ? end.level - 1 : L); level++) {
         LevelLists &ll = pl->lists[level];
         direct_sums(pl, level, ll.small, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1018-1020
     }
-    far_field(pl, bs.p, R, outs.p, row_begin, row_end, cut, s);                     // n_tree.cu:1021-1051, all levels
-    if (L > 0 && !cut) direct_sums(pl, L, pl->lists[L].keep, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1092-1094
+    far_field(pl, bs.p, R, outs.p, row_begin, row_end, cut, end.level ? end.level : L, s);   // n_tree.cu:1021-1051, all levels
+    if (L > 0 && !end.level) direct_sums(pl, L, pl->lists[L].keep, bs.p, R, outs.p, row_begin, row_end, s);   // n_tree.cu:1092-1094
 
     pl->last.begin(ST_UNPERMUTE, s);
     if (row_begin <= 0 && row_end >= N) scatter_rows(outs.p, tx.perm.p, out, N, R, s);
@@ -615,7 +641,7 @@ int f3m_plan_moments_range(f3m_plan *plan, const float *b, int32_t R, int64_t sr
         plan->moments_out = mom_out;
         plan->mom_begin = src_begin;
         plan->mom_end = src_end;
-        far_field(plan, bs.p, R, nullptr, 0, 0, 0, s);
+        far_field(plan, bs.p, R, nullptr, 0, 0, 0, plan->levels, s);
         F3M_CUDA(cudaStreamSynchronize(s));
     });
     plan->moments_out = nullptr;
@@ -757,7 +783,7 @@ int f3m_plan_shard_begin(f3m_plan *plan, const float *b, int32_t R, int64_t row_
             plan->mom_end = plan->h_pinned[1];
             plan->mom_box_begin = box_begin;
             plan->mom_box_end = box_end;
-            far_field(plan, sh.bs.p, R, nullptr, 0, 0, 0, s);
+            far_field(plan, sh.bs.p, R, nullptr, 0, 0, 0, plan->levels, s);
         }
         F3M_CUDA(cudaStreamSynchronize(s));
         sh.active = true;
@@ -798,7 +824,7 @@ int f3m_plan_shard_far(f3m_plan *plan, const float *mom, float *acc_sorted, void
         F3M_REQUIRE(sh.active, F3M_ERR_ARG, "f3m_plan_shard_far without f3m_plan_shard_begin");
         F3M_REQUIRE(mom || sh.all_sources, F3M_ERR_ARG, "this product exchanges moments: pass the gathered moment array");
         plan->ext_mom = sh.all_sources ? nullptr : mom;
-        far_field(plan, sh.bs.p, sh.R, acc_sorted, sh.row_begin, sh.row_end, 0, s);
+        far_field(plan, sh.bs.p, sh.R, acc_sorted, sh.row_begin, sh.row_end, 0, plan->levels, s);
         F3M_CUDA(cudaMemcpyAsync(plan->h_pinned, plan->d_flags + FL_ERR, sizeof(int), cudaMemcpyDeviceToHost, s));
         F3M_CUDA(cudaStreamSynchronize(s));
         F3M_REQUIRE(plan->h_pinned[0] == 0, F3M_ERR_INTERNAL, "device-side consistency check failed (code %d)", plan->h_pinned[0]);

@@ -396,6 +396,7 @@ struct f3m_plan {
     } shard;
     // a plan for one product (f3m_kmvm_f32): it may end at the level where that product will (far_stop_level), and b may have been sorted
     // with its points
+    bool one_product = false;
     int stop_level = 0;
     const float *carry_b = nullptr;
     f3m::DevBuf<float> carried_b;
@@ -416,6 +417,7 @@ struct Cube {
     float edge0 = 0.f;
     const unsigned *own = nullptr, *other = nullptr;
 };
+int sort_passes_for(int bits);
 bool sort_carries(int d, int depth);   // a sort to this depth takes a value per point along at less cost than a gather
 // b (or null): a value per point that travels along, in sorted order at b_out
 void build_sorted_tree(Tree &t, const float *X, int64_t n, int d, const Cube &cube, int math_mode, int depth, cudaStream_t s,
@@ -448,14 +450,29 @@ void build_levels(Tree &t, int l_last, f3m_plan *pl, cudaStream_t s);   // appen
 void lists_count(f3m_plan *pl, int level, cudaStream_t s);
 void lists_write(f3m_plan *pl, int level, const int64_t cap[3], cudaStream_t s);
 
+// near_nodes.cu: the direct lists of a level through interpolation nodes (whole products of one column)
+struct NodeChoice {
+    int p = 0;                          // nodes per axis, 0: no list of the level takes this form
+    bool small = false, keep = false;   // the lists that do (near list: last level only)
+    double seconds = 0.0;               // estimated time of the level's direct lists with this choice
+};
 // ---- far.cu ----------------------------------------------------------------------------------
 int nodes_per_dim(int d, int nr_interpolation);   // get_node_list for perfect powers, floor otherwise
 void far_field_level(f3m_plan *pl, int level, const float *b_sorted, int R, float *out_sorted,
                      int64_t row_begin, int64_t row_end, cudaStream_t s);   // per-level path (far.cu)
-void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut,
+// end: the last level whose far pairs are taken; cut == end: that level's small and kept pairs too
+void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut, int end,
                cudaStream_t s);                                               // whole product (far_fast.cu)
 int64_t far_moments_size(const f3m_plan *pl, int R);
-int far_cut_level(const f3m_plan *pl, int R);   // level at which a product over all rows may end, 0: none
+// Where a product over all rows may end before the last level of its tree.  nodes: the level's small and kept pairs go through that many
+// nodes of their own (near_nodes.cu); 0: all its pairs go through the far field's.
+struct CutChoice {
+    int level = 0;      // 0: the product visits all levels
+    NodeChoice nodes;
+};
+CutChoice far_cut(const f3m_plan *pl, int R, bool nodes_allowed = true);
+bool far_ends_with_nodes(const f3m_plan *pl, int level);   // a plan for one product: nothing below this level will be visited
+int far_node_end_level(const f3m_plan *pl, float edge0, int lmax);
 int far_stop_level(const f3m_plan *pl, int R, float edge0, const float *xmin, const float *ymin, int64_t n);   // before the tree is built
 
 // ---- shard.cu --------------------------------------------------------------------------------
@@ -484,13 +501,9 @@ void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, con
 bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted, int row_begin,
                  int row_end, cudaStream_t s);
 double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate, pairs or moments
-// near_nodes.cu: the direct lists of a level through interpolation nodes (whole products of one column)
-struct NodeChoice {
-    int p = 0;                          // nodes per axis, 0: no list of the level takes this form
-    bool small = false, keep = false;   // the lists that do (near list: last level only)
-    double seconds = 0.0;               // estimated time of the level's direct lists with this choice
-};
 NodeChoice node_choice(const f3m_plan *pl, int level, int R);
+// the same for a level at which the product ends: its small and kept pairs together, seconds their time (p = 0: not possible)
+NodeChoice node_end(const f3m_plan *pl, int level);
 bool node_sums(f3m_plan *pl, int level, const NodeChoice &choice, const float *b_sorted, float *out_sorted, cudaStream_t s);
 template <bool GRAD>
 void dense_f32(const float *X, int64_t N, const float *Y, int64_t M, const float *b, int R, int d, float ls, float *out,

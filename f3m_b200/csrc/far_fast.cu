@@ -1373,12 +1373,23 @@ int far_stop_level(const f3m_plan *pl, int R, float edge0, const float *xmin, co
     return 0;
 }
 
-int far_cut_level(const f3m_plan *pl, int R) {
+// A second way to end: at a level whose own nodes do not reproduce its near pairs, but whose children's do.  The far pairs of the levels
+// below are then as good as exact, so that the small and kept pairs of this level can take all that stands in for them: through
+// more nodes, the number near_nodes.cu needs (one column, three dimensions).  Mixture of 1e7 points, l = 0.5, 216 nodes: level 6
+// with 7 nodes for 4.0e6 pairs in place of level 7 and its 1.96e7, whole call 16.8 -> 7.9 ms (M2L 5.4 -> 0.9, levels 7 and 8 neither built nor sorted for).
+static bool ends_exactly_below(const f3m_plan *pl, double edge, int level) {
+    const int p = nodes_per_dim(pl->d, pl->prm.nr_interpolation);
+    bool wide;
+    return cut_kernels_fit(pl, 1, p, wide) && pl->same && cut_is_exact(pl->d, 0.5 * edge, (double)pl->lcs, nullptr, level + 1, p);
+}
+
+CutChoice far_cut(const f3m_plan *pl, int R, bool nodes_allowed) {
+    CutChoice best;
     const int L = pl->levels, d = pl->d;
-    if (L < 1) return 0;
+    if (L < 1) return best;
     const int p = pl->lists[1].p;
     bool wide;
-    if (!cut_kernels_fit(pl, R, p, wide)) return 0;
+    if (!cut_kernels_fit(pl, R, p, wide)) return best;
     int P = 1;
     for (int k = 0; k < d; k++) P *= p;
     double off[MAXD];
@@ -1392,22 +1403,55 @@ int far_cut_level(const f3m_plan *pl, int R) {
         direct[l] = node_choice(pl, l, R).seconds;
         full += direct[l] + m2l(pl->lists[l].far) + shifts(l);
     }
-    int best = 0;
     double best_t = full, head = 20e-6;
     for (int l = 1; l <= L; l++) {
         const LevelLists &ll = pl->lists[l];
         const double t = head + m2l(ll.far) + m2l(ll.small) + m2l(ll.keep) + shifts(l);
-        if (t < best_t && ll.far.count + ll.small.count + ll.keep.count <= 0x7fffffffLL && 
-            cut_is_exact(d, (double)pl->ty->levels[l].edge, (double)pl->lcs, pl->same ? nullptr : off, l, p)) { best = l; best_t = t; }
+        if (t < best_t && ll.far.count + ll.small.count + ll.keep.count <= 0x7fffffffLL &&
+            cut_is_exact(d, (double)pl->ty->levels[l].edge, (double)pl->lcs, pl->same ? nullptr : off, l, p)) {
+            best = CutChoice{};
+            best.level = l;
+            best_t = t;
+        }
+        if (nodes_allowed && R == 1 && l < L && ends_exactly_below(pl, (double)pl->ty->levels[l].edge, l)) {
+            const NodeChoice n = node_end(pl, l);
+            const double tn = head + m2l(ll.far) + shifts(l) + n.seconds;
+            if (n.p && tn < best_t) {
+                best.level = l;
+                best.nodes = n;
+                best_t = tn;
+            }
+        }
         head += direct[l] + m2l(ll.far) + shifts(l);
     }
     return best;
 }
 
+// The first level at which a product could end that way, from the cube's edge; 0: none within the key's depth
+int far_node_end_level(const f3m_plan *pl, float edge0, int lmax) {
+    for (int l = 1; l < lmax; l++)
+        if (ends_exactly_below(pl, ldexp((double)edge0, -l), l)) return pl->d == 3 ? l : 0;
+    return 0;
+}
+
+// While the tree of a plan for one product is built: may it end at this level, whose lists are there?  If it can (above) and going on
+// would cost more: one node-to-node step for every child pair of the kept pairs, of which there are 2^d or more per pair where its boxes
+// are populated, besides the lists and the deeper sort.
+bool far_ends_with_nodes(const f3m_plan *pl, int level) {
+    const int p = nodes_per_dim(pl->d, pl->prm.nr_interpolation);
+    if (!ends_exactly_below(pl, (double)pl->ty->levels[level].edge, level)) return false;
+    const NodeChoice n = node_end(pl, level);
+    if (!n.p) return false;
+    const LevelLists &ll = pl->lists[level];
+    const double P = pow((double)p, pl->d), small = ll.small.count ? direct_list_seconds(pl, level, ll.small, 1) : 0.0;
+    const double below = (double)ll.keep.count * (1 << pl->d) * P * 1.25e-12 + 2.0 * pl->tx.levels[level].nb * (1 << pl->d) / 2 * P * 8e-12;
+    return n.seconds <= small + below;
+}
+
 // Far field of the whole product.  Fast path when every level with far pairs uses the same p <= 8;
 // otherwise (var_compression switching node counts between levels, or more nodes per dimension) the
-// per-level path of far.cu.  cut > 0 (far_cut_level): the product ends at that level, all of whose pairs are taken here.
-void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut,
+// per-level path of far.cu.  cut > 0 (far_cut): the product ends at that level, all of whose pairs are taken here.
+void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, int64_t row_begin, int64_t row_end, int cut, int end,
                cudaStream_t s) {
     int lmin = 0, llast = 0, p = 0;
     bool uniform = true;
@@ -1419,7 +1463,7 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
         all.p = ll.p;
         pl->cut_level = cut;
     }
-    for (int l = 1; l <= (cut ? cut : pl->levels); l++) {
+    for (int l = 1; l <= end; l++) {
         if ((l == cut ? pl->cut_lists.far.count : pl->lists[l].far.count) == 0) continue;
         llast = l;
         if (!lmin) { lmin = l; p = pl->lists[l].p; }
@@ -1430,7 +1474,7 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
     for (int k = 0; k < pl->d; k++) P *= p;
     const bool fits = (size_t)3 * P * sizeof(float) + (size_t)pl->d * NOFF2 * mat_stride(p) * sizeof(float) <= 200 * 1024;
     if (!uniform || p > PMAX_FAST || p < 2 || !fits) {
-        for (int l = lmin; l <= pl->levels; l++) far_field_level(pl, l, b_sorted, R, out_sorted, row_begin, row_end, s);
+        for (int l = lmin; l <= end; l++) far_field_level(pl, l, b_sorted, R, out_sorted, row_begin, row_end, s);
         return;
     }
     const int rb = (int)row_begin, re = (int)row_end;

@@ -460,6 +460,18 @@ static double node_seconds(const f3m_plan *pl, int p, int64_t box_pairs) {
     return NODE_FIXED + (double)pl->tx.n * P * (p <= 8 ? 1.8e-13 : 2.4e-13) + (double)box_pairs * P * p * 1.1e-13;
 }
 
+NodeChoice node_end(const f3m_plan *pl, int level) {
+    NodeChoice c;
+    const LevelLists &ll = pl->lists[level];
+    if (pl->d != 3 || !pl->same || level < 1 || (pl->prm.flags & (F3M_FLAG_NEAR_MOMENTS | F3M_FLAG_NEAR_TENSOR_CORES))) return c;
+    c.p = nodes_needed((double)pl->tx.levels[level].edge * sqrt(2.0 * (double)pl->lcs));
+    if (!c.p) return c;
+    c.small = ll.small.count > 0;
+    c.keep = ll.keep.count > 0;
+    c.seconds = node_seconds(pl, c.p, ll.small.count + ll.keep.count);
+    return c;
+}
+
 NodeChoice node_choice(const f3m_plan *pl, int level, int R) {
     NodeChoice c;
     const LevelLists &ll = pl->lists[level];

@@ -679,6 +679,7 @@ constexpr int PLANE_BITS = 7;
 constexpr int64_t PLANE_POINTS = 1 << 21;
 static int sort_pass_count(int bits) { return (bits + RS_MAXBITS - 1) / RS_MAXBITS; }
 static int sort_digit_bits(int bits) { return (bits + sort_pass_count(bits) - 1) / sort_pass_count(bits); }
+int sort_passes_for(int bits) { return sort_pass_count(bits); }
 bool sort_carries(int d, int depth) { return sort_digit_bits(d * depth) <= PLANE_BITS; }
 
 // Keys and records [row0 + position, coordinates] of n points, sorted by the key bits [shift0, shift0 + bits).  With a tree, its

@@ -99,3 +99,51 @@ def test_small_workspace_sums_the_pairs(cuda):
             assert "workspace" in str(e)
             continue
         assert rel_l2(out.cpu(), want.cpu()) <= TOL
+
+
+def _mixture(n, g, width=0.06):
+    return torch.rand(20, 3, generator=g)[torch.randint(0, 20, (n,), generator=g)] + torch.randn(n, 3, generator=g) * width
+
+
+@pytest.mark.parametrize("n,p,ls", [(400_000, 6, 0.16), (500_000, 8, 0.25)])
+def test_products_that_end_above_the_exact_level(n, p, ls, cuda):
+    """The level whose children's interpolation is exact: its near pairs through more nodes, nothing below it is visited."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(p)
+    X = _mixture(n, g).to(cuda)
+    b = (torch.rand(n, 1, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, None, engine.make_params(ls, 100.0, p ** 3, False, 0.15, p ** 3))
+    out = plan.apply(b)
+    cut = plan.last_work()["cut_level"]
+    assert 0 < cut < plan.stats()["levels"] and plan.timings()["direct_launches"] > 0
+    half = n // 2 + 1
+    parts = plan.apply(b, row_range=(0, half)) + plan.apply(b, row_range=(half, n))   # slices visit all levels
+    # positive weights: the bound of the far pairs that are replaced (1.2e-7) besides those above
+    assert rel_l2(out.cpu(), parts.cpu()) <= 2 * TOL
+    assert torch.equal(plan.apply(b), out)
+    c = b.clone()
+    c[n // 3] = float("inf")
+    assert not torch.isfinite(plan.apply(c)).all()
+    assert torch.equal(plan.apply(b), out)
+
+
+def test_one_product_that_ends_above_the_exact_level(cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(11)
+    n = (1 << 21) + 77
+    X = _mixture(n, g).to(cuda)
+    b = (torch.rand(n, 1, generator=g) + 0.5).to(cuda)
+    prm = engine.make_params(0.16, 100.0, 216, False, 0.15, 216)
+    plan = engine.Plan(X, None, prm)
+    want = plan.apply(b)
+    assert 0 < plan.last_work()["cut_level"] < plan.stats()["levels"] and plan.timings()["direct_launches"] > 0
+    out = engine.kmvm(X, None, b, prm)
+    assert rel_l2(out.cpu(), want.cpu()) <= TOL
+    assert torch.equal(engine.kmvm(X, None, b, prm), out)
+    rows = torch.arange(0, n, n // 300, device=cuda)
+    exact = engine.rbf_dense(X[rows].double(), X.double(), b.double(), 0.16)
+    assert rel_l2(out[rows].cpu(), exact.cpu()) <= 1.2 * rel_l2(want[rows].cpu(), exact.cpu()) + TOL
+    # a weight of infinity: its neighbourhood is summed pair by pair
+    b[5] = float("inf")
+    out = engine.kmvm(X, None, b, prm)
+    assert not torch.isfinite(out[5]).any()
