@@ -259,6 +259,7 @@ struct LevelLists {
     DevBuf<int> far_oidx;
     bool far_ordered = false;
     DevBuf<float> T;   // axis matrices of the level (far_fast.cu), built on first use
+    bool T_ready = false;
 };
 
 // Device time per stage, from CUDA events recorded on the product's stream and read after its

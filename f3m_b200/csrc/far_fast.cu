@@ -35,20 +35,53 @@ namespace f3m {
 // ---------------------------------------------------------------------------------------------
 // T[k][o][i*p+j] = exp(-lcs (g_i - g_j - delta)^2), delta = (o + dqmin_k) edge + shift_k, g = node*edge/2
 // (setup_skip_conv n_tree.cu:433-486 adds the centres to the scaled nodes; the +edge/2 of n_tree.cu:510 cancels)
-__global__ void m2l_table2(NodeTab2 nt, int d, double edge, double lcs, Geom2 geo, float *T) {
-    const int p = nt.p, MS = mat_stride(p);
-    const int tot = d * NOFF2 * MS;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {
-        int q = e % MS, o = (e / MS) % NOFF2, k = e / (MS * NOFF2);
-        float v = 0.f;
-        if (q < p * p) {
-            int in = q / p, jn = q % p;
-            double delta = (double)(o + geo.dqmin[k]) * edge + geo.shift[k];
-            double diff = ((double)nt.node[in] - (double)nt.node[jn]) * edge * 0.5 - delta;
-            v = (float)exp(-lcs * diff * diff);
+// What the node-to-node steps of a product need of their levels: the tables, and the cells of the boxes of rows that have no order yet.
+// One launch for all levels (blockIdx.y), which also lays out the matrices between a box and its children.
+struct SetupLevel {
+    float *T;              // null: kept from an earlier product
+    double edge;
+    Geom2 geo;
+    const uint32_t *code[2];
+    int *cell[2];          // null: not needed
+    int nb[2], level;
+};
+struct ShiftTables { float a[2 * mat_stride(PMAX_FAST)], at[2 * mat_stride(PMAX_FAST)]; };
+struct SetupArgs {
+    SetupLevel lv[F3M_MAX_LEVELS];
+    ShiftTables shift;
+    float *shift_a, *shift_at;   // null: kept from an earlier product
+};
+__global__ void __launch_bounds__(256) setup_levels(NodeTab2 nt, int d, double lcs, const __grid_constant__ SetupArgs a) {
+    const SetupLevel &lv = a.lv[blockIdx.y];
+    const int p = nt.p, MS = mat_stride(p), first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (lv.T)
+        for (int e = first; e < d * NOFF2 * MS; e += step) {
+            const int q = e % MS, o = (e / MS) % NOFF2, k = e / (MS * NOFF2);
+            float v = 0.f;
+            if (q < p * p) {
+                const int in = q / p, jn = q % p;
+                const double delta = (double)(o + lv.geo.dqmin[k]) * lv.edge + lv.geo.shift[k];
+                const double diff = ((double)nt.node[in] - (double)nt.node[jn]) * lv.edge * 0.5 - delta;
+                v = (float)exp(-lcs * diff * diff);
+            }
+            lv.T[e] = v;
         }
-        T[e] = v;
-    }
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+        if (lv.cell[t])
+            for (int b = first; b < lv.nb[t]; b += step) {
+                const uint32_t c = lv.code[t][b];
+                for (int k = 0; k < d; k++) {
+                    int q = 0;
+                    for (int jb = 0; jb < lv.level; jb++) q |= (int)((c >> (d * jb + k)) & 1u) << jb;
+                    lv.cell[t][b * d + k] = q;
+                }
+            }
+    if (a.shift_a && blockIdx.y == 0)
+        for (int i = first; i < 2 * MS; i += step) {
+            a.shift_a[i] = a.shift.a[i];
+            a.shift_at[i] = a.shift.at[i];
+        }
 }
 
 // A[s][i*p+j] = L_i(xi), xi = (s ? +0.5 : -0.5) + 0.5 t_j ; AT is its transpose.  Exact Lagrange products in double.
@@ -67,15 +100,6 @@ static void make_shift_tables(const NodeTab2 &nt, std::vector<float> &A, std::ve
                 AT[s * MS + j * p + i] = (float)L;
             }
         }
-}
-
-// both tables in one kernel parameter: no copies from pageable host memory and no wait for them
-struct ShiftTables { float a[2 * mat_stride(PMAX_FAST)], at[2 * mat_stride(PMAX_FAST)]; };
-__global__ void shift_tables_kernel(ShiftTables t, int n, float *A, float *AT) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        A[i] = t.a[i];
-        AT[i] = t.at[i];
-    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -799,6 +823,12 @@ __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, i
     for (int k = 0; k < d; k++) c[k] = ctr[box * d + k];
     const int G = C >= NTH ? 1 : NTH / C;             // point groups
     const int g = C >= NTH ? 0 : threadIdx.x / C;
+    float acc[PP][RB];
+#pragma unroll
+    for (int i = 0; i < PP; i++)
+#pragma unroll
+        for (int r = 0; r < RB; r++) acc[i][r] = 0.f;
+    int chunks = 0;
     for (int base = s0; base < s1; base += TP) {
         const int cnt = min(TP, s1 - base);
         __syncthreads();
@@ -814,6 +844,9 @@ __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, i
             for (int r = 0; r < RB; r++) bsm[threadIdx.x * RB + r] = (r0 + r < R) ? bs[(size_t)i * R + r0 + r] : 0.f;
         }
         __syncthreads();
+        // A thread of a single combination keeps its sums over G chunks (128 terms), then adds them to the shared ones: added after every
+        // chunk, three terms at a time, the atomics of 2-D boxes took most of the kernel (6e4 sources, 36 nodes, three columns: 48.9 -> 29.5 us).
+        const bool flush = C > NTH || ++chunks == G || base + TP >= s1;
         if (g < G) {
             for (int cc = (C >= NTH ? (int)threadIdx.x : (int)threadIdx.x - g * C); cc < C; cc += NTH) {
                 const float *lp[MAXD];
@@ -823,11 +856,6 @@ __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, i
                     lp[k] = Ls;
                     if (k < d) { lp[k] = Ls + (size_t)(k * PP + rem % PP) * LS; rem /= PP; }
                 }
-                float acc[PP][RB];
-#pragma unroll
-                for (int i = 0; i < PP; i++)
-#pragma unroll
-                    for (int r = 0; r < RB; r++) acc[i][r] = 0.f;
                 for (int j = g; j < cnt; j += G) {
                     float w = 1.f;
 #pragma unroll
@@ -843,12 +871,17 @@ __global__ void __launch_bounds__(256) p2m_leaf(const float *__restrict__ pts, i
                         for (int r = 0; r < RB; r++) acc[i][r] = fmaf(l0, wb[r], acc[i][r]);
                     }
                 }
+                if (!flush) continue;
 #pragma unroll
                 for (int i = 0; i < PP; i++)
 #pragma unroll
-                    for (int r = 0; r < RB; r++) atomicAdd(&accsm[cc * CS + i * RB + r], acc[i][r]);
+                    for (int r = 0; r < RB; r++) {
+                        atomicAdd(&accsm[cc * CS + i * RB + r], acc[i][r]);
+                        acc[i][r] = 0.f;
+                    }
             }
         }
+        if (flush) chunks = 0;
     }
     __syncthreads();
     float *dst = lw.slot < 0 ? mom + (size_t)box * PR : part + lw.slot * PR;
@@ -999,9 +1032,18 @@ __global__ void __launch_bounds__(128) l2p_small3(const float *__restrict__ pts,
 }
 
 // lists of the small and the large boxes of the far field's last level, of one tree (0: targets, 1: sources); kept in the plan
+// (A few thousand boxes take a CTA each whatever they hold: the split and its read-back would cost more than it saves.)
+constexpr int LEAF_SPLIT = 4096;
 static void ensure_leaf_split(f3m_plan *pl, int which, int level, cudaStream_t s) {
     if (pl->leaf_level[which] == level) return;
     Level &lv = (which == 0 ? pl->tx : *pl->ty).levels[level];
+    if (lv.nb <= LEAF_SPLIT) {
+        pl->leaf_big[which].release();   // no list: all boxes
+        pl->n_leaf_big[which] = lv.nb;
+        pl->n_leaf_small[which] = 0;
+        pl->leaf_level[which] = level;
+        return;
+    }
     pl->leaf_small[which].alloc((size_t)lv.nb, s);
     pl->leaf_big[which].alloc((size_t)lv.nb, s);
     int *counts = pl->d_flags + FL_LEAF;
@@ -1098,18 +1140,64 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
         // the node-to-node kernels write every box of the levels they run on
         if ((l == cut ? pl->cut_lists : pl->lists[l]).far.count == 0) loc[l].zero();
     }
-    if (pl->shift_p != PP) {
-        std::vector<float> hA, hAT;
-        make_shift_tables(nt, hA, hAT);
-        pl->shift_p = 0;
-        pl->shift_a.alloc(hA.size(), s);
-        pl->shift_at.alloc(hAT.size(), s);
-        ShiftTables st{};
-        std::copy(hA.begin(), hA.end(), st.a);
-        std::copy(hAT.begin(), hAT.end(), st.at);
-        shift_tables_kernel<<<1, 128, 0, s>>>(st, (int)hA.size(), pl->shift_a.p, pl->shift_at.p);
-        F3M_LAUNCH_CHECK();
-        pl->shift_p = PP;
+    // tables and cells (setup_levels)
+    const bool nested = RB == 1 && (d == 2 || d == 3) && cfg.nf <= 64;
+    const bool rows = !nested && rows_form_available<PP, RB>(d);
+    std::vector<DevBuf<int>> cellx(L + 1), celly(L + 1);
+    auto level_rows = [&](int l) -> LevelLists & { return l == cut ? pl->cut_lists : pl->lists[l]; };
+    auto level_geometry = [&](int l) {
+        Geom2 geo{};
+        for (int k = 0; k < d; k++) {
+            double sh = pl->same ? 0.0 : (double)ty.origin[k] - (double)tx.origin[k];
+            geo.shift[k] = sh;
+            // pairs of level >= 2 descend from parent pairs closer than two parent edges, so their offset lies
+            // within a few boxes of -shift/edge; level-1 pairs are children of the root pair: offsets -1, 0, 1
+            geo.dqmin[k] = (l == 1 ? 0 : (int)floor(-sh / (double)tx.levels[l].edge)) - NOFF2 / 2 + 1;
+        }
+        return geo;
+    };
+    {
+        SetupArgs sa{};
+        int nlev = 0, most = d * NOFF2 * MS;
+        for (int l = lmin; l <= L; l++) {
+            LevelLists &ll = level_rows(l);
+            const bool cells = !(nested || rows) || !ll.far_ordered;   // the ordered rows hold the offsets
+            if (ll.far.count == 0 || (ll.T_ready && !cells)) continue;
+            SetupLevel &q = sa.lv[nlev++];
+            Level *lv[2] = {&tx.levels[l], &ty.levels[l]};
+            if (!ll.T_ready) {   // a constant of the plan: every product uses as many nodes on the level
+                ll.T.alloc((size_t)d * NOFF2 * MS, s);
+                q.T = ll.T.p;
+            }
+            q.edge = (double)lv[0]->edge;
+            q.geo = level_geometry(l);
+            q.level = l;
+            for (int t = 0; t < (pl->same ? 1 : 2) && cells; t++) {
+                DevBuf<int> &c = t ? celly[l] : cellx[l];
+                c.alloc((size_t)lv[t]->nb * d, s);
+                q.code[t] = lv[t]->code.p;
+                q.cell[t] = c.p;
+                q.nb[t] = lv[t]->nb;
+                most = std::max(most, lv[t]->nb);
+            }
+        }
+        if (pl->shift_p != PP) {
+            std::vector<float> hA, hAT;
+            make_shift_tables(nt, hA, hAT);
+            pl->shift_p = 0;
+            pl->shift_a.alloc(hA.size(), s);
+            pl->shift_at.alloc(hAT.size(), s);
+            std::copy(hA.begin(), hA.end(), sa.shift.a);
+            std::copy(hAT.begin(), hAT.end(), sa.shift.at);
+            sa.shift_a = pl->shift_a.p;
+            sa.shift_at = pl->shift_at.p;
+        }
+        if (nlev || sa.shift_a) {
+            setup_levels<<<dim3((unsigned)std::min((most + 255) / 256, 4 * NUM_SMS_HINT), std::max(nlev, 1)), 256, 0, s>>>(nt, d, (double)pl->lcs, sa);
+            F3M_LAUNCH_CHECK();
+            pl->shift_p = PP;
+            for (int l = lmin; l <= L; l++) level_rows(l).T_ready = level_rows(l).T.p != nullptr;
+        }
     }
     const float *A = pl->shift_a.p, *AT = pl->shift_at.p;
 
@@ -1160,14 +1248,13 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
             else { if (acc_reg) F3M_M2L_CALL(true, 0) else F3M_M2L_CALL(false, 0) }
 #undef F3M_M2L_CALL
         };
-        DevBuf<int> cellx, celly;
         for (int l = lmin; l <= L; l++) {
             const bool at_cut = l == cut;
             LevelLists &level_lists = pl->lists[l];
-            LevelLists &ll = at_cut ? pl->cut_lists : level_lists;
+            LevelLists &ll = level_rows(l);
             if (ll.far.count == 0) continue;
             if (r0 == 0) pl->last.box_pairs += ll.far.count;
-            Level &lx = tx.levels[l], &ly = ty.levels[l];
+            Level &lx = tx.levels[l];
             const ListSet ls{{level_lists.far.ptr.p, level_lists.small.ptr.p, level_lists.keep.ptr.p},
                              {level_lists.far.idx.p, level_lists.small.idx.p, level_lists.keep.idx.p}, at_cut ? 3 : 1};
             if (at_cut && !ll.far_ordered) {
@@ -1175,44 +1262,18 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                 add_list_ptrs<<<(lx.nb + 1 + 255) / 256, 256, 0, s>>>(lx.nb + 1, ls, ll.far.ptr.p);
                 F3M_LAUNCH_CHECK();
             }
-            Geom2 geo{};
-            for (int k = 0; k < d; k++) {
-                double sh = pl->same ? 0.0 : (double)ty.origin[k] - (double)tx.origin[k];
-                geo.shift[k] = sh;
-                // pairs of level >= 2 descend from parent pairs closer than two parent edges, so their offset lies
-                // within a few boxes of -shift/edge; level-1 pairs are children of the root pair: offsets -1, 0, 1
-                geo.dqmin[k] = (l == 1 ? 0 : (int)floor(-sh / (double)lx.edge)) - NOFF2 / 2 + 1;
-            }
-            if (!ll.T.p) {   // a constant of the plan: every product uses as many nodes on the level
-                ll.T.alloc((size_t)d * NOFF2 * MS, s);
-                m2l_table2<<<8, 256, 0, s>>>(nt, d, (double)lx.edge, (double)pl->lcs, geo, ll.T.p);
-                F3M_LAUNCH_CHECK();
-            }
+            const Geom2 geo = level_geometry(l);
             const float *T = ll.T.p;
-            const bool nested = RB == 1 && (d == 2 || d == 3) && cfg.nf <= 64;
-            const bool rows = !nested && rows_form_available<PP, RB>(d);
-            const int *cy = nullptr;
-            if (!(nested || rows) || !ll.far_ordered) {   // the ordered rows hold the offsets
-                cellx.alloc((size_t)lx.nb * d, s);
-                decode_cells_kernel<<<(lx.nb + 255) / 256, 256, 0, s>>>(lx.nb, l, d, lx.code.p, cellx.p);
-                F3M_LAUNCH_CHECK();
-                cy = cellx.p;
-                if (!pl->same) {
-                    celly.alloc((size_t)ly.nb * d, s);
-                    decode_cells_kernel<<<(ly.nb + 255) / 256, 256, 0, s>>>(ly.nb, l, d, ly.code.p, celly.p);
-                    F3M_LAUNCH_CHECK();
-                    cy = celly.p;
-                }
-            }
+            const int *cx = cellx[l].p, *cy = pl->same ? cx : celly[l].p;
             if (nested || rows) {
                 if (!ll.far_ordered) {
                     ll.far_okey.alloc((size_t)ll.far.count, s);
                     ll.far_oidx.alloc((size_t)ll.far.count, s);
                     if (d <= 4)
-                        far_order_kernel<4><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cellx.p, cy, geo,
+                        far_order_kernel<4><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cx, cy, geo,
                                                                            ll.far_okey.p, ll.far_oidx.p, pl->d_flags, lx.off.p, rb, re);
                     else
-                        far_order_kernel<32><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cellx.p, cy, geo,
+                        far_order_kernel<32><<<(lx.nb + 3) / 4, 128, 0, s>>>(lx.nb, d, ls, cx, cy, geo,
                                                                             ll.far_okey.p, ll.far_oidx.p, pl->d_flags, lx.off.p, rb, re);
                     F3M_LAUNCH_CHECK();
                     // kept for later products of this plan only when every box was ordered
@@ -1233,7 +1294,7 @@ static void far_fast_block(f3m_plan *pl, const float *bs, int R, int r0, float *
                                                                   T, momp[l], loc[l].p);
                 }
             } else
-                launch_m2l(lx.nb, ll.far.ptr.p, ll.far.idx.p, cellx.p, cy, lx.off.p, T, geo, momp[l], loc[l].p);
+                launch_m2l(lx.nb, ll.far.ptr.p, ll.far.idx.p, cx, cy, lx.off.p, T, geo, momp[l], loc[l].p);
             F3M_LAUNCH_CHECK();
         }
     }
@@ -1458,7 +1519,7 @@ void far_field(f3m_plan *pl, const float *b_sorted, int R, float *out_sorted, in
     if (cut && pl->cut_level != cut) {   // the number of columns can move the cut
         LevelLists &ll = pl->lists[cut], &all = pl->cut_lists;
         all.far_ordered = false;
-        all.T.release();
+        all.T_ready = false;
         all.far.count = ll.far.count + ll.small.count + ll.keep.count;
         all.p = ll.p;
         pl->cut_level = cut;
