@@ -19,7 +19,9 @@ namespace f3m {
 //     target tile a call of 2e4 points ran 157 four-warp CTAs on 148 SMs: most of the chip idle, then a second, nearly empty wave.
 //     The slices' partial sums are added in a fixed order by dense_combine, so results do not depend on scheduling.
 // Measured, product + gradient of 2e4 points, d = 3, 3 columns: 1280 -> 358 us on the device (171 + 181, floor 87 + 98 at nine and ten
-// FP32 lanes a pair); error against float64 5.4e-7 -> 3.1e-7.
+// FP32 lanes a pair); error against float64 5.4e-7 -> 3.1e-7.  With four source pairs in flight per thread and registers for them (six CTAs
+// per SM) instead of two (eight): 169 + 181 -> 160 + 168 us, the two calls 397 -> 373; one column of 2e4 points 120 -> 114, five dimensions
+// and 3 columns 212 -> 201; eight columns in three dimensions gain nothing and stay at two.
 constexpr int DNT = 128, DT = 2, DTILE = DNT * DT;
 constexpr int DST = 256;   // sources per shared-memory tile; also the length of the blocked partial sums
 
@@ -28,10 +30,10 @@ __host__ __device__ constexpr int dense_width(int D, int RB) { return (D + RB + 
 
 // dst: the product itself (stride R, column r0) when there is one slice, else partial sums (slices, N, RB)
 template <int D, int RB, bool GRAD>
-__global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float *__restrict__ X, int64_t n, const float *__restrict__ Y,
+__global__ void __launch_bounds__(DNT, RB <= 4 ? 6 : 4) dense_kernel(const float *__restrict__ X, int64_t n, const float *__restrict__ Y,
                                                                      const float *__restrict__ b, int64_t m, int64_t slice, float scale,
                                                                      float post, int R, int r0, float *dst) {
-    constexpr int W = dense_width(D, RB);
+    constexpr int W = dense_width(D, RB), UNROLL = RB <= 4 || D >= 4 ? 4 : 2;
     __shared__ __align__(16) float smem[DST * W];
     const int64_t i0 = (int64_t)blockIdx.x * DTILE + threadIdx.x;
     const int64_t m0 = (int64_t)blockIdx.y * slice, m1 = min(m, m0 + slice);
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(DNT, RB <= 4 ? 8 : 4) dense_kernel(const float
         for (int u = 0; u < DT; u++)
 #pragma unroll
             for (int r = 0; r < RB; r++) acc[u][r] = pack2(0.f, 0.f);
-#pragma unroll 2
+#pragma unroll UNROLL
         for (int p = 0; p < np; p++) {
             f32x2 col[W];
             const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(smem + p * 2 * W);
