@@ -268,7 +268,7 @@ struct ColCfg {
     static constexpr size_t smem = (size_t)(3 * NOFF2 * MS + 2 * NGRP * P) * sizeof(float);
 };
 
-// T[k][o][j * MSR + i] = exp(-lcs (g_i - g_j - delta)^2), delta = (o + dqmin) edge (m2l_table2 of far_fast.cu, columns first)
+// T[k][o][j * MSR + i] = exp(-lcs (g_i - g_j - delta)^2), delta = (o + dqmin) edge (the tables of setup_levels in far_fast.cu, columns first)
 static __global__ void column_table(NodeTab2 nt, double edge, double lcs, int dqmin, float *T) {
     const int p = nt.p, MSR = (p + 3) / 4 * 4, MS = p * MSR, tot = 3 * NOFF2 * MS;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {

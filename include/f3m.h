@@ -100,7 +100,7 @@ int f3m_kmvm_f32(const float *X, int64_t N, const float *Y, int64_t M, const flo
  * through torch, n_tree.cu:1061 and throughout; a host that hands out memory from its own
  * allocator passes a slice of it here).  workspace: device memory of workspace_bytes bytes, free for the duration
  * of the call; nothing is requested from or returned to the driver inside the call, apart from a per-device slot of
- * 1 KB of flags and pinned read-back words that the library creates the first time a device is used.
+ * 2.5 KB of flags and pinned read-back words that the library creates the first time a device is used.
  * f3m_workspace_bytes estimates the need for evenly spread points (sort buffers, tree, lists, packed sources,
  * moments); strongly clustered sets build deeper trees and need more.  A workspace that runs out ends the call
  * with F3M_ERR_TOO_LARGE and a message that names the request; f3m_last_workspace_peak returns the high-water
@@ -298,11 +298,12 @@ int f3m_plan_last_direct_launches(const f3m_plan *plan);
  * exponent, see near_field_run n_tree.cu:831-902 for the sums themselves): counts[0] expanded form with every
  * exponential on the special-function unit, [1] expanded form with 2/5 of the pairs on a degree-2 polynomial,
  * [2] with 1/3 on a degree-3 polynomial, [3] direct form (differences, wide boxes), [4] moment form (of degree 2 and 3 it
- * counts in [1] and [2] too: every exponent of the list is in that polynomial), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES). */
+ * counts in [1] and [2] too: every exponent of the list is in that polynomial), [5] tensor-core form (F3M_FLAG_NEAR_TENSOR_CORES).
+ * Lists summed through interpolation nodes are launches without a count here. */
 int f3m_plan_last_direct_variants(const f3m_plan *plan, int32_t counts[6]);
 /* What the last f3m_plan_apply visited: work[0] = pairs of points in the direct lists it summed pair by pair (whole lists, also
- * when a slice of the rows was asked for), [1] = box pairs of its far field, [2] = the level it ended at before the tree's last
- * one (0: none), [3] = direct-sum launches that took the kernel for several columns and short boxes (they count in counts[0] or
+ * when a slice of the rows was asked for; lists summed through moments or interpolation nodes visit none), [1] = box pairs of its far
+ * field, [2] = the level it ended at before the tree's last one (0: none), [3] = direct-sum launches that took the kernel for several columns and short boxes (they count in counts[0] or
  * counts[3] above too). */
 int f3m_plan_last_work(const f3m_plan *plan, int64_t work[4]);
 /* work[0] by the form that summed the pairs, in the order of f3m_plan_last_direct_variants (moments visit no pairs: pairs[4] = 0). */
