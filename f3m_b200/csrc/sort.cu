@@ -391,7 +391,7 @@ __host__ __device__ constexpr size_t rs_smem_bytes(int nbins, int rec_words, boo
 }
 
 // The keys of a tile are ranked first; records (and values) are read when their slots are known, so that they occupy no registers
-// while the ballots run: four blocks per SM instead of three.  PLANES: the last pass writes permutation and planes instead of
+// while the ballots run: up to four blocks per SM instead of three (sort_blocks_per_sm).  PLANES: the last pass writes permutation and planes instead of
 // records, where runs of equal digits are long enough for stores of single words.
 template <int D, bool PLANES, bool VALUE>
 __global__ void __launch_bounds__(RS_T, 4) rs_scatter(SortIO io, int64_t n, int shift, int dbits, int64_t chunk,
@@ -675,8 +675,14 @@ __global__ void __launch_bounds__(256) unpack_records(const void *__restrict__ r
 }
 
 // Stores of single words want runs: digits of at most PLANE_BITS bits, or arrays that stay in L2 until their lines are complete.
-constexpr int PLANE_BITS = 7;
+// Last pass of 1e8 points with 7 bits: planes 2.27 ms, records 1.05 and their unpacking 0.50; with 6 bits planes are ahead.
+constexpr int PLANE_BITS = 6;
 constexpr int64_t PLANE_POINTS = 1 << 21;
+
+// Blocks per SM of a pass.  Every block has one half-written line per digit and array open; when those of all blocks outgrow the L2,
+// lines go to memory in pieces.  Two passes over 1e8 points in three dimensions, 4 / 3 / 2 blocks: 9 bits 5.23 / 4.54 / 4.04 ms, 8 bits
+// 2.59 / 2.48 / 2.51, 7 bits 2.10 / 2.05 / 2.32.  Arrays that stay in L2 take as many blocks as fit.
+static int sort_blocks_per_sm(int64_t n, int dbits) { return n <= PLANE_POINTS || dbits <= 6 ? 4 : dbits <= 8 ? 3 : 2; }
 static int sort_pass_count(int bits) { return (bits + RS_MAXBITS - 1) / RS_MAXBITS; }
 static int sort_digit_bits(int bits) { return (bits + sort_pass_count(bits) - 1) / sort_pass_count(bits); }
 int sort_passes_for(int bits) { return sort_pass_count(bits); }
@@ -698,6 +704,7 @@ static void sort_records(const float *X, int64_t n, int row0, const MortonCfg &c
     F3M_CUDA(cudaFuncSetAttribute(rs_scatter<D, false, VALUE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     F3M_CUDA(cudaFuncSetAttribute(rs_scatter<D, true, VALUE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     F3M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rs_scatter<D, false, VALUE>, RS_T, smem));
+    occ = std::min(occ, sort_blocks_per_sm(n, dbits_all));
     const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
     const int64_t wave = (int64_t)sms * std::max(1, occ);
     const int64_t tpb = (ntiles + wave - 1) / wave;

@@ -52,3 +52,26 @@ def test_rows_of_b_follow_their_points(cuda):
     out = engine.kmvm(X, None, b, engine.make_params(1.0, 1000.0, 216, False, 0.15, 216))
     exact = engine.rbf_dense(X[rows].double(), X[rows].double(), b[rows].double(), 1.0)
     assert rel_l2(out[rows].cpu(), exact.cpu()) <= 2e-5     # six nodes per axis at l = 1: 2.5e-6 of the dense product and more for few weights
+
+
+@pytest.mark.parametrize("n", [(1 << 21) - 1, (1 << 21) + 4099])   # both sides of the size from which wide digits take fewer blocks
+@pytest.mark.parametrize("d,leaf,scale", [(3, 3e4, 1.0), (3, 4e3, 1.0), (3, 500.0, 1.0), (3, 60.0, 1.0), (2, 200.0, 1.0), (5, 3000.0, 1.0),
+                                          (3, 1000.0, 0.02)])
+def test_sorted_order_of_all_digit_widths(n, d, leaf, scale, cuda):
+    """The sorted points fill their boxes, box by box: 9 to 30 key bits in one to three passes of six to ten."""
+    from f3m_b200 import _lib, engine
+    g = torch.Generator(device=cuda).manual_seed(n % 1000 + d)
+    X = torch.rand(n, d, device=cuda, generator=g)
+    if scale < 1.0:   # clustered: sorted again to the full key depth
+        X = X * scale + torch.rand(10, d, device=cuda, generator=g)[torch.randint(0, 10, (n,), device=cuda, generator=g)]
+    plan = engine.Plan(X, None, engine.make_params(1.0, leaf, 8, False, 0.15, 8))
+    L = plan.stats()["levels"]
+    perm = torch.from_numpy(plan.array(L, 0, _lib.ARR_SORTED_INDEX)).long().to(cuda)
+    assert torch.equal(torch.sort(perm).values, torch.arange(n, device=cuda))
+    off = torch.from_numpy(plan.array(L, 0, _lib.ARR_BOX_OFFSETS)).long().to(cuda)
+    box = torch.repeat_interleave(torch.arange(off.numel() - 1, device=cuda), off.diff())
+    ctr = torch.from_numpy(plan.array(L, 0, _lib.ARR_BOX_CENTERS)).to(cuda)
+    lo, hi = X.min(0).values, X.max(0).values
+    half = (hi - lo).max() * 1.01 / 2 ** (L + 1)
+    # float32 centres and cells: a few roundings of coordinates of size one
+    assert ((X[perm] - ctr[box]).abs() <= half + 4e-6).all()
