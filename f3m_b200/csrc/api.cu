@@ -605,9 +605,22 @@ static int plan_create(f3m_plan **plan, const float *X, int64_t N, const float *
     return F3M_OK;
 }
 
+// A plan leaves the library with nothing of its build still running: its first product may be on another stream, and what it
+// gives back, at once or when it is destroyed, may go to any stream.  (plan_create alone is for calls whose product follows on the
+// same stream.)
+static int plan_built(f3m_plan **plan, int st, cudaStream_t s) {
+    if (st == F3M_OK) st = guarded([&] { F3M_CUDA(cudaStreamSynchronize(s)); });
+    if (st != F3M_OK) {
+        delete *plan;
+        *plan = nullptr;
+    }
+    return st;
+}
+
 int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, int64_t M, int32_t d,
                     const f3m_params *prm, void *stream) {
-    return plan_create(plan, X, N, Y, M, d, prm, 0, nullptr, stream);
+    const int st = plan_create(plan, X, N, Y, M, d, prm, 0, nullptr, stream);
+    return plan ? plan_built(plan, st, (cudaStream_t)stream) : st;
 }
 
 int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, int64_t row_begin, int64_t row_end,
@@ -718,7 +731,7 @@ int f3m_plan_create_from_cell_counts(f3m_plan **plan, const int32_t *cell_counts
         return st;
     }
     *plan = pl;
-    return F3M_OK;
+    return plan_built(plan, st, s);
 }
 
 int f3m_plan_attach_runs(f3m_plan *plan, const void *records, int64_t run_stride, void *stream) {
