@@ -316,14 +316,15 @@ struct Timings {
         last_end = -1;
         for (float &m : ms) m = 0.f;
     }
-    // Call after the stream has been synchronised.  A span that was never closed (the product failed in between)
-    // is dropped; a failed query must not stay behind as the runtime's last error, or the next launch check of an
-    // unrelated call would report it.
+    // Call after the stream has been synchronised (an event that has not passed all the same is waited for: a span once dropped is never
+    // read).  A span that was never closed (the product failed in between) is dropped; a failed query must not stay behind as the
+    // runtime's last error, or the next launch check of an unrelated call would report it.
     void resolve() {
         for (auto &sp : spans) {
             float t = 0.f;
             if (sp.b < 0) continue;
-            if (cudaEventElapsedTime(&t, (*events)[sp.a], (*events)[sp.b]) != cudaSuccess) (void)cudaGetLastError();
+            if (cudaEventSynchronize((*events)[sp.b]) != cudaSuccess || cudaEventElapsedTime(&t, (*events)[sp.a], (*events)[sp.b]) != cudaSuccess)
+                (void)cudaGetLastError();
             else if (sp.stage == ST_BUILD) build_ms = t;
             else ms[sp.stage] += t;
         }

@@ -48,3 +48,17 @@ def test_plans_dropped_at_once(cuda):
             plan = engine.Plan(Z, None, small)
             assert plan.stats()["levels"] > 0
             assert torch.equal(plan.apply(b), want)
+
+
+@pytest.mark.parametrize("n,m", [(50_000, 0), (2_000_003, 0), (2_000_003, 100)])
+def test_the_time_of_a_build_is_there_when_the_plan_is(n, m, cuda):
+    from f3m_b200 import engine
+    X = torch.rand(n, 3, device=cuda)
+    Y = torch.rand(m, 3, device=cuda) if m else None
+    prm = engine.make_params(0.3, 1000.0, 64, False, 0.15, 64)
+    for _ in range(20):
+        plan = engine.Plan(X, Y, prm)
+        ms = plan.stats()["build_ms"]
+        assert ms > 0
+        plan.apply(torch.ones(m or n, 1, device=cuda))
+        assert plan.stats()["build_ms"] == ms == plan.timings()["build"]
