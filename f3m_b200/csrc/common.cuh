@@ -500,7 +500,7 @@ double pair_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int 
 void column_sums(f3m_plan *pl, int level, const PairCSR &csr, bool expanded, const float *b_sorted, int R, int r0, float *out_sorted,
                  int row_begin, int row_end, cudaStream_t s);
 // near_moments.cu: sums a direct list through box moments when its geometry allows; false: sum the pairs
-bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *b_sorted, int R, float *out_sorted, int row_begin,
+bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, bool alone, const float *b_sorted, int R, float *out_sorted, int row_begin,
                  int row_end, cudaStream_t s);
 double direct_list_seconds(const f3m_plan *pl, int level, const PairCSR &csr, int R);   // estimate, pairs or moments
 NodeChoice node_choice(const f3m_plan *pl, int level, int R);

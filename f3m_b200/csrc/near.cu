@@ -803,10 +803,11 @@ static void direct_d(f3m_plan *pl, int level, const PairCSR &csr, const float *b
     }
 }
 
-static void direct_sums_plain(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out_sorted, int64_t row_begin,
-                 int64_t row_end, cudaStream_t s) {
+// moments or pairs; alone: the level's other list is not theirs to take along
+static void direct_sums_plain(f3m_plan *pl, int level, const PairCSR &csr, bool alone, const float *bs, int R, float *out_sorted,
+                              int64_t row_begin, int64_t row_end, cudaStream_t s) {
     const int rb = (int)row_begin, re = (int)row_end;
-    if (moment_sums(pl, level, csr, bs, R, out_sorted, rb, re, s)) return;
+    if (moment_sums(pl, level, csr, alone, bs, R, out_sorted, rb, re, s)) return;
     switch (pl->d) {
         case 1: direct_d<1>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
         case 2: direct_d<2>(pl, level, csr, bs, R, out_sorted, rb, re, s); break;
@@ -822,12 +823,14 @@ void direct_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, i
     LevelLists &ll = pl->lists[level];
     const bool keep = &csr == &ll.keep, whole = row_begin <= 0 && row_end >= pl->tx.n && !pl->shard.active && !pl->ext_mom;
     const NodeChoice c = whole && R == 1 && level > 0 ? node_choice(pl, level, R) : NodeChoice{};
+    // Nodes for one of the level's two lists: each is then summed by itself, also where the nodes are refused after all
+    const bool alone = c.p && c.small != c.keep;
     if (c.p && (keep ? c.keep : c.small)) {
         if (!keep && c.keep) return;   // summed with the near list
         if (node_sums(pl, level, c, bs, out_sorted, s)) return;
-        if (keep && c.small) direct_sums_plain(pl, level, ll.small, bs, R, out_sorted, row_begin, row_end, s);
+        if (keep && c.small) direct_sums_plain(pl, level, ll.small, alone, bs, R, out_sorted, row_begin, row_end, s);
     }
-    direct_sums_plain(pl, level, csr, bs, R, out_sorted, row_begin, row_end, s);
+    direct_sums_plain(pl, level, csr, alone, bs, R, out_sorted, row_begin, row_end, s);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -455,7 +455,8 @@ static void moment_degree(f3m_plan *pl, int level, int K, const PairCSR *l1, con
 
 // Sums the list through moments when its geometry allows; false: the caller sums the pairs.  On the last level the small
 // list waits for the near list when both take this form: one set of records and one pass over the rows then serve both.
-bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, int R, float *out, int rb, int re, cudaStream_t s) {
+// alone: the level's other list is summed elsewhere (near_nodes.cu), neither waited for nor taken along.
+bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, bool alone, const float *bs, int R, float *out, int rb, int re, cudaStream_t s) {
     if (level < 1) return false;
     LevelLists &ll = pl->lists[level];
     const bool keep = &csr == &ll.keep;
@@ -463,7 +464,7 @@ bool moment_sums(f3m_plan *pl, int level, const PairCSR &csr, const float *bs, i
     if (K == 0) return false;
     double h = list_exponent_bound(pl, level, keep);
     const PairCSR *other = nullptr;
-    if (level == pl->levels) {
+    if (level == pl->levels && !alone) {
         const int Ko = list_moment_degree(pl, level, !keep, R);
         if (Ko) {
             if (!keep) return true;   // summed with the near list

@@ -147,3 +147,30 @@ def test_one_product_that_ends_above_the_exact_level(cuda):
     b[5] = float("inf")
     out = engine.kmvm(X, None, b, prm)
     assert not torch.isfinite(out[5]).any()
+
+
+# A last level whose two lists both qualify for box moments (boxes of a tenth of a lengthscale) while one of them, or both, or none goes
+# through nodes: every pair is summed once.  Against slices of the rows, which take no nodes.
+@pytest.mark.parametrize("n,nodes,small,ls,leaf,by_nodes", [(3_000_000, 27, 27, 1.7, 1000.0, "keep"), (3_000_000, 27, 27, 3.0, 1000.0, "keep"),
+                                                            (8_000_000, 27, 27, 0.9, 1000.0, "keep"), (2_000_000, 27, 300, 1.5, 1000.0, "both"),
+                                                            (3_000_000, 8, 200, 1.7, 1000.0, None),
+                                                            (3_000_000, 8, 8, 1.7, 1000.0, None), (1_000_000, 27, 27, 2.0, 1000.0, None)])
+def test_one_list_through_nodes_and_one_through_moments(n, nodes, small, ls, leaf, by_nodes, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator(device=cuda).manual_seed(3)
+    X = torch.randn(n, 3, device=cuda, generator=g)
+    b = torch.rand(n, 1, device=cuda, generator=g) + 0.5
+    plan = engine.Plan(X, None, engine.make_params(ls, leaf, nodes, False, 0.15, small))
+    last = plan.level(plan.stats()["levels"])
+    assert last["n_small"] > 0 and last["n_keep"] > 0
+    out = plan.apply(b)
+    v, launches = plan.direct_variants(), plan.timings()["direct_launches"]
+    assert plan.last_work()["cut_level"] == 0
+    half = n // 2 + 1
+    parts = plan.apply(b, row_range=(0, half)) + plan.apply(b, row_range=(half, n))
+    # positive weights; both forms of a list are good to some 3e-7 of its sum
+    assert rel_l2(out.cpu(), parts.cpu()) <= 1e-6
+    assert rel_l2(engine.kmvm(X, None, b, engine.make_params(ls, leaf, nodes, False, 0.15, small)).cpu(), parts.cpu()) <= 1e-6
+    assert plan.direct_variants()["moments"] > 0
+    if by_nodes:
+        assert v["moments"] > 0 and launches > v["mufu"] + v["direct"] + v["moments"]   # a launch without a count is the nodes'
