@@ -1093,7 +1093,8 @@ static void p2m_level(f3m_plan *pl, Level &ly, int which, const float *bs, int R
 
 // Sources are interpolated at the first level from L on whose boxes hold at most this many points on average, and moved up by
 // M2M, which adds in a tree: with 375 000 sources per box summed at the cut, 3e6 points and l = 10 were 8.4e-7 from float64,
-// the finest level's 5.6e-7.
+// the finest level's 5.6e-7.  A tree that was built no deeper than the cut has no such level; what makes its sums as good are those of the
+// parts of long boxes, which keep their roundings (p2m_combine).
 constexpr int64_t SRC_LEAF = 8192;
 
 template <int PP, int RB>

@@ -190,15 +190,23 @@ __device__ __forceinline__ LeafWork leaf_work(const int *__restrict__ off, int n
     return w;
 }
 
-// moments of the long boxes: the sums of their parts, in the order of the rows
+// Moments of the long boxes: the sums of their parts, in the order of the rows, with the rounding of every addition carried along
+// (Knuth's two-sum; the loads of the parts take the time).  A tree that ends at a level whose boxes hold hundreds of thousands of points has hundreds of
+// parts per box, and a plain running sum was most of the product's error: error over sqrt(n), normal weights, l = 10, 300 products of
+// 3e6 points SRC3, of 1e7 SRC10; a kept plan, which interpolates its sources further down and adds them in a tree (far_fast.cu, SRC_LEAF), KEPT3
+// and KEPT10.
 static __global__ void __launch_bounds__(128) p2m_combine(const int *__restrict__ off, int nb, int n, int chunk, int PR, int src_begin, int src_end,
                                                   const float *__restrict__ part, float *mom) {
     const LongBox l = long_box_of_chunk(off, nb, n, chunk, blockIdx.x);
     if (l.box < 0 || off[l.box] < src_begin || off[l.box] >= src_end) return;
     for (int q = threadIdx.x; q < PR; q += 128) {
-        float v = part[l.first_slot * PR + q];
-        for (int64_t t = (l.first_slot | 1) + 1; t <= l.last_slot; t += 2) v += part[t * PR + q];
-        mom[(size_t)l.box * PR + q] = v;
+        float v = part[l.first_slot * PR + q], lost = 0.f;
+        for (int64_t t = (l.first_slot | 1) + 1; t <= l.last_slot; t += 2) {
+            const float x = part[t * PR + q], sum = __fadd_rn(v, x), w = __fsub_rn(sum, v);
+            lost += __fadd_rn(__fsub_rn(v, __fsub_rn(sum, w)), __fsub_rn(x, w));
+            v = sum;
+        }
+        mom[(size_t)l.box * PR + q] = isfinite(v) ? v + lost : v;
     }
 }
 
