@@ -61,21 +61,11 @@ __device__ __forceinline__ void wide_row_pair(const float (&xa)[3], const float 
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const f32x2 t = pack2(factor * c.from(xa[k], k), factor * c.from(xb[k], k));
-        f32x2 diff[PP], after[PP];
-#pragma unroll
-        for (int i = 0; i < PP; i++) diff[i] = add2(t, pack2(-nt.node[i], -nt.node[i]));
-#pragma unroll
-        for (int i = PP - 2; i >= 0; i--) after[i] = (i == PP - 2) ? diff[PP - 1] : mul2(after[i + 1], diff[i + 1]);
+        f32x2 L[PP];
+        lagrange_pair<PP>(t, nt, L);
         f32x2 *dst = reinterpret_cast<f32x2 *>(row + (k == 0 ? 0 : k == 1 ? G::AX0 : G::AX0 + G::AX1));
-        f32x2 before = diff[0];
 #pragma unroll
-        for (int i = 0; i < PP; i++) {
-            f32x2 cb = pack2(nt.c[i], nt.c[i]);
-            if (k == 2) cb = mul2(cb, f);
-            if (i > 0) cb = mul2(cb, before);
-            dst[i] = i == PP - 1 ? cb : mul2(cb, after[i]);
-            if (i > 0) before = mul2(before, diff[i]);
-        }
+        for (int i = 0; i < PP; i++) dst[i] = k == 2 ? mul2(L[i], f) : L[i];
         if (k == 1)
 #pragma unroll
             for (int i = PP; i < G::NG * G::G1; i++) dst[i] = 0ull;   // the last group's surplus

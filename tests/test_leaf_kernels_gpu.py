@@ -43,3 +43,25 @@ def test_chunks_of_points(p, tails, cuda):
     assert rel_l2(out, ref) <= TOL
     again = plan.apply(b.to(cuda)).cpu()
     assert torch.equal(out, again)
+
+
+# Positive weights under a kernel that is wide against the boxes: what is left are the roundings of the Lagrange rows (six per pair of
+# points, one per side and axis), of moments and of expansions.  Mean over ten right-hand sides.  Rows of plain products of differences, whose sum is off one
+# by some 1e-7: 2.2, 2.0, 2.2, 1.5e-7; normalised by division 1.3, 1.4, 1.7, 1.2e-7; rows that sum to one 1.0, 1.0, 1.4, 1.0e-7.
+@pytest.mark.parametrize("d,n,R,ls,bound", [(3, 1_000_000, 1, 10.0, 1.4e-7), (3, 1_000_000, 1, 4.0, 1.4e-7), (3, 300_000, 3, 4.0, 1.75e-7),
+                                            (2, 300_000, 3, 4.0, 1.2e-7)])
+def test_rows_sum_to_one(d, n, R, ls, bound, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator(device=cuda).manual_seed(99)
+    X = torch.rand(n, d, device=cuda, generator=g) * 12 ** 0.5
+    plan = engine.Plan(X, None, engine.make_params(ls, 1000.0, 6 ** d, False, 0.15, 6 ** d))
+    rows = torch.randperm(n, device=cuda, generator=g)[:64]
+    K = torch.exp(-((X[rows].double()[:, None, :] - X.double()[None]) ** 2).sum(-1) / (2 * ls * ls))
+    err = ref = 0.0
+    for _ in range(10):
+        b = torch.rand(n, R, device=cuda, generator=g) + 0.5
+        exact = K @ b.double()
+        err += float((plan.apply(b)[rows] - exact).square().sum())
+        ref += float(exact.square().sum())
+    assert plan.last_work()["cut_level"] > 0          # every pair through the rows
+    assert (err / ref) ** 0.5 <= bound, (err / ref) ** 0.5
