@@ -402,6 +402,7 @@ struct f3m_plan {
     int stop_level = 0;
     const float *carry_b = nullptr;
     f3m::DevBuf<float> carried_b;
+    long long launches_at_wait = -1;      // g_launches when the build last waited for its stream
     int *h_pinned = nullptr;              // pinned host words for count read-back (FLAG_WORDS ints)
     int *d_flags = nullptr;               // device status / counters (FLAG_WORDS ints, see FlagSlot)
     std::vector<cudaEvent_t> *events = nullptr;   // of the scratch slot, see Timings
