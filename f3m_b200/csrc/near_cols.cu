@@ -50,11 +50,11 @@ __global__ void __launch_bounds__(256) col_groups(int nbx, const int *__restrict
 }
 
 // items[b] = tiles of the rows of the group that begins with target box b inside [row_begin, row_end), times the parts its list is cut
-// into (chunk sources each, 0: not cut); a warp per box
+// into (chunk sources each, 0: not cut), slots[b] = as many where there is more than one part; a warp per box
 struct ColGroup { int boxes, parts; };
 __global__ void __launch_bounds__(256) col_items(int nbx, const int *__restrict__ off_x, const int *__restrict__ ptr, const int *__restrict__ idx,
                                                 const int *__restrict__ off_y, const int *__restrict__ first, int chunk, int row_begin,
-                                                int row_end, int *items, ColGroup *groups) {
+                                                int row_end, int *items, int *slots, ColGroup *groups) {
     const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b > nbx) return;
     int t = 0;
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(256) col_items(int nbx, const int *__restrict_
     }
     if (lane == 0) {
         items[b] = t * g.parts;
+        slots[b] = g.parts > 1 ? t * g.parts : 0;
         if (b < nbx) groups[b] = g;
     }
 }
@@ -90,11 +91,12 @@ __global__ void __launch_bounds__(256) pack_column_rows(const float *__restrict_
 // whole list: with X = s (x-c), Y = s (y-c) the exponent -|X-Y|^2 is, in the expanded form, (2 X.Y - |Y|^2) - |X|^2, whose last part
 // leaves the sum; |X|^2 is at most d/4 there (boxes up to one scaled unit), so the terms of the bracket cancel by no more than that and
 // no factor overflows.  Wide boxes take the differences.
-// A lane owns MT target rows, TR = 32 / G of them apart, and every G-th quadruple of sources; NC = 8 or 4 columns.
+// A lane owns MT target rows, TR = 32 / G of them apart, and every G-th quadruple of sources; NC = 8 or 4 columns.  slot: where in parts
+// a part of a list leaves its sums, or -1: they are added to out.
 template <int D, bool DIFF, int NC, int G, int MT>
 __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int n_x, float *stages, const int *__restrict__ idx, int e0,
                                             int e1, const int *__restrict__ off_y, const float *__restrict__ rows, const float (&c)[D],
-                                            float scale, int R, int r0, float *out, int t0, int nt, bool shared) {
+                                            float scale, int R, int r0, float *out, int t0, int nt, float *parts, int slot) {
     constexpr int TR = 32 / G, STEP = 4 * G;
     const int lane = threadIdx.x, g = lane % TR, h = lane / TR;
     float xr[MT][D];
@@ -271,32 +273,64 @@ __device__ __forceinline__ void column_tile(const float *__restrict__ xpts, int 
         if (i >= nt) continue;
         float *o = out + (size_t)(t0 + i) * R + r;
 #pragma unroll
-        for (int q = 0; q < CPL; q++)
-            if (r + q < R) {
-                if (shared) atomicAdd(o + q, f * sum[q]);   // the parts of a long list
-                else o[q] += f * sum[q];
-            }
+        for (int q = 0; q < CPL; q++) {
+            if (slot >= 0) parts[(size_t)slot * (CT * NC) + i * NC + CPL * h + q] = f * sum[q];
+            else if (r + q < R) o[q] += f * sum[q];
+        }
     }
+}
+
+// A group's rows inside the slice, dealt out evenly over its tiles, 16 at a time
+struct ColTile { int begin, rows; };
+__device__ __forceinline__ ColTile col_tile(const int *__restrict__ off_x, int box, int boxes, int tile, int ntiles, int row_begin, int row_end) {
+    const int a = max(off_x[box], row_begin), len = min(off_x[box + boxes], row_end) - a, units = (len + 15) >> 4;
+    const int t0 = a + 16 * (int)(((long long)units * tile) / ntiles);
+    return ColTile{t0, min(a + 16 * (int)(((long long)units * (tile + 1)) / ntiles), a + len) - t0};
+}
+
+// The sums of a list's parts, in the order of the list: a block per slot, those of a tile's first part work
+template <int NC>
+__global__ void __launch_bounds__(CT * NC / 4) col_parts_sum(const int *__restrict__ off_x, int nbx, const int *__restrict__ item_off,
+                                                    const int *__restrict__ slot_off, const ColGroup *__restrict__ groups,
+                                                    const float *__restrict__ parts, int R, int r0, float *out, int row_begin, int row_end) {
+    const int box = box_of_row(slot_off, nbx, blockIdx.x);
+    const ColGroup group = groups[box];
+    const int q = blockIdx.x - slot_off[box], np = group.parts;
+    if (q % np) return;
+    const ColTile t = col_tile(off_x, box, group.boxes, q / np, (item_off[box + 1] - item_off[box]) / np, row_begin, row_end);
+    const int e = threadIdx.x, i = e / (NC / 4), r = r0 + e % (NC / 4) * 4;   // four columns of a row
+    if (i >= t.rows) return;
+    const float4 *src = reinterpret_cast<const float4 *>(parts) + (size_t)blockIdx.x * (CT * NC / 4) + e;
+    float4 v = src[0];
+#pragma unroll 4
+    for (int p = 1; p < np; p++) {
+        const float4 w = src[(size_t)p * (CT * NC / 4)];
+        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+    }
+    const float sum[4] = {v.x, v.y, v.z, v.w};
+    float *o = out + (size_t)(t.begin + i) * R + r;
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        if (r + c < R) o[c] += sum[c];
 }
 
 template <int D, bool DIFF, int NC>
 __global__ void __launch_bounds__(32, 16) near_columns(const float *__restrict__ xpts, int n_x, const int *__restrict__ off_x, int nbx,
                                                        const float *__restrict__ ctr_x, const int *__restrict__ parent,
                                                        const float *__restrict__ parent_ctr, const int *__restrict__ item_off,
-                                                       const ColGroup *__restrict__ groups, const int *__restrict__ ptr, const int *__restrict__ idx,
-                                                       const int *__restrict__ off_y, const float *__restrict__ rows, float scale, int R,
-                                                       int r0, float *out, int row_begin, int row_end) {
+                                                       const int *__restrict__ slot_off, const ColGroup *__restrict__ groups,
+                                                       const int *__restrict__ ptr, const int *__restrict__ idx, const int *__restrict__ off_y,
+                                                       const float *__restrict__ rows, float scale, int R, int r0, float *out, float *parts,
+                                                       int row_begin, int row_end) {
     __shared__ __align__(16) float stage[2 * CST * CSTRIDE];
     const int item = blockIdx.x;
     if (item >= item_off[nbx]) return;      // the grid may be sized by a bound
     const int box = box_of_row(item_off, nbx, item);
     const ColGroup group = groups[box];
-    const int np = group.parts, part = (item - item_off[box]) % np, tile = (item - item_off[box]) / np;
-    // the group's rows are dealt out evenly over its tiles, 16 at a time
-    const int a = max(off_x[box], row_begin), len = min(off_x[box + group.boxes], row_end) - a;
-    const int ntiles = (item_off[box + 1] - item_off[box]) / np, units = (len + 15) >> 4;
-    const int t0 = a + 16 * (int)(((long long)units * tile) / ntiles);
-    const int nt = min(a + 16 * (int)(((long long)units * (tile + 1)) / ntiles), a + len) - t0;
+    const int np = group.parts, q = item - item_off[box], part = q % np;
+    const ColTile tile = col_tile(off_x, box, group.boxes, q / np, (item_off[box + 1] - item_off[box]) / np, row_begin, row_end);
+    const int t0 = tile.begin, nt = tile.rows;
+    const int slot = np > 1 ? slot_off[box] + q : -1;
     float c[D];
     const float *centre = group.boxes > 1 ? parent_ctr + parent[box] * D : ctr_x + box * D;
 #pragma unroll
@@ -304,7 +338,7 @@ __global__ void __launch_bounds__(32, 16) near_columns(const float *__restrict__
     const int p0 = ptr[box], n_entries = ptr[box + 1] - p0;
     const int e0 = p0 + (int)(((long long)n_entries * part) / np), e1 = p0 + (int)(((long long)n_entries * (part + 1)) / np);
 #define F3M_TILE(G_, MT_) \
-    column_tile<D, DIFF, NC, G_, MT_>(xpts, n_x, stage, idx, e0, e1, off_y, rows, c, scale, R, r0, out, t0, nt, np > 1)
+    column_tile<D, DIFF, NC, G_, MT_>(xpts, n_x, stage, idx, e0, e1, off_y, rows, c, scale, R, r0, out, t0, nt, parts, slot)
     if (nt > 48) F3M_TILE(2, 4);
     else if (nt > 32) F3M_TILE(2, 3);
     else if (nt > 24) F3M_TILE(4, 4);
@@ -321,29 +355,16 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
     Level &lx = tx.levels[level], &ly = ty.levels[level];
     const float scale = sqrtf(pl->lcs * 1.4426950408889634f);
     // Boxes in the middle of a cloud have lists a hundred times as long as the average: such a list, summed by one warp, outlasts all others.
-    // Lists of large calls are cut into parts (chunk sources or so each, some ten thousand items in all), and the host reads how
-    // many items there are; small calls launch a bound.
-    const int chunk = csr.pairs >= 100000000 ? (int)std::min<int64_t>(32768, std::max<int64_t>(1024, csr.pairs / 600000)) : 0;
+    // Lists of large calls are cut into parts (chunk sources or so each, some ten thousand items in all, and at most some 2^17: a part
+    // keeps 64 rows of sums until they are added up in the order of the list), and the host reads how many items there are; small
+    // calls launch a bound.
+    int chunk = 0;
+    if (csr.pairs >= 100000000) {
+        const int64_t even = std::min<int64_t>(32768, std::max<int64_t>(1024, csr.pairs / 600000));
+        chunk = (int)std::min<int64_t>(1 << 20, std::max<int64_t>(even, csr.pairs / (CT << 17)));
+    }
     // Groups of the expanded form: |X|^2 stays below d/4 times 1.25^2 around a parent's centre.
     const bool grouped = DIFF || scale * tx.levels[level - 1].edge <= 1.25f;
-    DevBuf<int> items, first;
-    DevBuf<ColGroup> groups;
-    items.alloc((size_t)lx.nb + 1, s);
-    first.alloc((size_t)lx.nb + 1, s);
-    groups.alloc((size_t)lx.nb, s);
-    const unsigned box_warps = (unsigned)(((int64_t)(lx.nb + 1) * 32 + 255) / 256);
-    col_groups<<<box_warps, 256, 0, s>>>(lx.nb, lx.parent.p, csr.ptr.p, csr.idx.p, grouped, first.p);
-    F3M_LAUNCH_CHECK();
-    col_items<<<box_warps, 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, csr.idx.p, ly.off.p, first.p, chunk, row_begin, row_end, items.p, groups.p);
-    F3M_LAUNCH_CHECK();
-    exclusive_scan_i32(items.p, items.p, (int64_t)lx.nb + 1, s);
-    int64_t max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1;
-    if (chunk) {
-        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, items.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
-        F3M_CUDA(cudaStreamSynchronize(s));
-        max_items = pl->h_pinned[0];
-        if (max_items <= 0) return;
-    }
     // one set of rows serves every list of the product
     f3m_plan::ColumnRows &cr = pl->column_rows;
     if (cr.r0 != r0) {
@@ -354,13 +375,58 @@ static void columns_impl(f3m_plan *pl, int level, const PairCSR &csr, const floa
         F3M_LAUNCH_CHECK();
         pl->last.end(s);
     }
+    const int nc = R - r0 <= 4 ? 4 : 8;
+    DevBuf<int> items, slots, first;
+    DevBuf<ColGroup> groups;
+    DevBuf<float> parts;
+    items.alloc((size_t)lx.nb + 1, s);
+    slots.alloc((size_t)lx.nb + 1, s);
+    first.alloc((size_t)lx.nb + 1, s);
+    groups.alloc((size_t)lx.nb, s);
+    const unsigned box_warps = (unsigned)(((int64_t)(lx.nb + 1) * 32 + 255) / 256);
+    col_groups<<<box_warps, 256, 0, s>>>(lx.nb, lx.parent.p, csr.ptr.p, csr.idx.p, grouped, first.p);
+    F3M_LAUNCH_CHECK();
+    int64_t max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1, nslots = 0;
+    while (true) {
+        col_items<<<box_warps, 256, 0, s>>>(lx.nb, lx.off.p, csr.ptr.p, csr.idx.p, ly.off.p, first.p, chunk, row_begin, row_end, items.p, slots.p,
+                                            groups.p);
+        F3M_LAUNCH_CHECK();
+        int *scanned[2] = {items.p, slots.p};
+        exclusive_scan_multi(scanned, chunk ? 2 : 1, (int64_t)lx.nb + 1, nullptr, s);
+        if (!chunk) break;
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned, items.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + 1, slots.p + lx.nb, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaStreamSynchronize(s));
+        max_items = pl->h_pinned[0];
+        nslots = pl->h_pinned[1];
+        if (max_items <= 0) return;
+        if (!nslots) break;
+        try {
+            parts.alloc((size_t)nslots * CT * nc, s);
+            break;
+        } catch (const Fail &) {   // no memory for the parts' sums: lists are not cut
+            cudaGetLastError();
+            chunk = 0;
+            nslots = 0;
+            max_items = (int64_t)(row_end - row_begin) / CT + lx.nb + 1;
+        }
+    }
     pl->last.begin(ST_DIRECT, s);
     auto launch = [&](auto kernel) {
         kernel<<<(unsigned)max_items, 32, 0, s>>>(tx.pts.p, (int)tx.n, lx.off.p, lx.nb, lx.ctr.p, lx.parent.p, tx.levels[level - 1].ctr.p, items.p,
-                                                 groups.p, csr.ptr.p, csr.idx.p, ly.off.p, cr.buf.p, scale, R, r0, out, row_begin, row_end);
+                                                 slots.p, groups.p, csr.ptr.p, csr.idx.p, ly.off.p, cr.buf.p, scale, R, r0, out, parts.p, row_begin,
+                                                 row_end);
     };
-    if (R - r0 <= 4) launch(near_columns<D, DIFF, 4>);
+    auto sum = [&](auto kernel) {
+        kernel<<<(unsigned)nslots, CT * nc / 4, 0, s>>>(tx.levels[level].off.p, lx.nb, items.p, slots.p, groups.p, parts.p, R, r0, out, row_begin, row_end);
+    };
+    if (nc == 4) launch(near_columns<D, DIFF, 4>);
     else launch(near_columns<D, DIFF, 8>);
+    if (nslots) {
+        F3M_LAUNCH_CHECK();
+        if (nc == 4) sum(col_parts_sum<4>);
+        else sum(col_parts_sum<8>);
+    }
     F3M_LAUNCH_CHECK();
     pl->last.end(s);
     pl->last.direct_launches++;

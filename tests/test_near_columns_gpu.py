@@ -164,3 +164,41 @@ def test_groups_and_parts_of_long_lists(d, n, R, ls, leaf, nodes, dist, cuda):
     one = torch.cat([sum(plan.apply(b[:, r:r + 1].contiguous(), row_range=(lo, hi)) for lo, hi in ((0, 7), (7, n))) for r in range(R)], 1)
     assert rel_l2(parts.cpu(), one.cpu()) <= 2e-6    # as in test_columns_of_many_short_boxes
     assert rel_l2(plan.apply(b).cpu(), one.cpu()) <= 2e-6
+
+
+# Lists of more than 1e8 pairs are cut into parts (ten here): the parts' sums are added in one order, however their warps end.  Lengthscales
+# of an eighth of a box: far pairs (whose moments are summed in any order) are below 1e-13 of a row's own weight.
+@pytest.mark.parametrize("d,R", [(3, 8), (3, 3), (3, 9), (2, 2), (2, 8)])
+def test_parts_of_long_lists_repeat_bit_by_bit(d, R, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(d + R)
+    n = 60007
+    ls = 1.01 / (4 if d == 3 else 8) / 8
+    X = torch.rand(n, d, generator=g).to(cuda)
+    b = (torch.rand(n, R, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, None, engine.make_params(ls, 2000.0, 3 ** d, False, 0.15, 3 ** d))
+    assert plan.stats()["direct_pairs"] > 200_000_000
+    out = plan.apply(b)
+    assert plan.last_work()["column_launches"] > 0
+    for _ in range(6):
+        assert torch.equal(plan.apply(b), out)
+    exact = engine.rbf_dense(X.double(), X.double(), b.double(), ls)
+    # ex2.approx 2.4e-7, exponents of the difference form to d + 2 roundings of a number whose share x e^-x is below 0.4
+    assert rel_l2(out.cpu(), exact.cpu()) <= 2e-6
+
+
+@pytest.mark.parametrize("d,n,R", [(5, 200003, 8), (4, 300007, 3), (4, 300007, 9), (3, 300007, 2)])
+def test_parts_of_long_lists_of_uneven_trees(d, n, R, cuda):
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(d)
+    X = torch.randn(n, d, generator=g).to(cuda)
+    b = (torch.rand(n, R, generator=g) + 0.5).to(cuda)
+    plan = engine.Plan(X, None, engine.make_params(0.3 if d == 3 else 1.0, 200.0 if d == 3 else 1000.0, 3 ** d, False, 0.15, 3 ** d))
+    assert plan.stats()["direct_pairs"] > 200_000_000
+    out = plan.apply(b)
+    assert plan.last_work()["column_launches"] > 0
+    one = torch.cat([plan.apply(b[:, r:r + 1].contiguous()) for r in range(R)], 1)
+    assert rel_l2(out.cpu(), one.cpu()) <= 2e-6
+    cuts = (0, 1017, n // 2 + 1, n)
+    parts = sum(plan.apply(b, row_range=(lo, hi)) for lo, hi in zip(cuts, cuts[1:]))
+    assert rel_l2(parts.cpu(), out.cpu()) <= 1e-6
