@@ -196,7 +196,7 @@ enum FlagSlot {
     FL_MMA_COUNTER = 32, // tile cursor of the tensor-core near kernel
     FL_LEAF = 40,        // 2 words: small / big finest-level boxes
     FL_NSMALL = 42,      // target tiles of at most 32 points
-    FL_WEIGHTS = 43,     // a weight is not finite, or near the largest float
+    FL_WEIGHTS = 43,     // a weight is not finite, or near the largest float; the next word: weights that are not zero
     FL_BBOX_Y = 48,      // 2 * MAXD words, the second point set
     FL_LVTOT = 64,       // boxes per level of the batch being built (F3M_MAX_LEVELS words)
     FL_LVMAX = 96,       // largest box per level (F3M_MAX_LEVELS words)
@@ -380,7 +380,7 @@ struct f3m_plan {
         f3m::DevBuf<uint32_t> okey;
     };
     std::vector<NodeRows> node_rows;
-    int weights_ok = -1;                  // of the product under way: all weights finite (-1: not looked at yet)
+    int weights_ok = -1;                  // of the product under way: finite, and not mostly zeros (-1: not looked at yet)
     // source rows of the several-column kernel (near_cols.cu; valid inside one product)
     struct ColumnRows {
         int r0 = -1;

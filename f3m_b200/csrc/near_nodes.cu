@@ -18,13 +18,18 @@ namespace f3m {
 // ---------------------------------------------------------------------------------------------
 // Nodes a list needs.  Per axis g(u) = exp(-u^2 / 2 l^2) is interpolated in x and in y over an edge e: with Cramer's inequality the
 // error is at most (1 + Lambda_p) 2 * 1.0865 (e / 4 l)^p / sqrt(p!), Lambda_p <= 1 + (2 / pi) ln p (the derivation stands in
-// far_fast.cu); the axes' errors add up.  The bound is taken against the kernel's largest value, 1: on one point set every row
-// holds its own weight with that factor, so the row's sum cannot be small against the error unless its weights cancel.  (The cut of
-// far_fast.cu bounds every pair against its own value, which these wide boxes cannot meet at their far corners.)
-// At the bound the products of 64 bits differ by a fifth of it in the 2-norm: boxes 1.09 l wide, 9 nodes, bound 3.1e-7, measured
-// 1e-8; 0.55 l, 7 nodes, bound 2.6e-7, measured 5e-8 -- below the rounding of the sums (3e-7).
+// far_fast.cu); the axes' errors add up.  The bound is taken against the kernel's largest value, 1: a row is off by at most NODE_EPS times the
+// sum of |b| over its list, besides roundings of the same kind.  (The cut of far_fast.cu bounds every pair against its own value,
+// which these wide boxes cannot meet at their far corners.)  At the bound the products of 64 bits differ by a fifth of it in the 2-norm:
+// boxes 1.09 l wide, 9 nodes, bound 3.1e-7, measured 1e-8; 0.55 l, 7 nodes, bound 2.6e-7, measured 5e-8 -- below the roundings.
+// Against float64, pairs of near.cu (whole products) / nodes, 2-norm, 1e-7: normal weights, 0.55 l 4.2 / 2.5, 1.09 l 3.3 / 2.6, 2.3 l 6.3 / 3.4;
+// positive ones 1.5 / 1.2, 1.7 / 1.6, 2.1 / 1.9; targets by themselves beside boxes of 2e4 points, worst row relative to its sum of
+// |K b|: 0.55 l 52 / 7, 1.09 l 134 / 85.  Few weights that are not zero make short sums, whose pairs are the more exact ones: one in
+// a hundred 1.8 / 2.5, 1.9 / 2.4, 5.4 / 3.1, a single one 1.0 / 1.6, 1.1 / 1.8, 4.2 / 2.5, and entries far below 1 keep their digits.  From
+// one in ten on they are even, so products of sparser weights sum the pairs.
 // ---------------------------------------------------------------------------------------------
 constexpr double NODE_EPS = 4e-7;
+constexpr int SPARSE_WEIGHTS = 10;   // fewer than one weight in so many not zero: pairs
 constexpr int PMIN_NODES = 5;
 
 static int nodes_needed(double edge_over_l) {
@@ -429,11 +434,27 @@ __global__ void __launch_bounds__(128) m2l_columns(const int *__restrict__ fptr,
     }
 }
 
-// true into *bad when a weight is not finite or so large that moments could overflow where the pairs' sums do not
-static __global__ void __launch_bounds__(256) weights_check(const float *__restrict__ b, int64_t n, int *bad) {
+// true into words[0] when a weight is not finite or so large that moments could overflow where the pairs' sums do not; words[1]: the
+// weights that are not zero
+static __global__ void __launch_bounds__(256) weights_check(const float *__restrict__ b, int64_t n, int *words) {
     bool any = false;
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) any |= !(fabsf(b[i]) <= 1e30f);
-    if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
+    int nonzero = 0;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+        any |= !(fabsf(b[i]) <= 1e30f);
+        nonzero += b[i] != 0.f;
+    }
+    any = __any_sync(0xffffffffu, any);
+    nonzero = __reduce_add_sync(0xffffffffu, nonzero);
+    __shared__ int sums[8];
+    if ((threadIdx.x & 31) == 0) {
+        sums[threadIdx.x >> 5] = nonzero;
+        if (any) atomicOr(words, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) nonzero += sums[w];
+        if (nonzero) atomicAdd(words + 1, nonzero);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -523,7 +544,8 @@ static void run_nodes(f3m_plan *pl, int level, const PairCSR *l1, const PairCSR 
 }
 
 // The level's lists that the choice names, added to out (sorted order).  false: nothing was added and the lists have to be summed directly
-// -- the memory for the moments is not to be had, or a weight is not finite (its box's moments would carry it with either sign).
+// -- the memory for the moments is not to be had, a weight is not finite (its box's moments would carry it with either sign), or few
+// weights are other than zero (above).
 bool node_sums(f3m_plan *pl, int level, const NodeChoice &choice, const float *bs, float *out, cudaStream_t s) {
     Tree &t = pl->tx;
     Level &lv = t.levels[level];
@@ -533,13 +555,13 @@ bool node_sums(f3m_plan *pl, int level, const NodeChoice &choice, const float *b
     const int64_t count = l1->count + (l2 ? l2->count : 0);
     if (count > 0x7fffffffLL) return false;
     if (pl->weights_ok < 0) {   // once per product
-        int *bad = pl->d_flags + FL_WEIGHTS;
-        F3M_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
-        weights_check<<<(unsigned)std::min<int64_t>((t.n + 1023) / 1024, 8 * NUM_SMS_HINT), 256, 0, s>>>(bs, t.n, bad);
+        int *words = pl->d_flags + FL_WEIGHTS;
+        F3M_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(int), s));
+        weights_check<<<(unsigned)std::min<int64_t>((t.n + 1023) / 1024, 8 * NUM_SMS_HINT), 256, 0, s>>>(bs, t.n, words);
         F3M_LAUNCH_CHECK();
-        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + FL_WEIGHTS, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+        F3M_CUDA(cudaMemcpyAsync(pl->h_pinned + FL_WEIGHTS, words, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
         F3M_CUDA(cudaStreamSynchronize(s));
-        pl->weights_ok = pl->h_pinned[FL_WEIGHTS] == 0;
+        pl->weights_ok = pl->h_pinned[FL_WEIGHTS] == 0 && (int64_t)pl->h_pinned[FL_WEIGHTS + 1] * SPARSE_WEIGHTS >= t.n;
     }
     if (!pl->weights_ok) return false;
     const int MS = p * ((p + 3) / 4 * 4), chunk = source_chunk(lv.max_count, t.n, false);

@@ -149,6 +149,48 @@ def test_one_product_that_ends_above_the_exact_level(cuda):
     assert not torch.isfinite(out[5]).any()
 
 
+@pytest.mark.parametrize("edge", [0.55, 1.09, 1.6])
+def test_few_weights_are_summed_pair_by_pair(edge, cuda):
+    """A column of K: entries far below 1 keep their digits, which interpolation against the kernel's largest value does not give."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(int(100 * edge))
+    X = torch.rand(30707, 3, generator=g) + 1.3
+    n = X.shape[0]
+    ls = float(torch.tensor(float((X.max(0).values - X.min(0).values).max()) * 1.01 / 4 / edge, dtype=torch.float32))
+    plan = _plan(X, ls, 300.0, 1000, cuda)
+    Xd = X.to(cuda).double()
+    for count in (1, n // 100):
+        b = torch.zeros(n, 1, device=cuda)
+        b[torch.randperm(n, generator=g)[:count].to(cuda)] = 0.75
+        out = plan.apply(b)
+        assert plan.last_work()["pairs"] == plan.stats()["direct_pairs"]
+        exact = engine.rbf_dense(Xd, Xd, b.double(), ls)
+        seen = exact > 1e-20
+        # exponents are differences of numbers up to 64 (in powers of two), good to some three roundings of them
+        assert float(((out.double() - exact).abs() / exact)[seen].max()) <= 2e-5
+    b = torch.rand(n, 1, device=cuda) + 0.5
+    plan.apply(b)
+    assert _used(plan)
+
+
+@pytest.mark.parametrize("edge", [0.55, 1.09])
+def test_targets_beside_dense_boxes(edge, cuda):
+    """Rows of single targets around two boxes of 2e4 points each: their error stays below the bound times the sum of the weights."""
+    from f3m_b200 import engine
+    g = torch.Generator().manual_seed(int(100 * edge))
+    dense = torch.rand(40000, 3, generator=g) * 0.25
+    dense[20000:, 0] += 0.25
+    X = torch.cat([dense, torch.rand(600, 3, generator=g), torch.zeros(1, 3), torch.ones(1, 3)]).to(cuda)
+    b = (torch.rand(X.shape[0], 1, generator=g) + 0.5).to(cuda)
+    b[40000:] *= 1e-3
+    ls = float(torch.tensor(1.01 / 4 / edge, dtype=torch.float32))
+    plan = engine.Plan(X, None, engine.make_params(ls, 21000.0, 45000, False, 0.15, 45000))
+    out = plan.apply(b)
+    assert _used(plan)
+    exact = engine.rbf_dense(X[40000:].double(), X.double(), b.double(), ls)
+    assert float((out[40000:].double() - exact).abs().max()) <= TOL * float(b.sum())
+
+
 # A last level whose two lists both qualify for box moments (boxes of a tenth of a lengthscale) while one of them, or both, or none goes
 # through nodes: every pair is summed once.  Against slices of the rows, which take no nodes.
 @pytest.mark.parametrize("n,nodes,small,ls,leaf,by_nodes", [(3_000_000, 27, 27, 1.7, 1000.0, "keep"), (3_000_000, 27, 27, 3.0, 1000.0, "keep"),
