@@ -219,12 +219,6 @@ __device__ __forceinline__ void flush_acc(float (&acc_reg)[2][PP], float acc_lef
     }
 }
 
-__device__ __forceinline__ void decode_cell2(uint32_t code, int level, int d, int *q) {
-    for (int k = 0; k < d; k++) q[k] = 0;
-    for (int jb = 0; jb < level; jb++)
-        for (int k = 0; k < d; k++) q[k] |= (int)((code >> (d * jb + k)) & 1u) << jb;
-}
-
 // ---------------------------------------------------------------------------------------------
 // M2L: one CTA per target box, its warps share the far row
 // ---------------------------------------------------------------------------------------------
@@ -1499,6 +1493,10 @@ int far_node_end_level(const f3m_plan *pl, float edge0, int lmax) {
 // While the tree of a plan for one product is built: may it end at this level, whose lists are there?  If it can (above) and going on
 // would cost more: one node-to-node step for every child pair of the kept pairs, of which there are 2^d or more per pair where its boxes
 // are populated, besides the lists and the deeper sort.
+// A product that refuses the nodes (node_sums) sums this level's lists pair by pair, in boxes wider than the full tree's.  Whole calls with one
+// infinite weight / finite, and of the full tree as it was: mixture of 1e7 points 24.4 / 13.5, 33 ms; 2e7 normal points, l = 0.3, 42.6 / 22.6,
+// 60 ms; twenty narrow clouds, 2e6 to 1e8 points, 1.0 to 2.2 times the finite call: where boxes are that full, small lists, box
+// moments and the far field's exact level (far_cut) are left.
 bool far_ends_with_nodes(const f3m_plan *pl, int level) {
     const int p = nodes_per_dim(pl->d, pl->prm.nr_interpolation);
     if (!ends_exactly_below(pl, (double)pl->ty->levels[level].edge, level)) return false;

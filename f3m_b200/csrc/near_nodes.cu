@@ -460,10 +460,11 @@ static __global__ void __launch_bounds__(256) weights_check(const float *__restr
 // ---------------------------------------------------------------------------------------------
 // Rule.  Estimated seconds of the lists of one level through nodes: the points' two passes, the pairs of boxes, and what the form pays
 // once (launches, the order of the rows, the check of the weights with its read-back).  Measured: 1.8e-13 s per point and node for
-// both passes up to eight nodes, 2.3e-13 beyond; 0.9e-13 to 1.2e-13 per pair of boxes and p^4 (p = 9, 4.15e6 pairs in rows of 127:
+// both passes up to eight nodes, 2.4e-13 beyond; 0.9e-13 to 1.2e-13 per pair of boxes and p^4 (p = 9, 4.15e6 pairs in rows of 127:
 // 2.28 ms; p = 7, 3.7e6 in rows of 63: 1.08 ms).  Whole calls, lists summed directly / here: 4e6 uniform points, boxes of 122, 1.09
 // lengthscales wide 18.2 / 5.4 ms; 2.9e7 points, l = 0.19 of sqrt12, 179 / 9.2 ms; 6e6 normal points 10.7 / 7.2 ms; 3.6e5 points 3.0 /
-// 0.87 ms; a mixture of 1e7 points 22.8 / 16.8 ms; 6e4 points, 1.5e8 to 7e8 pairs: even, so NODE_FIXED.
+// 0.87 ms; a mixture of 1e7 points that ends at its last level 22.8 / 16.8 ms (7.7 where it ends above, far_cut); 6e4 points, 1.5e8 to 7e8
+// pairs: even, so NODE_FIXED.
 // ---------------------------------------------------------------------------------------------
 constexpr double NODE_FIXED = 1e-4;
 static double node_seconds(const f3m_plan *pl, int p, int64_t box_pairs) {

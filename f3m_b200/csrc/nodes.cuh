@@ -230,10 +230,10 @@ __device__ __forceinline__ LeafWork leaf_work(const int *__restrict__ off, int n
 }
 
 // Moments of the long boxes: the sums of their parts, in the order of the rows, with the rounding of every addition carried along
-// (Knuth's two-sum; the loads of the parts take the time).  A tree that ends at a level whose boxes hold hundreds of thousands of points has hundreds of
-// parts per box, and a plain running sum was most of the product's error: error over sqrt(n), normal weights, l = 10, 300 products of
-// 3e6 points SRC3, of 1e7 SRC10; a kept plan, which interpolates its sources further down and adds them in a tree (far_fast.cu, SRC_LEAF), KEPT3
-// and KEPT10.
+// (Knuth's two-sum; the loads of the parts take the time).  A tree that ends at a level whose boxes hold hundreds of thousands of points has
+// hundreds of parts per box, and a plain running sum was most of the product's error.  Error over sqrt(n), normal weights, l = 10, 300
+// products each, plain / now: 3e6 points 3.65 / 2.46e-7, 1e7 3.77 / 2.77e-7, 3e7 4.53 / 2.74e-7; a kept plan, which interpolates its
+// sources further down and adds them in a tree (far_fast.cu, SRC_LEAF), 2.71, 3.24 and 3.45e-7 with plain sums.
 static __global__ void __launch_bounds__(128) p2m_combine(const int *__restrict__ off, int nb, int n, int chunk, int PR, int src_begin, int src_end,
                                                   const float *__restrict__ part, float *mom) {
     const LongBox l = long_box_of_chunk(off, nb, n, chunk, blockIdx.x);

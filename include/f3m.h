@@ -125,7 +125,10 @@ int f3m_plan_create(f3m_plan **plan, const float *X, int64_t N, const float *Y, 
  * row_begin/row_end restrict the product to the target boxes whose sorted point range starts
  * inside [row_begin,row_end) (a slice of the sorted target order, used to shard target boxes
  * over GPUs); rows outside the slice are written as 0.  Use 0, N for the whole product, which may end at the level whose
- * interpolation is exact for every pair (relative bound 1.2e-7); slices visit all levels.
+ * interpolation is exact for every pair (relative bound 1.2e-7); slices visit all levels.  In three dimensions, with one point
+ * set and one column, direct lists of populated boxes may go through interpolation nodes of their own: such a list's part of a row is within
+ * 4e-7 of the sum of |b| over the list (kernel values are at most 1), besides roundings; where fewer than one weight in ten is other
+ * than zero, or one is not finite, and in slices, its pairs are summed one by one.
  * A NaN in b makes every row it reaches NaN.  An infinity reaches rows through direct sums as infinity, through interpolation as NaN. */
 int f3m_plan_apply(f3m_plan *plan, const float *b, int32_t R, float *out, void *stream);
 int f3m_plan_apply_range(f3m_plan *plan, const float *b, int32_t R, float *out, int64_t row_begin,
